@@ -147,22 +147,29 @@ def _graph_module(case):
     return s.module
 
 
-def prepare(case, seed):
+def _inputs(case, seed):
+    """The operands of a case, made from the seed alone: [(A, B), ...] of a product, (q, k, v) of an attention."""
     gen = torch.Generator(device="cuda").manual_seed(int(seed))
     if case["kind"] in ("gemm", "fused"):
         m, n, k, dtype = case["m"], case["n"], case["k"], case["dtype"]
-        ta, tb, panels = case.get("ta", False), case.get("tb", True), case.get("panels", 1)
+        ta, tb = case.get("ta", False), case.get("tb", True)
         # activations N(0, 1) against weights N(0, 1/K): results of unit size, as in a model
-        pairs = [(_operand(gen, *((k, m) if ta else (m, k)), dtype, 1.0),
-                  _operand(gen, *((n, k) if tb else (k, n)), dtype, k ** -0.5)) for _ in range(panels)]
-        c = torch.empty(m, n, dtype=_DTYPE[case["out"]], device="cuda")
-        state = dict(kind=case["kind"], pairs=pairs, c=c, ta=ta, tb=tb)
+        return [(_operand(gen, *((k, m) if ta else (m, k)), dtype, 1.0),
+                 _operand(gen, *((n, k) if tb else (k, n)), dtype, k ** -0.5)) for _ in range(case.get("panels", 1))]
+    return tuple(_normal(gen, (case["b"], case["h"], s, case["d"]), case["dtype"], 1.0)
+                 for s in (case["s_q"], case["s_kv"], case["s_kv"]))
+
+
+def prepare(case, seed):
+    inputs = _inputs(case, seed)
+    if case["kind"] in ("gemm", "fused"):
+        c = torch.empty(case["m"], case["n"], dtype=_DTYPE[case["out"]], device="cuda")
+        state = dict(kind=case["kind"], pairs=inputs, c=c, ta=case.get("ta", False), tb=case.get("tb", True))
         if case["kind"] == "fused":
-            state.update(module=_fused_module(case), r=torch.empty(m, dtype=c.dtype, device="cuda"))
+            state.update(module=_fused_module(case), r=torch.empty(case["m"], dtype=c.dtype, device="cuda"))
         return state
-    shape = lambda s: (case["b"], case["h"], s, case["d"])  # noqa: E731
-    q, k, v = (_normal(gen, shape(s), case["dtype"], 1.0) for s in (case["s_q"], case["s_kv"], case["s_kv"]))
-    o = torch.empty(shape(case["s_q"]), dtype=_DTYPE[case["out"]], device="cuda")
+    q, k, v = inputs
+    o = torch.empty(q.shape, dtype=_DTYPE[case["out"]], device="cuda")
     if case["kind"] == "graph":
         return dict(kind="graph", module=_graph_module(case), tensors=[t[0, 0] for t in (q, k, v, o)])
     spec = dict(B=case["b"], H=case["h"], N=case["s_q"], D=case["d"], N_kv=case["s_kv"])
@@ -205,3 +212,27 @@ def tolerance(case):
         return {"rel": max(2e-6, 5e-9 * case["k"] * case["panels"])}
     # one rounding to the stored type for each panel
     return {"rel": {"fp16": 1e-3, "bf16": 8e-3}[case["out"]]}
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs, in 64 bits."""
+    inputs = _inputs(case, seed)
+    if case["kind"] in ("gemm", "fused"):
+        c = torch.full((case["m"], case["n"]), case.get("fill", 0.0), dtype=torch.float64, device="cuda")
+        for a, b in inputs:
+            c += (a.T if case.get("ta", False) else a).double() @ (b.T if case.get("tb", True) else b).double()
+        if case["kind"] == "gemm":
+            return c
+        return c, {"max": lambda: c.amax(1), "min": lambda: c.amin(1), "add": lambda: c.sum(1)}[case["reduce"]]()
+    q, k, v = (t.flatten(0, 1) for t in inputs)
+    s_q, s_kv = case["s_q"], case["s_kv"]
+    o = torch.empty(q.shape, dtype=torch.float64, device="cuda")
+    for i in range(q.shape[0]):
+        kd, vd = k[i].double(), v[i].double()
+        for r in range(0, s_q, 2048):  # query i sees s_kv - s_q + i + 1 keys where the case is causal
+            s = (q[i, r:r + 2048].double() @ kd.T) * case["d"] ** -0.5
+            if case["causal"]:
+                rows = torch.arange(r, r + s.shape[0], device="cuda")[:, None]
+                s.masked_fill_(torch.arange(s_kv, device="cuda")[None] > rows + (s_kv - s_q), -math.inf)
+            o[i, r:r + 2048] = torch.softmax(s, 1) @ vd
+    return o[0] if case["kind"] == "graph" else o.view(inputs[0].shape)
