@@ -17,9 +17,10 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units
 enum : unsigned { ST_ATTN_S = 0x201, ST_ATTN_P = 0x202, ST_ATTN_O = 0x203, ST_ATTN_KV = 0x204, ST_ATTN_Q = 0x205 };
 
 struct AttnParams {
-  int S_q, S_kv, n_pairs, causal;
+  int S_q, S_kv, causal;
+  int n_groups, group_rows;  // work items per (batch, head), and the query rows of one: two 128-row tiles or one
   int normalized;  // 1: two passes over the keys, P divided by the complete row sum before it is rounded
-  int64_t total_items;  // work items: pairs of 128-row query tiles of one (batch, head)
+  int64_t total_items;
   float scale_log2, scale;
   void* O;
   unsigned* status;
@@ -34,7 +35,9 @@ __device__ __forceinline__ float ex2f(float x) {
 
 // The reference's exponential (benchmark/layout/execution/tiled_attention.py:511-513 emits
 // ex2.approx.f32, and its qualification forbids .ftz): subnormal inputs and results are kept.
-// Used by the normalised mode, which follows the reference's arithmetic to the letter.
+// Used by the normalised mode, which follows the reference's arithmetic to the letter, where probabilities are
+// bf16.  (With fp16 probabilities a flushed exponential changes nothing: below 2^-126 it rounds to zero in fp16, and
+// the row sum it would join is at least 1.)
 __device__ __forceinline__ float ex2f_ieee_range(float x) {
   float y;
   asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -61,6 +64,40 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
       : "=l"(*reinterpret_cast<unsigned long long*>(&d))
       : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
   return d;
+}
+
+// the same pairs with subnormals kept and every operation rounded by itself (the normalised mode's arithmetic)
+__device__ __forceinline__ float2 mul2_rn(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(*reinterpret_cast<unsigned long long*>(&d))
+      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+  return d;
+}
+__device__ __forceinline__ float2 add2_rn(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(*reinterpret_cast<unsigned long long*>(&d))
+      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+  return d;
+}
+__device__ __forceinline__ float2 fma2_rn(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(*reinterpret_cast<unsigned long long*>(&d))
+      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
+        "l"(*reinterpret_cast<unsigned long long*>(&c)));
+  return d;
+}
+
+// a / l for a pair of numerators, without the branch a division per element brings (128 of them in a row of a key
+// tile ran one after the other).  Markstein's correction (IBM J. Res. Dev. 34(1), 1990): with inv the correctly
+// rounded reciprocal of l, q = a*inv is corrected by its exact remainder, and the result is the correctly rounded
+// quotient as long as the remainder is representable, a >= 2^-100 (here a <= 1 <= l, so nothing overflows); below
+// that the quotient, smaller than 2^-100, may be off by one unit of its last fp32 place before it is rounded to 16 bits.
+__device__ __forceinline__ float2 div2_by(float2 a, float2 neg_l, float2 inv) {
+  const float2 q = mul2_rn(a, inv);
+  return fma2_rn(fma2_rn(q, neg_l, a), inv, q);
 }
 
 template <bool BF16>

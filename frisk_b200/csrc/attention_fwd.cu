@@ -91,18 +91,18 @@ __global__ void __launch_bounds__(kThreads, 1)
   struct Item {
     int bh, m0, nq[2], n_max;
   };
-  const int bh_total = (int)(p.total_items / p.n_pairs);
+  const int bh_total = (int)(p.total_items / p.n_groups);
   auto decode = [&](int t) {
-    const int per_chunk = kHeadChunk * p.n_pairs;
+    const int per_chunk = kHeadChunk * p.n_groups;
     const int chunk = t / per_chunk;
     const int within = t - chunk * per_chunk;
     const int heads_here = min(kHeadChunk, bh_total - chunk * kHeadChunk);
-    const int pair = p.n_pairs - 1 - within / heads_here;
+    const int group = p.n_groups - 1 - within / heads_here;
     Item it;
     it.bh = chunk * kHeadChunk + within % heads_here;
-    it.m0 = pair * 2 * BM;
+    it.m0 = group * p.group_rows;
     it.nq[0] = kv_tiles_for(it.m0, p.S_q, p.S_kv, p.causal);
-    it.nq[1] = kv_tiles_for(it.m0 + BM, p.S_q, p.S_kv, p.causal);
+    it.nq[1] = p.group_rows > BM ? kv_tiles_for(it.m0 + BM, p.S_q, p.S_kv, p.causal) : 0;
     it.n_max = max(it.nq[0], it.nq[1]);
     return it;
   };
@@ -168,9 +168,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         const Item it = decode(t);
         // the Q tiles of the item before are free when both MMA threads have issued their last S of it
         if (n > 0 && !mbar_wait(q_empty, (n - 1) & 1, abort_flag, p.status, ST_ATTN_Q)) break;
-        mbar_expect_tx(q_full, 2 * L::kTileBytes);
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
+        const int q_tiles = it.nq[1] > 0 ? 2 : 1;  // (nothing reads the second tile's place where there is none)
+        mbar_expect_tx(q_full, q_tiles * L::kTileBytes);
+        for (int q = 0; q < q_tiles; ++q)
 #pragma unroll
           for (int b = 0; b < kBoxes; ++b)
             tma_load_3d(smem + L::kQ + q * L::kTileBytes + b * kBoxBytes, &tmap_q, q_full, b * 64, it.m0 + q * BM, it.bh);
@@ -332,9 +332,15 @@ __global__ void __launch_bounds__(kThreads, 1)
         // tail_attention_reference.py:74-78): score = fp32(dot) * scale; subtract the maximum of the
         // WHOLE row; e = ex2((score - max) * log2e); p = e / (sum of e over the whole row), IEEE
         // division; p rounded to 16 bits; then P.V.  Pass 0 finds max and sum, pass 1 forms P.
+        // The row of a key tile is worked on in packed pairs without branches: an IEEE division per element
+        // (__fdiv_rn branches) made this mode latency-bound, 16 heads x 1025 rows x D 64 took 154 us.
         const float kLog2e = 1.44269504088896340736f;
+        const float2 scale2 = make_float2(p.scale, p.scale), log2e2 = make_float2(kLog2e, kLog2e);
+        auto exp2_of = [](float x) { return BF16 ? ex2f_ieee_range(x) : ex2f(x); };
         float m_run = -INFINITY, l_run = 0.f;
         for (int pass = 0; pass < 2 && ok; ++pass) {
+          const float inv_l = __frcp_rn(l_run);  // (of use in pass 1 only)
+          const float2 inv2 = make_float2(inv_l, inv_l), negl2 = make_float2(-l_run, -l_run);
           for (int j = 0; j < n_tiles; ++j) {
             if (!mbar_wait(&s_full[q], steps & 1, abort_flag, p.status, ST_ATTN_S)) {
               ok = false;
@@ -346,51 +352,65 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(t_s + c * 32, sr[c]);
             tmem_ld_wait();
-            const int n0 = j * BN;
-            int limit = p.S_kv - 1;
-            if (p.causal) limit = min(limit, g_row + off);
-            limit -= n0;
             if (pass == 0) {
               // S_q is in registers: the MMA warp may overwrite it
               tc_fence_before_sync();
               mbar_arrive(&p_ready[q]);
               mbar_arrive(&p_ready_hi[q]);
-              float mx = -INFINITY;
+            }
+            const int n0 = j * BN;
+            if ((n0 + BN > p.S_kv) || (p.causal && (n0 + BN - 1 > m_tile + off))) {
+              int limit = p.S_kv - 1;
+              if (p.causal) limit = min(limit, g_row + off);
+              limit -= n0;  // columns > limit are hidden
 #pragma unroll
               for (int c = 0; c < 4; ++c)
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                  float sc = (c * 32 + i > limit) ? -INFINITY : __fmul_rn(__uint_as_float(sr[c][i]), p.scale);
-                  sr[c][i] = __float_as_uint(sc);
-                  mx = fmaxf(mx, sc);
-                }
-              const float m_new = fmaxf(m_run, mx);
-              float sum = 0.f;
-              if (m_new != -INFINITY) {
+                for (int i = 0; i < 32; ++i)
+                  if (c * 32 + i > limit) sr[c][i] = 0xff800000u;  // -inf
+            }
+            // (score - m) * log2e of a pair, rounded step by step; the scale is positive, so it keeps the order and
+            // the maximum of the scaled scores is the scaled maximum
+            auto arg2 = [&](int c, int i, float2 negm2) {
+              const float2 s2 = make_float2(__uint_as_float(sr[c][2 * i]), __uint_as_float(sr[c][2 * i + 1]));
+              return mul2_rn(add2_rn(mul2_rn(s2, scale2), negm2), log2e2);
+            };
+            if (pass == 0) {
+              float mxc[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
+                  mxc[c] = max3f(mxc[c], __uint_as_float(sr[c][2 * i]), __uint_as_float(sr[c][2 * i + 1]));
+              const float mx = __fmul_rn(max3f(mxc[0], mxc[1], fmaxf(mxc[2], mxc[3])), p.scale);
+              const float m_new = fmaxf(m_run, mx);
+              if (m_new != -INFINITY) {
+                const float2 negm2 = make_float2(-m_new, -m_new);
+                float2 sum[4];
 #pragma unroll
-                  for (int i = 0; i < 32; ++i)
-                    sum += ex2f_ieee_range(__fmul_rn(__fsub_rn(__uint_as_float(sr[c][i]), m_new), kLog2e));
+                for (int c = 0; c < 4; ++c) sum[c] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+#pragma unroll
+                  for (int c = 0; c < 4; ++c) {
+                    const float2 x = arg2(c, i, negm2);
+                    sum[c] = add2_rn(sum[c], make_float2(exp2_of(x.x), exp2_of(x.y)));
+                  }
+                const float2 all = add2_rn(add2_rn(sum[0], sum[1]), add2_rn(sum[2], sum[3]));
                 const float carry = (m_run == -INFINITY) ? 0.f : l_run * ex2f_ieee_range(__fmul_rn(__fsub_rn(m_run, m_new), kLog2e));
-                l_run = carry + sum;
+                l_run = carry + (all.x + all.y);
                 m_run = m_new;
               }
             } else {
+              const float2 negm2 = make_float2(-m_run, -m_run);
 #pragma unroll
               for (int c = 0; c < 4; ++c) {
                 uint32_t pk[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                  float pv[2];
-#pragma unroll
-                  for (int e = 0; e < 2; ++e) {
-                    const int col = c * 32 + 2 * i + e;
-                    const float sc = __fmul_rn(__uint_as_float(sr[c][2 * i + e]), p.scale);
-                    const float ex = (col > limit) ? 0.f : ex2f_ieee_range(__fmul_rn(__fsub_rn(sc, m_run), kLog2e));
-                    pv[e] = __fdiv_rn(ex, l_run);
-                  }
-                  pk[i] = pack16<BF16>(pv[0], pv[1]);
+                  const float2 x = arg2(c, i, negm2);
+                  const float2 pv = div2_by(make_float2(exp2_of(x.x), exp2_of(x.y)), negl2, inv2);
+                  pk[i] = pack16<BF16>(pv.x, pv.y);
                 }
                 tmem_st_32x32b_x16(t_s + c * 16, pk);
                 if (c & 1) {
@@ -627,9 +647,14 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q
   AttnParams p;
   p.S_q = d.S_q;
   p.S_kv = d.S_kv;
-  p.n_pairs = (d.S_q + 2 * BM - 1) / (2 * BM);
+  // Items of ONE query tile where that still leaves at most one item per SM: half the items' SMs would stand idle
+  // otherwise, and a tile alone on its SM takes about 0.6 of the time two tiles take side by side (so from one item
+  // per SM upwards pairs are the better use of it).
+  const int64_t tiles = (d.S_q + BM - 1) / BM;
+  p.group_rows = tiles * bh <= ctx->num_sms ? BM : 2 * BM;
+  p.n_groups = (d.S_q + p.group_rows - 1) / p.group_rows;
   p.causal = d.causal ? 1 : 0;
-  p.total_items = (int64_t)p.n_pairs * bh;
+  p.total_items = (int64_t)p.n_groups * bh;
   p.scale_log2 = d.scale * 1.4426950408889634f;
   p.scale = d.scale;
   p.normalized = d.normalize_p ? 1 : 0;

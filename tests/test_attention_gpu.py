@@ -161,6 +161,32 @@ def test_normalized_mode_large_heads(ctx):
     assert rel_frobenius(go.host(), ref) <= 2e-3
 
 
+@pytest.mark.parametrize("H,S_q,S_kv,causal,normalized", [
+    (37, 512, 512, True, False),    # 148 query tiles: one item per SM of one tile each
+    (37, 513, 640, False, True),    # 185 tiles: items of two tiles, the last one with a single row in its only tile
+    (74, 129, 257, True, True),     # 148 tiles, the second of every head with one row
+    (3, 1, 129, False, True),
+])
+def test_one_and_two_tile_items(ctx, H, S_q, S_kv, causal, normalized):
+    """Work items of one and of two query tiles, around the line between them, in both softmax modes."""
+    import torch
+    from oracle.numerics import to_storage
+    rng = np.random.default_rng(17)
+    q, k, v = (to_storage(rng.standard_normal((1, H, n, 64), dtype=np.float32), "bf16") for n in (S_q, S_kv, S_kv))
+    gq, gk, gv = (Guarded(x.shape, "bf16", fill=x) for x in (q, k, v))
+    go = Guarded(q.shape, "fp32")
+    go.view.fill_(float("nan"))
+    desc = capi.attn_desc(1, H, S_q, S_kv, 64, 0.125, causal, "bf16", "fp32", normalize_p=normalized)
+    s = torch.cuda.current_stream().cuda_stream
+    ctx.attention_fwd(desc, gq.view.data_ptr(), gk.view.data_ptr(), gv.view.data_ptr(), go.view.data_ptr(), stream=s)
+    ctx.check(s)
+    ref = ao.attention_fwd(q, k, v, "bf16", 0.125, causal=causal, mode="strict")
+    assert go.guards_intact()
+    # the strict mode rounds P after the division as the normalised mode does (exponentials and row sum agree to fp32);
+    # the single pass rounds it relative to a running maximum: an error of its own of the same size
+    assert rel_frobenius(go.host(), ref) <= (2e-3 if normalized else 5e-3)
+
+
 def test_properties_small(ctx):
     rng = np.random.default_rng(11)
     from oracle.numerics import to_storage
