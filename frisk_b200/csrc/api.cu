@@ -256,6 +256,9 @@ int frisk_b200_ctx_create(frisk_b200_ctx** out, int device) {
   ctx->num_sms = prop.multiProcessorCount;
   if ((e = cudaMalloc(&ctx->d_status, 256)) != cudaSuccess) return fail(e);
   if ((e = cudaMemset(ctx->d_status, 0, 256)) != cudaSuccess) return fail(e);
+  if ((e = cudaMalloc(&ctx->attn_scratch, attention_decode_scratch_bytes())) != cudaSuccess) return fail(e);
+  if ((e = cudaMemset(ctx->attn_scratch, 0, attention_decode_ticket_bytes())) != cudaSuccess) return fail(e);
+  if ((e = cudaStreamSynchronize(nullptr)) != cudaSuccess) return fail(e);  // cleared before any stream uses it
   if ((e = cudaMallocHost(&ctx->h_status, 256)) != cudaSuccess) return fail(e);
   ctx->h_status[0] = 0;
   if ((e = cudaStreamCreateWithFlags(&ctx->host_stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
@@ -274,6 +277,7 @@ int frisk_b200_ctx_destroy(frisk_b200_ctx* ctx) {
   for (auto& b : ctx->stage)
     if (b.ptr) cudaFree(b.ptr);
   if (ctx->d_status) cudaFree(ctx->d_status);
+  if (ctx->attn_scratch) cudaFree(ctx->attn_scratch);
   if (ctx->h_status) cudaFreeHost(ctx->h_status);
   for (auto& ev : ctx->ev)
     if (ev) cudaEventDestroy(ev);

@@ -701,6 +701,7 @@ int launch_out(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q
 
 int launch_attention_fwd(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K,
                          const void* V, void* O, cudaStream_t s) {
+  if (attention_decode_preferred(d)) return launch_attention_decode(ctx, d, Q, K, V, O, s);
   const bool bf = d.dtype_in == FRISK_B200_BF16;
   if (d.D == 128) return bf ? launch_out<true, 128>(ctx, d, Q, K, V, O, s) : launch_out<false, 128>(ctx, d, Q, K, V, O, s);
   if (d.D == 64) return bf ? launch_out<true, 64>(ctx, d, Q, K, V, O, s) : launch_out<false, 64>(ctx, d, Q, K, V, O, s);

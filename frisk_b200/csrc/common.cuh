@@ -75,6 +75,9 @@ struct frisk_b200_ctx {
   // staging for the *_host entry points and library-owned workspace
   fb::StagingBuffer stage[11];  // 0-2 A/B/C staging, 3 skinny scratch, 4 V staging, 5 GEMM tail scratch, 6 row partials,
                                 // 7 fp32 stream-K scratch, 8-10 fp32-on-tensor-cores: stacked A, stacked B, 3M x 3N product
+  // Scratch of fixed size, made with the context, so that a call that needs it never allocates; the tickets at its
+  // start are zero between launches.  attn: decode attention
+  void* attn_scratch = nullptr;
   cudaStream_t host_stream = nullptr;
   cudaStream_t copy_stream = nullptr;
   cudaStream_t out_stream = nullptr;
@@ -224,6 +227,13 @@ int launch_fill(void* C, int64_t M, int64_t N, int64_t ldc, float value, int dty
 
 int launch_attention_fwd(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K,
                          const void* V, void* O, cudaStream_t s);
+
+// a few queries per head against a long key/value cache (attention_decode.cu)
+bool attention_decode_preferred(const frisk_b200_attn_desc& d);
+size_t attention_decode_scratch_bytes();
+size_t attention_decode_ticket_bytes();  // the prefix of the scratch that starts at zero
+int launch_attention_decode(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K,
+                            const void* V, void* O, cudaStream_t s);
 
 int launch_convert_f32(const float* src, void* dst, int64_t n, int dtype, cudaStream_t s);
 

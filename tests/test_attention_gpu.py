@@ -187,6 +187,34 @@ def test_one_and_two_tile_items(ctx, H, S_q, S_kv, causal, normalized):
     assert rel_frobenius(go.host(), ref) <= (2e-3 if normalized else 5e-3)
 
 
+@pytest.mark.parametrize("B,H,S_q,S_kv,D,dtype,causal,out", [
+    (1, 1, 1, 1, 64, "fp16", True, "fp32"),       # one key
+    (1, 1, 16, 16, 128, "bf16", True, "bf16"),    # every row masked differently, whole warps without a visible key
+    (1, 3, 2, 63, 64, "bf16", False, "bf16"),     # below one key tile
+    (2, 2, 5, 65, 128, "fp16", True, "fp16"),     # one key beyond a tile
+    (1, 1, 7, 16384, 64, "bf16", True, "fp32"),   # one head shared by every CTA
+    (1, 149, 1, 192, 128, "bf16", True, "bf16"),  # CTA ranges that begin and end inside heads
+    (3, 100, 16, 100, 64, "fp16", False, "fp32"), # whole heads and shared ones in one CTA
+    (1, 2, 17, 300, 128, "bf16", True, "bf16"),   # one query too many: the two-tile kernel
+])
+def test_few_queries(ctx, B, H, S_q, S_kv, D, dtype, causal, out):
+    check(ctx, B, H, S_q, S_kv, D, dtype, causal, seed=41, out_dtype=out)
+
+
+def test_few_queries_rescale_and_rerun(ctx):
+    """Scores that keep growing along the keys (the reference maximum moves in every tile), and a
+    second launch on the same context: same bits, tickets left clean."""
+    from oracle.numerics import to_storage
+    rng = np.random.default_rng(43)
+    q, k, v = (rng.standard_normal((1, 2, n, 64), dtype=np.float32) for n in (3, 2000, 2000))
+    k *= np.linspace(0.1, 60.0, 2000, dtype=np.float32)[None, None, :, None]
+    q, k, v = (to_storage(x, "bf16") for x in (q, k, v))
+    got, ok = run_attention(ctx, q, k, v, "bf16", 0.125, True, "fp32")
+    again, _ = run_attention(ctx, q, k, v, "bf16", 0.125, True, "fp32")
+    assert ok and np.array_equal(got, again)
+    assert rel_frobenius(got, ao.attention_fwd(q, k, v, "bf16", 0.125, causal=True, mode="fp64")) <= TOL
+
+
 def test_properties_small(ctx):
     rng = np.random.default_rng(11)
     from oracle.numerics import to_storage
