@@ -392,6 +392,9 @@ int frisk_b200_gemm(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* d, const vo
   if (ranges_overlap(C, e.c, A, e.a) || ranges_overlap(C, e.c, B, e.b)) return FRISK_B200_E_OVERLAP;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   FB_DEVICE(ctx);
+  // (what an AUTO call runs; a call that names its kernel runs that)
+  if (d->algo == FRISK_B200_ALGO_AUTO && d->dtype_ab == FRISK_B200_F32)
+    algo = f32_split_beats_simt(*d) ? FRISK_B200_ALGO_F32_SPLIT : FRISK_B200_ALGO_SIMT_F32;
   switch (algo) {
     case FRISK_B200_ALGO_SIMT_F32:
       return launch_gemm_simt_f32(ctx, *d, static_cast<const float*>(A), static_cast<const float*>(B),

@@ -62,6 +62,33 @@ struct PerDeviceOnce {
   }
 };
 
+// How many clusters of `splits` (2, 4 or 8) CTAs of a kernel the device runs at a time; asked once per device and size.
+struct ClusterCapacity {
+  std::atomic<int> known[kMaxDevices][3] = {};  // capacity + 1
+  template <typename K>
+  int operator()(int device, K kern, int threads, int smem_bytes, int splits) {
+    if (device < 0 || device >= kMaxDevices) return 0;
+    std::atomic<int>& slot = known[device][splits == 2 ? 0 : splits == 4 ? 1 : 2];
+    int n = slot.load(std::memory_order_acquire) - 1;
+    if (n >= 0) return n;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)splits * kNumSMsDefault);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem_bytes;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) return 0;
+    slot.store(n + 1, std::memory_order_release);
+    return n;
+  }
+};
+
 }  // namespace fb
 
 struct frisk_b200_ctx {
@@ -73,8 +100,8 @@ struct frisk_b200_ctx {
   unsigned* d_status = nullptr;  // device status word (first failing wait records its code)
   unsigned* h_status = nullptr;  // pinned mirror
   // staging for the *_host entry points and library-owned workspace
-  fb::StagingBuffer stage[11];  // 0-2 A/B/C staging, 3 skinny scratch, 4 V staging, 5 GEMM tail scratch, 6 row partials,
-                                // 7 fp32 stream-K scratch, 8-10 fp32-on-tensor-cores: stacked A, stacked B, 3M x 3N product
+  fb::StagingBuffer stage[8];  // 0-2 A/B/C staging, 3 skinny scratch, 4 V staging, 5 GEMM tail scratch, 6 row partials,
+                               // 7 fp32 stream-K scratch
   // Scratch of fixed size, made with the context, so that a call that needs it never allocates; the tickets at its
   // start are zero between launches.  attn: decode attention
   void* attn_scratch = nullptr;
@@ -169,9 +196,10 @@ inline GemmExtents gemm_extents(const frisk_b200_gemm_desc& d) {
 // ---- kernel launchers (one per .cu file) --------------------------------------------
 int launch_gemm_simt_f32(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const float* A, const float* B,
                          float* C, cudaStream_t s);
-// fp32 GEMM as nine bf16 tensor-core products of exactly split operands (gemm_f32_split.cu)
-bool f32_split_supported(const frisk_b200_gemm_desc& d);
-bool f32_split_preferred(const frisk_b200_gemm_desc& d);
+// fp32 GEMM as six bf16 tensor-core products of split operands (gemm_f32_split.cu)
+bool f32_split_supported(const frisk_b200_gemm_desc& d);  // what F32_SPLIT accepts when it is asked for
+bool f32_split_preferred(const frisk_b200_gemm_desc& d);  // what AUTO reports as F32_SPLIT
+bool f32_split_beats_simt(const frisk_b200_gemm_desc& d);  // what an AUTO call runs on it
 int launch_gemm_f32_split(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const float* A, const float* B,
                           float* C, cudaStream_t s);
 

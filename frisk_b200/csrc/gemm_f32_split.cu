@@ -1,226 +1,555 @@
-// fp32 GEMM on the tensor cores: every fp32 operand element is split exactly into three bf16
-// terms (a = a1 + a2 + a3 up to 2^-26 |a|: 3 x 8 significant bits plus the signs), the nine
-// products A_s . B_t are one bf16 GEMM with fp32 accumulation in tensor memory over the stacked
-// operands [A1; A2; A3] (3M x K) and [B1; B2; B3] (3N x K), and the nine M x N blocks of that
-// product are added smallest first.  Products of bf16 terms are exact in fp32, so the result has
-// fp32-GEMM accuracy (relative Frobenius error a few 1e-7 against fp64, like the CUDA-core kernel)
-// at tensor-core speed.  Same contract as the CUDA-core kernel: `frisk.gemm` with f32 operands,
-// C <- (clear_accum ? 0 : C) + op(A).op(B) (lib/Dialect/Frisk/IR/FriskOps.cpp:406-426).
+// fp32 GEMM on the tensor cores: C <- (clear_accum ? 0 : C) + op(A).op(B) with fp32 accuracy, any size, pitch and
+// alignment, in ONE launch.  Contract: `frisk.gemm` with f32 operands (lib/Dialect/Frisk/IR/FriskOps.cpp:406-426).
 //
-// Three launches on the caller's stream: split (both operands), the tcgen05 GEMM, the 9-block sum.
-// Stacking keeps each operand's orientation: an operand stored [rows = MN][K] gets its planes one
-// below the other, an operand stored [K][MN] gets them side by side (row pitch 3 MN), so all four
-// transpose combinations reach the GEMM with the caller's flags unchanged.
+// Every element x of a tile is multiplied by 2^24 and split into three bf16 terms while it travels from global to shared
+// memory (x 2^24 = x0 + x1 + x2: 3 x 8 significant bits plus the signs, exact for every x below 2^104; the
+// factor keeps the terms of small elements out of the subnormals), and six of the nine term products run as
+// tcgen05.mma 128 x 128 x 16: A0B0, A0B1, A1B0, A1B1, A0B2, A2B0.  The three left out are at most 2^-26 |a||b| together,
+// a quarter of what ONE fp32 rounding of the product may lose.  Products of bf16 terms are exact in fp32.
+//
+// Accuracy is decided by the accumulation: tensor memory truncates every addition, a bias of half a unit per MMA along
+// a sum (1.0e-6 relative error at K = 1024 when the whole K stayed there).  So one 64-k block is
+// summed in tensor memory, small terms first, so that only the four A0B0 steps see a large accumulator, and then
+// added to fp32 registers with round-to-nearest: 1.0e-7 at K = 1024, 2.6e-7 on the CUDA cores.
+//
+// An element that is not finite, or so large that x 2^24 or a sum overflows, makes the result non-finite; such a result
+// is computed again by a plain fp32 loop over K, so infinities and NaN come out as IEEE arithmetic gives them.
+//
+// One CTA per SM, 16 warps with fixed roles (128 registers each, all of the SM's):
+//   warps 0-7   promotion: tensor memory -> fp32 registers (64 columns of one row per thread), stores.  One thread of
+//               warp 0 also issues the MMAs, of block i before the warp adds up block i - 1
+//   warps 8-15  loaders: global -> registers (one block ahead) -> split -> shared memory, in the 128-byte-swizzle image
+//               tcgen05 reads (K-major or MN-major, whichever way the operand lies in global memory)
+// Bound by shared memory: a block writes 96 KB of planes and its 24 MMAs read 192 KB, 2300 clk at 128 B/clk against 1540
+// clk of tensor pipe; 4096^3 takes 3700 clk a block (886 us, 155 TFLOP/s of fp32), a short K about 4000.
+//
+// Where the tiles are fewer than half the SMs a cluster of 2, 4 or 8 CTAs shares a tile's K; every CTA leaves its fp32 part
+// in its own shared memory and each finishes a share of the tile's 32-row pieces, adding the parts over distributed
+// shared memory in rank order (reproducible, no scratch).  Otherwise a CTA walks whole tiles.
 #include <cuda_bf16.h>
+#include <limits.h>
+
+#include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
+#include "gemm_common.cuh"
+#include "ptx.cuh"
 
 namespace fb {
 namespace {
+using gemm_detail::TileCoord;
+using gemm_detail::tile_coord;
 
-struct SplitOperand {
-  const float* src;
-  __nv_bfloat16* dst;
-  int64_t rows, cols, ld;       // as stored
-  int64_t dst_ld, plane;        // destination row pitch and distance between planes (elements)
-  int vec;                      // source rows 16-byte aligned and cols % 4 == 0
+constexpr int BT = 128;                       // tile edge
+constexpr int BK = 64;                        // k per block
+constexpr int kPlane = BT * BK * 2;           // one bf16 plane of an operand: 16 KB
+constexpr int kStageBytes = 6 * kPlane;       // three planes of A, three of B
+constexpr int kStages = 2;
+constexpr int kPromoWarps = 8, kLoadWarps = 8;
+constexpr int kThreads = 32 * (kPromoWarps + kLoadWarps);
+constexpr int kOutOffset = kStages * kStageBytes;
+constexpr int kOutPitch = 20;                 // floats: [32 rows][16 columns] per promotion warp, rows 16-byte aligned
+constexpr int kOutWarpBytes = 32 * kOutPitch * 4;
+constexpr int kBarOffset = kOutOffset + kPromoWarps * kOutWarpBytes;
+constexpr int kSmemTotal = kBarOffset + 256 + 1024;
+static_assert(kSmemTotal <= 232448, "stages and output buffers must fit");
+static_assert(kStages == 2, "stages and accumulators alternate together");
+constexpr float kScale = 16777216.f;          // 2^24, for both operands
+constexpr float kUnscale = 1.f / (kScale * kScale);
+constexpr float kFloatMax = 3.402823466e38f;
+
+struct Operand {
+  const float* p;
+  int64_t ld;
+  int rows, cols;  // as stored
 };
 
-__device__ __forceinline__ void split3(float x, __nv_bfloat16& p0, __nv_bfloat16& p1, __nv_bfloat16& p2) {
-  p0 = __float2bfloat16_rn(x);
-  const float r1 = x - __bfloat162float(p0);   // exact
-  p1 = __float2bfloat16_rn(r1);
-  const float r2 = r1 - __bfloat162float(p1);  // exact
-  p2 = __float2bfloat16_rn(r2);
+struct SplitArgs {
+  Operand a, b;
+  float* C;
+  int64_t ldc;
+  int M, N, K, accumulate, vec_c;
+  int tiles_m, tiles_n, kb;  // tiles, 64-k blocks per tile
+  int splits;                // CTAs of a cluster, which share a tile's K
+  unsigned* status;
+};
+
+// (x, y) 2^24 as three pairs of bf16 terms
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t (&w)[3]) {
+  x *= kScale;
+  y *= kScale;
+#pragma unroll
+  for (int t = 0; t < 3; ++t) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    w[t] = *reinterpret_cast<const uint32_t*>(&h);
+    x -= __uint_as_float(w[t] << 16);          // exact
+    y -= __uint_as_float(w[t] & 0xffff0000u);  // exact
+  }
 }
 
-// grid.y selects the operand; four consecutive columns per thread
-__global__ void __launch_bounds__(256) split_bf16x3_kernel(const SplitOperand a, const SplitOperand b) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  const SplitOperand& o = blockIdx.y == 0 ? a : b;
-  const int64_t quads_per_row = (o.cols + 3) / 4;
-  const int64_t total = o.rows * quads_per_row;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = i / quads_per_row, c = (i % quads_per_row) * 4;
-    const float* s = o.src + r * o.ld + c;
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    const int n = (int)(o.cols - c < 4 ? o.cols - c : 4);
-    if (o.vec && n == 4) {
-      const float4 t = __ldg(reinterpret_cast<const float4*>(s));
-      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    } else {
-      for (int j = 0; j < n; ++j) v[j] = __ldg(s + j);
-    }
-    __nv_bfloat16 p[3][4];
+// A block of an operand is 128 box rows of 64 elements: rows = MN and columns = k for an operand contiguous along K;
+// for one contiguous along MN, 64 rows = k of columns mn0..+63, then 64 rows of columns mn0+64..+127.  A loader thread
+// takes 32 elements of it.  VEC (16-byte aligned rows): eight groups of four columns, a warp reads two rows of 256 bytes;
+// otherwise columns lane and lane + 32 of 16 rows, a warp reads one row, one element per lane.
+template <bool MN, bool VEC>
+struct Loader {
+  static constexpr int kSteps = VEC ? 8 : 16;
+  static constexpr int kRowStep = 128 / kSteps;  // box rows from one step to the next
+  float r[32];
+  const float* base;  // this thread's first element of the block the next fetch() takes
+  int row, col;       // its place in the operand
+
+  __device__ __forceinline__ static int first_row(int tid) { return VEC ? tid >> 4 : tid >> 5; }
+  __device__ __forceinline__ static int first_col(int tid) { return VEC ? (tid & 15) * 4 : tid & 31; }
+  __device__ __forceinline__ void place(const Operand& o, int mn0, int k0, int tid) {
+    row = (MN ? k0 : mn0) + first_row(tid);
+    col = (MN ? mn0 : k0) + first_col(tid);
+    base = o.p + (int64_t)row * o.ld + col;
+  }
+  // `inside`: the whole block lies in the operand
+  __device__ __forceinline__ void fetch(const Operand& o, bool inside) {
+    const int64_t step = kRowStep * o.ld;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) split3(v[j], p[0][j], p[1][j], p[2][j]);
-    __nv_bfloat16* d = o.dst + r * o.dst_ld + c;
-#pragma unroll
-    for (int pl = 0; pl < 3; ++pl) {
-      // destination rows are 16-byte aligned and c is a multiple of 4: 8-byte stores
-      if (n == 4) {
-        uint2 w;
-        w.x = (uint32_t)__bfloat16_as_ushort(p[pl][0]) | ((uint32_t)__bfloat16_as_ushort(p[pl][1]) << 16);
-        w.y = (uint32_t)__bfloat16_as_ushort(p[pl][2]) | ((uint32_t)__bfloat16_as_ushort(p[pl][3]) << 16);
-        *reinterpret_cast<uint2*>(d + pl * o.plane) = w;
+    for (int v = 0; v < kSteps; ++v) {
+      const int rv = MN ? v % (kSteps / 2) : v, cv = MN ? v / (kSteps / 2) * 64 : 0;
+      const float* p = base + rv * step + cv;
+      if (VEC) {
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (inside) {
+          x = __ldg(reinterpret_cast<const float4*>(p));
+        } else if (row + rv * kRowStep < o.rows && col + cv < o.cols) {
+          if (col + cv + 3 < o.cols) {
+            x = __ldg(reinterpret_cast<const float4*>(p));
+          } else {
+            x.x = __ldg(p);
+            if (col + cv + 1 < o.cols) x.y = __ldg(p + 1);
+            if (col + cv + 2 < o.cols) x.z = __ldg(p + 2);
+          }
+        }
+        r[4 * v] = x.x; r[4 * v + 1] = x.y; r[4 * v + 2] = x.z; r[4 * v + 3] = x.w;
+      } else if (inside) {
+        r[2 * v] = __ldg(p);
+        r[2 * v + 1] = __ldg(p + 32);
       } else {
-        for (int j = 0; j < n; ++j) d[pl * o.plane + j] = p[pl][j];
+        const bool in_row = row + rv * kRowStep < o.rows;
+        r[2 * v] = in_row && col + cv < o.cols ? __ldg(p) : 0.f;
+        r[2 * v + 1] = in_row && col + cv + 32 < o.cols ? __ldg(p + 32) : 0.f;
       }
     }
+    base += MN ? BK * o.ld : (int64_t)BK;
+    if (MN) row += BK; else col += BK;
+  }
+  // the three planes of the block in the 128-byte-swizzle image: box row br at br * 128 bytes, 16-byte piece c at c ^ (br % 8)
+  __device__ __forceinline__ void store(unsigned char* s, int tid) const {
+    const int br = first_row(tid);  // (steps of 16 or 8 rows leave br % 8 as it is)
+    if (VEC) {
+      const int c4 = tid & 15;
+      unsigned char* d = s + br * 128 + ((((c4 >> 1) ^ (br & 7)) << 4) | ((c4 & 1) << 3));
+#pragma unroll
+      for (int v = 0; v < kSteps; ++v) {
+        uint32_t lo[3], hi[3];
+        split_pair(r[4 * v], r[4 * v + 1], lo);
+        split_pair(r[4 * v + 2], r[4 * v + 3], hi);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) *reinterpret_cast<uint2*>(d + v * (kRowStep * 128) + t * kPlane) = make_uint2(lo[t], hi[t]);
+      }
+    } else {
+      // neighbouring lanes swap: even lanes get columns (lane, lane + 1), odd lanes (lane + 31, lane + 32)
+      const int lane = tid & 31;
+      const bool odd = lane & 1;
+      const int word = odd ? 16 + (lane >> 1) : lane >> 1;  // of the row's 32
+      unsigned char* d = s + br * 128 + (((word >> 2) ^ (br & 7)) << 4) + (word & 3) * 4;
+#pragma unroll
+      for (int v = 0; v < kSteps; ++v) {
+        const float got = __shfl_xor_sync(0xffffffffu, odd ? r[2 * v] : r[2 * v + 1], 1);
+        uint32_t w[3];
+        split_pair(odd ? got : r[2 * v], odd ? r[2 * v + 1] : got, w);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) *reinterpret_cast<uint32_t*>(d + v * (kRowStep * 128) + t * kPlane) = w[t];
+      }
+    }
+  }
+};
+
+// one element of the product in plain fp32, for a result the split could not carry
+template <bool A_MN, bool B_MN>
+__device__ __forceinline__ float plain_dot(const SplitArgs& p, int row, int col) {
+  float acc = 0.f;
+#pragma unroll 1
+  for (int k = 0; k < p.K; ++k) {
+    const float a = A_MN ? p.a.p[(int64_t)k * p.a.ld + row] : p.a.p[(int64_t)row * p.a.ld + k];
+    const float b = B_MN ? p.b.p[(int64_t)k * p.b.ld + col] : p.b.p[(int64_t)col * p.b.ld + k];
+    acc = fmaf(a, b, acc);
+  }
+  return acc;
+}
+
+// The 32 x 16 piece of C at (r0, c0), lane = row: unscaled, added to C or written.  Four lanes write 64 consecutive
+// bytes of a row, through `out` ([32 rows][16 columns] of shared memory).
+template <bool A_MN, bool B_MN>
+__device__ __forceinline__ void store_piece(const SplitArgs& p, float (&v)[16], float* out, int r0, int c0, int lane) {
+  if (r0 >= p.M || c0 >= p.N) return;
+  bool finite = true;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) finite = finite && fabsf(v[i]) <= kFloatMax;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    *reinterpret_cast<float4*>(out + lane * kOutPitch + 4 * i) =
+        make_float4(v[4 * i] * kUnscale, v[4 * i + 1] * kUnscale, v[4 * i + 2] * kUnscale, v[4 * i + 3] * kUnscale);
+  if (!finite && r0 + lane < p.M)
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i) {
+      float& x = out[lane * kOutPitch + i];
+      if (!(fabsf(x) <= kFloatMax) && c0 + i < p.N) x = plain_dot<A_MN, B_MN>(p, r0 + lane, c0 + i);
+    }
+  __syncwarp();
+  if (p.vec_c) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int rl = j * 8 + (lane >> 2), row = r0 + rl, col = c0 + (lane & 3) * 4;
+      if (row >= p.M || col >= p.N) continue;
+      float4 x = *reinterpret_cast<const float4*>(out + rl * kOutPitch + (lane & 3) * 4);
+      float* dst = p.C + (int64_t)row * p.ldc + col;
+      if (col + 3 < p.N) {
+        if (p.accumulate) {
+          const float4 old = *reinterpret_cast<const float4*>(dst);
+          x.x += old.x; x.y += old.y; x.z += old.z; x.w += old.w;
+        }
+        *reinterpret_cast<float4*>(dst) = x;
+      } else {
+        const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+          if (col + e < p.N) dst[e] = p.accumulate ? dst[e] + xs[e] : xs[e];
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int rl = j * 2 + (lane >> 4), row = r0 + rl, col = c0 + (lane & 15);
+      if (row >= p.M || col >= p.N) continue;
+      const float x = out[rl * kOutPitch + (lane & 15)];
+      float* dst = p.C + (int64_t)row * p.ldc + col;
+      *dst = p.accumulate ? *dst + x : x;
+    }
+  }
+  __syncwarp();
+}
+
+template <bool A_MN, bool B_MN, bool VEC>
+__global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __grid_constant__ SplitArgs p) {
+  extern __shared__ unsigned char smem_unaligned[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kBarOffset);
+  uint64_t* empty_bar = full_bar + kStages;
+  uint64_t* acc_full = empty_bar + kStages;  // [2]
+  uint64_t* acc_empty = acc_full + 2;        // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int splits = p.splits, rank = splits > 1 ? (int)cluster_ctarank() : 0;
+  // this CTA's tiles (one, if K is shared) and its blocks of each
+  const int tile_first = (int)blockIdx.x / splits, tile_step = splits > 1 ? INT_MAX / 2 : (int)gridDim.x;
+  const int tiles = p.tiles_m * p.tiles_n;
+  const int kb0 = (int)((int64_t)p.kb * rank / splits), kb1 = (int)((int64_t)p.kb * (rank + 1) / splits);
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(&full_bar[i], kLoadWarps);
+      mbar_init(&empty_bar[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&acc_full[i], 1);
+      mbar_init(&acc_empty[i], kPromoWarps);
+    }
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, 2 * BT);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  // Launched with programmatic stream serialization: the set-up above may overlap the kernel before this one.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  if (warp < kPromoWarps) {
+    // ------------------------------------------------------------------ promotion and epilogue
+    const int quad = warp & 3, half = warp >> 2;  // tensor-memory lanes 32*quad.., columns 64*half..
+    const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
+    float* out = reinterpret_cast<float*>(smem + kOutOffset + warp * kOutWarpBytes);
+    int blocks = 0, issued = 0;  // blocks added up, blocks handed to the tensor core (by warp 0), over all tiles
+    const int n_mine = tile_first < tiles ? (tiles - 1 - tile_first) / tile_step + 1 : 0;
+    const int64_t total = (int64_t)n_mine * (kb1 - kb0);
+    bool ok = true;
+    // the MMAs of the next block: stage and accumulator alternate with the block's number
+    auto issue = [&]() {
+      constexpr uint32_t idesc = umma_idesc_f16(BT, BT, true, A_MN, B_MN);
+      // term products, smallest first; (term of A, term of B)
+      constexpr int ta[6] = {2, 0, 1, 1, 0, 0}, tb[6] = {0, 2, 1, 0, 1, 0};
+      const int i = issued & 1;
+      const uint32_t phase = (issued >> 1) & 1;
+      if (lane == 0 && mbar_wait(&full_bar[i], phase, abort_flag, p.status, ST_TIMEOUT_FULL) &&
+          mbar_wait(&acc_empty[i], phase ^ 1, abort_flag, p.status, ST_TIMEOUT_ACC_EMPTY)) {
+        tc_fence_after_sync();
+        const uint32_t sa = smem_u32(smem + i * kStageBytes), sb = sa + 3 * kPlane;
+        // descriptors differ only in the start address
+        const uint64_t da = A_MN ? umma_desc_mnmajor_sw128(sa, BK * 128, 1024) : umma_desc_kmajor_sw128(sa);
+        const uint64_t db = B_MN ? umma_desc_mnmajor_sw128(sb, BK * 128, 1024) : umma_desc_kmajor_sw128(sb);
+#pragma unroll
+        for (int t = 0; t < 6; ++t)
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k)
+            umma_f16_ss(tmem_base + i * BT, da + ((ta[t] * kPlane + k * (A_MN ? 16 * 128 : 32)) >> 4),
+                        db + ((tb[t] * kPlane + k * (B_MN ? 16 * 128 : 32)) >> 4), idesc, (t | k) != 0 ? 1u : 0u);
+        umma_commit(&empty_bar[i]);
+        umma_commit(&acc_full[i]);
+      }
+      __syncwarp();
+      ++issued;
+    };
+    if (warp == 0 && total > 0) issue();
+    for (int tile = tile_first; tile < tiles && ok; tile += tile_step) {
+      float v[64];
+#pragma unroll
+      for (int i = 0; i < 64; ++i) v[i] = 0.f;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (warp == 0 && issued < total) issue();
+        const int acc = blocks & 1;
+        if (!mbar_wait(&acc_full[acc], (blocks >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACC_FULL)) {
+          ok = false;
+          break;
+        }
+        ++blocks;
+        tc_fence_after_sync();
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t t[32];
+          tmem_ld_32x32b_x32(tmem_base + acc * BT + half * 64 + h * 32 + lane_addr, t);
+          tmem_ld_wait();
+          if (h == 1) {
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[acc]);
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[h * 32 + i] += __uint_as_float(t[i]);
+        }
+      }
+      if (!ok) break;
+      if (splits > 1) {
+        // the part goes into this CTA's shared memory, [32 groups of 4 columns][128 rows] float4.  The ring is free: the last
+        // accumulator is complete, so every MMA has read its stage, and no block follows.
+        float4* part = reinterpret_cast<float4*>(smem) + quad * 32 + lane;
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          part[(half * 16 + i) * BT] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+      } else {
+        const TileCoord tc = tile_coord(tile, p.tiles_m, p.tiles_n);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          float x[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) x[i] = v[u * 16 + i];
+          store_piece<A_MN, B_MN>(p, x, out, tc.m * BT + quad * 32, tc.n * BT + half * 64 + u * 16, lane);
+        }
+      }
+    }
+    if (splits > 1) {
+      // every role of every CTA of the cluster ends (its waits are bounded), so this meeting is reached
+      __syncwarp();
+      cluster_sync_all();
+      const TileCoord tc = tile_coord(tile_first, p.tiles_m, p.tiles_n);
+      // the tile's 32 pieces (32 rows x 16 columns) over the cluster's promotion warps
+      for (int x = rank * kPromoWarps + warp; x < 32; x += kPromoWarps * splits) {
+        const int g = x & 3, u = x >> 2;
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = 0.f;
+        const uint32_t at = smem_u32(smem) + ((u * 4) * BT + g * 32 + lane) * 16;
+        for (int c = 0; c < splits; ++c) {
+          const uint32_t peer = mapa_addr(at, c);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float4 t = ld_cluster_f4(peer + i * (BT * 16));
+            v[4 * i] += t.x; v[4 * i + 1] += t.y; v[4 * i + 2] += t.z; v[4 * i + 3] += t.w;
+          }
+        }
+        store_piece<A_MN, B_MN>(p, v, out, tc.m * BT + g * 32, tc.n * BT + u * 16, lane);
+      }
+      cluster_sync_all();  // the peers have read this CTA's part
+    }
+  } else {
+    // ------------------------------------------------------------------ loaders
+    const int tid = threadIdx.x - kPromoWarps * 32;
+    Loader<A_MN, VEC> la;
+    Loader<B_MN, VEC> lb;
+    int tile = tile_first, kb = kb0, stage = 0;
+    uint32_t phase = 0;
+    bool a_in = false, b_in = false;  // the tile's rows of A, columns of B lie inside the operands
+    auto place = [&]() {
+      const TileCoord tc = tile_coord(tile, p.tiles_m, p.tiles_n);
+      la.place(p.a, tc.m * BT, kb0 * BK, tid);
+      lb.place(p.b, tc.n * BT, kb0 * BK, tid);
+      a_in = (tc.m + 1) * BT <= p.M;
+      b_in = (tc.n + 1) * BT <= p.N;
+    };
+    bool more = tile < tiles;
+    if (more) {
+      place();
+      const bool k_in = (kb + 1) * BK <= p.K;
+      la.fetch(p.a, a_in && k_in);
+      lb.fetch(p.b, b_in && k_in);
+    }
+    while (more) {
+      if (++kb == kb1) {  // the block after the one in registers
+        kb = kb0;
+        tile += tile_step;
+        more = tile < tiles;
+        if (more) place();
+      }
+      if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+      __syncwarp();
+      unsigned char* sa = smem + stage * kStageBytes;
+      const bool k_in = (kb + 1) * BK <= p.K;
+      la.store(sa, tid);
+      if (more) la.fetch(p.a, a_in && k_in);
+      lb.store(sa + 3 * kPlane, tid);
+      if (more) lb.fetch(p.b, b_in && k_in);
+      fence_proxy_async_smem();  // the planes are read by the tensor core
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full_bar[stage]);
+      if (++stage == kStages) {
+        stage = 0;
+        phase ^= 1;
+      }
+    }
+    if (splits > 1) {
+      __syncwarp();
+      cluster_sync_all();
+      cluster_sync_all();
+    }
+  }
+
+  // ------------------------------------------------------------------ teardown
+  if (*abort_flag) {
+    unsigned long long t0 = globaltimer();
+    while (globaltimer() - t0 < 200000ull) __nanosleep(1000);
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    __syncwarp();
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, 2 * BT);
   }
 }
 
-// C[i][j] <- (accumulate ? C[i][j] : 0) + sum over the nine blocks P[s*M + i][t*N + j], smallest terms first
-__global__ void __launch_bounds__(256) sum9_kernel(const float* __restrict__ P, int64_t ldp, int64_t M, int64_t N,
-                                                   float* __restrict__ C, int64_t ldc, int accumulate, int vec_c) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int64_t quads = N / 4;  // N % 4 == 0 on this path
-  const int64_t total = M * quads;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = i / quads, c = (i % quads) * 4;
-    auto blk = [&](int s, int t) {
-      return __ldcs(reinterpret_cast<const float4*>(P + ((int64_t)s * M + r) * ldp + (int64_t)t * N + c));
-    };
-    // order of magnitude of A_s.B_t is 2^(-8 (s + t)): add from s + t = 4 down to 0
-    const float4 b22 = blk(2, 2), b21 = blk(2, 1), b12 = blk(1, 2), b20 = blk(2, 0), b02 = blk(0, 2),
-                 b11 = blk(1, 1), b10 = blk(1, 0), b01 = blk(0, 1), b00 = blk(0, 0);
-    float4 acc;
-#define FB_SUM9(f) acc.f = ((((((((b22.f + b21.f) + b12.f) + b20.f) + b02.f) + b11.f) + b10.f) + b01.f) + b00.f)
-    FB_SUM9(x); FB_SUM9(y); FB_SUM9(z); FB_SUM9(w);
-#undef FB_SUM9
-    float* dst = C + r * ldc + c;
-    if (vec_c) {
-      if (accumulate) {
-        const float4 old = *reinterpret_cast<const float4*>(dst);
-        acc.x += old.x; acc.y += old.y; acc.z += old.z; acc.w += old.w;
-      }
-      *reinterpret_cast<float4*>(dst) = acc;
-    } else {
-      const float v[4] = {acc.x, acc.y, acc.z, acc.w};
-      for (int j = 0; j < 4; ++j) dst[j] = accumulate ? dst[j] + v[j] : v[j];
-    }
-  }
+// K over the CTAs of a cluster while that leaves every CTA an SM and two blocks of its own (adding the parts up takes
+// about as long as one: 512 x 512 x 512 in 11.6 us with 2 blocks each on 4 CTAs a tile)
+int split_of(int64_t tiles, int64_t kb, int sms) {
+  int splits = 1;
+  while (splits < 8 && tiles * splits * 2 <= sms && kb >= splits * 4) splits *= 2;
+  return splits;
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-int own_buffer(frisk_b200_ctx* ctx, int slot, size_t bytes) {
-  StagingBuffer& b = ctx->stage[slot];
-  if (b.ptr && b.bytes >= bytes) return 0;
-  if (b.ptr) {
-    FB_CUDA(ctx, cudaFree(b.ptr));
-    b.ptr = nullptr;
-    b.bytes = 0;
-  }
-  const size_t want = (bytes + 255) / 256 * 256;
-  FB_CUDA(ctx, cudaMalloc(&b.ptr, want));
-  b.bytes = want;
+template <bool A_MN, bool B_MN, bool VEC>
+int launch_one(frisk_b200_ctx* ctx, SplitArgs a, cudaStream_t s) {
+  auto kern = gemm_f32_split_kernel<A_MN, B_MN, VEC>;
+  static PerDeviceOnce opt_in;
+  if (opt_in(ctx->device, [&] {
+        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTotal) == cudaSuccess ? 0 : 1;
+      }))
+    return FRISK_B200_E_CUDA;
+  static ClusterCapacity capacity;
+  const int sms = std::min(ctx->num_sms, kNumSMsDefault), tiles = a.tiles_m * a.tiles_n;
+  a.splits = split_of(tiles, a.kb, sms);
+  while (a.splits > 1 && capacity(ctx->device, kern, kThreads, kSmemTotal, a.splits) < tiles) a.splits /= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(a.splits > 1 ? tiles * a.splits : std::min(tiles, sms)));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmemTotal;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the kernel waits (griddepcontrol.wait) itself
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)a.splits;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = a.splits > 1 ? 2 : 1;
+  FB_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, a));
   return 0;
 }
 
-template <typename... Args>
-int launch_pdl(frisk_b200_ctx* ctx, void (*kern)(Args...), unsigned grid_x, unsigned grid_y, cudaStream_t s,
-               Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid_x, grid_y);
-  cfg.blockDim = dim3(256);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the kernels wait (griddepcontrol.wait) themselves
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  FB_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, args...));
-  return 0;
+template <bool A_MN, bool B_MN>
+int launch_vec(frisk_b200_ctx* ctx, const SplitArgs& a, bool vec, cudaStream_t s) {
+  return vec ? launch_one<A_MN, B_MN, true>(ctx, a, s) : launch_one<A_MN, B_MN, false>(ctx, a, s);
 }
 
 }  // namespace
 
-// TMA wants 16-byte row pitches of the stacked bf16 operands and the sum works on whole float4s
+// what `algo = FRISK_B200_ALGO_F32_SPLIT` accepts
 bool f32_split_supported(const frisk_b200_gemm_desc& d) {
   if (d.dtype_ab != FRISK_B200_F32 || d.dtype_c != FRISK_B200_F32) return false;
   if (d.M % 8 || d.N % 8 || d.K % 8) return false;
   return 3 * d.M <= INT32_MAX && 3 * d.N <= INT32_MAX && d.K <= INT32_MAX;
 }
 
-// Worth the two extra passes only when the product is large next to them
 bool f32_split_preferred(const frisk_b200_gemm_desc& d) {
   return f32_split_supported(d) && d.M >= 256 && d.N >= 256 && d.K >= 256;
 }
 
+// Both kernels estimated in microseconds from measurements.  CUDA cores: 4.3 for 64 x 64 x 64 and about 2.0 more for
+// every further 64 x 64 x 64 unit an SM takes, 2 to add up the parts of a shared tile (512^3 13.5, 1024^3 57, 2048^3 401).
+// Tensor cores: 5.5 and 2.1 for every 128 x 128 x 64 block a CTA takes, 2 more to add up the parts of a shared tile (64^3
+// 7.6, 128^3 9.9, 512^3 11.6, 1024^3 22.9, 2048^3 128); half as much again per block where rows are not 16-byte aligned.
+bool f32_split_beats_simt(const frisk_b200_gemm_desc& d) {
+  if (d.dtype_ab != FRISK_B200_F32 || d.dtype_c != FRISK_B200_F32) return false;
+  if (d.M > INT32_MAX / 4 || d.N > INT32_MAX / 4 || d.K > INT32_MAX / 4) return false;
+  const GemmDims g = resolve_dims(d);
+  const double sms = kNumSMsDefault;
+  const int64_t kb = (g.K + BK - 1) / BK, tiles = ((g.M + BT - 1) / BT) * ((g.N + BT - 1) / BT);
+  if (tiles > (int64_t)1 << 30) return false;
+  const double units = std::ceil((double)(((g.M + 63) / 64) * ((g.N + 63) / 64)) * (double)kb / sms);
+  const double simt = 4.3 + 2.0 * (units - 1) + (units < (double)kb ? 2.0 : 0.0);
+  const int splits = split_of(tiles, kb, kNumSMsDefault);
+  const double blocks = std::ceil((double)tiles / sms) * std::ceil((double)kb / splits);
+  const double block = g.lda % 4 || g.ldb % 4 ? 3.2 : 2.1;
+  return 5.5 + block * blocks + (splits > 1 ? 2.0 : 0.0) < simt;
+}
+
 int launch_gemm_f32_split(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const float* A, const float* B,
                           float* C, cudaStream_t s) {
-  if (!f32_split_supported(d)) return FRISK_B200_E_UNSUPPORTED;
   const GemmDims g = resolve_dims(d);
-  const int64_t M = g.M, N = g.N, K = g.K;
-
-  // context-owned scratch: the stacked operands, the 3M x 3N product, the GEMM's own tail scratch
-  frisk_b200_gemm_desc t = {};
-  t.M = 3 * M;
-  t.N = 3 * N;
-  t.K = K;
-  t.dtype_ab = FRISK_B200_BF16;
-  t.dtype_c = FRISK_B200_F32;
-  t.trans_a = d.trans_a;
-  t.trans_b = d.trans_b;
-  t.clear_accum = 1;
-  t.lda = d.trans_a ? 3 * M : K;
-  t.ldb = d.trans_b ? K : 3 * N;
-  t.ldc = 3 * N;
-  t.algo = tcgen05_2cta_preferred(t) ? FRISK_B200_ALGO_TCGEN05_PAIR : FRISK_B200_ALGO_TCGEN05;
-  const size_t tail = t.algo == FRISK_B200_ALGO_TCGEN05_PAIR ? tcgen05_2cta_workspace_bytes(t) : 0;
-  void *pa, *pb, *pp, *ws = nullptr;
-  size_t ws_bytes = 0;
-  {
-    std::lock_guard<std::recursive_mutex> lock(ctx->mu);
-    int rc;
-    if ((rc = own_buffer(ctx, 8, (size_t)3 * M * K * 2))) return rc;
-    if ((rc = own_buffer(ctx, 9, (size_t)3 * N * K * 2))) return rc;
-    if ((rc = own_buffer(ctx, 10, (size_t)9 * M * N * 4))) return rc;
-    if (tail) {
-      StagingBuffer& b = ctx->stage[5];
-      if (!b.ptr || b.bytes < tail) {
-        if ((rc = own_buffer(ctx, 5, tail))) return rc;
-        FB_CUDA(ctx, cudaMemsetAsync(b.ptr, 0, b.bytes, s));  // tickets start at zero; every launch leaves them so
-      }
-      ws = b.ptr;
-      ws_bytes = b.bytes;
-    }
-    pa = ctx->stage[8].ptr;
-    pb = ctx->stage[9].ptr;
-    pp = ctx->stage[10].ptr;
-  }
-
-  SplitOperand oa, ob;
-  oa.src = A;
-  oa.dst = static_cast<__nv_bfloat16*>(pa);
-  oa.rows = d.trans_a ? K : M;
-  oa.cols = d.trans_a ? M : K;
-  oa.ld = g.lda;
-  oa.dst_ld = t.lda;
-  oa.plane = d.trans_a ? M : M * K;
-  oa.vec = aligned16(A) && g.lda % 4 == 0;
-  ob.src = B;
-  ob.dst = static_cast<__nv_bfloat16*>(pb);
-  ob.rows = d.trans_b ? N : K;
-  ob.cols = d.trans_b ? K : N;
-  ob.ld = g.ldb;
-  ob.dst_ld = t.ldb;
-  ob.plane = d.trans_b ? N * K : N;
-  ob.vec = aligned16(B) && g.ldb % 4 == 0;
-  const int64_t quads = std::max(oa.rows * ((oa.cols + 3) / 4), ob.rows * ((ob.cols + 3) / 4));
-  const unsigned gx = (unsigned)std::min<int64_t>((quads + 255) / 256, (int64_t)ctx->num_sms * 8);
-  int rc = launch_pdl(ctx, split_bf16x3_kernel, gx, 2u, s, oa, ob);
-  if (rc) return rc;
-
-  rc = t.algo == FRISK_B200_ALGO_TCGEN05_PAIR ? launch_gemm_tcgen05_2cta(ctx, t, pa, pb, pp, ws, ws_bytes, s)
-                                              : launch_gemm_tcgen05(ctx, t, pa, pb, pp, s);
-  if (rc) return rc;
-
-  const int64_t out_quads = M * (N / 4);
-  const unsigned gs = (unsigned)std::min<int64_t>((out_quads + 255) / 256, (int64_t)ctx->num_sms * 8);
-  return launch_pdl(ctx, sum9_kernel, gs, 1u, s, static_cast<const float*>(pp), (int64_t)(3 * N), M, N, C, g.ldc,
-                    d.clear_accum ? 0 : 1, (int)(aligned16(C) && g.ldc % 4 == 0));
+  SplitArgs a;
+  a.a = Operand{A, g.lda, (int)(d.trans_a ? g.K : g.M), (int)(d.trans_a ? g.M : g.K)};
+  a.b = Operand{B, g.ldb, (int)(d.trans_b ? g.N : g.K), (int)(d.trans_b ? g.K : g.N)};
+  const bool vec = aligned16(A) && g.lda % 4 == 0 && aligned16(B) && g.ldb % 4 == 0;
+  a.C = C;
+  a.ldc = g.ldc;
+  a.M = (int)g.M; a.N = (int)g.N; a.K = (int)g.K;
+  a.accumulate = d.clear_accum ? 0 : 1;
+  a.vec_c = aligned16(C) && g.ldc % 4 == 0;
+  const int64_t tiles_m = (g.M + BT - 1) / BT, tiles_n = (g.N + BT - 1) / BT;
+  if (tiles_m * tiles_n > (int64_t)1 << 30) return FRISK_B200_E_UNSUPPORTED;
+  a.tiles_m = (int)tiles_m;
+  a.tiles_n = (int)tiles_n;
+  a.kb = (int)((g.K + BK - 1) / BK);
+  a.status = ctx->d_status;
+  const bool a_mn = d.trans_a != 0, b_mn = d.trans_b == 0;
+  if (a_mn) return b_mn ? launch_vec<true, true>(ctx, a, vec, s) : launch_vec<true, false>(ctx, a, vec, s);
+  return b_mn ? launch_vec<false, true>(ctx, a, vec, s) : launch_vec<false, false>(ctx, a, vec, s);
 }
 
 }  // namespace fb

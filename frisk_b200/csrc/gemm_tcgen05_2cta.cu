@@ -59,15 +59,6 @@ struct Smem2 {
 static_assert(Smem2::kTotalOut <= 232448, "the output boxes must fit next to the operand ring");
 
 // ---- cluster / cta_group::2 primitives
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // shared::cluster address of `p` (a shared-memory object of this CTA) in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t mapa_u32(const void* p, uint32_t rank) {
   uint32_t out;

@@ -80,6 +80,53 @@ def test_f32_split_transposes_accumulate_unaligned(ctx, ta, tb):
         check(ctx, 100, 77, 51, "fp32", "fp32", ta, tb, 11, algo=S)  # extents must be multiples of 8
 
 
+@pytest.mark.parametrize("M,N,K,acc", [
+    (512, 512, 512, False),    # a cluster of four CTAs per tile
+    (513, 640, 1000, True),    # two per tile, unaligned C and (transposed) operands, ragged rows and k
+    (1152, 2048, 65, False),   # 144 whole tiles, one k beyond a block
+    (2049, 1153, 200, False),  # more tiles than SMs, ragged everywhere
+    (384, 384, 4100, True),    # eight CTAs per tile
+])
+def test_f32_auto_on_the_tensor_cores(ctx, M, N, K, acc):
+    """Sizes an AUTO call runs on the split kernel: shared and whole tiles, every layout.  The bound is the error
+    of plain fp32 accumulation: K roundings of 2^-24 relative to the running sum, adding up like a random walk."""
+    for ta, tb in ((False, False), (False, True), (True, False), (True, True)):
+        assert check(ctx, M, N, K, "fp32", "fp32", ta, tb, 23, accumulate=acc) < 2.0 ** -24 * max(8, K ** 0.5)
+
+
+def test_f32_auto_extreme_values(ctx):
+    """Elements that are infinite, NaN, near the largest and the smallest normal numbers, and subnormal: the results fp32
+    arithmetic gives (products of 2^-100 and 2^100 keep their accuracy)."""
+    import torch
+
+    import frisk_b200 as F
+    n = 512
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a, b = (torch.randn(n, n, generator=g, device="cuda") for _ in range(2))
+    a[0] *= 2.0 ** -100
+    b[:, 1] *= 2.0 ** 100
+    a[2] *= 2.0 ** 110                       # beyond the split's range, results still finite (but in column 1)
+    a[3, 7], a[4, 9], a[5, 11] = float("inf"), float("nan"), -float("inf")
+    b[13, 6], b[15, 8] = float("inf"), float("nan")
+    a[6] = 2.0 ** -140                       # a subnormal row
+    a[7], b[:, 9] = 3.0e38, 1.0              # overflows
+    c = torch.empty(n, n, device="cuda")
+    F.gemm(a, b, c)
+    ref = a.double() @ b.double()
+    mag = a.double().abs() @ b.double().abs()
+    want = ref.float()
+    sure = ~torch.isfinite(ref) | (mag < 1e38) | (torch.isinf(want) & (ref.abs() > 1e39))  # no overflow on the way to be in doubt
+    sure &= ~((torch.arange(n, device="cuda") == 7)[:, None] & (torch.arange(n, device="cuda") != 9)[None])
+    sure[2, 1] = False                       # products that overflow with either sign
+    assert torch.equal(torch.isnan(c)[sure], torch.isnan(want)[sure])
+    assert torch.equal(torch.isinf(c)[sure], torch.isinf(want)[sure])
+    at = sure & torch.isinf(want)
+    assert torch.equal(c[at], want[at])
+    ok = torch.isfinite(want) & sure
+    # one rounding of the sum of the products' magnitudes per 64 k, and the smallest subnormal
+    assert ((c.double() - ref).abs()[ok] <= (mag * 2.0 ** -21 + 2.0 ** -148)[ok]).all()
+
+
 @pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
 def test_f32_simt_shared_k_ranges(ctx, ta, tb):
     """Shapes whose tiles are fewer than the SMs or do not divide among them: every tile's k range is shared
