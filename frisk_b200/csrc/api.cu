@@ -205,6 +205,31 @@ int prepare_owned_skinny_ws(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, 
   return 0;
 }
 
+// The calling stream's set of the row scratch; false when the sets belong to other streams (or the stream's handle does
+// not name one stream): the reduction is then composed from its own kernel.  A set stays its stream's for the context's life.
+bool row_scratch(frisk_b200_ctx* ctx, cudaStream_t s, RowEpilogue* out) {
+  if (s == cudaStreamPerThread) return false;
+  std::lock_guard<std::mutex> lock(ctx->row_mu);
+  int i = 0;
+  while (i < ctx->rows_owned && ctx->row_owner[i] != s) ++i;
+  if (i == ctx->rows_owned) {
+    if (i == kRowSets) return false;
+    ctx->row_owner[i] = s;
+    ++ctx->rows_owned;
+  }
+  unsigned char* base = static_cast<unsigned char*>(ctx->row_scratch) + i * kRowSetBytes;
+  out->row_tickets = reinterpret_cast<unsigned*>(base);
+  out->row_partials = reinterpret_cast<float*>(base + kRowTicketBytes);
+  return true;
+}
+
+// A C the TMA unit cannot address (base or rows off 16 bytes) always goes to the one-CTA kernel, whose warps write whole
+// rows; the pair kernel's threads write their own (3001 x 2055 x 1032 accumulating: 224 us).
+bool one_cta_preferred(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* C) {
+  if ((reinterpret_cast<uintptr_t>(C) & 15u) || resolve_dims(d).ldc * (int64_t)dtype_size(d.dtype_c) % 16) return true;
+  return tcgen05_clocks(ctx, d) < tcgen05_2cta_clocks(d);
+}
+
 }  // namespace
 }  // namespace fb
 
@@ -258,6 +283,10 @@ int frisk_b200_ctx_create(frisk_b200_ctx** out, int device) {
   if ((e = cudaMemset(ctx->d_status, 0, 256)) != cudaSuccess) return fail(e);
   if ((e = cudaMalloc(&ctx->attn_scratch, attention_decode_scratch_bytes())) != cudaSuccess) return fail(e);
   if ((e = cudaMemset(ctx->attn_scratch, 0, attention_decode_ticket_bytes())) != cudaSuccess) return fail(e);
+  if ((e = cudaMalloc(&ctx->row_scratch, kRowSets * kRowSetBytes)) != cudaSuccess) return fail(e);
+  for (int i = 0; i < kRowSets; ++i)
+    if ((e = cudaMemset(static_cast<unsigned char*>(ctx->row_scratch) + i * kRowSetBytes, 0, kRowTicketBytes)) != cudaSuccess)
+      return fail(e);
   if ((e = cudaStreamSynchronize(nullptr)) != cudaSuccess) return fail(e);  // cleared before any stream uses it
   if ((e = cudaMallocHost(&ctx->h_status, 256)) != cudaSuccess) return fail(e);
   ctx->h_status[0] = 0;
@@ -278,6 +307,7 @@ int frisk_b200_ctx_destroy(frisk_b200_ctx* ctx) {
     if (b.ptr) cudaFree(b.ptr);
   if (ctx->d_status) cudaFree(ctx->d_status);
   if (ctx->attn_scratch) cudaFree(ctx->attn_scratch);
+  if (ctx->row_scratch) cudaFree(ctx->row_scratch);
   if (ctx->h_status) cudaFreeHost(ctx->h_status);
   for (auto& ev : ctx->ev)
     if (ev) cudaEventDestroy(ev);
@@ -393,6 +423,8 @@ int frisk_b200_gemm(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* d, const vo
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   FB_DEVICE(ctx);
   // (what an AUTO call runs; a call that names its kernel runs that)
+  if (d->algo == FRISK_B200_ALGO_AUTO && (algo == FRISK_B200_ALGO_TCGEN05 || algo == FRISK_B200_ALGO_TCGEN05_PAIR))
+    algo = one_cta_preferred(ctx, *d, C) ? FRISK_B200_ALGO_TCGEN05 : FRISK_B200_ALGO_TCGEN05_PAIR;
   if (d->algo == FRISK_B200_ALGO_AUTO && d->dtype_ab == FRISK_B200_F32)
     algo = f32_split_beats_simt(*d) ? FRISK_B200_ALGO_F32_SPLIT : FRISK_B200_ALGO_SIMT_F32;
   switch (algo) {
@@ -673,6 +705,18 @@ int frisk_b200_gemm_fused(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* d, co
   FB_DEVICE(ctx);
   const bool use_fill = e->fill_enable && !d->clear_accum;  // a fill before an overwriting gemm is dead
   const float fill = round_fill(e->fill_value, d->dtype_c);
+  const int algo = frisk_b200_gemm_select(d);
+  if (d->algo == FRISK_B200_ALGO_AUTO && !workspace && (algo == FRISK_B200_ALGO_TCGEN05 || algo == FRISK_B200_ALGO_TCGEN05_PAIR) &&
+      one_cta_preferred(ctx, *d, C)) {
+    RowEpilogue re{};
+    re.has_fill = use_fill ? 1 : 0;
+    re.fill = fill;
+    re.reduce_kind = e->reduce_kind;
+    re.reduce_clear = e->reduce_clear;
+    re.reduce_dst = e->reduce_dst;
+    if (e->reduce_kind == FRISK_B200_REDUCE_NONE || (tcgen05_row_epilogue_fits(*d) && row_scratch(ctx, s, &re)))
+      return launch_gemm_tcgen05(ctx, *d, A, B, C, s, &re);
+  }
   if (fused == 0) {
     int rc = 0;
     if (use_fill && (rc = launch_fill(C, g.M, g.N, g.ldc, fill, d->dtype_c, s))) return rc;

@@ -47,6 +47,13 @@ struct TmapEntry {
 constexpr size_t kTmapCacheEntries = 64;
 constexpr int kMaxDevices = 64;
 
+// One set of the fused row reduction's scratch: a ticket per 128-row block (zero between launches), then row partials.
+constexpr int kRowSets = 4;
+constexpr int kRowTickets = 16384;
+constexpr size_t kRowTicketBytes = (size_t)kRowTickets * 4;
+constexpr size_t kRowPartialBytes = (size_t)4 << 20;
+constexpr size_t kRowSetBytes = kRowTicketBytes + kRowPartialBytes;
+
 // Per-kernel set-up that has to happen once per device (opting in to large dynamic shared
 // memory, an occupancy query): `run` returns 0 on success, and then never runs again for
 // that device.  Two threads may both run it the first time; the calls are idempotent.
@@ -105,6 +112,12 @@ struct frisk_b200_ctx {
   // Scratch of fixed size, made with the context, so that a call that needs it never allocates; the tickets at its
   // start are zero between launches.  attn: decode attention
   void* attn_scratch = nullptr;
+  // fused row reductions of the one-CTA GEMM: one set (tickets, row partials) per stream, for the first kRowSets streams
+  // the context is called on, so that calls on different streams do not meet in it
+  void* row_scratch = nullptr;
+  cudaStream_t row_owner[fb::kRowSets] = {};
+  int rows_owned = 0;
+  std::mutex row_mu;
   cudaStream_t host_stream = nullptr;
   cudaStream_t copy_stream = nullptr;
   cudaStream_t out_stream = nullptr;
@@ -216,8 +229,21 @@ int launch_gemm_skinny(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const
                        void* ws, size_t ws_bytes, cudaStream_t s, unsigned* status = nullptr);
 
 bool tcgen05_supported(const frisk_b200_gemm_desc& d);
+// fill and row reduction folded into the one-CTA kernel
+struct RowEpilogue {
+  int has_fill;   // C_in is the constant `fill` (already rounded to C's element type); C is not read
+  float fill;
+  int reduce_kind, reduce_clear;  // FRISK_B200_REDUCE_*; over the ROUNDED values that are stored
+  void* reduce_dst;
+  float* row_partials;     // [boxes of 128 bytes of columns][M]
+  unsigned* row_tickets;   // one per 128-row block, zero between launches
+};
 int launch_gemm_tcgen05(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* A, const void* B,
-                        void* C, cudaStream_t s);
+                        void* C, cudaStream_t s, const RowEpilogue* epi = nullptr);
+// clocks the two kernels are estimated at, for the choice between them
+double tcgen05_clocks(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d);
+double tcgen05_2cta_clocks(const frisk_b200_gemm_desc& d);
+bool tcgen05_row_epilogue_fits(const frisk_b200_gemm_desc& d);
 
 // Row blocks of the fp32 product are stored into up to 8 destination buffers instead of C:
 // destination i receives rows [i*rows_per_target, (i+1)*rows_per_target) (it may be a peer

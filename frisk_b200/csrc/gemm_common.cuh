@@ -19,6 +19,13 @@ __device__ __forceinline__ TileCoord tile_coord(int t, int tiles_m, int tiles_n)
   return TileCoord{first_m + r % gsize, r / gsize};
 }
 
+__device__ __forceinline__ float reduce_identity(int kind) {
+  return kind == FRISK_B200_REDUCE_MAX ? -INFINITY : kind == FRISK_B200_REDUCE_MIN ? INFINITY : 0.f;
+}
+__device__ __forceinline__ float reduce_combine(int kind, float a, float b) {
+  return kind == FRISK_B200_REDUCE_MAX ? fmaxf(a, b) : kind == FRISK_B200_REDUCE_MIN ? fminf(a, b) : a + b;
+}
+
 // the value an fp32 result takes once it is stored as TO
 template <typename TO>
 __device__ __forceinline__ float rounded_as(float v);
@@ -83,6 +90,16 @@ __device__ __forceinline__ float2 unpack2(uint32_t u, __half) {
 __device__ __forceinline__ float2 unpack2(uint32_t u, __nv_bfloat16) {
   return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u));
 }
+
+// two packed 16-bit values of type TO (the float form exists so that templates compile)
+template <typename TO>
+__device__ __forceinline__ float2 unpack_out(uint32_t u);
+template <>
+__device__ __forceinline__ float2 unpack_out<__half>(uint32_t u) { return unpack2(u, __half()); }
+template <>
+__device__ __forceinline__ float2 unpack_out<__nv_bfloat16>(uint32_t u) { return unpack2(u, __nv_bfloat16()); }
+template <>
+__device__ __forceinline__ float2 unpack_out<float>(uint32_t u) { return make_float2(__uint_as_float(u), 0.f); }
 
 template <typename T, typename T2>
 __device__ __forceinline__ void store_row_chunk16(T* p, const uint32_t (&v)[32], int valid, bool vec_ok,

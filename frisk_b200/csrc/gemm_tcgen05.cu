@@ -4,12 +4,25 @@
 // lib/Dialect/Frisk/IR/LegacyImportSemantics.cpp:26-44).
 //
 // One persistent CTA per SM, 6 warps with fixed roles:
-//   warp 0    TMA producer: A and B tiles -> 4-stage shared-memory ring (full/empty mbarriers)
+//   warp 0    TMA producer: A and B tiles -> shared-memory ring of 192 KB (full/empty mbarriers)
 //   warp 1    MMA issuer:   one thread issues tcgen05.mma (128 x BN x 16) per k16 slice,
 //                           tcgen05.commit releases the stage / publishes the accumulator
-//   warps 2-5 epilogue:     tcgen05.ld of the finished accumulator, conversion, global stores
+//   warps 2-5 epilogue:     tcgen05.ld of the finished accumulator, conversion, stores
 // Two accumulators (2 x BN TMEM columns) let the epilogue of tile i overlap the main loop of
-// tile i+1.
+// tile i+1.  Output tiles are 128 x 256 (12 KB of operands per 128 clk of MMA) or, where those are too few, 128 x 128
+// (8 KB per 64 clk, all that shared memory delivers).
+//
+// Whole rounds of tiles are dealt out tile by tile.  The tiles of a partial last round (all of them, where there are
+// fewer tiles than SMs) are shared by clusters of 2, 4 or 8 CTAs, each multiplying its part of K: every CTA leaves its fp32
+// accumulator in its own shared memory (the operand ring has done its work by then), and the parts are added up over
+// distributed shared memory, in rank order, for the CTAs that finish the tile's boxes of C (reproducible, no scratch, no
+// CTA waits for one outside its cluster).
+//
+// Every form of C leaves through a shared-memory box of 32 rows x 128 bytes per epilogue warp: an aligned C by TMA
+// stores (and its old values, where they are added, come in by TMA loads), any other C by whole-row accesses of the warp.
+// `frisk.fill` before and a row reduction after the gemm are folded in: the fill value is added in registers, every
+// (row, box of columns) leaves one fp32 partial of the reduction, and the CTA that finishes a row block's last column
+// tile combines them in column order.
 //
 // Shared-memory operand images are the canonical 128-byte-swizzle layouts (rows of 64
 // 16-bit elements, 1024-byte aligned stages): K-major for an operand that is contiguous
@@ -17,6 +30,10 @@
 // inference proposes for 16-bit MMA operands
 // (lib/Dialect/Frisk/Target/SM90/SM90GemmConstraints.cpp:121-138); TMA writes them directly.
 // No TMA load uses cluster multicast.
+#include <limits.h>
+
+#include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "common.cuh"
@@ -31,53 +48,47 @@ using namespace gemm_detail;
 constexpr int BM = 128;
 constexpr int BK = 64;       // one 128-byte swizzle span of 16-bit elements
 constexpr int UMMA_K = 16;
-constexpr int kStages = 4;
 constexpr int kThreads = 192;
+constexpr int kBoxBytes = 32 * 128;
 
 template <int BN>
 struct SmemLayout {
   static constexpr int kABytes = BM * BK * 2;
   static constexpr int kBBytes = BN * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
+  static constexpr int kStages = 196608 / kStageBytes;  // 4 at BN = 256, 6 at BN = 128
   static constexpr int kBarOffset = kStages * kStageBytes;
-  static constexpr int kTotal = kBarOffset + 256 + 1024;  // barriers + alignment slack
-  // TMA-store epilogue only: two [32 rows][128 bytes] output boxes per epilogue warp, 1024-byte aligned
+  // two [32 rows][128 bytes] boxes of C per epilogue warp, 1024-byte aligned
   static constexpr int kOutOffset = kBarOffset + 1024;
-  static constexpr int kOutWarpBytes = 2 * 32 * 128;
-  static constexpr int kTotalOut = kOutOffset + 4 * kOutWarpBytes + 1024;
-  static_assert(kTotalOut <= 232448, "the output boxes must fit next to the operand ring");
+  static constexpr int kTotal = kOutOffset + 4 * 2 * kBoxBytes + 1024;
+  static_assert(kTotal <= 232448, "the boxes of C must fit next to the operand ring");
+  // a shared tile: this CTA's part [BN/4][128 rows] float4, then the sums of the columns it finishes (at most half)
+  static constexpr int kSumOffset = BM * BN * 4;
+  static_assert(kSumOffset + BM * BN * 2 <= kBarOffset, "the parts and sums of a shared tile must fit in the ring");
 };
 
-// Work items: the first n_full items are whole 128xBN tiles; the tiles that would form a
-// partial last wave are cut into two 128x(BN/2) items each, so that the last wave takes half
-// as long (see the host side for when this pays).
-struct Item {
-  int m0, n0, bn;
+struct GemmArgs {
+  void* C;
+  int64_t ldc;
+  int M, N, K;
+  int accumulate;  // the old C is added
+  int tma_c;       // C goes through the TMA unit
+  int n_whole;     // tiles [0, n_whole) are walked whole, one by one
+  int splits;      // CTAs of a cluster, which share the K of one of the other tiles
+  RowEpilogue epi;
+  unsigned* status;
 };
-template <int BN>
-__device__ __forceinline__ Item get_item(int idx, int n_full, int tiles_m, int tiles_n) {
-  int t = idx, half = -1;
-  if (idx >= n_full) {
-    t = n_full + ((idx - n_full) >> 1);
-    half = (idx - n_full) & 1;
-  }
-  TileCoord tc = tile_coord(t, tiles_m, tiles_n);
-  Item it{tc.m * BM, tc.n * BN, BN};
-  if (half >= 0) {
-    it.n0 += half * (BN / 2);
-    it.bn = BN / 2;
-  }
-  return it;
-}
 
 // A_MN / B_MN: the operand is contiguous along M / N in global memory (MN-major image).
-// TMA_OUT: an overwriting store of an aligned C leaves through shared-memory boxes and TMA stores.
-template <typename TO, int BN, bool BF16, bool A_MN, bool B_MN, bool TMA_OUT>
+// PLAIN: an overwriting store of an aligned C, the usual call, without the code of every other epilogue.
+template <typename TO, int BN, bool BF16, bool A_MN, bool B_MN, bool PLAIN>
 __global__ void __launch_bounds__(kThreads, 1)
     gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                        const __grid_constant__ CUtensorMap tmap_c, TO* __restrict__ C, int M, int N, int K, int64_t ldc, int accumulate, int vec_c,
-                        int n_full, int n_items, unsigned* __restrict__ status) {
+                        const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ GemmArgs p) {
   using L = SmemLayout<BN>;
+  const bool tma_c = PLAIN || p.tma_c, accumulate = !PLAIN && p.accumulate, has_fill = !PLAIN && p.epi.has_fill;
+  const int reduce_kind = PLAIN ? FRISK_B200_REDUCE_NONE : p.epi.reduce_kind;
+  constexpr int kStages = L::kStages;
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -85,12 +96,33 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* empty_bar = full_bar + kStages;
   uint64_t* acc_full = empty_bar + kStages;   // [2]
   uint64_t* acc_empty = acc_full + 2;         // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* box_bar = acc_empty + 2;          // [4 warps][2] old values of C have landed in a box
+  uint64_t* epi_bar = box_bar + 8;            // the epilogue threads among themselves
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(epi_bar + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
+  volatile uint32_t* epi_word = tmem_slot + 2;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + BN - 1) / BN;
-  const int num_kb = (K + BK - 1) / BK;
+  const int tiles_m = (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN, tiles = tiles_m * tiles_n;
+  const int splits = p.splits, rank = splits > 1 ? (int)cluster_ctarank() : 0;
+  const int num_kb = (p.K + BK - 1) / BK;
+  // this CTA's work, item by item: its whole tiles, then its 64-k blocks of the tile its cluster shares
+  struct Item {
+    int tile, kb0, kb1;
+    bool shared;
+  };
+  auto get_item = [&](int i, Item& it) -> bool {
+    const int whole = (int)blockIdx.x + i * (int)gridDim.x;
+    if (whole < p.n_whole) {
+      it = Item{whole, 0, num_kb, false};
+      return true;
+    }
+    const int n_mine = (int)blockIdx.x < p.n_whole ? (p.n_whole - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int tile = p.n_whole + (int)blockIdx.x / splits;
+    if (i > n_mine || splits == 1 || tile >= tiles) return false;
+    it = Item{tile, (int)((int64_t)num_kb * rank / splits), (int)((int64_t)num_kb * (rank + 1) / splits), true};
+    return true;
+  };
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
@@ -101,11 +133,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(&acc_full[i], 1);
       mbar_init(&acc_empty[i], 4);
     }
+    for (int i = 0; i < 8; ++i) mbar_init(&box_bar[i], 1);
+    mbar_init(epi_bar, 128);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
-    if (TMA_OUT) tma_prefetch_desc(&tmap_c);
+    if (tma_c) tma_prefetch_desc(&tmap_c);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, 2 * BN);
@@ -126,17 +160,18 @@ __global__ void __launch_bounds__(kThreads, 1)
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < n_items && ok; t += gridDim.x) {
-        const Item it = get_item<BN>(t, n_full, tiles_m, tiles_n);
-        const int m0 = it.m0, n0 = it.n0;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, status, ST_TIMEOUT_EMPTY)) {
+      Item it;
+      for (int i = 0; ok && get_item(i, it); ++i) {
+        const TileCoord tc = tile_coord(it.tile, tiles_m, tiles_n);
+        const int m0 = tc.m * BM, n0 = tc.n * BN;
+        for (int kb = it.kb0; kb < it.kb1; ++kb) {
+          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) {
             ok = false;
             break;
           }
           unsigned char* sa = smem + stage * L::kStageBytes;
           unsigned char* sb = sa + L::kABytes;
-          mbar_expect_tx(&full_bar[stage], L::kABytes + it.bn * (BK * 2));
+          mbar_expect_tx(&full_bar[stage], L::kStageBytes);
           const int k0 = kb * BK;
           if (A_MN) {
 #pragma unroll
@@ -146,11 +181,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             tma_load_2d(sa, &tmap_a, &full_bar[stage], k0, m0);
           }
           if (B_MN) {
-            for (int j = 0; j < it.bn / 64; ++j)
+#pragma unroll
+            for (int j = 0; j < BN / 64; ++j)
               tma_load_2d(sb + j * (BK * 128), &tmap_b, &full_bar[stage], n0 + j * 64, k0);
           } else {
             // boxes of 128 rows: stacked 8-row groups, the same image as one taller box
-            for (int j = 0; j < it.bn / 128; ++j)
+#pragma unroll
+            for (int j = 0; j < BN / 128; ++j)
               tma_load_2d(sb + j * (128 * BK * 2), &tmap_b, &full_bar[stage], k0, n0 + j * 128);
           }
           if (++stage == kStages) {
@@ -163,20 +200,19 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      constexpr uint32_t idesc_full = umma_idesc_f16(BM, BN, BF16, A_MN, B_MN);
-      constexpr uint32_t idesc_half = umma_idesc_f16(BM, BN / 2, BF16, A_MN, B_MN);
+      constexpr uint32_t idesc = umma_idesc_f16(BM, BN, BF16, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < n_items && ok; t += gridDim.x) {
-        const uint32_t idesc = (t >= n_full) ? idesc_half : idesc_full;
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, status, ST_TIMEOUT_ACC_EMPTY)) break;
+      Item it;
+      for (int i = 0; ok && get_item(i, it); ++i) {
+        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.status, ST_TIMEOUT_ACC_EMPTY)) break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag, status, ST_TIMEOUT_FULL)) {
+        for (int kb = it.kb0; kb < it.kb1; ++kb) {
+          if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, ST_TIMEOUT_FULL)) {
             ok = false;
             break;
           }
@@ -189,7 +225,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                                : umma_desc_kmajor_sw128(sa + k * (UMMA_K * 2));
             uint64_t db = B_MN ? umma_desc_mnmajor_sw128(sb + k * (UMMA_K * 128), BK * 128, 1024)
                                : umma_desc_kmajor_sw128(sb + k * (UMMA_K * 2));
-            umma_f16_ss(d_tmem, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
+            umma_f16_ss(d_tmem, da, db, idesc, (kb > it.kb0 || k != 0) ? 1u : 0u);
           }
           umma_commit(&empty_bar[stage]);  // stage reusable once these MMAs have read it
           if (++stage == kStages) {
@@ -208,75 +244,292 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else {
     // ------------------------------------------------------------------ epilogue
     const int quad = warp & 3;  // TMEM lanes [32*quad, 32*quad+32) are this warp's
-    int box_sel = 0;            // which of the warp's two output boxes the next TMA store uses
+    constexpr int U = 128 / (int)sizeof(TO);  // columns of a box
+    unsigned char* boxes = smem + L::kOutOffset + quad * 2 * kBoxBytes;
+    uint64_t* bars = box_bar + quad * 2;
+    TO* const C = static_cast<TO*>(p.C);
+    int box_sel = 0;              // the box the next unit uses
+    uint32_t box_phases = 0;      // bit b: the phase box b's barrier is in
     int acc = 0;
-    uint32_t acc_phase = 0;
-    for (int t = blockIdx.x; t < n_items; t += gridDim.x) {
-      const Item it = get_item<BN>(t, n_full, tiles_m, tiles_n);
-      const int m0 = it.m0, n0 = it.n0;
-      if (!mbar_wait(&acc_full[acc], acc_phase, abort_flag, status, ST_TIMEOUT_ACC_FULL)) break;
-      tc_fence_after_sync();
-      const int row = m0 + quad * 32 + lane;
-      const uint32_t taddr = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);
-      if (TMA_OUT) {
-        // a lane holds 128 bytes of ONE row; the warp writes its 32 rows as a 128-byte-swizzle box and one lane
-        // hands the box to the TMA unit, which writes whole lines and clips at the edges of C
-        constexpr int kUnitCols = 128 / (int)sizeof(TO);
-        unsigned char* boxes = smem + L::kOutOffset + quad * L::kOutWarpBytes;
-#pragma unroll 1
-        for (int u = 0; u < it.bn / kUnitCols; ++u) {
-          const int c0 = n0 + u * kUnitCols, r0 = m0 + quad * 32;
-          if (c0 >= N || r0 >= M) break;  // wholly outside C (warp-uniform)
-          uint32_t w[32];
-          if (sizeof(TO) == 4) {
-            tmem_ld_32x32b_x32(taddr + u * 32, w);
-            tmem_ld_wait();
-          } else {
+    uint32_t acc_phase = 0, epi_phase = 0;
+    bool ok = true;
+    // bounded meeting point of this CTA's 128 epilogue threads
+    auto epi_sync = [&]() {
+      mbar_arrive(epi_bar);
+      if (ok) ok = mbar_wait(epi_bar, epi_phase, abort_flag, p.status, ST_TIMEOUT_MISC);
+      epi_phase ^= 1;
+    };
+    // byte offset of column j of a box's row r: 128-byte rows in the 128-byte-swizzle image
+    auto box_at = [](int r, int j) {
+      const int byte = j * (int)sizeof(TO);
+      return r * 128 + (((byte >> 4) ^ (r & 7)) << 4) + (byte & 15);
+    };
+    // the old values of the box at (r0, c0) on their way into box `sel`, whose last store has been read (one lane)
+    auto fetch_old = [&](int sel, int r0, int c0) {
+      tma_store_wait_read<0>();
+      mbar_expect_tx(&bars[sel], kBoxBytes);
+      tma_load_2d(boxes + sel * kBoxBytes, &tmap_c, &bars[sel], c0, r0);
+    };
+    // Finishes the box of C at (r0, c0): lane = row; values(h, v) gives the row's fp32 results of columns c0 + 32h..+31.
+    // Where the old C comes by TMA its load has been issued.
+    auto finish_box = [&](int r0, int c0, auto&& values) {
+      unsigned char* box = boxes + box_sel * kBoxBytes;
+      uint4* const my_row = reinterpret_cast<uint4*>(box + lane * 128);
+      float row_acc = reduce_identity(reduce_kind);
+      if (tma_c) {
+        if (!accumulate && lane == 0) tma_store_wait_read<1>();  // the store before the last one used this box
+        __syncwarp();
+      } else if (accumulate) {
+        // old values of C, a row piece at a time, into the same image
+#pragma unroll 16
+        for (int r = 0; r < 32; ++r) {
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-              uint32_t v[32];
-              tmem_ld_32x32b_x32(taddr + u * 64 + hh * 32, v);
-              tmem_ld_wait();
-#pragma unroll
-              for (int i = 0; i < 16; ++i)
-                w[hh * 16 + i] = pack_out<TO>(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
-            }
-          }
-          if (lane == 0) tma_store_wait_read<1>();  // the store before the last one used this box: it has been read
-          __syncwarp();
-          unsigned char* box = boxes + box_sel * (32 * 128);
-          box_sel ^= 1;
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<uint4*>(box + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-                make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            tma_store_2d(&tmap_c, box, c0, r0);
-            tma_store_commit();
+          for (int h = 0; h < U / 32; ++h) {
+            const int j = h * 32 + lane;
+            if (r0 + r < p.M && c0 + j < p.N) *reinterpret_cast<TO*>(box + box_at(r, j)) = C[(int64_t)(r0 + r) * p.ldc + c0 + j];
           }
         }
+        __syncwarp();
+      }
+      uint32_t w[32];
+#pragma unroll
+      for (int h = 0; h < U / 32; ++h) {
+        float v[32];
+        values(h, v);
+        if (accumulate) {
+          if (h == 0 && tma_c) {
+            if (ok) ok = mbar_wait(&bars[box_sel], (box_phases >> box_sel) & 1, abort_flag, p.status, ST_TIMEOUT_MISC);
+            box_phases ^= 1u << box_sel;
+            __syncwarp();
+          }
+          if (sizeof(TO) == 4) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const uint4 o = my_row[j ^ (lane & 7)];
+              v[4 * j] += __uint_as_float(o.x); v[4 * j + 1] += __uint_as_float(o.y);
+              v[4 * j + 2] += __uint_as_float(o.z); v[4 * j + 3] += __uint_as_float(o.w);
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint4 o = my_row[(h * 4 + j) ^ (lane & 7)];
+              const uint32_t ow[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float2 f = unpack_out<TO>(ow[e]);
+                v[8 * j + 2 * e] += f.x;
+                v[8 * j + 2 * e + 1] += f.y;
+              }
+            }
+          }
+        } else if (has_fill) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] += p.epi.fill;
+        }
+        if (sizeof(TO) == 4) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) w[i] = __float_as_uint(v[i]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) w[(h & 1) * 16 + i] = pack_out<TO>(v[2 * i], v[2 * i + 1]);
+        }
+        if (reduce_kind) {  // over the values as they are stored
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (c0 + h * 32 + i < p.N) row_acc = reduce_combine(reduce_kind, row_acc, rounded_as<TO>(v[i]));
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) my_row[j ^ (lane & 7)] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+      if (tma_c) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(&tmap_c, box, c0, r0);  // clipped at the edges of C
+          tma_store_commit();
+        }
       } else {
+        __syncwarp();
+#pragma unroll 8
+        for (int r = 0; r < 32; ++r) {
+#pragma unroll
+          for (int h = 0; h < U / 32; ++h) {
+            const int j = h * 32 + lane;
+            if (r0 + r < p.M && c0 + j < p.N) C[(int64_t)(r0 + r) * p.ldc + c0 + j] = *reinterpret_cast<const TO*>(box + box_at(r, j));
+          }
+        }
+        __syncwarp();
+      }
+      box_sel ^= 1;
+      if (reduce_kind && r0 + lane < p.M) __stcg(p.epi.row_partials + (int64_t)(c0 / U) * p.M + r0 + lane, row_acc);
+    };
+    // A column tile of row block tc.m has left its partials: whoever draws the last ticket combines the row block's
+    auto combine_rows = [&](const TileCoord& tc) {
+      epi_sync();
+      if (warp == 2 && lane == 0) {
+        __threadfence();
+        const bool last = atomicAdd(p.epi.row_tickets + tc.m, 1u) == (unsigned)tiles_n - 1;
+        if (last) {
+          p.epi.row_tickets[tc.m] = 0;  // clean for the next launch
+          __threadfence();
+        }
+        *epi_word = last ? 1u : 0u;
+      }
+      epi_sync();
+      const bool combine = ok && *epi_word != 0;
+      epi_sync();  // everybody has read it
+      const int row = tc.m * BM + quad * 32 + lane;
+      if (combine && row < p.M) {
+        TO* const dst = static_cast<TO*>(p.epi.reduce_dst);
+        float r = p.epi.reduce_clear ? reduce_identity(reduce_kind) : static_cast<float>(dst[row]);
+        const int n = (p.N + U - 1) / U;
+#pragma unroll 4
+        for (int t = 0; t < n; ++t) r = reduce_combine(reduce_kind, r, __ldcg(p.epi.row_partials + (int64_t)t * p.M + row));
+        dst[row] = static_cast<TO>(r);
+      }
+    };
+
+    Item it;
+    TileCoord shared_tile{-1, -1};
+    for (int i = 0; ok && get_item(i, it); ++i) {
+      const TileCoord tc = tile_coord(it.tile, tiles_m, tiles_n);
+      const int m0 = tc.m * BM, n0 = tc.n * BN;
+      if (!mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.status, ST_TIMEOUT_ACC_FULL)) break;
+      tc_fence_after_sync();
+      __syncwarp();
+      const uint32_t taddr = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);
+      if (it.shared) {
+        // this CTA's last item: its part goes into the ring, every stage of which has been read
+        float4* part = reinterpret_cast<float4*>(smem) + quad * 32 + lane;
 #pragma unroll 1
-        for (int c = 0; c < it.bn / 32; ++c) {
+        for (int c = 0; c < BN / 32; ++c) {
           uint32_t v[32];
           tmem_ld_32x32b_x32(taddr + c * 32, v);
           tmem_ld_wait();
-          const int col = n0 + c * 32;
-          if (row < M && col < N)
-            store_row_chunk<TO>(C + (int64_t)row * ldc + col, v, min(32, N - col), vec_c != 0, accumulate != 0);
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            part[(c * 8 + i) * BM] = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
+                                                 __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
         }
+        shared_tile = tc;
+        break;
+      }
+      const int r0 = m0 + quad * 32;
+      const int units = r0 < p.M ? (min(BN, p.N - n0) + U - 1) / U : 0;
+      const bool old_by_tma = accumulate && tma_c;
+      if (old_by_tma && units > 0 && lane == 0) fetch_old(box_sel, r0, n0);
+#pragma unroll 1
+      for (int u = 0; u < units; ++u) {
+        if (old_by_tma && u + 1 < units && lane == 0) fetch_old(box_sel ^ 1, r0, n0 + (u + 1) * U);
+        finish_box(r0, n0 + u * U, [&](int h, float (&v)[32]) {
+          uint32_t t[32];
+          tmem_ld_32x32b_x32(taddr + u * U + h * 32, t);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(t[i]);
+        });
       }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[acc]);
+      if (reduce_kind) combine_rows(tc);
       if (++acc == 2) {
         acc = 0;
         acc_phase ^= 1;
       }
     }
-    if (TMA_OUT && lane == 0) tma_store_wait<0>();  // the boxes are read and written out before the CTA leaves
+    if (splits > 1) {
+      // every role of every CTA of the cluster ends (its waits are bounded), so these meetings are reached
+      __syncwarp();
+      cluster_sync_all();  // the parts are complete
+      const TileCoord tc = shared_tile;
+      const bool shared = tc.m >= 0;  // (the same for the whole cluster, unless a wait ran out)
+      const int r0 = tc.m * BM + quad * 32;
+      // Column groups (4 columns) rank, rank + splits, ...: the parts of this warp's rows, S x kDeep loads in flight, summed
+      // in rank order and handed to the CTA that finishes their box (boxes are dealt out column by column)
+      auto add_up = [&](auto splits_c) {
+        constexpr int S = decltype(splits_c)::value, kDeep = 16 / S;
+        const uint32_t own = smem_u32(smem) + (quad * 32 + lane) * 16;
+        for (int cg0 = rank; cg0 < BN / 4; cg0 += S * kDeep) {
+          float4 t[kDeep][S];
+#pragma unroll
+          for (int j = 0; j < kDeep; ++j)
+#pragma unroll
+            for (int c = 0; c < S; ++c) t[j][c] = ld_cluster_f4(mapa_addr(own + (cg0 + j * S) * (BM * 16), c));
+#pragma unroll
+          for (int j = 0; j < kDeep; ++j) {
+            float4 sum = t[j][0];
+#pragma unroll
+            for (int c = 1; c < S; ++c) {
+              sum.x += t[j][c].x; sum.y += t[j][c].y; sum.z += t[j][c].z; sum.w += t[j][c].w;
+            }
+            const int cg = cg0 + j * S, u = cg / (U / 4);  // box column u: finished by CTA u % S, as its u / S-th
+            st_cluster_f4(mapa_addr(own + L::kSumOffset + ((u / S) * (U / 4) + cg % (U / 4)) * (BM * 16), u % S), sum);
+          }
+        }
+      };
+      // Where every CTA finishes a box column, it reads the parts of its boxes itself; otherwise (more CTAs than box
+      // columns) all of them add up first.
+      const bool direct = BN / U >= splits;
+      if (shared && r0 < p.M && !direct) {
+        if (splits == 2) add_up(std::integral_constant<int, 2>());
+        else if (splits == 4) add_up(std::integral_constant<int, 4>());
+        else add_up(std::integral_constant<int, 8>());
+      }
+      if (!direct) {
+        __syncwarp();
+        cluster_sync_all();  // the sums are complete
+      }
+      if (shared) {
+#pragma unroll 1
+        for (int u = rank; u < BN / U; u += splits) {
+          const int c0 = tc.n * BN + u * U;
+          if (r0 >= p.M || c0 >= p.N) continue;
+          if (accumulate && tma_c && lane == 0) fetch_old(box_sel, r0, c0);
+          finish_box(r0, c0, [&](int h, float (&v)[32]) {
+            if (direct) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[i] = 0.f;
+              const uint32_t at = smem_u32(smem) + ((u * U + h * 32) / 4 * BM + quad * 32 + lane) * 16;
+              for (int c = 0; c < splits; c += 2) {  // two parts' loads in flight, added in rank order
+                float4 t[2][8];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                  const uint32_t peer = mapa_addr(at, c + j);
+#pragma unroll
+                  for (int i = 0; i < 8; ++i) t[j][i] = ld_cluster_f4(peer + i * (BM * 16));
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                  for (int i = 0; i < 8; ++i) {
+                    v[4 * i] += t[j][i].x; v[4 * i + 1] += t[j][i].y; v[4 * i + 2] += t[j][i].z; v[4 * i + 3] += t[j][i].w;
+                  }
+              }
+              return;
+            }
+            const float4* sums = reinterpret_cast<const float4*>(smem + L::kSumOffset) +
+                                 ((u / splits) * (U / 4) + h * 8) * BM + quad * 32 + lane;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float4 t = sums[i * BM];
+              v[4 * i] = t.x; v[4 * i + 1] = t.y; v[4 * i + 2] = t.z; v[4 * i + 3] = t.w;
+            }
+          });
+        }
+      }
+      if (reduce_kind) __threadfence();  // the row partials, before rank 0 takes the ticket for the cluster
+      __syncwarp();
+      cluster_sync_all();  // nobody reads a peer any more
+      if (reduce_kind && shared && rank == 0) combine_rows(tc);
+    }
+    if (tma_c && lane == 0) tma_store_wait<0>();  // the boxes are read and written out before the CTA leaves
+  }
+  if (warp < 2 && splits > 1) {
+    __syncwarp();
+    cluster_sync_all();
+    if (BN * (int)sizeof(TO) / 128 < splits) cluster_sync_all();
+    cluster_sync_all();
   }
 
   // ------------------------------------------------------------------ teardown
@@ -288,6 +541,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) {
+    __syncwarp();
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 2 * BN);
   }
@@ -295,9 +549,58 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Which tile, and how many CTAs share the K of a tile of the last round: the least of these estimates, in clocks of about
+// 1.9 GHz beyond the launch.
+struct Plan {
+  int bn, splits, n_whole, grid;
+  double clocks;
+};
+// The plan for tiles of bn columns and clusters of `splits` CTAs, of which the device runs `clusters`.  A 64-k block takes
+// its MMAs (512 clk at 256 columns, 256 at 128) and, the more SMs are at it, what L2 adds: 770 at 2048^3 and 4096^3 with
+// the chip full, 1100 where rows begin off 128-byte lines (3000^3: two requests of the TMA unit a row).  Sharing costs
+// barriers, parts and sums: 3.5 us at 128 rows (128 x 512 x 512 over clusters of four took 8.7 us, whole 6.7), less
+// with fewer rows (17 x 1024 x 1024 6.8, 128 x 1024 x 1024 9.1 over clusters of eight).
+Plan plan_of(const GemmDims& g, int64_t tiles, int sms, int bn, int splits, int clusters) {
+  const int64_t kb = (g.K + BK - 1) / BK;
+  const bool aligned = g.lda % 64 == 0 && g.ldb % 64 == 0;
+  Plan p{bn, splits, 0, 0, 1e300};
+  double blocks, extra;
+  if (splits == 1) {
+    p.n_whole = (int)tiles;
+    p.grid = (int)std::min<int64_t>(tiles, sms);
+    blocks = std::ceil((double)tiles / sms) * (double)kb;
+    extra = bn == 256 ? 3500 : 1800;
+  } else {
+    const int grid = splits * std::min(clusters, sms / splits);
+    if (grid == 0 || kb < 2 * splits) return p;
+    const int64_t rounds = tiles / grid, rest = tiles % grid;
+    if (rest == 0 || rest > grid / splits) return p;
+    p.n_whole = (int)(rounds * grid);
+    p.grid = rounds > 0 ? grid : (int)rest * splits;
+    blocks = (double)rounds * (double)kb + std::ceil((double)kb / splits);
+    extra = (bn == 256 ? 4500 : 3500) + 3000.0 * (double)std::min<int64_t>(g.M, BM) / BM;
+  }
+  const double busy = (double)p.grid / sms;
+  p.clocks = blocks * (bn == 256 ? 520 + (aligned ? 250 : 580) * busy : 270 + (aligned ? 200 : 450) * busy) + extra;
+  return p;
+}
+template <typename F>
+Plan make_plan(const GemmDims& g, int sms, F&& clusters) {
+  Plan best{256, 1, 0, 0, 1e300};
+  for (int bn : {256, 128}) {
+    const int64_t tiles = ((g.M + BM - 1) / BM) * ((g.N + bn - 1) / bn);
+    if (tiles > INT32_MAX / 2) continue;
+    for (int splits : {1, 2, 4, 8}) {
+      const Plan p = plan_of(g, tiles, sms, bn, splits, splits > 1 ? clusters(bn, splits) : 0);
+      if (p.clocks < best.clocks) best = p;
+    }
+  }
+  return best;
+}
+
 template <typename TO, int BN, bool BF16, bool A_MN, bool B_MN>
 int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* A, const void* B, void* C,
-               cudaStream_t s) {
+               const Plan& plan, const RowEpilogue* epi, cudaStream_t s) {
   GemmDims g = resolve_dims(d);
   CUtensorMap ta, tb;
   int rc;
@@ -306,72 +609,100 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* A
     rc = encode_tmap_2d(ctx, &ta, d.dtype_ab, A, (uint64_t)g.M, (uint64_t)g.K, (uint64_t)g.lda * 2, 64, BK, true);
   else
     rc = encode_tmap_2d(ctx, &ta, d.dtype_ab, A, (uint64_t)g.K, (uint64_t)g.M, (uint64_t)g.lda * 2, BK, BM, true);
-  if (rc) { if (ctx) ctx->last_cuda = rc; return FRISK_B200_E_CUDA; }
+  if (rc) { ctx->last_cuda = rc; return FRISK_B200_E_CUDA; }
   if (B_MN)
     rc = encode_tmap_2d(ctx, &tb, d.dtype_ab, B, (uint64_t)g.N, (uint64_t)g.K, (uint64_t)g.ldb * 2, 64, BK, true);
   else
     rc = encode_tmap_2d(ctx, &tb, d.dtype_ab, B, (uint64_t)g.K, (uint64_t)g.N, (uint64_t)g.ldb * 2, BK, 128, true);
-  if (rc) { if (ctx) ctx->last_cuda = rc; return FRISK_B200_E_CUDA; }
+  if (rc) { ctx->last_cuda = rc; return FRISK_B200_E_CUDA; }
 
-  // an overwriting store of a C whose base and row pitch are 16-byte aligned goes out through the TMA unit
-  const bool tma_out = d.clear_accum && aligned16(C) && (g.ldc * sizeof(TO)) % 16 == 0;
+  GemmArgs a{};
+  // a C whose base and row pitch are 16-byte aligned goes through the TMA unit
+  a.tma_c = aligned16(C) && (g.ldc * sizeof(TO)) % 16 == 0;
   CUtensorMap tc = ta;  // unused otherwise
-  if (tma_out) {
+  if (a.tma_c) {
     const int out_dtype = sizeof(TO) == 4 ? FRISK_B200_F32 : (std::is_same<TO, __half>::value ? FRISK_B200_F16 : FRISK_B200_BF16);
     rc = encode_tmap_2d(ctx, &tc, out_dtype, C, (uint64_t)g.N, (uint64_t)g.M, (uint64_t)g.ldc * sizeof(TO),
                         128 / sizeof(TO), 32, true);
-    if (rc) { if (ctx) ctx->last_cuda = rc; return FRISK_B200_E_CUDA; }
+    if (rc) { ctx->last_cuda = rc; return FRISK_B200_E_CUDA; }
   }
+  a.C = C;
+  a.ldc = g.ldc;
+  a.M = (int)g.M; a.N = (int)g.N; a.K = (int)g.K;
+  a.accumulate = d.clear_accum || (epi && epi->has_fill) ? 0 : 1;
+  if (epi) a.epi = *epi;
+  a.status = ctx->d_status;
+  a.splits = plan.splits;
+  a.n_whole = plan.n_whole;
   using L = SmemLayout<BN>;
-  int tiles = (int)(((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN));
-  int grid = tiles < ctx->num_sms ? tiles : ctx->num_sms;
-  // A partial last wave of at most grid/2 tiles runs as twice as many half-width items: the
-  // wave then costs half a tile time instead of a whole one.
-  int rem = tiles % grid;
-  int n_full = tiles, n_items = tiles;
-  if (tiles > grid && rem > 0 && 2 * rem <= grid) {
-    n_full = tiles - rem;
-    n_items = n_full + 2 * rem;
-  }
-  int vec_c = aligned16(C) && (g.ldc * sizeof(TO)) % 16 == 0;
-  auto launch = [&](auto kern, int smem_bytes, PerDeviceOnce& opt_in) -> int {
+  auto launch = [&](auto kern, PerDeviceOnce& opt_in) -> int {
     if (opt_in(ctx->device, [&] {
-          return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) == cudaSuccess ? 0 : 1;
+          return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal) == cudaSuccess ? 0 : 1;
         }))
       return FRISK_B200_E_CUDA;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = dim3((unsigned)plan.grid);
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem_bytes;
+    cfg.dynamicSmemBytes = L::kTotal;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the kernel waits (griddepcontrol.wait) itself
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)plan.splits;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    TO* Cp = static_cast<TO*>(C);
-    int Mi = (int)g.M, Ni = (int)g.N, Ki = (int)g.K, acc = d.clear_accum ? 0 : 1;
-    int64_t ldc = g.ldc;
-    unsigned* st = ctx->d_status;
-    FB_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, Cp, Mi, Ni, Ki, ldc, acc, vec_c, n_full, n_items, st));
+    cfg.numAttrs = plan.splits > 1 ? 2 : 1;
+    FB_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, a));
     return 0;
   };
-  static PerDeviceOnce opt_in_plain, opt_in_tma;  // one pair per instantiation
-  if (tma_out) return launch(gemm_tcgen05_kernel<TO, BN, BF16, A_MN, B_MN, true>, L::kTotalOut, opt_in_tma);
-  return launch(gemm_tcgen05_kernel<TO, BN, BF16, A_MN, B_MN, false>, L::kTotal, opt_in_plain);
+  static PerDeviceOnce opt_in_plain, opt_in_general;  // one pair per instantiation
+  if (a.tma_c && !a.accumulate && !a.epi.has_fill && !a.epi.reduce_kind)
+    return launch(gemm_tcgen05_kernel<TO, BN, BF16, A_MN, B_MN, true>, opt_in_plain);
+  return launch(gemm_tcgen05_kernel<TO, BN, BF16, A_MN, B_MN, false>, opt_in_general);
 }
 
-template <typename TO, int BN, bool BF16>
+template <typename TO, bool BF16, int BN>
 int launch_major(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* A, const void* B, void* C,
-                 cudaStream_t s) {
+                 const Plan& plan, const RowEpilogue* epi, cudaStream_t s) {
   bool a_mn = d.trans_a != 0;   // A stored [K,M]
   bool b_mn = d.trans_b == 0;   // B stored [K,N]
   if (a_mn) {
-    if (b_mn) return launch_cfg<TO, BN, BF16, true, true>(ctx, d, A, B, C, s);
-    return launch_cfg<TO, BN, BF16, true, false>(ctx, d, A, B, C, s);
+    if (b_mn) return launch_cfg<TO, BN, BF16, true, true>(ctx, d, A, B, C, plan, epi, s);
+    return launch_cfg<TO, BN, BF16, true, false>(ctx, d, A, B, C, plan, epi, s);
   }
-  if (b_mn) return launch_cfg<TO, BN, BF16, false, true>(ctx, d, A, B, C, s);
-  return launch_cfg<TO, BN, BF16, false, false>(ctx, d, A, B, C, s);
+  if (b_mn) return launch_cfg<TO, BN, BF16, false, true>(ctx, d, A, B, C, plan, epi, s);
+  return launch_cfg<TO, BN, BF16, false, false>(ctx, d, A, B, C, plan, epi, s);
+}
+
+// Clusters the device runs at a time.  Every instantiation has one CTA per SM (shared memory decides), so one of them
+// answers for all of the same tile.
+int clusters_of(int device, int bn, int splits) {
+  static ClusterCapacity wide, narrow;
+  static PerDeviceOnce opt_wide, opt_narrow;
+  auto ask = [&](auto kern, int smem, ClusterCapacity& capacity, PerDeviceOnce& opt_in) {
+    if (opt_in(device, [&] {
+          return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess ? 0 : 1;
+        }))
+      return 0;
+    return capacity(device, kern, kThreads, smem, splits);
+  };
+  return bn == 256 ? ask(gemm_tcgen05_kernel<__half, 256, false, false, false, true>, SmemLayout<256>::kTotal, wide, opt_wide)
+                   : ask(gemm_tcgen05_kernel<__half, 128, false, false, false, true>, SmemLayout<128>::kTotal, narrow, opt_narrow);
+}
+Plan plan_for(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d) {
+  return make_plan(resolve_dims(d), std::min(ctx->num_sms, kNumSMsDefault),
+                   [&](int bn, int splits) { return clusters_of(ctx->device, bn, splits); });
+}
+
+template <typename TO, bool BF16>
+int launch_tile(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* A, const void* B, void* C,
+                const RowEpilogue* epi, cudaStream_t s) {
+  const Plan plan = plan_for(ctx, d);
+  if (plan.grid == 0) return FRISK_B200_E_UNSUPPORTED;
+  return plan.bn == 256 ? launch_major<TO, BF16, 256>(ctx, d, A, B, C, plan, epi, s)
+                        : launch_major<TO, BF16, 128>(ctx, d, A, B, C, plan, epi, s);
 }
 
 }  // namespace
@@ -385,15 +716,25 @@ bool tcgen05_supported(const frisk_b200_gemm_desc& d) {
   return true;
 }
 
+// clocks the plan is estimated at (frisk_b200_gemm weighs it against the pair kernel)
+double tcgen05_clocks(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d) { return plan_for(ctx, d).clocks; }
+
+// the row reduction keeps one fp32 per (box of columns, row) and one ticket per row block
+bool tcgen05_row_epilogue_fits(const frisk_b200_gemm_desc& d) {
+  const GemmDims g = resolve_dims(d);
+  const int64_t box = 128 / (int64_t)dtype_size(d.dtype_c);
+  return (g.N + box - 1) / box * g.M * 4 <= (int64_t)kRowPartialBytes && (g.M + BM - 1) / BM <= kRowTickets;
+}
+
 int launch_gemm_tcgen05(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* A, const void* B,
-                        void* C, cudaStream_t s) {
+                        void* C, cudaStream_t s, const RowEpilogue* epi) {
   if (!tcgen05_supported(d)) return FRISK_B200_E_UNSUPPORTED;
   if (!aligned16(A) || !aligned16(B)) return FRISK_B200_E_ALIGN;
   const bool bf = d.dtype_ab == FRISK_B200_BF16;
   if (d.dtype_c == FRISK_B200_F32)
-    return bf ? launch_major<float, 256, true>(ctx, d, A, B, C, s) : launch_major<float, 256, false>(ctx, d, A, B, C, s);
-  if (bf) return launch_major<__nv_bfloat16, 256, true>(ctx, d, A, B, C, s);
-  return launch_major<__half, 256, false>(ctx, d, A, B, C, s);
+    return bf ? launch_tile<float, true>(ctx, d, A, B, C, epi, s) : launch_tile<float, false>(ctx, d, A, B, C, epi, s);
+  if (bf) return launch_tile<__nv_bfloat16, true>(ctx, d, A, B, C, epi, s);
+  return launch_tile<__half, false>(ctx, d, A, B, C, epi, s);
 }
 
 }  // namespace fb

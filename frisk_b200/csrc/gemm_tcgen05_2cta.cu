@@ -122,7 +122,7 @@ __device__ __forceinline__ Item2 get_item2(int i, int n_full, int num_kb) {
 
 // MODE: what the epilogue does with a finished tile.  Separate instantiations, so that the plain
 // store keeps its register budget and code exactly as if the other two did not exist.
-enum { kStore = 0, kPush = 1, kFused = 2, kStoreTma = 3, kStoreTmaWide = 4, kPushWide = 5 };
+enum { kStore = 0, kPush = 1, kFused = 2, kStoreTma = 3, kStoreTmaWide = 4, kPushWide = 5, kAccTma = 6 };
 // kStoreTmaWide, kPushWide: deep-K products.  A work item is a 256 x 512 tile: both accumulators (all 512 tensor-memory columns)
 // belong to ONE item, whose two 256-column halves share every A k-block, so per MMA each SM's shared memory takes
 // 6 KB of TMA writes instead of 8.  The price is that the epilogue no longer overlaps the next item's MMAs, which a
@@ -140,7 +140,8 @@ __global__ void __launch_bounds__(kThreads2, 1)
   using L = Smem2;
   constexpr bool WIDE = MODE == kStoreTmaWide || MODE == kPushWide;
   constexpr bool PUSH = MODE == kPush || MODE == kPushWide;
-  constexpr bool TMA_OUT = MODE == kStoreTma || MODE == kStoreTmaWide;
+  constexpr bool ADD_OLD = MODE == kAccTma;  // the old C is added, through the TMA unit both ways
+  constexpr bool TMA_OUT = MODE == kStoreTma || MODE == kStoreTmaWide || ADD_OLD;
   constexpr int TILE_N = WIDE ? kWideN : BN2;                       // columns of a work item
   constexpr int NST = WIDE ? kStagesWide : kStages2;                // ring depth
   constexpr int STAGE = WIDE ? L::kABytes + 2 * L::kBBytes : L::kStageBytes;
@@ -156,6 +157,7 @@ __global__ void __launch_bounds__(kThreads2, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(epi_bar + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile uint32_t* epi_word = tmem_slot + 2;
+  uint64_t* box_bar = epi_bar + 3;  // [4 warps][2] TMA-store mode: old values of C have landed in a box
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
@@ -173,6 +175,8 @@ __global__ void __launch_bounds__(kThreads2, 1)
       mbar_init(&acc_empty[i], 8);  // 4 epilogue warps of each CTA
     }
     mbar_init(epi_bar, 128);
+    if (ADD_OLD)
+      for (int i = 0; i < 8; ++i) mbar_init(&box_bar[i], 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_a);
@@ -303,6 +307,7 @@ __global__ void __launch_bounds__(kThreads2, 1)
     // ------------------------------------------------------------------ epilogue (own 128 rows)
     const int quad = warp & 3;
     int box_sel = 0;  // which of the warp's two output boxes the next TMA store uses
+    uint32_t box_phases = 0;  // bit b: the phase box b's barrier is in
     int acc = 0;
     uint32_t acc_phase = 0;
     const uint32_t leader_acc_empty0 = mapa_u32(&acc_empty[0], 0), leader_acc_empty1 = mapa_u32(&acc_empty[1], 0);
@@ -360,11 +365,26 @@ __global__ void __launch_bounds__(kThreads2, 1)
         // [32 rows][128 bytes] box in the 128-byte-swizzle image and one lane hands the box to the TMA unit,
         // which writes whole lines and clips the box at the edges of C.  Two boxes per warp alternate.
         constexpr int kUnitCols = 128 / (int)sizeof(TO);
+        // Where C accumulates, its old values come the same way, a box ahead.
         unsigned char* boxes = smem + L::kOutOffset + quad * L::kOutWarpBytes;
+        uint64_t* bars = box_bar + quad * 2;
+        auto fetch_old = [&](int sel, int c0, int r0) {  // (one lane) once the box's last store has been read
+          tma_store_wait_read<0>();
+          mbar_expect_tx(&bars[sel], 32 * 128);
+          tma_load_2d(boxes + sel * (32 * 128), &tmap_c, &bars[sel], c0, r0);
+        };
+        if (ADD_OLD && lane == 0 && n0 < N && m0 + quad * 32 < M) fetch_old(box_sel, n0, m0 + quad * 32);
 #pragma unroll 1
         for (int u = 0; u < TILE_N / kUnitCols; ++u) {
           const int c0 = n0 + u * kUnitCols, r0 = m0 + quad * 32;
           if (c0 >= N || r0 >= M) break;  // wholly outside C (warp-uniform)
+          if (ADD_OLD) {
+            if (lane == 0 && u + 1 < TILE_N / kUnitCols && c0 + kUnitCols < N) fetch_old(box_sel ^ 1, c0 + kUnitCols, r0);
+            if (epi_ok) epi_ok = mbar_wait(&bars[box_sel], (box_phases >> box_sel) & 1, abort_flag, status, ST_TIMEOUT_MISC);
+            box_phases ^= 1u << box_sel;
+            __syncwarp();
+          }
+          const uint4* old_row = reinterpret_cast<const uint4*>(boxes + box_sel * (32 * 128) + lane * 128);
           uint32_t w[32];
           if (sizeof(TO) == 4) {
             tmem_ld_32x32b_x32(taddr + u * 32, w);
@@ -377,6 +397,16 @@ __global__ void __launch_bounds__(kThreads2, 1)
                 w[4 * i + 1] = __float_as_uint(__uint_as_float(w[4 * i + 1]) + o.y);
                 w[4 * i + 2] = __float_as_uint(__uint_as_float(w[4 * i + 2]) + o.z);
                 w[4 * i + 3] = __float_as_uint(__uint_as_float(w[4 * i + 3]) + o.w);
+              }
+            }
+            if (ADD_OLD) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const uint4 o = old_row[j ^ (lane & 7)];
+                w[4 * j] = __float_as_uint(__uint_as_float(w[4 * j]) + __uint_as_float(o.x));
+                w[4 * j + 1] = __float_as_uint(__uint_as_float(w[4 * j + 1]) + __uint_as_float(o.y));
+                w[4 * j + 2] = __float_as_uint(__uint_as_float(w[4 * j + 2]) + __uint_as_float(o.z));
+                w[4 * j + 3] = __float_as_uint(__uint_as_float(w[4 * j + 3]) + __uint_as_float(o.w));
               }
             }
           } else {
@@ -395,13 +425,26 @@ __global__ void __launch_bounds__(kThreads2, 1)
                   v[4 * i + 3] = __float_as_uint(__uint_as_float(v[4 * i + 3]) + o.w);
                 }
               }
+              if (ADD_OLD) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const uint4 o = old_row[(hh * 4 + j) ^ (lane & 7)];
+                  const uint32_t ow[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+                  for (int e = 0; e < 4; ++e) {
+                    const float2 f = unpack_out<TO>(ow[e]);
+                    v[8 * j + 2 * e] = __float_as_uint(__uint_as_float(v[8 * j + 2 * e]) + f.x);
+                    v[8 * j + 2 * e + 1] = __float_as_uint(__uint_as_float(v[8 * j + 2 * e + 1]) + f.y);
+                  }
+                }
+              }
 #pragma unroll
               for (int i = 0; i < 16; ++i)
                 w[hh * 16 + i] = pack_out<TO>(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
             }
           }
           // the store before the last one used this box: it has been read
-          if (lane == 0) tma_store_wait_read<1>();
+          if (!ADD_OLD && lane == 0) tma_store_wait_read<1>();
           __syncwarp();
           unsigned char* box = boxes + box_sel * (32 * 128);
           box_sel ^= 1;
@@ -568,7 +611,7 @@ int launch_cfg2(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* 
   if (rc) { ctx->last_cuda = rc; return FRISK_B200_E_CUDA; }
 
   CUtensorMap tc = ta;  // unused by the other modes
-  if (MODE == kStoreTma || MODE == kStoreTmaWide) {
+  if (MODE == kStoreTma || MODE == kStoreTmaWide || MODE == kAccTma) {
     // C as [M][N] with boxes of 32 rows x 128 bytes in the 128-byte-swizzle image the epilogue writes
     const int out_dtype = sizeof(TO) == 4 ? FRISK_B200_F32 : (std::is_same<TO, __half>::value ? FRISK_B200_F16 : FRISK_B200_BF16);
     rc = encode_tmap_2d(ctx, &tc, out_dtype, C, (uint64_t)g.N, (uint64_t)g.M, (uint64_t)g.ldc * sizeof(TO),
@@ -578,7 +621,7 @@ int launch_cfg2(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* 
 
   auto kern = gemm_tcgen05_2cta_kernel<TO, BF16, A_MN, B_MN, MODE>;
   constexpr int kSmemBytes = (MODE == kPush || MODE == kPushWide) ? Smem2::kTotalPush
-                             : (MODE == kStoreTma || MODE == kStoreTmaWide) ? Smem2::kTotalOut : Smem2::kTotal;
+                             : (MODE == kStoreTma || MODE == kStoreTmaWide || MODE == kAccTma) ? Smem2::kTotalOut : Smem2::kTotal;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -664,6 +707,20 @@ bool tcgen05_2cta_preferred(const frisk_b200_gemm_desc& d) {
   return 2 * tiles <= kPairsAssumed && (d.K + BK - 1) / BK >= kMinKbAllHalved;
 }
 
+// Clocks (at about 1.9 GHz, beyond the launch) a product is estimated at, to weigh against tcgen05_clocks.  Measured: 4096^3
+// 92.5 us, 2048^3 16.6, 3000^3 46.6 (rows off 128-byte lines cost the TMA unit two requests each), 1024 x 1024 x 4096
+// 22.6 with all tiles halved.
+double tcgen05_2cta_clocks(const frisk_b200_gemm_desc& d) {
+  const int64_t tiles = ((d.M + BM2 - 1) / BM2) * ((d.N + BN2 - 1) / BN2), kb = (d.K + BK - 1) / BK;
+  const GemmDims g = resolve_dims(d);
+  const double block = g.lda % 64 == 0 && g.ldb % 64 == 0 ? 730 : 840, tail = 3000, hand_over = 9000;
+  if (2 * tiles <= kPairsAssumed && kb >= kMinKbAllHalved) return (double)((kb + 1) / 2) * block + tail + hand_over;
+  const int64_t rem = tiles % kPairsAssumed;
+  const bool halved = tiles > kPairsAssumed && rem > 0 && 2 * rem <= kPairsAssumed && kb >= 8;
+  const double rounds = (double)(tiles / kPairsAssumed) + (rem == 0 ? 0.0 : halved ? 0.5 : 1.0);
+  return rounds * (double)kb * block + tail + (halved ? hand_over : 0);
+}
+
 // Split-K across GPUs: the same kernel, its epilogue storing every fp32 tile into this rank's slot at the row's owner.
 int launch_gemm_tcgen05_2cta_push(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* A, const void* B,
                                   const PushTargets& push, cudaStream_t s) {
@@ -710,11 +767,18 @@ int launch_gemm_tcgen05_2cta(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d,
     if (bf) return launch_major2<__nv_bfloat16, true, kFused>(ctx, d, A, B, C, ws, ws_bytes, s, epi);
     return launch_major2<__half, false, kFused>(ctx, d, A, B, C, ws, ws_bytes, s, epi);
   }
-  // an overwriting store of a C whose base and row pitch are 16-byte aligned goes out through the TMA unit
+  // a C whose base and row pitch are 16-byte aligned goes through the TMA unit (accumulating through the threads' own
+  // 16-byte accesses, 3000^3 took 55 us where overwriting took 47)
   const GemmDims g = resolve_dims(d);
   const size_t cs = dtype_size(d.dtype_c);
-#ifndef FB_NO_TMA_STORE
-  if (d.clear_accum && aligned16(C) && (g.ldc * cs) % 16 == 0) {
+  if (aligned16(C) && (g.ldc * cs) % 16 == 0) {
+    if (!d.clear_accum) {
+      if (d.dtype_c == FRISK_B200_F32)
+        return bf ? launch_major2<float, true, kAccTma>(ctx, d, A, B, C, ws, ws_bytes, s, nullptr)
+                  : launch_major2<float, false, kAccTma>(ctx, d, A, B, C, ws, ws_bytes, s, nullptr);
+      if (bf) return launch_major2<__nv_bfloat16, true, kAccTma>(ctx, d, A, B, C, ws, ws_bytes, s, nullptr);
+      return launch_major2<__half, false, kAccTma>(ctx, d, A, B, C, ws, ws_bytes, s, nullptr);
+    }
     // deep K and enough 256 x 512 items to keep every CTA pair busy for several rounds: the wide items
     const int64_t tiles_w = ((g.M + BM2 - 1) / BM2) * ((g.N + kWideN - 1) / kWideN);
     // (at 8192 x 8192 the wide items lose 2-7 % for K <= 4096, where the exposed epilogue outweighs the saved writes)
@@ -731,7 +795,6 @@ int launch_gemm_tcgen05_2cta(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d,
     if (bf) return launch_major2<__nv_bfloat16, true, kStoreTma>(ctx, d, A, B, C, ws, ws_bytes, s, nullptr);
     return launch_major2<__half, false, kStoreTma>(ctx, d, A, B, C, ws, ws_bytes, s, nullptr);
   }
-#endif
   if (d.dtype_c == FRISK_B200_F32)
     return bf ? launch_major2<float, true, kStore>(ctx, d, A, B, C, ws, ws_bytes, s, nullptr)
               : launch_major2<float, false, kStore>(ctx, d, A, B, C, ws, ws_bytes, s, nullptr);

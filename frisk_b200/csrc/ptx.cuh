@@ -169,6 +169,11 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t cluster_addr) {
                : "memory");
   return v;
 }
+__device__ __forceinline__ void st_cluster_f4(uint32_t cluster_addr, float4 v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};"
+               ::"r"(cluster_addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+               : "memory");
+}
 
 // ---------------------------------------------------------------- TMEM
 // One full warp allocates `cols` (power of two, 32..512) columns; the base address lands in

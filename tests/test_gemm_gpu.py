@@ -595,6 +595,25 @@ def test_splitk_push_two_gpus(tmp_path):
         assert float((tmp_path / f"err{r}.txt").read_text()) <= TOL["bf16"]
 
 
+@pytest.mark.parametrize("M,N,K", [
+    (17, 1024, 1000),    # few rows, K over eight CTAs, a ragged last block
+    (100, 4104, 2048),   # rows of a box beyond M
+    (520, 776, 4104),    # K over four CTAs
+    (1000, 1000, 136),   # whole tiles of 128 columns, edges in both directions
+    (2200, 4000, 264),   # more tiles than SMs
+    (64, 128, 64),       # one block
+])
+@pytest.mark.parametrize("dtype,out", [("bf16", "bf16"), ("fp16", "fp32")])
+def test_one_cta_plans(ctx, M, N, K, dtype, out):
+    """Whole tiles and tiles whose K a cluster shares, every layout, overwriting and accumulating, a C that goes through
+    TMA and one that does not (rows or base off 16 bytes)."""
+    for ta, tb in ((False, False), (False, True), (True, False), (True, True)):
+        m, n = (M + 7 & ~7 if ta else M), (N if tb else N + 7 & ~7)
+        check(ctx, m, n, K, dtype, out, ta, tb, 31, accumulate=ta != tb)
+        if tb:
+            check(ctx, m, n + 1, K, dtype, out, ta, tb, 32, accumulate=not ta)
+
+
 # ------------------------------------------------------------------ fill / row-reduce next to the gemm
 def run_fused(ctx, M, N, K, dtype_ab, dtype_c, seed, *, fill=None, kind=None, clear=True, clear_accum=True,
               algo=capi.ALGO_AUTO, c_init=None, expect_fused=None):
@@ -643,6 +662,20 @@ def test_fused_row_reduce_in_pair_epilogue(ctx, kind, dtype_c):
         c, r, ref, r0 = run_fused(ctx, 2304, N, 512, "fp16", dtype_c, 70, kind=kind, clear=clear, expect_fused=1)
         assert rel_frobenius(from_storage(c, dtype_c), ref) <= TOL["fp16"]
         check_reduce(c, r, dtype_c, kind, clear, r0)
+
+
+@pytest.mark.parametrize("M,N,K,dtype,out,kind", [
+    (130, 264, 200, "fp16", "fp16", "max"),    # a cluster shares K, ragged rows and columns
+    (513, 390, 72, "bf16", "fp32", "add"),     # whole tiles, C with rows that are not 16-byte multiples
+    (3000, 2056, 136, "bf16", "bf16", "min"),  # several tiles per CTA
+    (100, 65, 4096, "fp16", "fp16", "add"),    # eight CTAs per tile, one column beyond a box
+])
+def test_fused_on_the_one_cta_kernel(ctx, M, N, K, dtype, out, kind):
+    """Fill and row reduction folded into the one-CTA kernel (twice: its tickets are left clean)."""
+    for fill, clear in ((0.25, True), (-1.5, False)):
+        c, r, ref, r0 = run_fused(ctx, M, N, K, dtype, out, 81, fill=fill, kind=kind, clear_accum=False, clear=clear)
+        assert rel_frobenius(from_storage(c, out), ref) <= TOL[dtype]
+        check_reduce(c, r, out, kind, clear, r0)
 
 
 def test_fused_fill_replaces_the_read_of_c(ctx):
