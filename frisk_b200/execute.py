@@ -50,8 +50,13 @@ def context_for(device_index):
 
 def _stream_ptr(stream, device):
     torch = _torch()
-    s = stream if stream is not None else torch.cuda.current_stream(device)
-    return s.cuda_stream if hasattr(s, "cuda_stream") else int(s)
+    if stream is None:
+        # the current stream's handle, without the Stream object around it
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        if raw is not None and device.index is not None:
+            return raw(device.index)
+        stream = torch.cuda.current_stream(device)
+    return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
 
 
 def _find_gemm(kernel):
@@ -175,9 +180,10 @@ def execute(module_or_kernel, *tensors, stream=None, name=None, algo=capi.ALGO_A
     """Run the kernel on CUDA tensors bound positionally to its memref arguments."""
     torch = _torch()
     kernel = _kernel_of(module_or_kernel, name)
-    attention = any(isinstance(op, tensor_ops.MmaOp) for op in tensor_ops._ops_of(kernel))
+    ops = tensor_ops._ops_of(kernel)
+    attention = any(isinstance(op, tensor_ops.MmaOp) for op in ops)
     if attention:
-        spec, arg_idx = tensor_ops.attention_plan(kernel)
+        spec, arg_idx = tensor_ops.attention_plan(kernel, ops)
     else:
         desc, (ia, ib, ic), epilogue = fused_plan(kernel, algo=algo)
     arg_types = kernel.attrs["function_type"].inputs
@@ -217,22 +223,24 @@ def execute(module_or_kernel, *tensors, stream=None, name=None, algo=capi.ALGO_A
 
 def gemm(a, b, c, *, trans_a=False, trans_b=False, clear_accum=True, algo=capi.ALGO_AUTO, stream=None):
     """Direct GEMM on CUDA tensors (the op ``create_gemm_op`` describes), bypassing IR."""
-    torch = _torch()
-    code = {torch.float32: capi.F32, torch.float16: capi.F16, torch.bfloat16: capi.BF16}
-    m = a.shape[1] if trans_a else a.shape[0]
-    k = a.shape[0] if trans_a else a.shape[1]
-    n = b.shape[0] if trans_b else b.shape[1]
-    rc, msg = capi.gemm_check_memrefs(list(a.shape), code.get(a.dtype, -1), list(b.shape), code.get(b.dtype, -2),
-                                      list(c.shape), code.get(c.dtype, -3), trans_a, trans_b, m, n, k)
+    _torch()
+    code = _TORCH_DTYPE
+    sa, sb, sc = a.shape, b.shape, c.shape
+    m = sa[1] if trans_a else sa[0]
+    k = sa[0] if trans_a else sa[1]
+    n = sb[0] if trans_b else sb[1]
+    da, dc = code.get(a.dtype, -1), code.get(c.dtype, -3)
+    rc, msg = capi.gemm_check_memrefs(sa, da, sb, code.get(b.dtype, -2), sc, dc, trans_a, trans_b, m, n, k)
     if rc:
         raise ValueError(msg)
-    for t in (a, b, c):
-        if not t.is_cuda or t.stride(-1) != 1:
+    strides = a.stride(), b.stride(), c.stride()
+    for t, st in zip((a, b, c), strides):
+        if not t.is_cuda or st[-1] != 1:
             raise ValueError("frisk-b200-execute: operands must be row-major CUDA tensors")
-    desc = capi.gemm_desc(m, n, k, code[a.dtype], code[c.dtype], trans_a, trans_b, clear_accum,
-                          lda=a.stride(0), ldb=b.stride(0), ldc=c.stride(0), algo=algo)
-    ctx = context_for(c.device.index or 0)
-    ctx.gemm(desc, a.data_ptr(), b.data_ptr(), c.data_ptr(), stream=_stream_ptr(stream, c.device))
+    desc = capi.gemm_desc(m, n, k, da, dc, trans_a, trans_b, clear_accum,
+                          lda=strides[0][0], ldb=strides[1][0], ldc=strides[2][0], algo=algo)
+    device = c.device
+    context_for(device.index or 0).gemm(desc, a.data_ptr(), b.data_ptr(), c.data_ptr(), stream=_stream_ptr(stream, device))
     return c
 
 
@@ -254,7 +262,7 @@ def attention_forward(spec, q, k, v, out, *, scale=None, causal=False, normalize
     torch = _torch()
     b, h, n, d = attention_geometry(spec)
     n_kv = int(spec.get("N_kv", n))
-    code = {torch.float32: capi.F32, torch.float16: capi.F16, torch.bfloat16: capi.BF16}
+    code = _TORCH_DTYPE
     for t, s in ((q, n), (k, n_kv), (v, n_kv), (out, n)):
         if not t.is_cuda or not t.is_contiguous() or list(t.shape) != [b, h, s, d]:
             raise ValueError("attention operands must be compact BHSD CUDA tensors")

@@ -86,7 +86,18 @@ class type:  # noqa: N801  (name kept from the reference binding)
         return ("function", tuple(t._key() for t in self.inputs), tuple(t._key() for t in self.results))
 
     def __eq__(self, other):
-        return isinstance(other, type) and self._key() == other._key()
+        if self is other:
+            return True
+        if not isinstance(other, type) or self.kind != other.kind:
+            return False
+        if self.kind in ("float", "int"):  # (the comparison verifiers make most, without building keys)
+            return self.name == other.name
+        if self.kind in ("memref", "tensor"):
+            mine, its = getattr(self, "map", None), getattr(other, "map", None)
+            return (list(self.shape) == list(other.shape) and self.element == other.element
+                    and (mine is its or (mine and str(mine)) == (its and str(its)))
+                    and getattr(self, "space", 0) == getattr(other, "space", 0))
+        return self._key() == other._key()
 
     def __hash__(self):
         return hash(self._key())
@@ -682,64 +693,103 @@ class builder:  # noqa: N801
 # ------------------------------------------------------------------------ verification
 
 
+def _verify_parallel(op):  # FriskOps.cpp:224-234
+    if op.attrs["threads"] not in _SUPPORTED_THREADS:
+        raise ValueError("threads must be one of 32,64,128,256,512,1024")
+    if not op.attrs["ranges"] or any(r <= 0 for r in op.attrs["ranges"]):
+        raise ValueError("ranges must contain positive static extents")
+    if op.regions[0].empty() or len(op.regions[0].front().arguments) != len(op.attrs["ranges"]):
+        raise ValueError("range count must match the region induction arguments")
+
+
+def _verify_alloc(op):  # FriskOps.cpp:481-489
+    a = op.attrs["alignment"]
+    if a < 0:
+        raise ValueError("alignment must be non-negative")
+    if a > 0 and a & (a - 1):
+        raise ValueError("alignment must be a power of 2")
+
+
+def _verify_gemm(op):  # FriskOps.cpp:406-414
+    attrs = op.attrs
+    if attrs["policy"] == GemmWarpPolicy.Auto:
+        raise ValueError("Auto policy requires frisk.mma; legacy gemm has deterministic partitioning")
+    a, b, c = (v.type for v in op.operands)
+    code, msg = capi.gemm_check_memrefs(a.shape, _gemm_dtype(a), b.shape, _gemm_dtype(b), c.shape,
+                                        _gemm_dtype(c), attrs["transA"], attrs["transB"],
+                                        attrs["M"], attrs["N"], attrs["K"])
+    if code:
+        raise ValueError(msg)
+
+
+def _verify_fill(op):  # FriskOps.cpp:684-699
+    if op.operands[0].type.element != op.attrs["value"][1]:
+        raise ValueError(f"value type {op.attrs['value'][1]} does not match memref element type "
+                         f"{op.operands[0].type.element}")
+
+
+def _verify_reduce(op):  # FriskOps.cpp:728-762
+    src, dst = op.operands[0].type, op.operands[1].type
+    kind, dim = op.attrs["kind"], op.attrs["dim"]
+    if src.kind != "memref" or dst.kind != "memref":
+        raise ValueError("source and destination must be memref types")
+    if dim < 0 or dim >= len(src.shape):
+        raise ValueError(f"dimension {dim} is out of range for source of rank {len(src.shape)}")
+    if kind not in ("add", "mul", "min", "max"):
+        raise ValueError(f"unsupported reduce kind: {kind}. Supported: add, mul, min, max")
+    if len(src.shape) != len(dst.shape) + 1:
+        raise ValueError("destination rank must be one less than source rank. Got: "
+                         f"{len(dst.shape)} vs {len(src.shape)}")
+    kept = [i for i in range(len(src.shape)) if i != dim]
+    for j, i in enumerate(kept):
+        if src.shape[i] != dst.shape[j]:
+            raise ValueError(f"non-reduced dimension mismatch: source[{i}] = {src.shape[i]} vs "
+                             f"destination[{j}] = {dst.shape[j]}")
+    if src.element != dst.element:
+        raise ValueError("source and destination must have the same element type")
+
+
+def _verify_copy(op):  # FriskOps.cpp:662-679
+    if len(op.get_src_indices()) != op.attrs["srcMap"].get_num_inputs():
+        raise ValueError("source index count does not match the source map")
+    if len(op.get_dst_indices()) != op.attrs["dstMap"].get_num_inputs():
+        raise ValueError("destination index count does not match the destination map")
+
+
+def _verifier_of(cls):
+    """The verifier the ops of a class go through (None: nothing to check)."""
+    for base, check in ((ParallelOp, _verify_parallel), (AllocBufferOp, _verify_alloc), (GemmOp, _verify_gemm),
+                        (FillOp, _verify_fill), (ReduceOp, _verify_reduce)):
+        if issubclass(cls, base):
+            return check
+    if hasattr(cls, "verify_op"):  # the tensor-level ops (tensor_ops.py) carry their own verifiers
+        return cls.verify_op
+    return _verify_copy if issubclass(cls, CopyOp) else None
+
+
+_verifiers = {}  # class -> its verifier
+
+
+def _check(op):
+    cls = op.__class__
+    try:
+        check = _verifiers[cls]
+    except KeyError:
+        check = _verifiers[cls] = _verifier_of(cls)
+    if check is not None:
+        check(op)
+
+
 def _verify(op):
     """Raise ValueError with the verifier message of the first failing op."""
-    if isinstance(op, ParallelOp):  # FriskOps.cpp:224-234
-        if op.attrs["threads"] not in _SUPPORTED_THREADS:
-            raise ValueError("threads must be one of 32,64,128,256,512,1024")
-        if not op.attrs["ranges"] or any(r <= 0 for r in op.attrs["ranges"]):
-            raise ValueError("ranges must contain positive static extents")
-        if op.regions[0].empty() or len(op.regions[0].front().arguments) != len(op.attrs["ranges"]):
-            raise ValueError("range count must match the region induction arguments")
-    elif isinstance(op, AllocBufferOp):  # FriskOps.cpp:481-489
-        a = op.attrs["alignment"]
-        if a < 0:
-            raise ValueError("alignment must be non-negative")
-        if a > 0 and a & (a - 1):
-            raise ValueError("alignment must be a power of 2")
-    elif isinstance(op, GemmOp):  # FriskOps.cpp:406-414
-        if op.attrs["policy"] == GemmWarpPolicy.Auto:
-            raise ValueError("Auto policy requires frisk.mma; legacy gemm has deterministic partitioning")
-        a, b, c = (v.type for v in op.operands)
-        code, msg = capi.gemm_check_memrefs(a.shape, _gemm_dtype(a), b.shape, _gemm_dtype(b), c.shape,
-                                            _gemm_dtype(c), op.attrs["transA"], op.attrs["transB"],
-                                            op.attrs["M"], op.attrs["N"], op.attrs["K"])
-        if code:
-            raise ValueError(msg)
-    elif isinstance(op, FillOp):  # FriskOps.cpp:684-699
-        if op.operands[0].type.element != op.attrs["value"][1]:
-            raise ValueError(f"value type {op.attrs['value'][1]} does not match memref element type "
-                             f"{op.operands[0].type.element}")
-    elif isinstance(op, ReduceOp):  # FriskOps.cpp:728-762
-        src, dst = op.operands[0].type, op.operands[1].type
-        kind, dim = op.attrs["kind"], op.attrs["dim"]
-        if src.kind != "memref" or dst.kind != "memref":
-            raise ValueError("source and destination must be memref types")
-        if dim < 0 or dim >= len(src.shape):
-            raise ValueError(f"dimension {dim} is out of range for source of rank {len(src.shape)}")
-        if kind not in ("add", "mul", "min", "max"):
-            raise ValueError(f"unsupported reduce kind: {kind}. Supported: add, mul, min, max")
-        if len(src.shape) != len(dst.shape) + 1:
-            raise ValueError("destination rank must be one less than source rank. Got: "
-                             f"{len(dst.shape)} vs {len(src.shape)}")
-        kept = [i for i in range(len(src.shape)) if i != dim]
-        for j, i in enumerate(kept):
-            if src.shape[i] != dst.shape[j]:
-                raise ValueError(f"non-reduced dimension mismatch: source[{i}] = {src.shape[i]} vs "
-                                 f"destination[{j}] = {dst.shape[j]}")
-        if src.element != dst.element:
-            raise ValueError("source and destination must have the same element type")
-    elif hasattr(op, "verify_op"):  # the tensor-level ops (tensor_ops.py) carry their own verifiers
-        op.verify_op()
-    elif isinstance(op, CopyOp):  # FriskOps.cpp:662-679
-        if len(op.get_src_indices()) != op.attrs["srcMap"].get_num_inputs():
-            raise ValueError("source index count does not match the source map")
-        if len(op.get_dst_indices()) != op.attrs["dstMap"].get_num_inputs():
-            raise ValueError("destination index count does not match the destination map")
+    _check(op)
     for r in op.regions:
         for b in r.blocks:
             for child in b.operations:
-                _verify(child)
+                if child.regions:
+                    _verify(child)
+                else:
+                    _check(child)
 
 
 # ------------------------------------------------------------------------ printing

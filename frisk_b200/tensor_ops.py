@@ -43,7 +43,7 @@ class MmaOp(OpState):
         ta, tb, ti = (v.type for v in self.operands)
         tr = self.results[0].type
         for t in (ta, tb, ti, tr):
-            if not _shaped(t) or len(t.shape) != 2 or any(e <= 0 for e in t.shape) or t.element.kind != "float":
+            if not _shaped(t) or len(t.shape) != 2 or min(t.shape) <= 0 or t.element.kind != "float":
                 raise ValueError("mma-shape: requires positive static rank-2 floating matrices")
         if ta.element != tb.element or ti.element != tr.element or _float_bits(ti.element) < _float_bits(ta.element):
             raise ValueError("mma-shape: incompatible input/accumulator element types")
@@ -75,7 +75,7 @@ class ReduceTensorOp(OpState):
         if getattr(src.element, "name", "") not in ("f16", "bf16", "f32") or src.element != dst.element:
             raise ValueError("reduce-shape: requires matching f16/bf16/f32 element types")
         for t in (src, dst):
-            if any(not _is_pow2(e) for e in t.shape):
+            if not all(map(_is_pow2, t.shape)):
                 raise ValueError("reduce-shape: requires static positive power-of-two extents")
         if list(dst.shape) != [e for i, e in enumerate(src.shape) if i != dim]:
             raise ValueError("reduce-shape: result must delete the reduction axis")
@@ -139,6 +139,8 @@ class UpstreamOp(OpState):
 
     def verify_op(self):
         n = self.op_name
+        if n in ("arith.constant", "tensor.empty", "memref.alloc", "math.exp"):
+            return
         if n in ("arith.mulf", "arith.subf", "arith.divf"):
             a, b = (v.type for v in self.operands)
             if a != b or a != self.results[0].type:
@@ -302,7 +304,8 @@ def _ops_of(kernel):
             for blk in r.blocks:
                 for child in blk.operations:
                     out.append(child)
-                    visit(child)
+                    if child.regions:
+                        visit(child)
     visit(kernel)
     return out
 
@@ -311,12 +314,14 @@ def _fail(what):
     raise ValueError(f"frisk-b200-execute: not the attention graph: {what}")
 
 
-def attention_plan(kernel):
+def attention_plan(kernel, ops=None):
     """Host-only.  Resolve a kernel that holds the attention graph to
     ``(dict(S_q, S_kv, D, scale, dtype_in, dtype_out), (iq, ik, iv, io))`` (argument indices), following the
-    use-def chain back from the ``frisk.tile_store``; raises ValueError naming the first deviation."""
+    use-def chain back from the ``frisk.tile_store``; raises ValueError naming the first deviation.
+    ``ops``: the kernel's ops, where the caller has just listed them."""
     ir._verify(kernel)
-    ops = _ops_of(kernel)
+    if ops is None:
+        ops = _ops_of(kernel)
     entry = kernel.regions[0].front()
     copies = [op for op in ops if isinstance(op, ir.CopyOp)]
 
