@@ -641,7 +641,7 @@ def secondary(ctx, torch, stream, peaks, args, sampler, headline_sets, headline_
         return total / (n or steps)
 
     # fp32 GEMM 1024^3 (12 MiB of operands: rotate enough sets to stay ahead of L2), by both of its kernels:
-    # the default (operands split exactly into bf16 terms, nine tensor-core products) and the CUDA cores
+    # the default (operands split exactly into bf16 terms, six tensor-core products) and the CUDA cores
     for key, algo in (("gemm_f32_1024", capi.ALGO_AUTO), ("gemm_f32_1024_cuda_cores", capi.ALGO_SIMT_F32)):
         try:
             M = 1024
@@ -659,7 +659,7 @@ def secondary(ctx, torch, stream, peaks, args, sampler, headline_sets, headline_
             from oracle.numerics import rel_frobenius
             err = rel_frobenius(c.double().cpu().numpy(), a.double().cpu().numpy() @ b.double().cpu().numpy())
             res[key] = {"ms": round(ms, 5), "tflops": round(2.0 * M ** 3 / ms / 1e9, 2),
-                        "algo": {capi.ALGO_F32_SPLIT: "split_bf16x9_tcgen05", capi.ALGO_SIMT_F32: "cuda_cores"}[
+                        "algo": {capi.ALGO_F32_SPLIT: "split_bf16x6_tcgen05", capi.ALGO_SIMT_F32: "cuda_cores"}[
                             capi.load().frisk_b200_gemm_select(desc)],
                         "frac_of_nominal_fp32_simt": round(2.0 * M ** 3 / ms / 1e9 / 80.0, 4),
                         "err": float(f"{err:.3e}"), "checked": err <= 1e-3}

@@ -19,8 +19,8 @@
  * input (benchmark/layout/execution/tiled_execution.py:113-139).
  *
  * One context serves one stream of calls: the context holds scratch that its kernels share
- * (the attention kernel's work counter, the fp32 and skinny GEMMs' tickets and partial sums when
- * no workspace is passed, the device status word), so two calls on the same context must not
+ * (the attention kernels' work counter and partial results, the CUDA-core fp32, skinny and pair GEMMs' tickets and
+ * partial sums when no workspace is passed, the device status word), so two calls on the same context must not
  * run on the GPU at the same time.  Use one context per concurrent stream.  Every entry point
  * leaves the calling thread's current device as it found it.
  */
@@ -39,16 +39,17 @@ typedef struct frisk_b200_ctx frisk_b200_ctx;
 /* element types: the float types python/frisk/common/utils.py:156-170 can name */
 enum { FRISK_B200_F32 = 0, FRISK_B200_F16 = 1, FRISK_B200_BF16 = 2 };
 
-/* kernel selection for frisk_b200_gemm (AUTO picks by type and shape).  f32 operands: AUTO takes F32_SPLIT when
- * M, N and K are multiples of 8 and at least 256, else SIMT_F32.  F32_SPLIT and SIMT_F32 keep their scratch (stacked
- * bf16 operands and the 3M x 3N fp32 product; tickets and partial tiles) in the context, whatever `workspace` is. */
+/* kernel selection for frisk_b200_gemm.  AUTO runs the kernel its estimates name the faster for the operands at hand:
+ * TCGEN05 or TCGEN05_PAIR (SKINNY for M <= 16) for 16-bit operands, F32_SPLIT or SIMT_F32 for f32.  A descriptor that
+ * names F32_SPLIT has extents that are multiples of 8.  SIMT_F32 keeps its scratch (tickets and partial tiles) in the
+ * context, whatever `workspace` is; TCGEN05 and F32_SPLIT need none. */
 enum {
   FRISK_B200_ALGO_AUTO = 0,
   FRISK_B200_ALGO_SIMT_F32 = 1, /* fp32 CUDA-core GEMM                                   */
-  FRISK_B200_ALGO_TCGEN05 = 2,  /* fp16/bf16 tcgen05 + TMEM + TMA ring, one CTA per tile */
+  FRISK_B200_ALGO_TCGEN05 = 2,  /* fp16/bf16 tcgen05 + TMEM + TMA ring, one CTA or a K-sharing cluster per tile */
   FRISK_B200_ALGO_SKINNY = 3,   /* M<=16: weights streamed by TMA into tcgen05, stream-K  */
   FRISK_B200_ALGO_TCGEN05_PAIR = 4, /* tcgen05 with CTA pairs (cta_group::2), 256x256 tiles */
-  FRISK_B200_ALGO_F32_SPLIT = 5 /* fp32 operands split exactly into 3 bf16 terms, 9 tcgen05 products, fp32 sums */
+  FRISK_B200_ALGO_F32_SPLIT = 5 /* fp32 operands split exactly into 3 bf16 terms, 6 tcgen05 products, fp32 sums */
 };
 
 /* error codes (negative: host-side contract checks) */
@@ -138,8 +139,9 @@ int frisk_b200_gemm_check_memrefs(int32_t a_rank, const int64_t* a_shape, int32_
                                   int32_t c_rank, const int64_t* c_shape, int32_t c_dtype,
                                   int32_t trans_a, int32_t trans_b, int64_t m, int64_t n, int64_t k,
                                   const char** message);
-/* Which kernel AUTO resolves to for this descriptor (FRISK_B200_ALGO_*), or a negative
- * error.  Host-only. */
+/* A kernel that takes this descriptor (FRISK_B200_ALGO_*), or a negative error.  Host-only.  For AUTO it goes by type,
+ * layout and extents alone; the launch, which also knows the device and C's address, may run the other kernel of the
+ * same element type. */
 int frisk_b200_gemm_select(const frisk_b200_gemm_desc* desc);
 /* Bytes of caller-provided, ZERO-INITIALISED scratch this descriptor needs (0 = none).
  * The kernels leave their control words zero again, so one memset at allocation suffices
