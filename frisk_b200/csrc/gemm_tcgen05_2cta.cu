@@ -374,6 +374,17 @@ __global__ void __launch_bounds__(kThreads2, 1)
           tma_load_2d(boxes + sel * (32 * 128), &tmap_c, &bars[sel], c0, r0);
         };
         if (ADD_OLD && lane == 0 && n0 < N && m0 + quad * 32 < M) fetch_old(box_sel, n0, m0 + quad * 32);
+        // the other K half of the box after the current one is on its way while this one is finished (loaded when it
+        // was needed, each 32 columns cost an L2 round trip)
+        float4 ahead[kUnitCols / 32][8];
+        auto fetch_other = [&](int u, int h) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) ahead[h][i] = __ldcg(other + ((u * (kUnitCols / 32) + h) * 8 + i) * BMC);
+        };
+        if (other != nullptr) {
+#pragma unroll
+          for (int h = 0; h < kUnitCols / 32; ++h) fetch_other(0, h);
+        }
 #pragma unroll 1
         for (int u = 0; u < TILE_N / kUnitCols; ++u) {
           const int c0 = n0 + u * kUnitCols, r0 = m0 + quad * 32;
@@ -392,12 +403,13 @@ __global__ void __launch_bounds__(kThreads2, 1)
             if (other != nullptr) {
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
-                const float4 o = __ldcg(other + (u * 8 + i) * BMC);
+                const float4 o = ahead[0][i];
                 w[4 * i] = __float_as_uint(__uint_as_float(w[4 * i]) + o.x);
                 w[4 * i + 1] = __float_as_uint(__uint_as_float(w[4 * i + 1]) + o.y);
                 w[4 * i + 2] = __float_as_uint(__uint_as_float(w[4 * i + 2]) + o.z);
                 w[4 * i + 3] = __float_as_uint(__uint_as_float(w[4 * i + 3]) + o.w);
               }
+              if (u + 1 < TILE_N / kUnitCols) fetch_other(u + 1, 0);
             }
             if (ADD_OLD) {
 #pragma unroll
@@ -418,12 +430,13 @@ __global__ void __launch_bounds__(kThreads2, 1)
               if (other != nullptr) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                  const float4 o = __ldcg(other + ((u * 2 + hh) * 8 + i) * BMC);
+                  const float4 o = ahead[hh & (kUnitCols / 32 - 1)][i];
                   v[4 * i] = __float_as_uint(__uint_as_float(v[4 * i]) + o.x);
                   v[4 * i + 1] = __float_as_uint(__uint_as_float(v[4 * i + 1]) + o.y);
                   v[4 * i + 2] = __float_as_uint(__uint_as_float(v[4 * i + 2]) + o.z);
                   v[4 * i + 3] = __float_as_uint(__uint_as_float(v[4 * i + 3]) + o.w);
                 }
+                if (u + 1 < TILE_N / kUnitCols) fetch_other(u + 1, hh & (kUnitCols / 32 - 1));
               }
               if (ADD_OLD) {
 #pragma unroll
