@@ -69,13 +69,14 @@ struct PerDeviceOnce {
   }
 };
 
-// How many clusters of `splits` (2, 4 or 8) CTAs of a kernel the device runs at a time; asked once per device and size.
+constexpr int kMaxCluster = 8;  // portable cluster size
+// How many clusters of `splits` CTAs of a kernel the device runs at a time; asked once per device and size.
 struct ClusterCapacity {
-  std::atomic<int> known[kMaxDevices][3] = {};  // capacity + 1
+  std::atomic<int> known[kMaxDevices][kMaxCluster + 1] = {};  // capacity + 1
   template <typename K>
   int operator()(int device, K kern, int threads, int smem_bytes, int splits) {
-    if (device < 0 || device >= kMaxDevices) return 0;
-    std::atomic<int>& slot = known[device][splits == 2 ? 0 : splits == 4 ? 1 : 2];
+    if (device < 0 || device >= kMaxDevices || splits < 1 || splits > kMaxCluster) return 0;
+    std::atomic<int>& slot = known[device][splits];
     int n = slot.load(std::memory_order_acquire) - 1;
     if (n >= 0) return n;
     cudaLaunchConfig_t cfg = {};

@@ -23,7 +23,7 @@
 // Bound by shared memory: a block writes 96 KB of planes and its 24 MMAs read 192 KB, 2300 clk at 128 B/clk against 1540
 // clk of tensor pipe; 4096^3 takes 3700 clk a block (886 us, 155 TFLOP/s of fp32), a short K about 4000.
 //
-// Where the tiles are fewer than half the SMs a cluster of 2, 4 or 8 CTAs shares a tile's K; every CTA leaves its fp32 part
+// Where the tiles are fewer than half the SMs a cluster of 2 to 8 CTAs shares a tile's K; every CTA leaves its fp32 part
 // in its own shared memory and each finishes a share of the tile's 32-row pieces, adding the parts over distributed
 // shared memory in rank order (reproducible, no scratch).  Otherwise a CTA walks whole tiles.
 #include <cuda_bf16.h>
@@ -452,12 +452,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
   }
 }
 
-// K over the CTAs of a cluster while that leaves every CTA an SM and two blocks of its own (adding the parts up takes
-// about as long as one: 512 x 512 x 512 in 11.6 us with 2 blocks each on 4 CTAs a tile)
-int split_of(int64_t tiles, int64_t kb, int sms) {
-  int splits = 1;
-  while (splits < 8 && tiles * splits * 2 <= sms && kb >= splits * 4) splits *= 2;
-  return splits;
+// How many CTAs of a cluster share a tile's K: as many as leave every CTA an SM and two blocks of its own (adding the
+// parts up takes about as long as one: 512 x 512 x 512 in 11.6 us with 2 blocks each on 4 CTAs a tile), and of those the
+// fewest that give the same number of blocks.  `fits(n)`: the device runs a cluster of n for every tile at a time.
+template <typename F>
+int split_of(int64_t tiles, int64_t kb, int sms, F&& fits) {
+  int best = 1;
+  for (int n = 2; n <= kMaxCluster && tiles * n <= sms && kb >= 2 * n; ++n)
+    if ((kb + n - 1) / n < (kb + best - 1) / best && fits(n)) best = n;
+  return best;
 }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -472,8 +475,7 @@ int launch_one(frisk_b200_ctx* ctx, SplitArgs a, cudaStream_t s) {
     return FRISK_B200_E_CUDA;
   static ClusterCapacity capacity;
   const int sms = std::min(ctx->num_sms, kNumSMsDefault), tiles = a.tiles_m * a.tiles_n;
-  a.splits = split_of(tiles, a.kb, sms);
-  while (a.splits > 1 && capacity(ctx->device, kern, kThreads, kSmemTotal, a.splits) < tiles) a.splits /= 2;
+  a.splits = split_of(tiles, a.kb, sms, [&](int n) { return capacity(ctx->device, kern, kThreads, kSmemTotal, n) >= tiles; });
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(a.splits > 1 ? tiles * a.splits : std::min(tiles, sms)));
   cfg.blockDim = dim3(kThreads);
@@ -523,7 +525,7 @@ bool f32_split_beats_simt(const frisk_b200_gemm_desc& d) {
   if (tiles > (int64_t)1 << 30) return false;
   const double units = std::ceil((double)(((g.M + 63) / 64) * ((g.N + 63) / 64)) * (double)kb / sms);
   const double simt = 4.3 + 2.0 * (units - 1) + (units < (double)kb ? 2.0 : 0.0);
-  const int splits = split_of(tiles, kb, kNumSMsDefault);
+  const int splits = split_of(tiles, kb, kNumSMsDefault, [](int) { return true; });
   const double blocks = std::ceil((double)tiles / sms) * std::ceil((double)kb / splits);
   const double block = g.lda % 4 || g.ldb % 4 ? 3.2 : 2.1;
   return 5.5 + block * blocks + (splits > 1 ? 2.0 : 0.0) < simt;
