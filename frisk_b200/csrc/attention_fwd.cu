@@ -148,6 +148,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  // Launched with programmatic stream serialization: the set-up above may run while the kernel in front of this one
+  // drains; nothing touches global memory (the operands, the work counter) before that kernel is complete.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 
   // the TMA/MMA warpgroup hands registers to the two softmax warpgroups (a full row of S per thread)
   if (warp >= 8) {
@@ -333,7 +337,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // WHOLE row; e = ex2((score - max) * log2e); p = e / (sum of e over the whole row), IEEE
         // division; p rounded to 16 bits; then P.V.  Pass 0 finds max and sum, pass 1 forms P.
         // The row of a key tile is worked on in packed pairs without branches: an IEEE division per element
-        // (__fdiv_rn branches) made this mode latency-bound, 16 heads x 1025 rows x D 64 took 154 us.
+        // (__fdiv_rn branches) made this mode latency-bound, 16 heads x 1025 rows x D 64 took 154 us, 31 so.
         const float kLog2e = 1.44269504088896340736f;
         const float2 scale2 = make_float2(p.scale, p.scale), log2e2 = make_float2(kLog2e, kLog2e);
         auto exp2_of = [](float x) { return BF16 ? ex2f_ieee_range(x) : ex2f(x); };
@@ -681,8 +685,17 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q
   });
   if (bad) return bad;
   const unsigned grid = (unsigned)std::min<int64_t>(p.total_items, ctx->num_sms);
-  kern<<<grid, kThreads, L::kTotal, s>>>(tq, tk, tv, to, p);
-  FB_CUDA(ctx, cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = L::kTotal;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the kernel waits (griddepcontrol.wait) itself
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  FB_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, to, p));
   return 0;
 }
 
