@@ -678,6 +678,26 @@ def test_fused_on_the_one_cta_kernel(ctx, M, N, K, dtype, out, kind):
         check_reduce(c, r, out, kind, clear, r0)
 
 
+def test_fused_reduction_on_more_streams_than_scratch_sets(ctx):
+    """Every stream gets the same bits, whether it owns a set of the reduction's scratch or is served by the composed form."""
+    import torch
+    M, N, K = 300, 520, 256
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a, b = (torch.randn(x, K, generator=g, device="cuda").half() for x in (M, N))
+    results = []
+    torch.cuda.synchronize()
+    for _ in range(6):
+        st = torch.cuda.Stream()
+        c, r = torch.empty(M, N, dtype=torch.half, device="cuda"), torch.empty(M, dtype=torch.half, device="cuda")
+        epi = capi.gemm_epilogue(reduce="max", reduce_dst=r.data_ptr())
+        ctx.gemm_fused(capi.gemm_desc(M, N, K, "fp16", "fp16", False, True), epi, a.data_ptr(), b.data_ptr(), c.data_ptr(),
+                       stream=st.cuda_stream)
+        ctx.check(st.cuda_stream)
+        results.append((c, r))
+    for c, r in results:
+        assert torch.equal(c, results[0][0]) and torch.equal(r, c.amax(1))
+
+
 def test_fused_fill_replaces_the_read_of_c(ctx):
     # C holds NaN: a fused fill must not read it.  bf16 output, then with a reduction on top.
     c, _, ref, _ = run_fused(ctx, 2304, 2560, 256, "bf16", "bf16", 71, fill=0.75, clear_accum=False, expect_fused=1)
