@@ -90,18 +90,20 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&w)[3]) {
 
 // A block of an operand is 128 box rows of 64 elements: rows = MN and columns = k for an operand contiguous along K;
 // for one contiguous along MN, 64 rows = k of columns mn0..+63, then 64 rows of columns mn0+64..+127.  A loader thread
-// takes 32 elements of it.  VEC (16-byte aligned rows): eight groups of four columns, a warp reads two rows of 256 bytes;
-// otherwise columns lane and lane + 32 of 16 rows, a warp reads one row, one element per lane.
+// takes 32 elements of it, eight groups of four columns (a warp has two rows of 256 bytes at a time): as 16-byte loads where
+// the rows are aligned (VEC), otherwise as four loads of 32 bits (spread over whole rows, one element a lane, the loads
+// touch fewer lines each but the halves have to be exchanged and stored in pieces: 1151 x 2047 x 1023 69 us so, 43 this way,
+// 37 for the aligned neighbour).
 template <bool MN, bool VEC>
 struct Loader {
-  static constexpr int kSteps = VEC ? 8 : 16;
+  static constexpr int kSteps = 8;
   static constexpr int kRowStep = 128 / kSteps;  // box rows from one step to the next
   float r[32];
   const float* base;  // this thread's first element of the block the next fetch() takes
   int row, col;       // its place in the operand
 
-  __device__ __forceinline__ static int first_row(int tid) { return VEC ? tid >> 4 : tid >> 5; }
-  __device__ __forceinline__ static int first_col(int tid) { return VEC ? (tid & 15) * 4 : tid & 31; }
+  __device__ __forceinline__ static int first_row(int tid) { return tid >> 4; }
+  __device__ __forceinline__ static int first_col(int tid) { return (tid & 15) * 4; }
   __device__ __forceinline__ void place(const Operand& o, int mn0, int k0, int tid) {
     row = (MN ? k0 : mn0) + first_row(tid);
     col = (MN ? mn0 : k0) + first_col(tid);
@@ -114,60 +116,32 @@ struct Loader {
     for (int v = 0; v < kSteps; ++v) {
       const int rv = MN ? v % (kSteps / 2) : v, cv = MN ? v / (kSteps / 2) * 64 : 0;
       const float* p = base + rv * step + cv;
-      if (VEC) {
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (inside) {
-          x = __ldg(reinterpret_cast<const float4*>(p));
-        } else if (row + rv * kRowStep < o.rows && col + cv < o.cols) {
-          if (col + cv + 3 < o.cols) {
-            x = __ldg(reinterpret_cast<const float4*>(p));
-          } else {
-            x.x = __ldg(p);
-            if (col + cv + 1 < o.cols) x.y = __ldg(p + 1);
-            if (col + cv + 2 < o.cols) x.z = __ldg(p + 2);
-          }
-        }
-        r[4 * v] = x.x; r[4 * v + 1] = x.y; r[4 * v + 2] = x.z; r[4 * v + 3] = x.w;
-      } else if (inside) {
-        r[2 * v] = __ldg(p);
-        r[2 * v + 1] = __ldg(p + 32);
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      const int left = row + rv * kRowStep < o.rows ? o.cols - (col + cv) : 0;  // columns of the row from here on
+      if (VEC && (inside || left > 3)) {
+        x = __ldg(reinterpret_cast<const float4*>(p));
       } else {
-        const bool in_row = row + rv * kRowStep < o.rows;
-        r[2 * v] = in_row && col + cv < o.cols ? __ldg(p) : 0.f;
-        r[2 * v + 1] = in_row && col + cv + 32 < o.cols ? __ldg(p + 32) : 0.f;
+        if (inside || left > 0) x.x = __ldg(p);
+        if (inside || left > 1) x.y = __ldg(p + 1);
+        if (inside || left > 2) x.z = __ldg(p + 2);
+        if (inside || left > 3) x.w = __ldg(p + 3);
       }
+      r[4 * v] = x.x; r[4 * v + 1] = x.y; r[4 * v + 2] = x.z; r[4 * v + 3] = x.w;
     }
     base += MN ? BK * o.ld : (int64_t)BK;
     if (MN) row += BK; else col += BK;
   }
   // the three planes of the block in the 128-byte-swizzle image: box row br at br * 128 bytes, 16-byte piece c at c ^ (br % 8)
   __device__ __forceinline__ void store(unsigned char* s, int tid) const {
-    const int br = first_row(tid);  // (steps of 16 or 8 rows leave br % 8 as it is)
-    if (VEC) {
-      const int c4 = tid & 15;
-      unsigned char* d = s + br * 128 + ((((c4 >> 1) ^ (br & 7)) << 4) | ((c4 & 1) << 3));
+    const int br = first_row(tid), c4 = tid & 15;  // (steps of 16 rows leave br % 8 as it is)
+    unsigned char* d = s + br * 128 + ((((c4 >> 1) ^ (br & 7)) << 4) | ((c4 & 1) << 3));
 #pragma unroll
-      for (int v = 0; v < kSteps; ++v) {
-        uint32_t lo[3], hi[3];
-        split_pair(r[4 * v], r[4 * v + 1], lo);
-        split_pair(r[4 * v + 2], r[4 * v + 3], hi);
+    for (int v = 0; v < kSteps; ++v) {
+      uint32_t lo[3], hi[3];
+      split_pair(r[4 * v], r[4 * v + 1], lo);
+      split_pair(r[4 * v + 2], r[4 * v + 3], hi);
 #pragma unroll
-        for (int t = 0; t < 3; ++t) *reinterpret_cast<uint2*>(d + v * (kRowStep * 128) + t * kPlane) = make_uint2(lo[t], hi[t]);
-      }
-    } else {
-      // neighbouring lanes swap: even lanes get columns (lane, lane + 1), odd lanes (lane + 31, lane + 32)
-      const int lane = tid & 31;
-      const bool odd = lane & 1;
-      const int word = odd ? 16 + (lane >> 1) : lane >> 1;  // of the row's 32
-      unsigned char* d = s + br * 128 + (((word >> 2) ^ (br & 7)) << 4) + (word & 3) * 4;
-#pragma unroll
-      for (int v = 0; v < kSteps; ++v) {
-        const float got = __shfl_xor_sync(0xffffffffu, odd ? r[2 * v] : r[2 * v + 1], 1);
-        uint32_t w[3];
-        split_pair(odd ? got : r[2 * v], odd ? r[2 * v + 1] : got, w);
-#pragma unroll
-        for (int t = 0; t < 3; ++t) *reinterpret_cast<uint32_t*>(d + v * (kRowStep * 128) + t * kPlane) = w[t];
-      }
+      for (int t = 0; t < 3; ++t) *reinterpret_cast<uint2*>(d + v * (kRowStep * 128) + t * kPlane) = make_uint2(lo[t], hi[t]);
     }
   }
 };
@@ -515,7 +489,7 @@ bool f32_split_preferred(const frisk_b200_gemm_desc& d) {
 // Both kernels estimated in microseconds from measurements.  CUDA cores: 4.3 for 64 x 64 x 64 and about 2.0 more for
 // every further 64 x 64 x 64 unit an SM takes, 2 to add up the parts of a shared tile (512^3 13.5, 1024^3 57, 2048^3 401).
 // Tensor cores: 5.5 and 2.1 for every 128 x 128 x 64 block a CTA takes, 2 more to add up the parts of a shared tile (64^3
-// 7.6, 128^3 9.9, 512^3 11.6, 1024^3 22.9, 2048^3 128); half as much again per block where rows are not 16-byte aligned.
+// 7.6, 128^3 9.9, 512^3 11.6, 1024^3 22.9, 2048^3 128); 2.4 per block where rows are not 16-byte aligned (1151 x 2047 x 1023 43).
 bool f32_split_beats_simt(const frisk_b200_gemm_desc& d) {
   if (d.dtype_ab != FRISK_B200_F32 || d.dtype_c != FRISK_B200_F32) return false;
   if (d.M > INT32_MAX / 4 || d.N > INT32_MAX / 4 || d.K > INT32_MAX / 4) return false;
@@ -527,7 +501,7 @@ bool f32_split_beats_simt(const frisk_b200_gemm_desc& d) {
   const double simt = 4.3 + 2.0 * (units - 1) + (units < (double)kb ? 2.0 : 0.0);
   const int splits = split_of(tiles, kb, kNumSMsDefault, [](int) { return true; });
   const double blocks = std::ceil((double)tiles / sms) * std::ceil((double)kb / splits);
-  const double block = g.lda % 4 || g.ldb % 4 ? 3.2 : 2.1;
+  const double block = g.lda % 4 || g.ldb % 4 ? 2.4 : 2.1;
   return 5.5 + block * blocks + (splits > 1 ? 2.0 : 0.0) < simt;
 }
 
