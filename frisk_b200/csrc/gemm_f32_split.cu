@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
     bool more = tile < tiles;
     if (more) {
       place();
-      const bool k_in = (kb + 1) * BK <= p.K;
+      const bool k_in = (unsigned)(kb + 1) * BK <= (unsigned)p.K;
       la.fetch(p.a, a_in && k_in);
       lb.fetch(p.b, b_in && k_in);
     }
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
       if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
       __syncwarp();
       unsigned char* sa = smem + stage * kStageBytes;
-      const bool k_in = (kb + 1) * BK <= p.K;
+      const bool k_in = (unsigned)(kb + 1) * BK <= (unsigned)p.K;
       la.store(sa, tid);
       if (more) la.fetch(p.a, a_in && k_in);
       lb.store(sa + 3 * kPlane, tid);
