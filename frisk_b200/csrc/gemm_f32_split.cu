@@ -21,9 +21,9 @@
 //   warps 8-15  loaders: global -> registers (one block ahead) -> split -> shared memory, in the 128-byte-swizzle image
 //               tcgen05 reads (K-major or MN-major, whichever way the operand lies in global memory)
 // Shared memory would allow a block in 2300 clk (96 KB of planes written, 192 KB read by 24 MMAs, at 128 B/clk; 1540 clk of
-// tensor pipe).  4096^3 takes 3700 (886 us, 155 TFLOP/s of fp32): with two stages of 96 KB a stage is filled only when its
-// MMAs are done, so a block costs half of MMAs + loading + hand-over.  2048^3 126 us; 118 without the conversions, 120 without the
-// loads, 112 with a sixth of the MMAs.
+// tensor pipe).  4096^3 takes 3700 (886 us, 155 TFLOP/s of fp32).  No single part is the limit: 2048^3 takes 126 us, 118
+// without the conversions, 120 without the loads, 112 with a sixth of the MMAs; four stages of 32 k instead of two of 64
+// take 154.
 //
 // Where the tiles are fewer than half the SMs a cluster of 2 to 8 CTAs shares a tile's K; every CTA leaves its fp32 part
 // in its own shared memory and each finishes a share of the tile's 32-row pieces, adding the parts over distributed
