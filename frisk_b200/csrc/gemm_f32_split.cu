@@ -12,8 +12,10 @@
 // summed in tensor memory, small terms first, so that only the four A0B0 steps see a large accumulator, and then
 // added to fp32 registers with round-to-nearest: 1.0e-7 at K = 1024, 2.6e-7 on the CUDA cores.
 //
-// An element that is not finite, or so large that x 2^24 or a sum overflows, makes the result non-finite; such a result
-// is computed again by a plain fp32 loop over K, so infinities and NaN come out as IEEE arithmetic gives them.
+// An element that is not finite, or so large that x 2^24 or a sum overflows, makes the result non-finite.  The 32 x 16
+// piece of C it lies in is not stored but noted, and when a CTA's tiles are done (no wait of the pipeline is open any
+// more, however long K is) all its warps compute the noted pieces as 64-bit sums, rounded once: infinities and NaN come out
+// as IEEE arithmetic gives them, and the finite results of such a piece are no further off than the others.
 //
 // One CTA per SM, 16 warps with fixed roles (128 registers each, all of the SM's):
 //   warps 0-7   promotion: tensor memory -> fp32 registers (64 columns of one row per thread), stores.  One thread of
@@ -53,7 +55,9 @@ constexpr int kThreads = 32 * (kPromoWarps + kLoadWarps);
 constexpr int kOutOffset = kStages * kStageBytes;
 constexpr int kOutPitch = 20;                 // floats: [32 rows][16 columns] per promotion warp, rows 16-byte aligned
 constexpr int kOutWarpBytes = 32 * kOutPitch * 4;
-constexpr int kBarOffset = kOutOffset + kPromoWarps * kOutWarpBytes;
+constexpr int kRedoOffset = kOutOffset + kPromoWarps * kOutWarpBytes;
+constexpr int kMaxTilesPerCta = 2048;         // a word of noted pieces each; larger products take several launches
+constexpr int kBarOffset = kRedoOffset + kMaxTilesPerCta * 4;
 constexpr int kSmemTotal = kBarOffset + 256 + 1024;
 static_assert(kSmemTotal <= 232448, "stages and output buffers must fit");
 static_assert(kStages == 2, "stages and accumulators alternate together");
@@ -73,6 +77,7 @@ struct SplitArgs {
   int64_t ldc;
   int M, N, K, accumulate, vec_c;
   int tiles_m, tiles_n, kb;  // tiles, 64-k blocks per tile
+  int tile0, tile1;          // the tiles of this launch
   int splits;                // CTAs of a cluster, which share a tile's K
   unsigned* status;
 };
@@ -148,37 +153,19 @@ struct Loader {
   }
 };
 
-// one element of the product in plain fp32, for a result the split could not carry
-template <bool A_MN, bool B_MN>
-__device__ __forceinline__ float plain_dot(const SplitArgs& p, int row, int col) {
-  float acc = 0.f;
-#pragma unroll 1
-  for (int k = 0; k < p.K; ++k) {
-    const float a = A_MN ? p.a.p[(int64_t)k * p.a.ld + row] : p.a.p[(int64_t)row * p.a.ld + k];
-    const float b = B_MN ? p.b.p[(int64_t)k * p.b.ld + col] : p.b.p[(int64_t)col * p.b.ld + k];
-    acc = fmaf(a, b, acc);
-  }
-  return acc;
-}
-
 // The 32 x 16 piece of C at (r0, c0), lane = row: unscaled, added to C or written.  Four lanes write 64 consecutive
-// bytes of a row, through `out` ([32 rows][16 columns] of shared memory).
-template <bool A_MN, bool B_MN>
-__device__ __forceinline__ void store_piece(const SplitArgs& p, float (&v)[16], float* out, int r0, int c0, int lane) {
-  if (r0 >= p.M || c0 >= p.N) return;
+// bytes of a row, through `out` ([32 rows][16 columns] of shared memory).  Returns false, with C as it was, where a result
+// is not finite.
+__device__ __forceinline__ bool store_piece(const SplitArgs& p, float (&v)[16], float* out, int r0, int c0, int lane) {
+  if (r0 >= p.M || c0 >= p.N) return true;
   bool finite = true;
 #pragma unroll
   for (int i = 0; i < 16; ++i) finite = finite && fabsf(v[i]) <= kFloatMax;
+  if (__any_sync(0xffffffffu, !finite && r0 + lane < p.M)) return false;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
     *reinterpret_cast<float4*>(out + lane * kOutPitch + 4 * i) =
         make_float4(v[4 * i] * kUnscale, v[4 * i + 1] * kUnscale, v[4 * i + 2] * kUnscale, v[4 * i + 3] * kUnscale);
-  if (!finite && r0 + lane < p.M)
-#pragma unroll 1
-    for (int i = 0; i < 16; ++i) {
-      float& x = out[lane * kOutPitch + i];
-      if (!(fabsf(x) <= kFloatMax) && c0 + i < p.N) x = plain_dot<A_MN, B_MN>(p, r0 + lane, c0 + i);
-    }
   __syncwarp();
   if (p.vec_c) {
 #pragma unroll
@@ -211,6 +198,87 @@ __device__ __forceinline__ void store_piece(const SplitArgs& p, float (&v)[16], 
     }
   }
   __syncwarp();
+  return true;
+}
+
+// The noted pieces of this CTA's tiles (bit 16 h + w of a tile's word: columns 64h + 16 (w / 4), rows 32 (w % 4)) as
+// 64-bit sums in the order of k, by all 16 warps, one piece of a half tile each; a lane has 4 x 4 results.
+// 4096^3 takes 0.83 ms, with one infinite element 1.75 and with every result above 2^80 11.7 (53 and 451 when the thread
+// that met such a result summed it up on the spot); the 64-bit units bound it.
+template <bool A_MN, bool B_MN>
+__device__ __noinline__ void redo_pieces(const SplitArgs& p, unsigned char* smem, const uint32_t* noted, int first, int step,
+                                         int count) {
+  constexpr int kPitchA = BT + 2, kPitchB = BT / 2 + 2;  // 4 banks from one k to the next
+  static_assert(BK * (kPitchA + kPitchB) * 8 <= kOutOffset, "a block in 64 bits must fit in the stages");
+  double* sa = reinterpret_cast<double*>(smem);          // [64 k][128 rows]
+  double* sb = sa + BK * kPitchA;                        // [64 k][64 columns]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int t = 0; t < 2 * count; ++t) {
+    const uint32_t mask = (noted[t >> 1] >> (16 * (t & 1))) & 0xffffu;
+    if (mask == 0) continue;  // (the same for every thread)
+    const TileCoord tc = tile_coord(first + (t >> 1) * step, p.tiles_m, p.tiles_n);
+    const int m0 = tc.m * BT, n0 = tc.n * BT + (t & 1) * (BT / 2);
+    // A thread's elements of a block: where k is contiguous, 8 k of 4 rows a warp (32-byte sectors, all banks); otherwise rows
+    auto row_of = [&](bool mn, int rows, int j) { return mn ? (int)threadIdx.x % rows : (lane >> 3) + 4 * warp + 64 * (j >> 3); };
+    auto k_of = [&](bool mn, int rows, int j) {
+      return mn ? (int)threadIdx.x / rows + j * (kThreads / rows) : (lane & 7) + 8 * (j & 7);
+    };
+    auto element = [&](const Operand& o, bool mn, int r, int k, int rows) {
+      return r < rows && k < p.K ? __ldg(o.p + (mn ? (int64_t)k * o.ld + r : (int64_t)r * o.ld + k)) : 0.f;
+    };
+    float pa[16], pb[8];
+    auto fetch = [&](int k0) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) pa[j] = element(p.a, A_MN, m0 + row_of(A_MN, BT, j), k0 + k_of(A_MN, BT, j), p.M);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) pb[j] = element(p.b, B_MN, n0 + row_of(B_MN, BT / 2, j), k0 + k_of(B_MN, BT / 2, j), p.N);
+    };
+    double acc[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[r][c] = 0.0;
+    // the pieces of a row block, as those of a column block, are four different schedulers'; rows and columns of a lane come
+    // in pairs, so that the reads of a warp are consecutive
+    const int pm = (warp + (warp >> 2)) & 3, pn = warp >> 2;
+    const int row = pm * 32 + (lane & 7) * 2, col = pn * 16 + (lane >> 3) * 2;
+    const bool mine = (mask >> (pn * 4 + pm)) & 1u;
+    fetch(0);
+    for (int kb = 0; kb < p.kb; ++kb) {
+      __syncthreads();  // the block before this one has been read
+#pragma unroll
+      for (int j = 0; j < 16; ++j) sa[k_of(A_MN, BT, j) * kPitchA + row_of(A_MN, BT, j)] = pa[j];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sb[k_of(B_MN, BT / 2, j) * kPitchB + row_of(B_MN, BT / 2, j)] = pb[j];
+      __syncthreads();
+      if (kb + 1 < p.kb) fetch((kb + 1) * BK);
+      if (mine) {
+#pragma unroll 2
+        for (int k = 0; k < BK; ++k) {
+          const double2* a2 = reinterpret_cast<const double2*>(sa + k * kPitchA + row);
+          const double2* b2 = reinterpret_cast<const double2*>(sb + k * kPitchB + col);
+          const double a[4] = {a2[0].x, a2[0].y, a2[8].x, a2[8].y}, b[4] = {b2[0].x, b2[0].y, b2[4].x, b2[4].y};
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+        }
+      }
+    }
+    if (mine)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int rr = m0 + row + (r >> 1) * 16 + (r & 1), cc = n0 + col + (c >> 1) * 8 + (c & 1);
+          if (rr < p.M && cc < p.N) {
+            float* dst = p.C + (int64_t)rr * p.ldc + cc;
+            const float x = static_cast<float>(acc[r][c]);
+            *dst = p.accumulate ? *dst + x : x;
+          }
+        }
+    __syncthreads();
+  }
 }
 
 template <bool A_MN, bool B_MN, bool VEC>
@@ -224,11 +292,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
   uint64_t* acc_empty = acc_full + 2;        // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
+  volatile uint32_t* any_noted = tmem_slot + 2;
+  uint32_t* noted = reinterpret_cast<uint32_t*>(smem + kRedoOffset);  // pieces of each of this CTA's tiles to compute again
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int splits = p.splits, rank = splits > 1 ? (int)cluster_ctarank() : 0;
   // this CTA's tiles (one, if K is shared) and its blocks of each
-  const int tile_first = (int)blockIdx.x / splits, tile_step = splits > 1 ? INT_MAX / 2 : (int)gridDim.x;
-  const int tiles = p.tiles_m * p.tiles_n;
+  const int tile_first = p.tile0 + (int)blockIdx.x / splits, tile_step = splits > 1 ? INT_MAX / 2 : (int)gridDim.x;
+  const int tiles = p.tile1;
+  const int n_mine = tile_first < tiles ? (tiles - 1 - tile_first) / tile_step + 1 : 0;
   const int kb0 = (int)((int64_t)p.kb * rank / splits), kb1 = (int)((int64_t)p.kb * (rank + 1) / splits);
 
   if (threadIdx.x == 0) {
@@ -241,8 +312,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
       mbar_init(&acc_empty[i], kPromoWarps);
     }
     *abort_flag = 0;
+    *any_noted = 0;
     mbar_fence_init();
   }
+  for (int i = threadIdx.x; i < n_mine; i += kThreads) noted[i] = 0;
   if (warp == 0) {
     tmem_alloc(tmem_slot, 2 * BT);
     tmem_relinquish();
@@ -261,9 +334,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     float* out = reinterpret_cast<float*>(smem + kOutOffset + warp * kOutWarpBytes);
     int blocks = 0, issued = 0;  // blocks added up, blocks handed to the tensor core (by warp 0), over all tiles
-    const int n_mine = tile_first < tiles ? (tiles - 1 - tile_first) / tile_step + 1 : 0;
     const int64_t total = (int64_t)n_mine * (kb1 - kb0);
     bool ok = true;
+    auto note = [&](int tile, int piece) {
+      if (lane == 0) {
+        atomicOr(&noted[(tile - tile_first) / tile_step], 1u << piece);
+        *any_noted = 1;
+      }
+    };
     // the MMAs of the next block: stage and accumulator alternate with the block's number
     auto issue = [&]() {
       constexpr uint32_t idesc = umma_idesc_f16(BT, BT, true, A_MN, B_MN);
@@ -334,7 +412,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
           float x[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) x[i] = v[u * 16 + i];
-          store_piece<A_MN, B_MN>(p, x, out, tc.m * BT + quad * 32, tc.n * BT + half * 64 + u * 16, lane);
+          if (!store_piece(p, x, out, tc.m * BT + quad * 32, tc.n * BT + half * 64 + u * 16, lane))
+            note(tile, half * 16 + u * 4 + quad);
         }
       }
     }
@@ -358,7 +437,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
             v[4 * i] += t.x; v[4 * i + 1] += t.y; v[4 * i + 2] += t.z; v[4 * i + 3] += t.w;
           }
         }
-        store_piece<A_MN, B_MN>(p, v, out, tc.m * BT + g * 32, tc.n * BT + u * 16, lane);
+        if (!store_piece(p, v, out, tc.m * BT + g * 32, tc.n * BT + u * 16, lane)) note(tile_first, x);
       }
       cluster_sync_all();  // the peers have read this CTA's part
     }
@@ -414,6 +493,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
     }
   }
 
+  // ------------------------------------------------------------------ results the split cannot carry
+  __syncthreads();  // every role is done, and the peers of a cluster with this CTA's shared memory
+  if (*any_noted && !*abort_flag) redo_pieces<A_MN, B_MN>(p, smem, noted, tile_first, tile_step, n_mine);
+
   // ------------------------------------------------------------------ teardown
   if (*abort_flag) {
     unsigned long long t0 = globaltimer();
@@ -453,7 +536,6 @@ int launch_one(frisk_b200_ctx* ctx, SplitArgs a, cudaStream_t s) {
   const int sms = std::min(ctx->num_sms, kNumSMsDefault), tiles = a.tiles_m * a.tiles_n;
   a.splits = split_of(tiles, a.kb, sms, [&](int n) { return capacity(ctx->device, kern, kThreads, kSmemTotal, n) >= tiles; });
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(a.splits > 1 ? tiles * a.splits : std::min(tiles, sms)));
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = kSmemTotal;
   cfg.stream = s;
@@ -466,7 +548,12 @@ int launch_one(frisk_b200_ctx* ctx, SplitArgs a, cudaStream_t s) {
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = a.splits > 1 ? 2 : 1;
-  FB_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, a));
+  for (a.tile0 = 0; a.tile0 < tiles; a.tile0 = a.tile1) {
+    a.tile1 = (int)std::min<int64_t>(tiles, (int64_t)a.tile0 + (int64_t)sms * kMaxTilesPerCta);
+    const int n = a.tile1 - a.tile0;
+    cfg.gridDim = dim3((unsigned)(a.splits > 1 ? n * a.splits : std::min(n, sms)));
+    FB_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, a));
+  }
   return 0;
 }
 

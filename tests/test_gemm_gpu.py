@@ -128,6 +128,55 @@ def test_f32_auto_extreme_values(ctx):
 
 
 @pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("M,N,K,acc", [
+    (2304, 2569, 323, False),  # two or three whole tiles a CTA, the last column tile 9 wide
+    (2049, 1153, 392, True),   # the same, added to C
+    (391, 520, 1027, True),    # K shared by a cluster: every CTA has some of a tile's pieces
+])
+def test_f32_results_the_split_cannot_carry(ctx, M, N, K, acc, ta, tb):
+    """Infinities, NaN and finite results above 2^80 among ordinary ones, in several tiles of a CTA.  The elements are whole
+    numbers (times a power of two a row), so that every finite result is exact in any order."""
+    import torch
+
+    import frisk_b200 as F
+    from frisk_b200.execute import context_for
+    g = torch.Generator(device="cuda").manual_seed(9)
+    a = torch.randint(-8, 9, (M, K), generator=g, device="cuda").float()
+    b = torch.randint(-8, 9, (K, N), generator=g, device="cuda").float()
+    c0 = torch.randint(-99, 99, (M, N), generator=g, device="cuda").float()
+    a[40:80] *= 2.0 ** 90                       # finite, beyond what the scaled split can carry
+    c0[40:80] = 0
+    a[5, K // 2], a[M - 1, 0], a[130, K - 1] = float("inf"), -float("inf"), float("nan")
+    b[K // 3, N - 2], b[1, 7] = float("inf"), float("nan")
+    want = (a.double() @ b.double()).float() + (c0 if acc else 0)
+    c = c0.clone() if acc else torch.full((M, N), 7.0, device="cuda")
+    F.gemm(a.T.contiguous() if ta else a, b.T.contiguous() if tb else b, c, trans_a=ta, trans_b=tb, clear_accum=not acc)
+    context_for(0).check(torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(torch.isnan(c), torch.isnan(want))
+    ok = ~torch.isnan(want)
+    assert torch.equal(c[ok], want[ok]) and torch.isinf(want[ok]).any()
+
+
+def test_f32_every_result_above_what_the_split_can_carry(ctx):
+    """360 tiles of results above 2^80: all are computed again, tile by tile.  2304 x 2560 x 4096 should take 2 ms, and is
+    allowed ten times that; a thread that summed up its 64 results one by one would need a hundred times as much."""
+    import torch
+    M, N, K = 2304, 2560, 4096
+    a, b = torch.full((M, K), 2.0 ** 45, device="cuda"), torch.full((K, N), 2.0 ** 45, device="cuda")
+    c = torch.empty(M, N, device="cuda")
+    desc = capi.gemm_desc(M, N, K, "fp32", "fp32", algo=capi.ALGO_F32_SPLIT)
+    s = torch.cuda.current_stream().cuda_stream
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    for _ in range(2):
+        e0.record()
+        ctx.gemm(desc, a.data_ptr(), b.data_ptr(), c.data_ptr(), stream=s)
+        e1.record()
+        ctx.check(s)
+    assert (c == 2.0 ** 102).all()
+    assert e0.elapsed_time(e1) < 20
+
+
+@pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
 def test_f32_simt_shared_k_ranges(ctx, ta, tb):
     """Shapes whose tiles are fewer than the SMs or do not divide among them: every tile's k range is shared
     between workers (tickets, partial tiles), with ragged edges and a ragged last k stage."""
