@@ -10,7 +10,9 @@
 // Accuracy is decided by the accumulation: tensor memory truncates every addition, a bias of half a unit per MMA along
 // a sum (1.0e-6 relative error at K = 1024 when the whole K stayed there).  So one 64-k block is
 // summed in tensor memory, small terms first, so that only the four A0B0 steps see a large accumulator, and then
-// added to fp32 registers with round-to-nearest: 1.0e-7 at K = 1024, 2.6e-7 on the CUDA cores.
+// added to fp32 registers with round-to-nearest: 1.0e-7 at K = 1024, 2.6e-7 on the CUDA cores.  Sums whose terms share a
+// sign feel the truncations more: below K = 640 a block is summed in two halves, each in an accumulator of its own
+// (TWO; 22.4 us instead of 21.8 at 1024^3), and below K = 320 the CUDA cores are the more accurate (split_accurate).
 //
 // An element that is not finite, or so large that x 2^24 or a sum overflows, makes the result non-finite.  The 32 x 16
 // piece of C it lies in is not stored but noted, and when a CTA's tiles are done (no wait of the pipeline is open any
@@ -281,7 +283,8 @@ __device__ __noinline__ void redo_pieces(const SplitArgs& p, unsigned char* smem
   }
 }
 
-template <bool A_MN, bool B_MN, bool VEC>
+// TWO: a block's 32-k halves are summed in accumulators of their own
+template <bool A_MN, bool B_MN, bool VEC, bool TWO>
 __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __grid_constant__ SplitArgs p) {
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
@@ -294,6 +297,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile uint32_t* any_noted = tmem_slot + 2;
   uint32_t* noted = reinterpret_cast<uint32_t*>(smem + kRedoOffset);  // pieces of each of this CTA's tiles to compute again
+  constexpr int kHalves = TWO ? 2 : 1, kAccCols = kHalves * BT;  // of an accumulator
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int splits = p.splits, rank = splits > 1 ? (int)cluster_ctarank() : 0;
   // this CTA's tiles (one, if K is shared) and its blocks of each
@@ -317,7 +321,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
   }
   for (int i = threadIdx.x; i < n_mine; i += kThreads) noted[i] = 0;
   if (warp == 0) {
-    tmem_alloc(tmem_slot, 2 * BT);
+    tmem_alloc(tmem_slot, 2 * kAccCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
@@ -360,8 +364,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
         for (int t = 0; t < 6; ++t)
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
-            umma_f16_ss(tmem_base + i * BT, da + ((ta[t] * kPlane + k * (A_MN ? 16 * 128 : 32)) >> 4),
-                        db + ((tb[t] * kPlane + k * (B_MN ? 16 * 128 : 32)) >> 4), idesc, (t | k) != 0 ? 1u : 0u);
+            umma_f16_ss(tmem_base + i * kAccCols + (TWO && k >= 2 ? BT : 0), da + ((ta[t] * kPlane + k * (A_MN ? 16 * 128 : 32)) >> 4),
+                        db + ((tb[t] * kPlane + k * (B_MN ? 16 * 128 : 32)) >> 4), idesc, (t | (TWO ? k & 1 : k)) != 0 ? 1u : 0u);
         umma_commit(&empty_bar[i]);
         umma_commit(&acc_full[i]);
       }
@@ -384,17 +388,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
         tc_fence_after_sync();
         __syncwarp();
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < 2 * kHalves; ++h) {
           uint32_t t[32];
-          tmem_ld_32x32b_x32(tmem_base + acc * BT + half * 64 + h * 32 + lane_addr, t);
+          tmem_ld_32x32b_x32(tmem_base + acc * kAccCols + (h >> 1) * BT + half * 64 + (h & 1) * 32 + lane_addr, t);
           tmem_ld_wait();
-          if (h == 1) {
+          if (h == 2 * kHalves - 1) {
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[acc]);
           }
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[h * 32 + i] += __uint_as_float(t[i]);
+          for (int i = 0; i < 32; ++i) v[(h & 1) * 32 + i] += __uint_as_float(t[i]);
         }
       }
       if (!ok) break;
@@ -507,7 +511,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
   if (warp == 0) {
     __syncwarp();
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 2 * BT);
+    tmem_dealloc(tmem_base, 2 * kAccCols);
   }
 }
 
@@ -522,11 +526,12 @@ int split_of(int64_t tiles, int64_t kb, int sms, F&& fits) {
   return best;
 }
 
+constexpr int kTwoBelowK = 640;
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-template <bool A_MN, bool B_MN, bool VEC>
+template <bool A_MN, bool B_MN, bool VEC, bool TWO>
 int launch_one(frisk_b200_ctx* ctx, SplitArgs a, cudaStream_t s) {
-  auto kern = gemm_f32_split_kernel<A_MN, B_MN, VEC>;
+  auto kern = gemm_f32_split_kernel<A_MN, B_MN, VEC, TWO>;
   static PerDeviceOnce opt_in;
   if (opt_in(ctx->device, [&] {
         return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTotal) == cudaSuccess ? 0 : 1;
@@ -559,7 +564,9 @@ int launch_one(frisk_b200_ctx* ctx, SplitArgs a, cudaStream_t s) {
 
 template <bool A_MN, bool B_MN>
 int launch_vec(frisk_b200_ctx* ctx, const SplitArgs& a, bool vec, cudaStream_t s) {
-  return vec ? launch_one<A_MN, B_MN, true>(ctx, a, s) : launch_one<A_MN, B_MN, false>(ctx, a, s);
+  if (a.K < kTwoBelowK)
+    return vec ? launch_one<A_MN, B_MN, true, true>(ctx, a, s) : launch_one<A_MN, B_MN, false, true>(ctx, a, s);
+  return vec ? launch_one<A_MN, B_MN, true, false>(ctx, a, s) : launch_one<A_MN, B_MN, false, false>(ctx, a, s);
 }
 
 }  // namespace
@@ -575,12 +582,18 @@ bool f32_split_preferred(const frisk_b200_gemm_desc& d) {
   return f32_split_supported(d) && d.M >= 256 && d.N >= 256 && d.K >= 256;
 }
 
+// Where the error is no larger than that of the CUDA cores' fp32 sums, whatever the signs.  Relative to theirs it is, for
+// terms of either sign / of one sign / of sizes e^3 apart: 0.9 / 1.7 / 1.4 at K = 64, 0.8 / 1.5 / 1.2 at 128 with one
+// accumulator a block; 0.54 / 1.06 / 0.7 at 256, 0.52 / 0.96 / 0.65 at 320, 0.45 / 0.87 / 0.57 at 512 with two; 0.45 / 0.98 /
+// 0.7 at 640, 0.38 / 0.86 / 0.6 at 1024 with one (1024 x 1024 x K, 2-norm; CUDA cores 8e-8 at 64, 2.6e-7 at 1024).
+bool split_accurate(const frisk_b200_gemm_desc& d) { return d.K >= 320 || f32_split_preferred(d); }
+
 // Both kernels estimated in microseconds from measurements.  CUDA cores: 4.3 for 64 x 64 x 64 and about 2.0 more for
 // every further 64 x 64 x 64 unit an SM takes, 2 to add up the parts of a shared tile (512^3 13.5, 1024^3 57, 2048^3 401).
 // Tensor cores: 5.5 and 2.1 for every 128 x 128 x 64 block a CTA takes, 2 more to add up the parts of a shared tile (64^3
 // 7.6, 128^3 9.9, 512^3 11.6, 1024^3 22.9, 2048^3 128); 2.4 per block where rows are not 16-byte aligned (1151 x 2047 x 1023 43).
 bool f32_split_beats_simt(const frisk_b200_gemm_desc& d) {
-  if (d.dtype_ab != FRISK_B200_F32 || d.dtype_c != FRISK_B200_F32) return false;
+  if (d.dtype_ab != FRISK_B200_F32 || d.dtype_c != FRISK_B200_F32 || !split_accurate(d)) return false;
   if (d.M > INT32_MAX / 4 || d.N > INT32_MAX / 4 || d.K > INT32_MAX / 4) return false;
   const GemmDims g = resolve_dims(d);
   const double sms = kNumSMsDefault;

@@ -83,8 +83,8 @@ def test_f32_split_transposes_accumulate_unaligned(ctx, ta, tb):
 @pytest.mark.parametrize("M,N,K,acc", [
     (512, 512, 512, False),    # a cluster of four CTAs per tile
     (513, 640, 1000, True),    # two per tile, unaligned C and (transposed) operands, ragged rows and k
-    (1152, 2048, 65, False),   # 144 whole tiles, one k beyond a block
-    (2049, 1153, 200, False),  # more tiles than SMs, ragged everywhere
+    (1152, 2048, 321, False),  # 144 whole tiles, one k beyond a block
+    (2049, 1153, 392, False),  # more tiles than SMs, ragged everywhere
     (384, 384, 4100, True),    # eight CTAs per tile
 ])
 def test_f32_auto_on_the_tensor_cores(ctx, M, N, K, acc):
@@ -92,6 +92,40 @@ def test_f32_auto_on_the_tensor_cores(ctx, M, N, K, acc):
     of plain fp32 accumulation: K roundings of 2^-24 relative to the running sum, adding up like a random walk."""
     for ta, tb in ((False, False), (False, True), (True, False), (True, True)):
         assert check(ctx, M, N, K, "fp32", "fp32", ta, tb, 23, accumulate=acc) < 2.0 ** -24 * max(8, K ** 0.5)
+
+
+def test_f32_auto_short_k_is_the_cuda_cores_sum(ctx):
+    """Below K = 320 (other than multiples of 8 from 256 up) an AUTO call adds in fp32 with round-to-nearest, whatever the
+    other kernel would take: K = 1 is the correctly rounded product."""
+    import torch
+
+    import frisk_b200 as F
+    g = torch.Generator(device="cuda").manual_seed(6)
+    for M, N, K in ((2048, 2048, 1), (2048, 2048, 8), (2048, 2048, 64), (2048, 2048, 248), (2047, 2049, 319)):
+        a, b = torch.rand(M, K, generator=g, device="cuda"), torch.rand(K, N, generator=g, device="cuda")
+        c, cores = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+        F.gemm(a, b, c)
+        F.gemm(a, b, cores, algo=capi.ALGO_SIMT_F32)
+        assert torch.equal(c, cores) and (K > 1 or torch.equal(c, a * b))
+
+
+@pytest.mark.parametrize("K", [320, 512, 639, 640, 1023])
+def test_f32_auto_is_no_further_off_than_the_cuda_cores(ctx, K):
+    """Sums whose terms share a sign, where truncated additions show most (1.02 allows for the draw of the inputs: the error is
+    a 2-norm over a million results)."""
+    import torch
+
+    import frisk_b200 as F
+    g = torch.Generator(device="cuda").manual_seed(K)
+    for shift in (0.0, 1.0, -0.5):
+        a, b = (torch.rand(s, generator=g, device="cuda") + shift for s in ((1024, K), (K, 1032)))
+        ref = a.double() @ b.double()
+        err = []
+        for algo in (capi.ALGO_AUTO, capi.ALGO_SIMT_F32):
+            c = torch.empty(1024, 1032, device="cuda")
+            F.gemm(a, b, c, algo=algo)
+            err.append((c.double() - ref).norm().item())
+        assert 0 < err[0] <= 1.02 * err[1], (shift, err)
 
 
 def test_f32_auto_extreme_values(ctx):
