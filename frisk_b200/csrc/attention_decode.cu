@@ -10,7 +10,8 @@
 //   * the (head, 64-key tile) units are numbered head-major and CTA c takes a contiguous range of them, so every SM
 //     streams the same number of bytes whatever the head count and the cache length; a head shared by several CTAs is
 //     finished by the contributor that draws the last ticket, which adds the partial results in contributor order
-//     (reproducible).  No CTA waits for another;
+//     (reproducible).  No CTA waits for another, and one whose own wait ran out still draws the tickets it owes, so
+//     that they are zero again when the launch ends however it ends;
 //   * K and V tiles arrive by TMA in a ring of 192 KB (6 stages of 64 keys at D = 128, 12 at D = 64);
 //   * four warps work on every tile, warp w on its keys 16w..16w+15 with its own reference maximum, row sums and fp32
 //     O, so nothing but the ring ties them together before the end of a head's range.  The products use
@@ -22,6 +23,7 @@
 
 #include "common.cuh"
 #include "ptx.cuh"
+#include "work_split.cuh"
 
 #include "attention_common.cuh"
 
@@ -54,16 +56,11 @@ struct DecParams {
   const void* Q;
   void* O;
   int S_q, S_kv, n_tiles, causal;
-  unsigned q, r;  // units = grid * q + r: the first r CTAs take q + 1
+  WorkSplit work;  // (head, key tile) units over the CTAs
   float scale_log2;
   unsigned* tickets;  // one per head, zero between launches
   float* partials;    // two per CTA
   unsigned* status;
-  __host__ __device__ unsigned start(unsigned c) const { return c * q + (c < r ? c : r); }
-  __device__ unsigned worker_of(unsigned u) const {
-    const unsigned big = r * (q + 1);
-    return u < big ? u / (q + 1) : r + (u - big) / q;
-  }
 };
 
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
@@ -116,7 +113,7 @@ __global__ void __launch_bounds__(kDecThreads, 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned n_tiles = (unsigned)p.n_tiles;
-  const unsigned u_begin = p.start(blockIdx.x), u_end = p.start(blockIdx.x + 1);
+  const unsigned u_begin = p.work.start(blockIdx.x), u_end = p.work.start(blockIdx.x + 1);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < L::kStages; ++i) {
@@ -180,8 +177,15 @@ __global__ void __launch_bounds__(kDecThreads, 1)
     const uint32_t k_off = k_row * 128, v_off = v_row * 128;
     int stage = 0;
     uint32_t phase = 0;
+    // (one thread) this CTA's draw of a shared head's ticket; true for the last of the head's contributors
+    auto draw = [&](unsigned head, unsigned partners) {
+      const bool last = atomicAdd(&p.tickets[head], 1u) == partners;
+      if (last) p.tickets[head] = 0;  // clean for the next launch
+      return last;
+    };
 
-    for (unsigned u = u_begin; u < u_end && ok;) {
+    unsigned u = u_begin;  // the tickets of the units before u are drawn
+    while (u < u_end && ok) {
       const unsigned head = u / n_tiles, tile0 = u % n_tiles;
       const unsigned tile1 = min(n_tiles, tile0 + (u_end - u));  // this CTA's tiles of the head: [tile0, tile1)
 
@@ -333,20 +337,19 @@ __global__ void __launch_bounds__(kDecThreads, 1)
         }
       }
       if (!whole) {
-        const unsigned h0 = head * n_tiles;
-        const unsigned c_first = p.worker_of(h0), c_last = p.worker_of(h0 + n_tiles - 1);
+        const unsigned h0 = head * n_tiles, partners = p.work.partners(h0, n_tiles), c_first = p.work.worker_of(h0);
         meet();  // the partial is written ...
         if (threadIdx.x == 0) {
           __threadfence();  // ... and visible device-wide before the ticket is taken
-          *ticket_word = atomicAdd(&p.tickets[head], 1u);
+          *ticket_word = draw(head, partners) ? 1u : 0u;
         }
         meet();
-        if (ok && *ticket_word == c_last - c_first) {
+        if (ok && *ticket_word) {
           __threadfence();
-          const int n_contrib = (int)(c_last - c_first) + 1;
+          const int n_contrib = (int)partners + 1;
           // (a contributor whose range begins before the head has it as the head its range ends in)
           auto slot_of = [&](unsigned c) {
-            return p.partials + ((size_t)c * 2 + (p.start(c) >= h0 ? 0 : 1)) * kPartialFloats;
+            return p.partials + ((size_t)c * 2 + (p.work.start(c) >= h0 ? 0 : 1)) * kPartialFloats;
           };
           // weights of the contributors, eight threads to a row
           const int row = threadIdx.x >> 3, sub = threadIdx.x & 7;
@@ -382,12 +385,13 @@ __global__ void __launch_bounds__(kDecThreads, 1)
             store4<BF16, OUT_F32>(p.O, ((size_t)head * p.S_q + r) * D + c4 * 4,
                                   make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
           }
-          if (threadIdx.x == 0) p.tickets[head] = 0;  // clean for the next launch
         }
       }
       meet();  // the reduction area may be written again
       u += tile1 - tile0;
     }
+    // what a wait that ran out has left over
+    if (threadIdx.x == 0) p.work.draw_owed(u, u_end, n_tiles, draw);
   }
 
   // ------------------------------------------------------------------ teardown
@@ -427,8 +431,8 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q
   p.scale_log2 = d.scale * 1.4426950408889634f;
   const unsigned units = (unsigned)bh * (unsigned)p.n_tiles;  // < 2^31 (attention_decode_preferred)
   const unsigned grid = std::min<unsigned>(units, (unsigned)std::min(ctx->num_sms, kNumSMsDefault));
-  p.q = units / grid;
-  p.r = units % grid;
+  p.work.q = units / grid;
+  p.work.r = units % grid;
   p.tickets = static_cast<unsigned*>(ctx->attn_scratch);
   p.partials = reinterpret_cast<float*>(static_cast<unsigned char*>(ctx->attn_scratch) + kTicketBytes);
   p.status = ctx->d_status;
