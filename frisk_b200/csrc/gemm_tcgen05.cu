@@ -40,6 +40,7 @@
 
 #include "gemm_common.cuh"
 #include "ptx.cuh"
+#include "work_split.cuh"
 
 namespace fb {
 namespace {
@@ -106,23 +107,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int tiles_m = (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN, tiles = tiles_m * tiles_n;
   const int splits = p.splits, rank = splits > 1 ? (int)cluster_ctarank() : 0;
   const int num_kb = (p.K + BK - 1) / BK;
-  // this CTA's work, item by item: its whole tiles, then its 64-k blocks of the tile its cluster shares
-  struct Item {
-    int tile, kb0, kb1;
-    bool shared;
-  };
-  auto get_item = [&](int i, Item& it) -> bool {
-    const int whole = (int)blockIdx.x + i * (int)gridDim.x;
-    if (whole < p.n_whole) {
-      it = Item{whole, 0, num_kb, false};
-      return true;
-    }
-    const int n_mine = (int)blockIdx.x < p.n_whole ? (p.n_whole - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    const int tile = p.n_whole + (int)blockIdx.x / splits;
-    if (i > n_mine || splits == 1 || tile >= tiles) return false;
-    it = Item{tile, (int)((int64_t)num_kb * rank / splits), (int)((int64_t)num_kb * (rank + 1) / splits), true};
-    return true;
-  };
+  // this CTA's work, item by item
+  const TileWalk walk{tiles, num_kb, p.n_whole, splits, (int)gridDim.x};
+  auto get_item = [&](int i, TileItem& it) { return walk.get((int)blockIdx.x, rank, i, it); };
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
@@ -160,7 +147,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      Item it;
+      TileItem it;
       for (int i = 0; ok && get_item(i, it); ++i) {
         const TileCoord tc = tile_coord(it.tile, tiles_m, tiles_n);
         const int m0 = tc.m * BM, n0 = tc.n * BN;
@@ -206,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      Item it;
+      TileItem it;
       for (int i = 0; ok && get_item(i, it); ++i) {
         if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.status, ST_TIMEOUT_ACC_EMPTY)) break;
         tc_fence_after_sync();
@@ -363,18 +350,23 @@ __global__ void __launch_bounds__(kThreads, 1)
       box_sel ^= 1;
       if (reduce_kind && r0 + lane < p.M) __stcg(p.epi.row_partials + (int64_t)(c0 / U) * p.M + r0 + lane, row_acc);
     };
+    // (one thread) a draw of row block m's ticket; true for the last of its column tiles
+    auto draw_row = [&](int m) {
+      const bool last = atomicAdd(p.epi.row_tickets + m, 1u) == (unsigned)tiles_n - 1;
+      if (last) p.epi.row_tickets[m] = 0;  // clean for the next launch
+      return last;
+    };
+    int drawn = 0;  // items whose tickets this CTA has drawn
     // A column tile of row block tc.m has left its partials: whoever draws the last ticket combines the row block's
     auto combine_rows = [&](const TileCoord& tc) {
       epi_sync();
       if (warp == 2 && lane == 0) {
         __threadfence();
-        const bool last = atomicAdd(p.epi.row_tickets + tc.m, 1u) == (unsigned)tiles_n - 1;
-        if (last) {
-          p.epi.row_tickets[tc.m] = 0;  // clean for the next launch
-          __threadfence();
-        }
+        const bool last = draw_row(tc.m);
+        if (last) __threadfence();
         *epi_word = last ? 1u : 0u;
       }
+      ++drawn;
       epi_sync();
       const bool combine = ok && *epi_word != 0;
       epi_sync();  // everybody has read it
@@ -389,7 +381,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     };
 
-    Item it;
+    TileItem it;
     TileCoord shared_tile{-1, -1};
     for (int i = 0; ok && get_item(i, it); ++i) {
       const TileCoord tc = tile_coord(it.tile, tiles_m, tiles_n);
@@ -523,6 +515,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       cluster_sync_all();  // nobody reads a peer any more
       if (reduce_kind && shared && rank == 0) combine_rows(tc);
     }
+    // what a wait that ran out has left over: the tickets are zero again however the launch ends
+    if (reduce_kind && warp == 2 && lane == 0)
+      walk.draw_owed((int)blockIdx.x, rank, drawn, [&](int tile) { draw_row(tile_coord(tile, tiles_m, tiles_n).m); });
     if (tma_c && lane == 0) tma_store_wait<0>();  // the boxes are read and written out before the CTA leaves
   }
   if (warp < 2 && splits > 1) {

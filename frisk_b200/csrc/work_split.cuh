@@ -1,6 +1,7 @@
 // How work is dealt to CTAs, and which tickets a CTA owes.  Plain arithmetic, for the host as well.
 //
 // WorkSplit: units, numbered group after group (a group: the key tiles of a head), in contiguous ranges.
+// TileWalk: output tiles, whole ones round by round and the rest to clusters that share each one's K.
 //
 // What several CTAs work on has a ticket, zero between launches: each contributor draws it EXACTLY ONCE, whatever
 // happens to the CTA in between (draw_owed), and the last draw puts it back to zero.
@@ -32,6 +33,36 @@ struct WorkSplit {
       if (left >= end - u) break;
       u += left;
     }
+  }
+};
+
+struct TileItem {
+  int tile, kb0, kb1;  // 64-k blocks [kb0, kb1) of the tile
+  bool shared;         // the other blocks are the cluster's other CTAs'
+};
+
+struct TileWalk {
+  int tiles, num_kb;          // in all; 64-k blocks of a tile
+  int n_whole, splits, grid;  // tiles [0, n_whole) are walked whole; a cluster of `splits` CTAs shares each of the others
+  // item i of CTA `cta`, which has `rank` in its cluster: its whole tiles, then its part of one shared tile
+  FB_HOST_DEVICE bool get(int cta, int rank, int i, TileItem& it) const {
+    const int whole = cta + i * grid;
+    if (whole < n_whole) {
+      it = TileItem{whole, 0, num_kb, false};
+      return true;
+    }
+    const int n_mine = cta < n_whole ? (n_whole - 1 - cta) / grid + 1 : 0;
+    const int tile = n_whole + cta / splits;
+    if (i > n_mine || splits == 1 || tile >= tiles) return false;
+    it = TileItem{tile, (int)((long long)num_kb * rank / splits), (int)((long long)num_kb * (rank + 1) / splits), true};
+    return true;
+  }
+  // draw(tile) for the tiles from item i on whose tickets this CTA draws: all of its own, and rank 0 the cluster's
+  template <typename Draw>
+  FB_HOST_DEVICE void draw_owed(int cta, int rank, int i, Draw&& draw) const {
+    TileItem it;
+    for (; get(cta, rank, i, it); ++i)
+      if (!it.shared || rank == 0) draw(it.tile);
   }
 };
 

@@ -55,6 +55,47 @@ int main() {
       if (merged[g] != (contributors > 1 ? 1u : 0u)) return 6;
     }
   }
+  // tiles: whole rounds, then clusters that share the K of the rest
+  for (int round = 0; round < 20000; ++round) {
+    const int splits = 1 << pick(0, 3), sms = 148, kb = (int)pick(2 * splits, 64), tiles_n = (int)pick(1, 30);
+    const int tiles = tiles_n * (int)pick(1, 30), full = sms / splits * splits;
+    int grid, n_whole;
+    if (splits == 1) {
+      grid = tiles < sms ? tiles : sms;
+      n_whole = tiles;
+    } else {
+      const int rest = tiles % full;
+      if (rest == 0 || rest > full / splits) continue;
+      n_whole = tiles - rest;
+      grid = n_whole > 0 ? full : rest * splits;
+    }
+    const fb::TileWalk w{tiles, kb, n_whole, splits, grid};
+    std::vector<int> blocks(tiles, 0);
+    std::vector<unsigned> ticket(tiles / tiles_n, 0), merged(tiles / tiles_n, 0);
+    auto draw = [&](int tile) {
+      const bool last = ticket[tile / tiles_n]++ == (unsigned)tiles_n - 1;
+      if (last) { ticket[tile / tiles_n] = 0; ++merged[tile / tiles_n]; }
+    };
+    const bool stops = round % 2;
+    for (int c = 0; c < grid; ++c) {
+      fb::TileItem it;
+      int drawn = 0, i = 0;
+      bool stopped = false;
+      for (; w.get(c, c % splits, i, it); ++i) {
+        blocks[it.tile] += it.kb1 - it.kb0;
+        if (it.kb0 >= it.kb1 || it.kb1 > kb || (it.shared && (splits == 1 || w.get(c, c % splits, i + 1, it)))) return 7;
+        if (stops && rng() % 4 == 0) stopped = true;
+        if (stopped) continue;
+        if (!it.shared || c % splits == 0) draw(it.tile);
+        ++drawn;
+      }
+      w.draw_owed(c, c % splits, drawn, draw);
+    }
+    for (int t = 0; t < tiles; ++t)
+      if (blocks[t] != kb) return 8;
+    for (size_t m = 0; m < ticket.size(); ++m)
+      if (ticket[m] != 0 || merged[m] != 1) return 9;
+  }
   puts("ok");
   return 0;
 }
