@@ -205,22 +205,34 @@ int prepare_owned_skinny_ws(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, 
   return 0;
 }
 
-// The calling stream's set of the row scratch; false when the sets belong to other streams (or the stream's handle does
-// not name one stream): the reduction is then composed from its own kernel.  A set stays its stream's for the context's life.
-bool row_scratch(frisk_b200_ctx* ctx, cudaStream_t s, RowEpilogue* out) {
-  if (s == cudaStreamPerThread) return false;
-  std::lock_guard<std::mutex> lock(ctx->row_mu);
-  int i = 0;
-  while (i < ctx->rows_owned && ctx->row_owner[i] != s) ++i;
-  if (i == ctx->rows_owned) {
-    if (i == kRowSets) return false;
-    ctx->row_owner[i] = s;
-    ++ctx->rows_owned;
+// A set of the row scratch for a launch on `s`: the one `s` used last (the stream keeps the two in order), else one whose last
+// use is complete.  -1 where there is none, and under capture, since a graph may be replayed on any stream at any time:
+// the reduction is then composed from its own kernel.  The caller holds row_mu until it has recorded the use.
+int take_row_set(frisk_b200_ctx* ctx, cudaStream_t s) {
+  cudaStreamCaptureStatus capture;
+  unsigned long long id;
+  if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone ||
+      cudaStreamGetId(s, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
   }
-  unsigned char* base = static_cast<unsigned char*>(ctx->row_scratch) + i * kRowSetBytes;
-  out->row_tickets = reinterpret_cast<unsigned*>(base);
-  out->row_partials = reinterpret_cast<float*>(base + kRowTicketBytes);
-  return true;
+  for (int i = 0; i < kRowSets; ++i)
+    if (ctx->row_sets[i].used && ctx->row_sets[i].stream == id) return i;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // a query must not disturb another thread's capture
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  int idle = -1;
+  for (int i = 0; i < kRowSets && idle < 0; ++i) {
+    if (!ctx->row_sets[i].used || cudaEventQuery(ctx->row_sets[i].done) == cudaSuccess)
+      idle = i;
+    else
+      cudaGetLastError();  // (cudaErrorNotReady: in use)
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (idle >= 0) {
+    ctx->row_sets[idle].used = true;
+    ctx->row_sets[idle].stream = id;
+  }
+  return idle;
 }
 
 // A C the TMA unit cannot address (base or rows off 16 bytes) always goes to the one-CTA kernel, whose warps write whole
@@ -295,6 +307,8 @@ int frisk_b200_ctx_create(frisk_b200_ctx** out, int device) {
   if ((e = cudaStreamCreateWithFlags(&ctx->out_stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
   for (auto& ev : ctx->ev)
     if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return fail(e);
+  for (auto& set : ctx->row_sets)
+    if ((e = cudaEventCreateWithFlags(&set.done, cudaEventDisableTiming)) != cudaSuccess) return fail(e);
   *out = ctx;
   return 0;
 }
@@ -311,6 +325,8 @@ int frisk_b200_ctx_destroy(frisk_b200_ctx* ctx) {
   if (ctx->h_status) cudaFreeHost(ctx->h_status);
   for (auto& ev : ctx->ev)
     if (ev) cudaEventDestroy(ev);
+  for (auto& set : ctx->row_sets)
+    if (set.done) cudaEventDestroy(set.done);
   if (ctx->host_stream) cudaStreamDestroy(ctx->host_stream);
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   if (ctx->out_stream) cudaStreamDestroy(ctx->out_stream);
@@ -714,8 +730,19 @@ int frisk_b200_gemm_fused(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* d, co
     re.reduce_kind = e->reduce_kind;
     re.reduce_clear = e->reduce_clear;
     re.reduce_dst = e->reduce_dst;
-    if (e->reduce_kind == FRISK_B200_REDUCE_NONE || (tcgen05_row_epilogue_fits(*d) && row_scratch(ctx, s, &re)))
-      return launch_gemm_tcgen05(ctx, *d, A, B, C, s, &re);
+    if (e->reduce_kind == FRISK_B200_REDUCE_NONE) return launch_gemm_tcgen05(ctx, *d, A, B, C, s, &re);
+    if (tcgen05_row_epilogue_fits(*d)) {
+      std::lock_guard<std::mutex> lock(ctx->row_mu);
+      const int set = take_row_set(ctx, s);
+      if (set >= 0) {
+        unsigned char* base = static_cast<unsigned char*>(ctx->row_scratch) + set * kRowSetBytes;
+        re.row_tickets = reinterpret_cast<unsigned*>(base);
+        re.row_partials = reinterpret_cast<float*>(base + kRowTicketBytes);
+        const int rc = launch_gemm_tcgen05(ctx, *d, A, B, C, s, &re);
+        FB_CUDA(ctx, cudaEventRecord(ctx->row_sets[set].done, s));
+        return rc;
+      }
+    }
   }
   if (fused == 0) {
     int rc = 0;

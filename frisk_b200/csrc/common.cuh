@@ -53,6 +53,11 @@ constexpr int kRowTickets = 16384;
 constexpr size_t kRowTicketBytes = (size_t)kRowTickets * 4;
 constexpr size_t kRowPartialBytes = (size_t)4 << 20;
 constexpr size_t kRowSetBytes = kRowTicketBytes + kRowPartialBytes;
+struct RowSet {
+  bool used = false;
+  unsigned long long stream = 0;  // id of the stream that used it last (a handle can come again, an id cannot)
+  cudaEvent_t done = nullptr;     // behind that use
+};
 
 // Per-kernel set-up that has to happen once per device (opting in to large dynamic shared
 // memory, an occupancy query): `run` returns 0 on success, and then never runs again for
@@ -113,11 +118,10 @@ struct frisk_b200_ctx {
   // Scratch of fixed size, made with the context, so that a call that needs it never allocates; the tickets at its
   // start are zero between launches.  attn: decode attention
   void* attn_scratch = nullptr;
-  // fused row reductions of the one-CTA GEMM: one set (tickets, row partials) per stream, for the first kRowSets streams
-  // the context is called on, so that calls on different streams do not meet in it
+  // fused row reductions of the one-CTA GEMM: sets of tickets and row partials, each in the use of one stream at a time
+  // (take_row_set in api.cu), so that calls on different streams do not meet in one
   void* row_scratch = nullptr;
-  cudaStream_t row_owner[fb::kRowSets] = {};
-  int rows_owned = 0;
+  fb::RowSet row_sets[fb::kRowSets];
   std::mutex row_mu;
   cudaStream_t host_stream = nullptr;
   cudaStream_t copy_stream = nullptr;

@@ -761,24 +761,75 @@ def test_fused_on_the_one_cta_kernel(ctx, M, N, K, dtype, out, kind):
         check_reduce(c, r, out, kind, clear, r0)
 
 
-def test_fused_reduction_on_more_streams_than_scratch_sets(ctx):
-    """Every stream gets the same bits, whether it owns a set of the reduction's scratch or is served by the composed form."""
+def _fused_max_problem(M, N, K, seed):
     import torch
-    M, N, K = 300, 520, 256
-    g = torch.Generator(device="cuda").manual_seed(3)
+    g = torch.Generator(device="cuda").manual_seed(seed)
     a, b = (torch.randn(x, K, generator=g, device="cuda").half() for x in (M, N))
+    return capi.gemm_desc(M, N, K, "fp16", "fp16", False, True), a, b, (a.float() @ b.float().T).half()
+
+
+def _fused_max(ctx, problem, stream):
+    import torch
+    desc, a, b, _ = problem
+    c, r = torch.empty(desc.M, desc.N, dtype=torch.half, device="cuda"), torch.empty(desc.M, dtype=torch.half, device="cuda")
+    epi = capi.gemm_epilogue(reduce="max", reduce_dst=r.data_ptr())
+    ctx.gemm_fused(desc, epi, a.data_ptr(), b.data_ptr(), c.data_ptr(), stream=stream)
+    return c, r
+
+
+# row blocks with 1 to 9 column tiles, so that tickets of one call would not do for another
+FUSED_SHAPES = [(300, 520, 2048), (300, 1100, 1024), (200, 130, 2048), (700, 260, 1024)]
+
+
+def test_fused_reductions_overlapping_on_many_streams(ctx):
+    """Calls in flight on more streams than there are sets of scratch, on streams that come and go (a handle comes again, work of
+    the destroyed stream still running): every call reduces its own C."""
+    import ctypes
+
+    import torch
+    cuda = ctypes.CDLL("libcuda.so.1")
+    problems = [_fused_max_problem(*shape, seed=i) for i, shape in enumerate(FUSED_SHAPES)]
+    pool = [torch.cuda.Stream() for _ in range(6)]
     results = []
     torch.cuda.synchronize()
-    for _ in range(6):
-        st = torch.cuda.Stream()
-        c, r = torch.empty(M, N, dtype=torch.half, device="cuda"), torch.empty(M, dtype=torch.half, device="cuda")
-        epi = capi.gemm_epilogue(reduce="max", reduce_dst=r.data_ptr())
-        ctx.gemm_fused(capi.gemm_desc(M, N, K, "fp16", "fp16", False, True), epi, a.data_ptr(), b.data_ptr(), c.data_ptr(),
-                       stream=st.cuda_stream)
-        ctx.check(st.cuda_stream)
-        results.append((c, r))
-    for c, r in results:
-        assert torch.equal(c, results[0][0]) and torch.equal(r, c.amax(1))
+    for i in range(160):
+        problem = problems[i % len(problems)]
+        if i % 2:
+            results.append((problem, *_fused_max(ctx, problem, pool[i // 2 % len(pool)].cuda_stream)))
+            continue
+        handle = ctypes.c_void_p()
+        assert cuda.cuStreamCreate(ctypes.byref(handle), 1) == 0
+        results.append((problem, *_fused_max(ctx, problem, handle.value)))
+        assert cuda.cuStreamDestroy_v2(handle) == 0
+    torch.cuda.synchronize()
+    ctx.check(torch.cuda.current_stream().cuda_stream)
+    for (_, _, _, ref), c, r in results:
+        assert (c.float() - ref.float()).norm() <= 1e-3 * ref.float().norm() and torch.equal(r, c.amax(1))
+
+
+def test_fused_reduction_captured_and_replayed_beside_other_calls(ctx):
+    """A graph may be replayed on another stream than it was captured on, while that one goes on."""
+    import torch
+    problems = [_fused_max_problem(*shape, seed=i) for i, shape in enumerate(FUSED_SHAPES)]
+    home, other = torch.cuda.Stream(), torch.cuda.Stream()
+    _fused_max(ctx, problems[0], home.cuda_stream)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=home):
+        captured = [_fused_max(ctx, p, home.cuda_stream) for p in problems]
+    for _, r in captured:
+        r.zero_()
+    torch.cuda.synchronize()
+    live = []
+    for i in range(20):
+        with torch.cuda.stream(other):
+            graph.replay()
+        live.append(_fused_max(ctx, problems[i % len(problems)], home.cuda_stream))
+    torch.cuda.synchronize()
+    for c, r in captured + live:
+        assert torch.equal(r, c.amax(1))
+    for (c, _), (_, _, _, ref) in zip(captured, problems):
+        assert (c.float() - ref.float()).norm() <= 1e-3 * ref.float().norm()
 
 
 def test_fused_fill_replaces_the_read_of_c(ctx):
