@@ -660,7 +660,7 @@ def secondary(ctx, torch, stream, peaks, args, sampler, headline_sets, headline_
             err = rel_frobenius(c.double().cpu().numpy(), a.double().cpu().numpy() @ b.double().cpu().numpy())
             res[key] = {"ms": round(ms, 5), "tflops": round(2.0 * M ** 3 / ms / 1e9, 2),
                         "algo": {capi.ALGO_F32_SPLIT: "split_bf16x6_tcgen05", capi.ALGO_SIMT_F32: "cuda_cores"}[
-                            capi.load().frisk_b200_gemm_select(desc)],
+                            ctx.gemm_plan(desc, c.data_ptr()).algo],
                         "frac_of_nominal_fp32_simt": round(2.0 * M ** 3 / ms / 1e9 / 80.0, 4),
                         "err": float(f"{err:.3e}"), "checked": err <= 1e-3}
             del sets

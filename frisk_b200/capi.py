@@ -28,6 +28,7 @@ EXPORTS = (
     "frisk_b200_gemm_skinny_static", "frisk_b200_gemm_push", "frisk_b200_sum_slots",
     "frisk_b200_peer_buffer_create", "frisk_b200_peer_buffer_open", "frisk_b200_peer_buffer_close",
     "frisk_b200_gemm_fused_select", "frisk_b200_gemm_fused_workspace_bytes", "frisk_b200_gemm_fused",
+    "frisk_b200_gemm_plan",
 )
 
 
@@ -42,6 +43,12 @@ class GemmDesc(ctypes.Structure):
 class GemmEpilogue(ctypes.Structure):
     _fields_ = [("fill_enable", ctypes.c_int32), ("fill_value", ctypes.c_float), ("reduce_kind", ctypes.c_int32),
                 ("reduce_clear", ctypes.c_int32), ("reduce_dst", ctypes.c_void_p)]
+
+
+class GemmPlanInfo(ctypes.Structure):
+    _fields_ = [("algo", ctypes.c_int32), ("tile_n", ctypes.c_int32), ("splits", ctypes.c_int32), ("ctas", ctypes.c_int32),
+                ("tiles", ctypes.c_int64), ("whole_tiles", ctypes.c_int64),
+                ("clocks", ctypes.c_double), ("pair_clocks", ctypes.c_double)]
 
 
 REDUCE_KIND = {None: 0, "max": 1, "min": 2, "add": 3}
@@ -113,6 +120,7 @@ def load():
         "frisk_b200_gemm_fused_select": (ctypes.c_int, [gd, ge]),
         "frisk_b200_gemm_fused_workspace_bytes": (sz, [gd, ge]),
         "frisk_b200_gemm_fused": (ctypes.c_int, [vp, gd, ge, vp, vp, vp, vp, sz, vp]),
+        "frisk_b200_gemm_plan": (ctypes.c_int, [vp, gd, vp, ctypes.POINTER(GemmPlanInfo)]),
     }
     for name, (res, args) in sig.items():
         fn = getattr(lib, name)
@@ -188,6 +196,12 @@ class Context:
         rc = load().frisk_b200_gemm_fused(self.handle, ctypes.byref(desc), ctypes.byref(epi), a_ptr, b_ptr, c_ptr,
                                           ws_ptr, ws_bytes, stream)
         raise_for(rc, self._h)
+
+    def gemm_plan(self, desc, c_ptr):
+        """What ``gemm`` runs for this descriptor and C (``GemmPlanInfo``); launches nothing."""
+        info = GemmPlanInfo()
+        raise_for(load().frisk_b200_gemm_plan(self.handle, ctypes.byref(desc), c_ptr, ctypes.byref(info)), self._h)
+        return info
 
     def gemm_host(self, desc, a_ptr, b_ptr, c_ptr):
         raise_for(load().frisk_b200_gemm_host(self.handle, ctypes.byref(desc), a_ptr, b_ptr, c_ptr), self._h)

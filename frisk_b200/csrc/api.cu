@@ -242,6 +242,16 @@ bool one_cta_preferred(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const
   return tcgen05_clocks(ctx, d) < tcgen05_2cta_clocks(d);
 }
 
+// What a gemm into C runs.  `selected` is frisk_b200_gemm_select's answer: a call that names its kernel runs that, an AUTO call
+// the one of the same element type that is estimated the faster on this device.
+int launched_algo(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, int selected, const void* C) {
+  if (d.algo != FRISK_B200_ALGO_AUTO) return selected;
+  if (selected == FRISK_B200_ALGO_TCGEN05 || selected == FRISK_B200_ALGO_TCGEN05_PAIR)
+    return one_cta_preferred(ctx, d, C) ? FRISK_B200_ALGO_TCGEN05 : FRISK_B200_ALGO_TCGEN05_PAIR;
+  if (d.dtype_ab == FRISK_B200_F32) return f32_split_beats_simt(d) ? FRISK_B200_ALGO_F32_SPLIT : FRISK_B200_ALGO_SIMT_F32;
+  return selected;
+}
+
 }  // namespace
 }  // namespace fb
 
@@ -438,12 +448,7 @@ int frisk_b200_gemm(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* d, const vo
   if (ranges_overlap(C, e.c, A, e.a) || ranges_overlap(C, e.c, B, e.b)) return FRISK_B200_E_OVERLAP;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   FB_DEVICE(ctx);
-  // (what an AUTO call runs; a call that names its kernel runs that)
-  if (d->algo == FRISK_B200_ALGO_AUTO && (algo == FRISK_B200_ALGO_TCGEN05 || algo == FRISK_B200_ALGO_TCGEN05_PAIR))
-    algo = one_cta_preferred(ctx, *d, C) ? FRISK_B200_ALGO_TCGEN05 : FRISK_B200_ALGO_TCGEN05_PAIR;
-  if (d->algo == FRISK_B200_ALGO_AUTO && d->dtype_ab == FRISK_B200_F32)
-    algo = f32_split_beats_simt(*d) ? FRISK_B200_ALGO_F32_SPLIT : FRISK_B200_ALGO_SIMT_F32;
-  switch (algo) {
+  switch (algo = launched_algo(ctx, *d, algo, C)) {
     case FRISK_B200_ALGO_SIMT_F32:
       return launch_gemm_simt_f32(ctx, *d, static_cast<const float*>(A), static_cast<const float*>(B),
                                   static_cast<float*>(C), s);
@@ -481,6 +486,20 @@ int frisk_b200_gemm(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* d, const vo
   return FRISK_B200_E_UNSUPPORTED;
 }
 
+int frisk_b200_gemm_plan(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* d, const void* C, frisk_b200_gemm_plan_info* out) {
+  if (!ctx || !d || !out) return FRISK_B200_E_ARG;
+  const int algo = frisk_b200_gemm_select(d);
+  if (algo < 0) return algo;
+  FB_DEVICE(ctx);
+  *out = frisk_b200_gemm_plan_info{};
+  out->algo = launched_algo(ctx, *d, algo, C);
+  if (out->algo == FRISK_B200_ALGO_TCGEN05 || out->algo == FRISK_B200_ALGO_TCGEN05_PAIR) {
+    tcgen05_describe(ctx, *d, out);
+    out->pair_clocks = tcgen05_2cta_clocks(*d);
+  }
+  return 0;
+}
+
 int frisk_b200_gemm_host(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* d, const void* A, const void* B,
                          void* C) {
   if (!ctx || !d || !A || !B || !C) return FRISK_B200_E_ARG;
@@ -494,6 +513,7 @@ int frisk_b200_gemm_host(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* d, con
   if ((rc = ensure_stage(ctx, 1, e.b, false))) return rc;
   if ((rc = ensure_stage(ctx, 2, e.c, false))) return rc;
   cudaStream_t s = ctx->host_stream, s2 = ctx->copy_stream, s3 = ctx->out_stream;
+  algo = launched_algo(ctx, *d, algo, ctx->stage[2].ptr);
   if (algo == FRISK_B200_ALGO_SKINNY && (rc = prepare_owned_skinny_ws(ctx, *d, s))) return rc;
   if (size_t need = (algo == FRISK_B200_ALGO_TCGEN05_PAIR ? tcgen05_2cta_workspace_bytes(*d) : 0))
     if ((rc = ensure_stage(ctx, 5, need, true, s))) return rc;
@@ -721,9 +741,8 @@ int frisk_b200_gemm_fused(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* d, co
   FB_DEVICE(ctx);
   const bool use_fill = e->fill_enable && !d->clear_accum;  // a fill before an overwriting gemm is dead
   const float fill = round_fill(e->fill_value, d->dtype_c);
-  const int algo = frisk_b200_gemm_select(d);
-  if (d->algo == FRISK_B200_ALGO_AUTO && !workspace && (algo == FRISK_B200_ALGO_TCGEN05 || algo == FRISK_B200_ALGO_TCGEN05_PAIR) &&
-      one_cta_preferred(ctx, *d, C)) {
+  if (d->algo == FRISK_B200_ALGO_AUTO && !workspace &&
+      launched_algo(ctx, *d, frisk_b200_gemm_select(d), C) == FRISK_B200_ALGO_TCGEN05) {
     RowEpilogue re{};
     re.has_fill = use_fill ? 1 : 0;
     re.fill = fill;

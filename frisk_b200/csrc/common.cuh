@@ -248,6 +248,7 @@ int launch_gemm_tcgen05(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, cons
 // clocks the two kernels are estimated at, for the choice between them
 double tcgen05_clocks(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d);
 double tcgen05_2cta_clocks(const frisk_b200_gemm_desc& d);
+void tcgen05_describe(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, frisk_b200_gemm_plan_info* out);
 bool tcgen05_row_epilogue_fits(const frisk_b200_gemm_desc& d);
 
 // Row blocks of the fp32 product are stored into up to 8 destination buffers instead of C:

@@ -714,6 +714,17 @@ bool tcgen05_supported(const frisk_b200_gemm_desc& d) {
 // clocks the plan is estimated at (frisk_b200_gemm weighs it against the pair kernel)
 double tcgen05_clocks(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d) { return plan_for(ctx, d).clocks; }
 
+void tcgen05_describe(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, frisk_b200_gemm_plan_info* out) {
+  const Plan p = plan_for(ctx, d);
+  const GemmDims g = resolve_dims(d);
+  out->tile_n = p.bn;
+  out->splits = p.splits;
+  out->ctas = p.grid;
+  out->tiles = ((g.M + BM - 1) / BM) * ((g.N + p.bn - 1) / p.bn);
+  out->whole_tiles = p.n_whole;
+  out->clocks = p.clocks;
+}
+
 // the row reduction keeps one fp32 per (box of columns, row) and one ticket per row block
 bool tcgen05_row_epilogue_fits(const frisk_b200_gemm_desc& d) {
   const GemmDims g = resolve_dims(d);

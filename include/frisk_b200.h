@@ -143,6 +143,17 @@ int frisk_b200_gemm_check_memrefs(int32_t a_rank, const int64_t* a_shape, int32_
  * layout and extents alone; the launch, which also knows the device and C's address, may run the other kernel of the
  * same element type. */
 int frisk_b200_gemm_select(const frisk_b200_gemm_desc* desc);
+/* What frisk_b200_gemm (and frisk_b200_gemm_host) runs for this descriptor, this C and this context's device: `algo` is
+ * the kernel.  For the tcgen05 kernels of 16-bit operands the rest describes the one-CTA kernel's plan (128 x tile_n tiles,
+ * the first whole_tiles of them walked whole, each of the others shared by a cluster of `splits` of the `ctas` CTAs) and
+ * the two estimates the choice between the kernels goes by, in clocks beyond the launch.  Launches nothing. */
+typedef struct frisk_b200_gemm_plan_info {
+  int32_t algo, tile_n, splits, ctas;
+  int64_t tiles, whole_tiles;
+  double clocks, pair_clocks;
+} frisk_b200_gemm_plan_info;
+int frisk_b200_gemm_plan(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* desc, const void* C,
+                         frisk_b200_gemm_plan_info* out);
 /* Bytes of caller-provided, ZERO-INITIALISED scratch this descriptor needs (0 = none).
  * The kernels leave their control words zero again, so one memset at allocation suffices
  * for repeated launches of the SAME descriptor; a scratch buffer that is reused with
@@ -221,11 +232,13 @@ int frisk_b200_gemm_push(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* desc, 
  * (a fill before a gemm that overwrites C is dead: clear_accum wins)
  *     reduce_dst[i] <- (reduce_clear ? identity : reduce_dst[i]) (+) reduce_j C[i][j]
  * with the reduction taken over the values of C as stored (rounded to its element type) and
- * accumulated in fp32.  On the tcgen05 pair kernel both happen in the GEMM's epilogue (C is
- * not read for the fill; the reduction costs one fp32 per row and 256 columns, combined in a
- * fixed order); for the other kernels, and for a reduction after an accumulate that reads C,
- * the same result is produced by a fill kernel before and a row-reduction kernel after the
- * GEMM.  Kind `mul` of the reference has no kernel here (FRISK_B200_E_UNSUPPORTED). */
+ * accumulated in fp32.  On the tcgen05 kernels both happen in the GEMM's epilogue (C is
+ * not read for the fill; the reduction costs one fp32 per row and 256 columns, or 128 bytes of
+ * columns, combined in a fixed order): on the pair kernel unless the reduction follows an
+ * accumulate that reads C, on the one-CTA kernel for AUTO calls without a workspace outside
+ * stream capture, while one of the context's sets of scratch is free.  Otherwise, and for
+ * the other kernels, a fill kernel before and a row-reduction kernel after the GEMM produce
+ * the same result.  Kind `mul` of the reference has no kernel here (FRISK_B200_E_UNSUPPORTED). */
 enum {
   FRISK_B200_REDUCE_NONE = 0,
   FRISK_B200_REDUCE_MAX = 1,
@@ -239,12 +252,13 @@ typedef struct frisk_b200_gemm_epilogue {
   int32_t reduce_clear; /* 1: overwrite reduce_dst; 0: combine with what it holds */
   void* reduce_dst;     /* M elements of C's element type; may be NULL when reduce_kind is NONE */
 } frisk_b200_gemm_epilogue;
-/* 1 when the descriptor/epilogue pair runs fused in the GEMM epilogue, 0 when it is composed
- * from separate kernels, negative error code otherwise.  Host-only. */
+/* 1 when the descriptor/epilogue pair runs fused in the PAIR kernel's epilogue where that kernel runs, 0 when
+ * it is composed from separate kernels there, negative error code otherwise.  Host-only. */
 int frisk_b200_gemm_fused_select(const frisk_b200_gemm_desc* desc, const frisk_b200_gemm_epilogue* epi);
 size_t frisk_b200_gemm_fused_workspace_bytes(const frisk_b200_gemm_desc* desc,
                                              const frisk_b200_gemm_epilogue* epi);
-/* workspace may be NULL: the context then owns the scratch (allocated on first use). */
+/* workspace may be NULL: the context then owns the scratch (the pair kernel's is allocated on first use).  A
+ * caller's workspace serves the pair kernel; such a call does not use the one-CTA kernel's fused form. */
 int frisk_b200_gemm_fused(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* desc,
                           const frisk_b200_gemm_epilogue* epi, const void* A, const void* B, void* C,
                           void* workspace, size_t workspace_bytes, void* stream);

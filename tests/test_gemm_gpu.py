@@ -531,6 +531,21 @@ def test_gemm_host_entry_short_last_panel_and_explicit_algo(ctx):
         assert np.isfinite(c).all() and rel_frobenius(c, ref) <= TOL["fp16"], algo
 
 
+@pytest.mark.parametrize("M,N,K,dtype,ta,tb", [
+    (515, 771, 1003, "fp32", True, True),     # tensor cores, though no extent is a multiple of 8
+    (64, 1024, 4096, "bf16", False, True),    # K shared by clusters of the one-CTA kernel
+    (300, 1003, 512, "fp16", False, True),    # a C the pair kernel would write element by element
+    (520, 2560, 1024, "fp16", False, True),
+])
+def test_gemm_host_runs_the_kernel_that_gemm_runs(ctx, M, N, K, dtype, ta, tb):
+    """One AUTO for both entries: the same bits."""
+    a, b = inputs.gemm_inputs(M, N, K, dtype, ta, tb, 46, "uniform" if dtype == "fp32" else "normal_rsqrt_k")
+    c = np.zeros((M, N), a.dtype)
+    ctx.gemm_host(capi.gemm_desc(M, N, K, dtype, dtype, ta, tb), a.ctypes.data, b.ctypes.data, c.ctypes.data)
+    device, ok = run_gemm(ctx, a, b, dtype, dtype, M, N, K, ta, tb)
+    assert ok and np.array_equal(c.view(np.uint8), device.view(np.uint8))
+
+
 def test_contract_errors_before_launch(ctx):
     import torch
     a = torch.zeros(128, 64, dtype=torch.float16, device="cuda")  # room for a shifted 64x64 view
