@@ -66,7 +66,7 @@ def test_f32_config_1024(ctx, algo):
     spec = inputs.WORKLOADS["gemm_f32_1024"]
     err = check(ctx, spec["M"], spec["N"], spec["K"], "fp32", "fp32", False, False, spec["seed"], algo=algo)
     assert err < 1e-5  # fp32 accumulation of 1024 terms is far inside the 1e-3 budget
-    # the tensor-core path adds nine exact-product GEMMs of a three-term bf16 split: fp32-GEMM accuracy
+    # the tensor-core path adds six exact-product GEMMs of a three-term bf16 split: fp32-GEMM accuracy
     assert err < 2e-6 or algo == capi.ALGO_SIMT_F32, err
 
 
@@ -304,11 +304,29 @@ def test_tc_many_tiles_persistent(ctx, algo):
 
 
 @pytest.mark.parametrize("tb", [True, False])
-def test_tc_tail_wave_of_half_tiles(ctx, tb):
-    # 16 x 10 = 160 tiles on 148 SMs: the 12 tiles of the last wave run as 24 half-width items
+def test_tc_more_tiles_than_ctas(ctx, tb):
+    # a little over one and two rounds of whole tiles, too little K to share the rest; ragged N
     check(ctx, 2048, 2560, 192, "bf16", "bf16", False, tb, 29, algo=capi.ALGO_TCGEN05, dist="normal_rsqrt_k")
-    # ragged N: the second half of the last tile column lies wholly outside the matrix
     check(ctx, 2048, 2400, 64, "fp16", "fp32", False, tb, 30, algo=capi.ALGO_TCGEN05, dist="normal_rsqrt_k")
+
+
+@pytest.mark.parametrize("M,N,K,dtype,out", [
+    (2048, 2560, 1024, "bf16", "bf16"),  # one round of 128 x 256 tiles, then 28 shared ones
+    (2048, 2560, 1024, "fp16", "fp32"),
+    (3920, 1472, 840, "bf16", "bf16"),   # ragged rows and columns
+    (2048, 2561, 2048, "fp16", "fp16"),  # two rounds of 128 x 128 tiles, a C off 16 bytes
+    (2048, 2561, 2048, "bf16", "fp32"),
+])
+def test_tc_whole_rounds_then_shared_tiles(ctx, M, N, K, dtype, out):
+    """A CTA of the one-CTA kernel walks whole tiles and then joins a cluster that shares the K of one of the rest (or has
+    none and takes part in the cluster's meetings only): ring, accumulators and boxes go on from one to the other."""
+    desc = capi.gemm_desc(M, N, K, dtype, out, False, True, algo=capi.ALGO_TCGEN05)
+    plan = ctx.gemm_plan(desc, 4096)
+    assert plan.algo == capi.ALGO_TCGEN05 and plan.splits > 1 and plan.ctas <= plan.whole_tiles < plan.tiles
+    assert (plan.tiles - plan.whole_tiles) * plan.splits <= plan.ctas
+    for accumulate in (False, True):
+        check(ctx, M, N, K, dtype, out, False, True, 40 + accumulate, accumulate=accumulate, algo=capi.ALGO_TCGEN05,
+              dist="normal_rsqrt_k")
 
 
 @pytest.mark.parametrize("algo", [capi.ALGO_TCGEN05, capi.ALGO_TCGEN05_PAIR])
@@ -328,10 +346,10 @@ def test_tc_pair_few_tiles_all_split_in_k(ctx, tb):
     meet through the fp32 scratch (ragged edges, fp32 and 16-bit outputs, accumulate, repeat on the same scratch)."""
     P = capi.ALGO_TCGEN05_PAIR
     for _ in range(2):
-        check(ctx, 1024, 2048, 4096, "fp16", "fp16", False, tb, 61, algo=capi.ALGO_AUTO, dist="normal_rsqrt_k")
+        check(ctx, 1024, 2048, 4096, "fp16", "fp16", False, tb, 61, algo=P, dist="normal_rsqrt_k")
     check(ctx, 1000, 1800, 2048, "bf16", "fp32", False, tb, 62, algo=P, dist="normal_rsqrt_k")
     check(ctx, 520, 304, 1024, "bf16", "bf16", False, tb, 63, accumulate=True, algo=P, dist="normal_rsqrt_k")
-    check(ctx, 256, 256, 8192, "fp16", "fp16", False, tb, 64, algo=capi.ALGO_AUTO, dist="normal_rsqrt_k")
+    check(ctx, 256, 256, 8192, "fp16", "fp16", False, tb, 64, algo=P, dist="normal_rsqrt_k")
 
 
 @pytest.mark.parametrize("tb", [True, False])
@@ -705,11 +723,12 @@ def test_splitk_push_two_gpus(tmp_path):
 def test_one_cta_plans(ctx, M, N, K, dtype, out):
     """Whole tiles and tiles whose K a cluster shares, every layout, overwriting and accumulating, a C that goes through
     TMA and one that does not (rows or base off 16 bytes)."""
+    A = capi.ALGO_TCGEN05
     for ta, tb in ((False, False), (False, True), (True, False), (True, True)):
         m, n = (M + 7 & ~7 if ta else M), (N if tb else N + 7 & ~7)
-        check(ctx, m, n, K, dtype, out, ta, tb, 31, accumulate=ta != tb)
+        check(ctx, m, n, K, dtype, out, ta, tb, 31, accumulate=ta != tb, algo=A)
         if tb:
-            check(ctx, m, n + 1, K, dtype, out, ta, tb, 32, accumulate=not ta)
+            check(ctx, m, n + 1, K, dtype, out, ta, tb, 32, accumulate=not ta, algo=A)
 
 
 # ------------------------------------------------------------------ fill / row-reduce next to the gemm
@@ -757,19 +776,32 @@ def check_reduce(got_c, got_r, dtype_c, kind, clear, r_init):
 def test_fused_row_reduce_in_pair_epilogue(ctx, kind, dtype_c):
     # 9 x 10 tiles on 74 pairs: whole tiles and a K-split tail wave; ragged N masks the last columns
     for N, clear in ((2560, True), (2496, False)):
-        c, r, ref, r0 = run_fused(ctx, 2304, N, 512, "fp16", dtype_c, 70, kind=kind, clear=clear, expect_fused=1)
+        c, r, ref, r0 = run_fused(ctx, 2304, N, 512, "fp16", dtype_c, 70, kind=kind, clear=clear, expect_fused=1,
+                                  algo=capi.ALGO_TCGEN05_PAIR)
         assert rel_frobenius(from_storage(c, dtype_c), ref) <= TOL["fp16"]
         check_reduce(c, r, dtype_c, kind, clear, r0)
 
 
-@pytest.mark.parametrize("M,N,K,dtype,out,kind", [
-    (130, 264, 200, "fp16", "fp16", "max"),    # a cluster shares K, ragged rows and columns
-    (513, 390, 72, "bf16", "fp32", "add"),     # whole tiles, C with rows that are not 16-byte multiples
-    (3000, 2056, 136, "bf16", "bf16", "min"),  # several tiles per CTA
-    (100, 65, 4096, "fp16", "fp16", "add"),    # eight CTAs per tile, one column beyond a box
+@pytest.mark.parametrize("M,N,K,dtype,out,kind,plan", [
+    (130, 264, 200, "fp16", "fp16", "max", "whole"),     # ragged rows and columns
+    (513, 390, 72, "bf16", "fp32", "add", "whole"),      # C with rows that are not 16-byte multiples
+    (100, 65, 4096, "fp16", "fp16", "add", "shared"),    # eight CTAs per tile, one column beyond a box
+    (200, 520, 2048, "bf16", "bf16", "max", "shared"),   # the same, five column tiles
+    (200, 520, 2048, "bf16", "fp32", "min", "shared"),
+    (2300, 2569, 136, "fp16", "fp16", "max", "rounds"),  # several whole tiles per CTA
+    (2300, 2569, 136, "bf16", "fp32", "add", "rounds"),
+    (2048, 2561, 2048, "fp16", "fp16", "min", "both"),   # whole rounds, then shared tiles of the same row blocks
+    (2048, 2561, 2048, "bf16", "fp32", "max", "both"),
+    (3000, 2056, 136, "bf16", "bf16", "min", "pair"),    # (and a size the choice leaves to the pair kernel)
 ])
-def test_fused_on_the_one_cta_kernel(ctx, M, N, K, dtype, out, kind):
+def test_fused_on_the_one_cta_kernel(ctx, M, N, K, dtype, out, kind, plan):
     """Fill and row reduction folded into the one-CTA kernel (twice: its tickets are left clean)."""
+    p = ctx.gemm_plan(capi.gemm_desc(M, N, K, dtype, out, False, True), 4096)
+    assert (p.algo == capi.ALGO_TCGEN05_PAIR) == (plan == "pair")
+    if plan != "pair":
+        shared = p.tiles - p.whole_tiles
+        assert plan == ("both" if shared and p.whole_tiles else "shared" if shared else
+                        "rounds" if p.tiles > p.ctas else "whole")
     for fill, clear in ((0.25, True), (-1.5, False)):
         c, r, ref, r0 = run_fused(ctx, M, N, K, dtype, out, 81, fill=fill, kind=kind, clear_accum=False, clear=clear)
         assert rel_frobenius(from_storage(c, out), ref) <= TOL[dtype]
@@ -847,18 +879,23 @@ def test_fused_reduction_captured_and_replayed_beside_other_calls(ctx):
         assert (c.float() - ref.float()).norm() <= 1e-3 * ref.float().norm()
 
 
-def test_fused_fill_replaces_the_read_of_c(ctx):
-    # C holds NaN: a fused fill must not read it.  bf16 output, then with a reduction on top.
-    c, _, ref, _ = run_fused(ctx, 2304, 2560, 256, "bf16", "bf16", 71, fill=0.75, clear_accum=False, expect_fused=1)
+@pytest.mark.parametrize("algo", [capi.ALGO_AUTO, capi.ALGO_TCGEN05_PAIR])
+def test_fused_fill_replaces_the_read_of_c(ctx, algo):
+    # C holds NaN: a fused fill must not read it.  bf16 output, then with a reduction on top; fp32 and ragged.
+    c, _, ref, _ = run_fused(ctx, 2304, 2560, 256, "bf16", "bf16", 71, fill=0.75, clear_accum=False, expect_fused=1, algo=algo)
     assert rel_frobenius(from_storage(c, "bf16"), ref) <= TOL["bf16"]
     c, r, ref, r0 = run_fused(ctx, 2304, 2560, 256, "bf16", "bf16", 72, fill=-1.5, kind="max", clear_accum=False,
-                              expect_fused=1)
+                              expect_fused=1, algo=algo)
     assert rel_frobenius(from_storage(c, "bf16"), ref) <= TOL["bf16"]
     check_reduce(c, r, "bf16", "max", True, r0)
+    c, r, ref, r0 = run_fused(ctx, 2311, 2569, 520, "fp16", "fp32", 73, fill=0.25, kind="add", clear_accum=False, clear=False,
+                              expect_fused=1, algo=algo)
+    assert rel_frobenius(from_storage(c, "fp32"), ref) <= TOL["fp16"]
+    check_reduce(c, r, "fp32", "add", False, r0)
 
 
 def test_fill_and_reduce_composed_for_the_other_kernels(ctx):
-    # one-CTA tcgen05 kernel, fp32 SIMT kernel, skinny kernel, and a reduction after an accumulate that reads C
+    # (folded into the one-CTA kernel, see above), fp32 CUDA cores, skinny kernel, and a reduction after an accumulate that reads C
     c, r, ref, r0 = run_fused(ctx, 384, 520, 192, "fp16", "fp16", 73, fill=0.25, kind="add", clear_accum=False,
                               clear=False, expect_fused=0)
     assert rel_frobenius(from_storage(c, "fp16"), ref) <= TOL["fp16"]
