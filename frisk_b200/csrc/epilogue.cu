@@ -9,9 +9,12 @@
 #include <cuda_fp16.h>
 
 #include "common.cuh"
+#include "gemm_common.cuh"
 
 namespace fb {
 namespace {
+using gemm_detail::reduce_combine;
+using gemm_detail::reduce_identity;
 
 __device__ __forceinline__ float to_f(float v) { return v; }
 __device__ __forceinline__ float to_f(__half v) { return __half2float(v); }
@@ -24,13 +27,6 @@ template <>
 __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half_rn(v); }
 template <>
 __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
-
-__device__ __forceinline__ float reduce_identity(int kind) {
-  return kind == FRISK_B200_REDUCE_MAX ? -INFINITY : kind == FRISK_B200_REDUCE_MIN ? INFINITY : 0.f;
-}
-__device__ __forceinline__ float reduce_combine(int kind, float a, float b) {
-  return kind == FRISK_B200_REDUCE_MAX ? fmaxf(a, b) : kind == FRISK_B200_REDUCE_MIN ? fminf(a, b) : a + b;
-}
 
 // dst[row] = (clear ? id : dst[row]) (+) partials[0][row] (+) partials[1][row] ...
 template <typename T>

@@ -59,12 +59,6 @@ struct Smem2 {
 static_assert(Smem2::kTotalOut <= 232448, "the output boxes must fit next to the operand ring");
 
 // ---- cluster / cta_group::2 primitives
-// shared::cluster address of `p` (a shared-memory object of this CTA) in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t mapa_u32(const void* p, uint32_t rank) {
-  uint32_t out;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_u32(p)), "r"(rank));
-  return out;
-}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -219,7 +213,7 @@ __global__ void __launch_bounds__(kThreads2, 1)
           unsigned char* sb = sa + L::kABytes;
           // the leader's barrier collects the bytes of both CTAs
           if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * STAGE);
-          const uint32_t bar = mapa_u32(&full_bar[stage], 0);
+          const uint32_t bar = mapa_addr(smem_u32(&full_bar[stage]), 0);
           const int k0 = kb * BK;
           if (A_MN) {
 #pragma unroll
@@ -310,7 +304,7 @@ __global__ void __launch_bounds__(kThreads2, 1)
     uint32_t box_phases = 0;  // bit b: the phase box b's barrier is in
     int acc = 0;
     uint32_t acc_phase = 0;
-    const uint32_t leader_acc_empty0 = mapa_u32(&acc_empty[0], 0), leader_acc_empty1 = mapa_u32(&acc_empty[1], 0);
+    const uint32_t leader_acc_empty0 = mapa_addr(smem_u32(&acc_empty[0]), 0), leader_acc_empty1 = mapa_addr(smem_u32(&acc_empty[1]), 0);
     uint32_t epi_phase = 0;
     bool epi_ok = true;
     // bounded meeting point of this CTA's 128 epilogue threads
