@@ -106,7 +106,8 @@ typedef struct frisk_b200_attn_desc {
   int32_t dtype_out; /* == dtype_in, or F32              */
   /* 0: single pass, P rounded relative to a running maximum (fast path).
    * 1: the reference's semantics to the letter: two passes over the keys, every probability is
-   *    divided by the COMPLETE row sum (IEEE division) before it is rounded to 16 bits
+   *    divided by the COMPLETE row sum before it is rounded to 16 bits (the IEEE quotient; below 2^-100
+   *    it may be one unit of its last fp32 place off before that rounding)
    *    (tiled_attention.py:697-698, tail_attention_reference.py:74-78); the reference's analytic
    *    fixtures then match bit for bit. */
   int32_t normalize_p;

@@ -277,6 +277,34 @@ def test_normalized_mode_long_sequence(ctx):
     assert np.array_equal(got[0, 0, 0], from_storage(v, "bf16")[0, 0, 0])  # query 0 sees only key 0: P = 1 exactly
 
 
+def test_normalized_mode_tiny_probabilities_bf16(ctx):
+    """bf16 keeps probabilities down to 2^-126: each is the IEEE quotient exp / sum rounded to bf16, read off one by one through a
+    diagonal V (quotients between 2^-126 and 2^-100, where the correction's remainder is not exact; the exponential is the device's own)."""
+    import torch
+    BH, S, D, scale = 512, 64, 64, 0.125
+    g = torch.Generator(device="cuda").manual_seed(8)
+    t = 0.95 + 0.1 * torch.rand(BH, S, generator=g, device="cuda")  # score of key j for query i: -c_i t_j
+    t[:, :3] = 0                                                    # three keys with the maximum: the sum is 3
+    c = 560 + 130 * torch.rand(BH, S, generator=g, device="cuda")
+    q, k, v = (torch.zeros(1, BH, S, D, dtype=torch.bfloat16, device="cuda") for _ in range(3))
+    q[0, :, :, 0], k[0, :, :, 0] = c.bfloat16(), -t.bfloat16()
+    v[0] = torch.eye(S, device="cuda") * 2.0 ** 110
+    o = torch.empty(1, BH, S, D, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    ctx.attention_fwd(capi.attn_desc(1, BH, S, S, D, scale, False, "bf16", "fp32", normalize_p=True), q.data_ptr(), k.data_ptr(),
+                      v.data_ptr(), o.data_ptr(), stream=stream)
+    ctx.check(stream)
+    dot = q[0, :, :, :1].float() * k[0, :, None, :, 0].float()    # exact: 8-bit factors
+    e = torch.exp2((dot * scale) * 1.44269504088896340736)
+    p = (e / 3).bfloat16().double()
+    normal = p >= 2.0 ** -126
+    tiny = normal & (p < 2.0 ** -100)
+    assert tiny.sum() > 200_000
+    got = o[0].double() / 2.0 ** 110
+    wrong = (got != p) & normal
+    assert not wrong.any(), (int(wrong.sum()), int(tiny.sum()), got[wrong][:4], p[wrong][:4])
+
+
 def test_launch_contract_refusals(ctx):
     """The launch validation of benchmark/layout/execution/tiled_execution.py:113-139: an output that
     overlaps an input, or a base address that is not 16-byte aligned, is refused before anything runs."""
