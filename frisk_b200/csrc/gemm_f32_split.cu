@@ -15,9 +15,9 @@
 // (TWO; 22.4 us instead of 21.8 at 1024^3), and below K = 320 the CUDA cores are the more accurate (split_accurate).
 //
 // An element that is not finite, or so large that x 2^24 or a sum overflows, makes the result non-finite.  The 32 x 16
-// piece of C it lies in is not stored but noted, and when a CTA's tiles are done (no wait of the pipeline is open any
-// more, however long K is) all its warps compute the noted pieces as 64-bit sums, rounded once: infinities and NaN come out
-// as IEEE arithmetic gives them, and the finite results of such a piece are no further off than the others.
+// piece of C it lies in is noted, and when a CTA's tiles are done (no wait of the pipeline is open any more, however long
+// K is) all its warps compute such results as plain fp32 sums over k, so infinities and NaN come out as IEEE arithmetic
+// gives them.
 //
 // One CTA per SM, 16 warps with fixed roles (128 registers each, all of the SM's):
 //   warps 0-7   promotion: tensor memory -> fp32 registers (64 columns of one row per thread), stores.  One thread of
@@ -156,14 +156,15 @@ struct Loader {
 };
 
 // The 32 x 16 piece of C at (r0, c0), lane = row: unscaled, added to C or written.  Four lanes write 64 consecutive
-// bytes of a row, through `out` ([32 rows][16 columns] of shared memory).  Returns false, with C as it was, where a result
-// is not finite.
+// bytes of a row, through `out` ([32 rows][16 columns] of shared memory).  Returns false where a result is not finite: the
+// piece then stands in C as it is, or has not been added to C.
 __device__ __forceinline__ bool store_piece(const SplitArgs& p, float (&v)[16], float* out, int r0, int c0, int lane) {
   if (r0 >= p.M || c0 >= p.N) return true;
   bool finite = true;
 #pragma unroll
   for (int i = 0; i < 16; ++i) finite = finite && fabsf(v[i]) <= kFloatMax;
-  if (__any_sync(0xffffffffu, !finite && r0 + lane < p.M)) return false;
+  const bool whole = !__any_sync(0xffffffffu, !finite && r0 + lane < p.M);
+  if (!whole && p.accumulate) return false;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
     *reinterpret_cast<float4*>(out + lane * kOutPitch + 4 * i) =
@@ -200,20 +201,22 @@ __device__ __forceinline__ bool store_piece(const SplitArgs& p, float (&v)[16], 
     }
   }
   __syncwarp();
-  return true;
+  return whole;
 }
 
-// The noted pieces of this CTA's tiles (bit 16 h + w of a tile's word: columns 64h + 16 (w / 4), rows 32 (w % 4)) as
-// 64-bit sums in the order of k, by all 16 warps, one piece of a half tile each; a lane has 4 x 4 results.
-// 4096^3 takes 0.83 ms, with one infinite element 1.75 and with every result above 2^80 11.7 (53 and 451 when the thread
-// that met such a result summed it up on the spot); the 64-bit units bound it.
+// The non-finite results (where C is added to: all) of the noted pieces of this CTA's tiles, bit 16 h + w of a tile's word:
+// columns 64h + 16 (w / 4), rows 32 (w % 4).  Plain fp32 sums by all 16 warps, half a tile at a time, a lane with 4 x 4
+// results of a piece; where few pieces are noted, two or four warps share a block's k and their sums are added in order.
+// 4096^3 takes 0.83 ms, with one infinite element 1.5 and with every result above 2^80 8.4 (53 and 451 when the thread that
+// met such a result summed it up on the spot); 1024^3 24 us, 167 and 232.
 template <bool A_MN, bool B_MN>
 __device__ __noinline__ void redo_pieces(const SplitArgs& p, unsigned char* smem, const uint32_t* noted, int first, int step,
                                          int count) {
-  constexpr int kPitchA = BT + 2, kPitchB = BT / 2 + 2;  // 4 banks from one k to the next
-  static_assert(BK * (kPitchA + kPitchB) * 8 <= kOutOffset, "a block in 64 bits must fit in the stages");
-  double* sa = reinterpret_cast<double*>(smem);          // [64 k][128 rows]
-  double* sb = sa + BK * kPitchA;                        // [64 k][64 columns]
+  constexpr int kPitchA = BT + 4, kPitchB = BT / 2 + 4;  // 4 banks from one k to the next
+  float* sa = reinterpret_cast<float*>(smem);            // [64 k][128 rows]
+  float* sb = sa + BK * kPitchA;                         // [64 k][64 columns]
+  float* sums = sb + BK * kPitchB;                       // [16 warps][16 results][32 lanes]
+  static_assert((BK * (kPitchA + kPitchB) + 16 * 512) * 4 <= kOutOffset, "a block and the sums must fit in the stages");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int t = 0; t < 2 * count; ++t) {
     const uint32_t mask = (noted[t >> 1] >> (16 * (t & 1))) & 0xffffu;
@@ -235,16 +238,14 @@ __device__ __noinline__ void redo_pieces(const SplitArgs& p, unsigned char* smem
 #pragma unroll
       for (int j = 0; j < 8; ++j) pb[j] = element(p.b, B_MN, n0 + row_of(B_MN, BT / 2, j), k0 + k_of(B_MN, BT / 2, j), p.N);
     };
-    double acc[4][4];
+    const int pieces = __popc(mask), sharers = pieces <= 4 ? 4 : pieces <= 8 ? 2 : 1;  // warps of a piece
+    const int slot = warp / sharers, part = warp % sharers;
+    const int piece = slot < pieces ? (int)__fns(mask, 0, slot + 1) : -1;  // the slot-th noted piece
+    const int row = (piece & 3) * 32 + (lane & 7) * 4, col = (piece >> 2) * 16 + (lane >> 3) * 4;
+    const int k_first = part * (BK / sharers), k_last = k_first + BK / sharers;
+    float acc[16];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[r][c] = 0.0;
-    // the pieces of a row block, as those of a column block, are four different schedulers'; rows and columns of a lane come
-    // in pairs, so that the reads of a warp are consecutive
-    const int pm = (warp + (warp >> 2)) & 3, pn = warp >> 2;
-    const int row = pm * 32 + (lane & 7) * 2, col = pn * 16 + (lane >> 3) * 2;
-    const bool mine = (mask >> (pn * 4 + pm)) & 1u;
+    for (int i = 0; i < 16; ++i) acc[i] = 0.f;
     fetch(0);
     for (int kb = 0; kb < p.kb; ++kb) {
       __syncthreads();  // the block before this one has been read
@@ -254,31 +255,37 @@ __device__ __noinline__ void redo_pieces(const SplitArgs& p, unsigned char* smem
       for (int j = 0; j < 8; ++j) sb[k_of(B_MN, BT / 2, j) * kPitchB + row_of(B_MN, BT / 2, j)] = pb[j];
       __syncthreads();
       if (kb + 1 < p.kb) fetch((kb + 1) * BK);
-      if (mine) {
-#pragma unroll 2
-        for (int k = 0; k < BK; ++k) {
-          const double2* a2 = reinterpret_cast<const double2*>(sa + k * kPitchA + row);
-          const double2* b2 = reinterpret_cast<const double2*>(sb + k * kPitchB + col);
-          const double a[4] = {a2[0].x, a2[0].y, a2[8].x, a2[8].y}, b[4] = {b2[0].x, b2[0].y, b2[4].x, b2[4].y};
+      if (piece >= 0) {
+#pragma unroll 4
+        for (int k = k_first; k < k_last; ++k) {
+          const float4 a4 = *reinterpret_cast<const float4*>(sa + k * kPitchA + row);
+          const float4 b4 = *reinterpret_cast<const float4*>(sb + k * kPitchB + col);
+          const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
-          for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+          for (int i = 0; i < 16; ++i) acc[i] = fmaf(a[i >> 2], b[i & 3], acc[i]);
         }
       }
     }
-    if (mine)
+    if (sharers > 1) {
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
+      for (int i = 0; i < 16; ++i) sums[(warp * 16 + i) * 32 + lane] = acc[i];
+      __syncthreads();
+      for (int q = 1; q < sharers; ++q)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int rr = m0 + row + (r >> 1) * 16 + (r & 1), cc = n0 + col + (c >> 1) * 8 + (c & 1);
-          if (rr < p.M && cc < p.N) {
-            float* dst = p.C + (int64_t)rr * p.ldc + cc;
-            const float x = static_cast<float>(acc[r][c]);
-            *dst = p.accumulate ? *dst + x : x;
-          }
-        }
+        for (int i = 0; i < 16; ++i)
+          if (part == 0) acc[i] += sums[((warp + q) * 16 + i) * 32 + lane];
+    }
+    if (piece >= 0 && part == 0)
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int r = m0 + row + (i >> 2), c = n0 + col + (i & 3);
+        if (r >= p.M || c >= p.N) continue;
+        float* dst = p.C + (int64_t)r * p.ldc + c;
+        if (p.accumulate)
+          *dst += acc[i];
+        else if (!(fabsf(*dst) <= kFloatMax))
+          *dst = acc[i];
+      }
     __syncthreads();
   }
 }
