@@ -4,7 +4,8 @@
 
 Each ``csrc/*.cu`` is compiled to an object (in parallel, only when it or a header
 is newer than the object) and linked into ``frisk_b200/lib/libfrisk_b200.so``.
-nvcc cross-compiles without a GPU.
+nvcc cross-compiles without a GPU.  ``csrc/recognise.cpp``, a host-only CPython module, is compiled by g++ into
+``frisk_b200/lib/_recognise.so``.
 """
 import concurrent.futures
 import os
@@ -12,11 +13,13 @@ import pathlib
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = pathlib.Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "build"
 LIB = PKG / "lib" / "libfrisk_b200.so"
+RECOGNISE = PKG / "lib" / "_recognise.so"
 INCLUDE = PKG.parent / "include"
 
 NVCC_FLAGS = [
@@ -71,6 +74,14 @@ def build(force=False, verbose=False):
         if res.returncode:
             sys.stderr.write(res.stdout + res.stderr)
             raise RuntimeError("link of libfrisk_b200.so failed")
+    host = CSRC / "recognise.cpp"
+    if force or _stale(RECOGNISE, [host]):
+        cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"],
+               str(host), "-o", str(RECOGNISE)]
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode:
+            sys.stderr.write(res.stdout + res.stderr)
+            raise RuntimeError("g++ failed on recognise.cpp")
     return LIB
 
 

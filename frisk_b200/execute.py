@@ -23,7 +23,7 @@ Device memory, streams and process groups come from torch; the arithmetic does n
 """
 import math
 
-from . import capi, ir, tensor_ops
+from . import capi, ir, recognise, tensor_ops
 
 _TORCH_DTYPE = None
 
@@ -176,19 +176,45 @@ def gemm_plan(module_or_kernel, name=None, algo=capi.ALGO_AUTO):
     return desc, idx
 
 
+_ELEMENTS = (capi.F16, capi.BF16, capi.F32)  # the codes of recognise.plan
+
+
+def _plan_of(kernel, algo):
+    """(True, (descriptor, argument indices of q, k, v, o)) of an attention graph, (False, ``fused_plan``'s answer) of a gemm."""
+    known = recognise.plan(kernel)
+    if known is None:
+        ops = tensor_ops._ops_of(kernel)
+        if any(isinstance(op, tensor_ops.MmaOp) for op in ops):
+            spec, idx = tensor_ops.attention_plan(kernel, ops)
+            return True, (capi.attn_desc(1, 1, spec["S_q"], spec["S_kv"], spec["D"], spec["scale"], False, spec["dtype_in"],
+                                         spec["dtype_out"], normalize_p=True), idx)
+        return False, fused_plan(kernel, algo=algo)
+    if not known[0]:
+        _, s_q, s_kv, d, scale, e_in, e_out, *idx = known
+        return True, (capi.attn_desc(1, 1, s_q, s_kv, d, scale, False, _ELEMENTS[e_in], _ELEMENTS[e_out], normalize_p=True), idx)
+    _, m, n, k, e_ab, e_c, trans_a, trans_b, clear, policy, ia, ib, ic, fill, kind, reduce_arg, reduce_clear = known
+    desc = capi.gemm_desc(m, n, k, _ELEMENTS[e_ab], _ELEMENTS[e_c], trans_a, trans_b, clear, algo=algo)
+    desc.policy = policy
+    epilogue = None
+    if fill is not None or kind is not None:
+        epilogue = {"fill": fill, "reduce": kind, "reduce_arg": None if kind is None else reduce_arg,
+                    "reduce_clear": bool(reduce_clear)}
+    return False, (desc, (ia, ib, ic), epilogue)
+
+
 def execute(module_or_kernel, *tensors, stream=None, name=None, algo=capi.ALGO_AUTO):
     """Run the kernel on CUDA tensors bound positionally to its memref arguments."""
     torch = _torch()
     kernel = _kernel_of(module_or_kernel, name)
-    ops = tensor_ops._ops_of(kernel)
-    attention = any(isinstance(op, tensor_ops.MmaOp) for op in ops)
+    attention, plan = _plan_of(kernel, algo)
     if attention:
-        spec, arg_idx = tensor_ops.attention_plan(kernel, ops)
+        adesc, arg_idx = plan
     else:
-        desc, (ia, ib, ic), epilogue = fused_plan(kernel, algo=algo)
+        desc, (ia, ib, ic), epilogue = plan
     arg_types = kernel.attrs["function_type"].inputs
     if len(tensors) != len(arg_types):
         raise ValueError(f"frisk-b200-execute: kernel takes {len(arg_types)} tensors, got {len(tensors)}")
+    dtypes = {"f16": torch.float16, "bf16": torch.bfloat16, "f32": torch.float32}
     for t, ty in zip(tensors, arg_types):
         if t is None:
             continue
@@ -196,13 +222,10 @@ def execute(module_or_kernel, *tensors, stream=None, name=None, algo=capi.ALGO_A
             raise ValueError("frisk-b200-execute: tensors must live on a CUDA device (there is no CPU path)")
         if list(t.shape) != list(ty.shape) or not t.is_contiguous():
             raise ValueError(f"frisk-b200-execute: tensor of shape {list(t.shape)} does not match {ty}")
-        want = {"f16": torch.float16, "bf16": torch.bfloat16, "f32": torch.float32}.get(ty.element.name)
-        if t.dtype != want:
+        if t.dtype != dtypes.get(ty.element.name):
             raise ValueError(f"frisk-b200-execute: tensor dtype {t.dtype} does not match {ty}")
     if attention:
         q, k, v, o = (tensors[i] for i in arg_idx)
-        adesc = capi.attn_desc(1, 1, spec["S_q"], spec["S_kv"], spec["D"], spec["scale"], False, spec["dtype_in"],
-                               spec["dtype_out"], normalize_p=True)
         ctx = context_for(o.device.index or 0)
         ctx.attention_fwd(adesc, q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
                           stream=_stream_ptr(stream, o.device))
