@@ -235,10 +235,10 @@ int take_row_set(frisk_b200_ctx* ctx, cudaStream_t s) {
   return idle;
 }
 
-// A C the TMA unit cannot address (base or rows off 16 bytes) always goes to the one-CTA kernel, whose warps write whole
+// A C the TMA unit cannot write (base, pitch or rows off 16 bytes) always goes to the one-CTA kernel, whose warps write whole
 // rows; the pair kernel's threads write their own (3001 x 2055 x 1032 accumulating: 224 us).
 bool one_cta_preferred(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* C) {
-  if ((reinterpret_cast<uintptr_t>(C) & 15u) || resolve_dims(d).ldc * (int64_t)dtype_size(d.dtype_c) % 16) return true;
+  if (!tma_writes_c(d, C)) return true;
   return tcgen05_clocks(ctx, d) < tcgen05_2cta_clocks(d);
 }
 

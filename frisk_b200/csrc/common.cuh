@@ -186,6 +186,14 @@ inline GemmDims resolve_dims(const frisk_b200_gemm_desc& d) {
   return g;
 }
 
+// C may be written and read by the TMA unit: base, pitch AND rows are multiples of 16 bytes.  A store clips at 16 bytes, not at the
+// last column: where a row of C ends inside 16 bytes of a wider buffer, the rest of them becomes zero.
+inline bool tma_writes_c(const frisk_b200_gemm_desc& d, const void* C) {
+  const GemmDims g = resolve_dims(d);
+  const int64_t size = (int64_t)dtype_size(d.dtype_c);
+  return (reinterpret_cast<uintptr_t>(C) & 15u) == 0 && g.ldc * size % 16 == 0 && g.N * size % 16 == 0;
+}
+
 // ---- byte extents of the operands, for the output-overlaps-input refusal every entry makes
 inline bool ranges_overlap(const void* a, size_t an, const void* b, size_t bn) {
   uintptr_t a0 = reinterpret_cast<uintptr_t>(a), b0 = reinterpret_cast<uintptr_t>(b);

@@ -612,8 +612,7 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* A
   if (rc) { ctx->last_cuda = rc; return FRISK_B200_E_CUDA; }
 
   GemmArgs a{};
-  // a C whose base and row pitch are 16-byte aligned goes through the TMA unit
-  a.tma_c = aligned16(C) && (g.ldc * sizeof(TO)) % 16 == 0;
+  a.tma_c = tma_writes_c(d, C);
   CUtensorMap tc = ta;  // unused otherwise
   if (a.tma_c) {
     const int out_dtype = sizeof(TO) == 4 ? FRISK_B200_F32 : (std::is_same<TO, __half>::value ? FRISK_B200_F16 : FRISK_B200_BF16);

@@ -774,11 +774,10 @@ int launch_gemm_tcgen05_2cta(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d,
     if (bf) return launch_major2<__nv_bfloat16, true, kFused>(ctx, d, A, B, C, ws, ws_bytes, s, epi);
     return launch_major2<__half, false, kFused>(ctx, d, A, B, C, ws, ws_bytes, s, epi);
   }
-  // a C whose base and row pitch are 16-byte aligned goes through the TMA unit (accumulating through the threads' own
+  // through the TMA unit where it can take C (accumulating through the threads' own
   // 16-byte accesses, 3000^3 took 55 us where overwriting took 47)
   const GemmDims g = resolve_dims(d);
-  const size_t cs = dtype_size(d.dtype_c);
-  if (aligned16(C) && (g.ldc * cs) % 16 == 0) {
+  if (tma_writes_c(d, C)) {
     if (!d.clear_accum) {
       if (d.dtype_c == FRISK_B200_F32)
         return bf ? launch_major2<float, true, kAccTma>(ctx, d, A, B, C, ws, ws_bytes, s, nullptr)

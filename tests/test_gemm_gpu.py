@@ -957,3 +957,26 @@ def test_fused_epilogue_with_caller_workspace(ctx):
                           gemm_oracle.row_reduce(got, "fp16", "max"))
     with pytest.raises(ValueError):
         ctx.gemm_fused(desc, epi, da.data_ptr(), db.data_ptr(), dc.data_ptr(), ws.data_ptr(), need - 4096, stream=s)
+
+
+# ------------------------------------------------------------------ a C that is part of a wider buffer
+@pytest.mark.parametrize("algo", [capi.ALGO_AUTO] + TC_ALGOS)
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("dtype_c,N,pitch", [("bf16", 130, 136), ("bf16", 125, 128), ("fp32", 129, 132), ("fp32", 62, 64), ("bf16", 128, 136)])
+def test_columns_beyond_n_keep_their_values(ctx, algo, accumulate, dtype_c, N, pitch):
+    """C's rows end inside 16 bytes of a row of the buffer: what follows is not C's."""
+    import torch
+    M, K = 300, 192
+    a, b = inputs.gemm_inputs(M, N, K, "bf16", False, True, 5 + N)
+    ga, gb = Guarded(a.shape, "bf16", fill=a), Guarded(b.shape, "bf16", fill=b)
+    old = to_storage(np.random.default_rng(N).standard_normal((M, pitch), dtype=np.float32), dtype_c)
+    gc = Guarded((M, pitch), dtype_c, fill=old)
+    desc = capi.gemm_desc(M, N, K, "bf16", dtype_c, False, True, clear_accum=not accumulate, ldc=pitch, algo=algo)
+    s = torch.cuda.current_stream().cuda_stream
+    ctx.gemm(desc, ga.view.data_ptr(), gb.view.data_ptr(), gc.view.data_ptr(), stream=s)
+    ctx.check(s)
+    got = gc.host()
+    assert gc.guards_intact() and np.array_equal(got[:, N:], old[:, N:])
+    mine = np.ascontiguousarray(old[:, :N])
+    ref = gemm_oracle.gemm_fp64(a, b, "bf16", False, True, mine if accumulate else None, dtype_c)
+    assert rel_frobenius(from_storage(np.ascontiguousarray(got[:, :N]), dtype_c), ref) <= TOL["bf16"]
