@@ -10,7 +10,7 @@
 //   warps 2-5 epilogue:     tcgen05.ld of the finished accumulator, conversion, stores
 // Two accumulators (2 x BN TMEM columns) let the epilogue of tile i overlap the main loop of
 // tile i+1.  Output tiles are 128 x 256 (12 KB of operands per 128 clk of MMA) or, where those are too few, 128 x 128
-// (8 KB per 64 clk, all that shared memory delivers).
+// (8 KB per 64 clk, all that shared memory delivers) or 128 x 64.
 //
 // Whole rounds of tiles are dealt out tile by tile.  The tiles of a partial last round (all of them, where there are
 // fewer tiles than SMs) are shared by clusters of 2, 4 or 8 CTAs, each multiplying its part of K: every CTA leaves its fp32
@@ -57,15 +57,17 @@ struct SmemLayout {
   static constexpr int kABytes = BM * BK * 2;
   static constexpr int kBBytes = BN * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = 196608 / kStageBytes;  // 4 at BN = 256, 6 at BN = 128
+  static constexpr int kStages = 196608 / kStageBytes;  // 4 at BN = 256, 6 at BN = 128, 8 at BN = 64
+  static constexpr int kBoxRowsB = BN < 128 ? BN : 128;  // rows of B that one TMA instruction brings
   static constexpr int kBarOffset = kStages * kStageBytes;
   // two [32 rows][128 bytes] boxes of C per epilogue warp, 1024-byte aligned
   static constexpr int kOutOffset = kBarOffset + 1024;
   static constexpr int kTotal = kOutOffset + 4 * 2 * kBoxBytes + 1024;
   static_assert(kTotal <= 232448, "the boxes of C must fit next to the operand ring");
-  // a shared tile: this CTA's part [BN/4][128 rows] float4, then the sums of the columns it finishes (at most half)
+  // a shared tile: this CTA's part [BN/4][128 rows] float4, then the sums of the columns it finishes (at most half, but at
+  // BN = 64 and 16 bits, a single box wide, all)
   static constexpr int kSumOffset = BM * BN * 4;
-  static_assert(kSumOffset + BM * BN * 2 <= kBarOffset, "the parts and sums of a shared tile must fit in the ring");
+  static_assert(kSumOffset + BM * (BN == 64 ? BN : BN / 2) * 4 <= kBarOffset, "the parts and sums of a shared tile must fit in the ring");
 };
 
 struct GemmArgs {
@@ -172,10 +174,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int j = 0; j < BN / 64; ++j)
               tma_load_2d(sb + j * (BK * 128), &tmap_b, &full_bar[stage], n0 + j * 64, k0);
           } else {
-            // boxes of 128 rows: stacked 8-row groups, the same image as one taller box
+            // boxes of at most 128 rows: stacked 8-row groups, the same image as one taller box
 #pragma unroll
-            for (int j = 0; j < BN / 128; ++j)
-              tma_load_2d(sb + j * (128 * BK * 2), &tmap_b, &full_bar[stage], k0, n0 + j * 128);
+            for (int j = 0; j < BN / L::kBoxRowsB; ++j)
+              tma_load_2d(sb + j * (L::kBoxRowsB * BK * 2), &tmap_b, &full_bar[stage], k0, n0 + j * L::kBoxRowsB);
           }
           if (++stage == kStages) {
             stage = 0;
@@ -554,7 +556,10 @@ struct Plan {
 // its MMAs (512 clk at 256 columns, 256 at 128) and, the more SMs are at it, what L2 adds: 770 at 2048^3 and 4096^3 with
 // the chip full, 1100 where rows begin off 128-byte lines (3000^3: two requests of the TMA unit a row).  Sharing costs
 // barriers, parts and sums: 3.5 us at 128 rows (128 x 512 x 512 over clusters of four took 8.7 us, whole 6.7), less
-// with fewer rows (17 x 1024 x 1024 6.8, 128 x 1024 x 1024 9.1 over clusters of eight).
+// with fewer rows (17 x 1024 x 1024 6.8, 128 x 1024 x 1024 9.1 over clusters of eight).  Tiles of 64 columns take as long for a
+// block (MMAs paced by the 6 KB of operands each) but put twice the SMs to work and have half the parts to add up: they are for products
+// with few columns and rows (128 x 2048 x 2048 in clusters of four 9.9 us, 11.2 with 128 columns; 64 x 2048 x 4096 11.4, 12.3;
+// 256 x 1024 x 4096 12.1, 13.4; whole 300 x 1000 x 1000 9.2, 9.9).
 Plan plan_of(const GemmDims& g, int64_t tiles, int sms, int bn, int splits, int clusters) {
   const int64_t kb = (g.K + BK - 1) / BK;
   const bool aligned = g.lda % 64 == 0 && g.ldb % 64 == 0;
@@ -564,7 +569,7 @@ Plan plan_of(const GemmDims& g, int64_t tiles, int sms, int bn, int splits, int 
     p.n_whole = (int)tiles;
     p.grid = (int)std::min<int64_t>(tiles, sms);
     blocks = std::ceil((double)tiles / sms) * (double)kb;
-    extra = bn == 256 ? 3500 : 1800;
+    extra = bn == 256 ? 3500 : bn == 128 ? 1800 : 1500;
   } else {
     const int grid = splits * std::min(clusters, sms / splits);
     if (grid == 0 || kb < 2 * splits) return p;
@@ -573,16 +578,18 @@ Plan plan_of(const GemmDims& g, int64_t tiles, int sms, int bn, int splits, int 
     p.n_whole = (int)(rounds * grid);
     p.grid = rounds > 0 ? grid : (int)rest * splits;
     blocks = (double)rounds * (double)kb + std::ceil((double)kb / splits);
-    extra = (bn == 256 ? 4500 : 3500) + 3000.0 * (double)std::min<int64_t>(g.M, BM) / BM;
+    extra = (bn == 256 ? 4500 : bn == 128 ? 3500 : 2500) + (bn == 64 ? 1500.0 : 3000.0) * (double)std::min<int64_t>(g.M, BM) / BM;
   }
   const double busy = (double)p.grid / sms;
-  p.clocks = blocks * (bn == 256 ? 520 + (aligned ? 250 : 580) * busy : 270 + (aligned ? 200 : 450) * busy) + extra;
+  const double mma = bn == 256 ? 520 : bn == 128 ? 270 : 250;
+  const double l2 = bn == 256 ? (aligned ? 250 : 580) : bn == 128 ? (aligned ? 200 : 450) : aligned ? 150 : 340;
+  p.clocks = blocks * (mma + l2 * busy) + extra;
   return p;
 }
 template <typename F>
 Plan make_plan(const GemmDims& g, int sms, F&& clusters) {
   Plan best{256, 1, 0, 0, 1e300};
-  for (int bn : {256, 128}) {
+  for (int bn : {256, 128, 64}) {
     const int64_t tiles = ((g.M + BM - 1) / BM) * ((g.N + bn - 1) / bn);
     if (tiles > INT32_MAX / 2) continue;
     for (int splits : {1, 2, 4, 8}) {
@@ -608,7 +615,8 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* A
   if (B_MN)
     rc = encode_tmap_2d(ctx, &tb, d.dtype_ab, B, (uint64_t)g.N, (uint64_t)g.K, (uint64_t)g.ldb * 2, 64, BK, true);
   else
-    rc = encode_tmap_2d(ctx, &tb, d.dtype_ab, B, (uint64_t)g.K, (uint64_t)g.N, (uint64_t)g.ldb * 2, BK, 128, true);
+    rc = encode_tmap_2d(ctx, &tb, d.dtype_ab, B, (uint64_t)g.K, (uint64_t)g.N, (uint64_t)g.ldb * 2, BK,
+                        SmemLayout<BN>::kBoxRowsB, true);
   if (rc) { ctx->last_cuda = rc; return FRISK_B200_E_CUDA; }
 
   GemmArgs a{};
@@ -673,8 +681,8 @@ int launch_major(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void*
 // Clusters the device runs at a time.  Every instantiation has one CTA per SM (shared memory decides), so one of them
 // answers for all of the same tile.
 int clusters_of(int device, int bn, int splits) {
-  static ClusterCapacity wide, narrow;
-  static PerDeviceOnce opt_wide, opt_narrow;
+  static ClusterCapacity wide, narrow, thin;
+  static PerDeviceOnce opt_wide, opt_narrow, opt_thin;
   auto ask = [&](auto kern, int smem, ClusterCapacity& capacity, PerDeviceOnce& opt_in) {
     if (opt_in(device, [&] {
           return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess ? 0 : 1;
@@ -682,8 +690,9 @@ int clusters_of(int device, int bn, int splits) {
       return 0;
     return capacity(device, kern, kThreads, smem, splits);
   };
-  return bn == 256 ? ask(gemm_tcgen05_kernel<__half, 256, false, false, false, true>, SmemLayout<256>::kTotal, wide, opt_wide)
-                   : ask(gemm_tcgen05_kernel<__half, 128, false, false, false, true>, SmemLayout<128>::kTotal, narrow, opt_narrow);
+  if (bn == 256) return ask(gemm_tcgen05_kernel<__half, 256, false, false, false, true>, SmemLayout<256>::kTotal, wide, opt_wide);
+  if (bn == 128) return ask(gemm_tcgen05_kernel<__half, 128, false, false, false, true>, SmemLayout<128>::kTotal, narrow, opt_narrow);
+  return ask(gemm_tcgen05_kernel<__half, 64, false, false, false, true>, SmemLayout<64>::kTotal, thin, opt_thin);
 }
 Plan plan_for(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d) {
   return make_plan(resolve_dims(d), std::min(ctx->num_sms, kNumSMsDefault),
@@ -695,8 +704,9 @@ int launch_tile(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc& d, const void* 
                 const RowEpilogue* epi, cudaStream_t s) {
   const Plan plan = plan_for(ctx, d);
   if (plan.grid == 0) return FRISK_B200_E_UNSUPPORTED;
-  return plan.bn == 256 ? launch_major<TO, BF16, 256>(ctx, d, A, B, C, plan, epi, s)
-                        : launch_major<TO, BF16, 128>(ctx, d, A, B, C, plan, epi, s);
+  if (plan.bn == 256) return launch_major<TO, BF16, 256>(ctx, d, A, B, C, plan, epi, s);
+  if (plan.bn == 128) return launch_major<TO, BF16, 128>(ctx, d, A, B, C, plan, epi, s);
+  return launch_major<TO, BF16, 64>(ctx, d, A, B, C, plan, epi, s);
 }
 
 }  // namespace

@@ -980,3 +980,18 @@ def test_columns_beyond_n_keep_their_values(ctx, algo, accumulate, dtype_c, N, p
     mine = np.ascontiguousarray(old[:, :N])
     ref = gemm_oracle.gemm_fp64(a, b, "bf16", False, True, mine if accumulate else None, dtype_c)
     assert rel_frobenius(from_storage(np.ascontiguousarray(got[:, :N]), dtype_c), ref) <= TOL["bf16"]
+
+
+# ------------------------------------------------------------------ tiles of 64 columns
+@pytest.mark.parametrize("M,N,K,ta,tb,dtype_c", [
+    (128, 2048, 2048, False, True, "bf16"),   # clusters of four, one box column: the parts are added up by all
+    (64, 2048, 4096, False, True, "fp32"),    # two box columns
+    (300, 1000, 1000, False, False, "bf16"),  # whole tiles, ragged columns
+    (192, 64, 8192, True, True, "bf16"),      # one tile column
+    (96, 72, 1192, False, False, "fp32"),
+])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_tiles_of_64_columns(ctx, M, N, K, ta, tb, dtype_c, accumulate):
+    desc = capi.gemm_desc(M, N, K, "bf16", dtype_c, ta, tb, clear_accum=not accumulate, algo=capi.ALGO_TCGEN05)
+    assert ctx.gemm_plan(desc, 4096).tile_n == 64
+    check(ctx, M, N, K, "bf16", dtype_c, ta, tb, M + N, accumulate=accumulate, algo=capi.ALGO_TCGEN05)
