@@ -82,6 +82,118 @@ struct GemmArgs {
   unsigned* status;
 };
 
+// A 32-row box (128 bytes a row, a 32-bit word a lane) of a C that the TMA unit cannot address: its rows begin on a multiple
+// of the element's size and no more.  16-bit elements go in pairs wherever they lie on 4 bytes: of a row that begins
+// there lane l has elements 2l and 2l + 1, of an odd row 2l + 1 and 2l + 2, and its first and last element go by themselves.
+// Which rows are odd is one of four patterns, the same for the whole box: an epilogue warp has its scheduler to itself, so its
+// time is the number of instructions, and rows that decide for themselves took 1200 of them a box (1.9 us).  With 2-byte accesses
+// 4000 x 4092 x 512 took 51.7 us, 33.3 so, 22.9 with 4096 columns by TMA; 4095 columns 51.7 and 39.8.  The old values used to be
+// loaded one after the other, each behind the shared-memory store of the one before: two panels of 6543 x 4546 x 2296
+// 872 us, 359 so; fp32 3000 x 2055 x 1032 186 and 73.
+struct BoxRows {
+  bool first_odd, second_odd;
+  template <typename TO>
+  __device__ __forceinline__ BoxRows(const TO* row, int64_t pitch)
+      : first_odd(sizeof(TO) == 2 && (reinterpret_cast<uintptr_t>(row) & 2u)),
+        second_odd(sizeof(TO) == 2 && (reinterpret_cast<uintptr_t>(row + pitch) & 2u)) {}
+  // f(first row odd, second row odd), the answers as types
+  template <typename F>
+  __device__ __forceinline__ void pattern(F&& f) const {
+    if (first_odd) {
+      if (second_odd) f(std::true_type(), std::true_type()); else f(std::true_type(), std::false_type());
+    } else {
+      if (second_odd) f(std::false_type(), std::true_type()); else f(std::false_type(), std::false_type());
+    }
+  }
+};
+// the old values of a box, cols x rows of which lie in C (all loads on their way before the first is used), into its image:
+// put(r, word of row r)
+template <typename TO, typename Put>
+__device__ __forceinline__ void load_box_rows(const TO* row, int64_t pitch, int rows, int cols, int lane, Put&& put) {
+  uint32_t w[32];
+  if (sizeof(TO) == 4) {
+#pragma unroll
+    for (int r = 0; r < 32; ++r) w[r] = r < rows && lane < cols ? *reinterpret_cast<const uint32_t*>(row + r * pitch + lane) : 0u;
+#pragma unroll
+    for (int r = 0; r < 32; ++r) put(r, w[r]);
+    return;
+  }
+  const unsigned short* p = reinterpret_cast<const unsigned short*>(row);
+  // lane r: the first element of row r
+  const uint32_t firsts = lane < rows ? p[lane * pitch] : 0u;
+  BoxRows(row, pitch).pattern([&](auto odd0, auto odd1) {
+#pragma unroll
+    for (int r = 0; r < 32; ++r) {
+      const bool odd = r % 2 ? decltype(odd1)::value : decltype(odd0)::value;
+      const int j = 2 * lane + (odd ? 1 : 0);
+      w[r] = 0u;
+      if (r < rows && j + 1 < cols) w[r] = *reinterpret_cast<const uint32_t*>(p + r * pitch + j);
+      if (r < rows && j + 1 == cols) w[r] = p[r * pitch + j];
+    }
+#pragma unroll
+    for (int r = 0; r < 32; ++r) {
+      const bool odd = r % 2 ? decltype(odd1)::value : decltype(odd0)::value;
+      if (odd) {
+        const uint32_t before = __shfl_up_sync(0xffffffffu, w[r], 1), first = __shfl_sync(0xffffffffu, firsts, r);
+        w[r] = (lane == 0 ? first : before >> 16) | (w[r] << 16);
+      }
+      put(r, w[r]);
+    }
+  });
+}
+// a box back to C: get(r) gives this lane's word of row r
+template <typename TO, typename Get>
+__device__ __forceinline__ void store_box_rows(TO* row, int64_t pitch, int rows, int cols, int lane, Get&& get) {
+  constexpr int kStep = 8;
+  if (sizeof(TO) == 4) {
+#pragma unroll 1
+    for (int r = 0; r < rows; r += kStep, row += kStep * pitch) {
+      uint32_t w[kStep];
+#pragma unroll
+      for (int i = 0; i < kStep; ++i) w[i] = get(r + i);
+#pragma unroll
+      for (int i = 0; i < kStep; ++i)
+        if (r + i < rows && lane < cols) *reinterpret_cast<uint32_t*>(row + i * pitch + lane) = w[i];
+    }
+    return;
+  }
+  unsigned short* p = reinterpret_cast<unsigned short*>(row);
+  // an odd row's pairs, and what is left over: lane 0 has the first element, the lane of the last column the last where cols is even
+  const bool pair_even = 2 * lane + 1 < cols, pair_odd = 2 * lane + 2 < cols, one_even = 2 * lane + 1 == cols;
+  const bool one_odd = lane == 0 || 2 * lane + 2 == cols;
+  const int one_at = lane == 0 ? 0 : 2 * lane + 1;
+  BoxRows(row, pitch).pattern([&](auto odd0, auto odd1) {
+#pragma unroll 1
+    for (int r = 0; r < rows; r += kStep, p += kStep * pitch) {
+      uint32_t w[kStep];
+#pragma unroll
+      for (int i = 0; i < kStep; ++i) w[i] = get(r + i);
+#pragma unroll
+      for (int i = 0; i < kStep; ++i) {
+        const bool odd = i % 2 ? decltype(odd1)::value : decltype(odd0)::value;
+        unsigned short* q = p + i * pitch;
+        const bool in = r + i < rows;
+        if (odd) {
+          const uint32_t after = __shfl_down_sync(0xffffffffu, w[i], 1);
+          if (in && pair_odd) *reinterpret_cast<uint32_t*>(q + 2 * lane + 1) = __funnelshift_r(w[i], after, 16);
+          if (in && one_odd) q[one_at] = (unsigned short)(lane == 0 ? w[i] : w[i] >> 16);
+        } else {
+          if (in && pair_even) *reinterpret_cast<uint32_t*>(q + 2 * lane) = w[i];
+          if (in && one_even) q[2 * lane] = (unsigned short)w[i];
+        }
+      }
+    }
+    // (cols = 2: lane 0 has both ends of an odd row)
+    if (cols == 2 && (decltype(odd0)::value || decltype(odd1)::value)) {
+      unsigned short* q = reinterpret_cast<unsigned short*>(row);
+      for (int r = 0; r < rows; ++r) {
+        const uint32_t w = get(r);
+        if (lane == 0 && (r % 2 ? decltype(odd1)::value : decltype(odd0)::value)) q[r * pitch + 1] = (unsigned short)(w >> 16);
+      }
+    }
+  });
+}
+
 // A_MN / B_MN: the operand is contiguous along M / N in global memory (MN-major image).
 // PLAIN: an overwriting store of an aligned C, the usual call, without the code of every other epilogue.
 template <typename TO, int BN, bool BF16, bool A_MN, bool B_MN, bool PLAIN>
@@ -233,7 +345,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else {
     // ------------------------------------------------------------------ epilogue
     const int quad = warp & 3;  // TMEM lanes [32*quad, 32*quad+32) are this warp's
-    constexpr int U = 128 / (int)sizeof(TO);  // columns of a box
+    constexpr int U = 128 / (int)sizeof(TO);     // columns of a box
+    constexpr int kPer = 4 / (int)sizeof(TO);    // of a lane's 32-bit word of a box row
     unsigned char* boxes = smem + L::kOutOffset + quad * 2 * kBoxBytes;
     uint64_t* bars = box_bar + quad * 2;
     TO* const C = static_cast<TO*>(p.C);
@@ -269,15 +382,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (!accumulate && lane == 0) tma_store_wait_read<1>();  // the store before the last one used this box
         __syncwarp();
       } else if (accumulate) {
-        // old values of C, a row piece at a time, into the same image
-#pragma unroll 16
-        for (int r = 0; r < 32; ++r) {
-#pragma unroll
-          for (int h = 0; h < U / 32; ++h) {
-            const int j = h * 32 + lane;
-            if (r0 + r < p.M && c0 + j < p.N) *reinterpret_cast<TO*>(box + box_at(r, j)) = C[(int64_t)(r0 + r) * p.ldc + c0 + j];
-          }
-        }
+        // old values of C, a row at a time, into the same image; all loads are on their way before the first is stored
+        load_box_rows(C + (int64_t)r0 * p.ldc + c0, p.ldc, min(32, p.M - r0), min(U, p.N - c0), lane, [&](int r, uint32_t w) {
+          *reinterpret_cast<uint32_t*>(box + box_at(r, lane * kPer)) = w;
+        });
         __syncwarp();
       }
       uint32_t w[32];
@@ -339,14 +447,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       } else {
         __syncwarp();
-#pragma unroll 8
-        for (int r = 0; r < 32; ++r) {
-#pragma unroll
-          for (int h = 0; h < U / 32; ++h) {
-            const int j = h * 32 + lane;
-            if (r0 + r < p.M && c0 + j < p.N) C[(int64_t)(r0 + r) * p.ldc + c0 + j] = *reinterpret_cast<const TO*>(box + box_at(r, j));
-          }
-        }
+        store_box_rows(C + (int64_t)r0 * p.ldc + c0, p.ldc, min(32, p.M - r0), min(U, p.N - c0), lane, [&](int r) {
+          return *reinterpret_cast<const uint32_t*>(box + box_at(r, lane * kPer));
+        });
         __syncwarp();
       }
       box_sel ^= 1;

@@ -982,6 +982,44 @@ def test_columns_beyond_n_keep_their_values(ctx, algo, accumulate, dtype_c, N, p
     assert rel_frobenius(from_storage(np.ascontiguousarray(got[:, :N]), dtype_c), ref) <= TOL["bf16"]
 
 
+# ------------------------------------------------------------------ C whose rows do not begin on 16 bytes
+@pytest.mark.parametrize("dtype_ab,dtype_c", [("fp16", "fp16"), ("bf16", "bf16"), ("bf16", "fp32")])
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("M,N,pitch,offset", [
+    (33, 1, 1, 0),          # one column: a row in two begins between two 32-bit words
+    (130, 65, 65, 0),       # one element more than a box of 16-bit elements
+    (64, 63, 67, 2),        # a base between two words, columns beyond N that are not C's
+    (257, 127, 130, 4),     # rows on 4 bytes
+    (100, 130, 132, 8),     # rows on 8 bytes
+    (31, 259, 259, 2),
+    (300, 514, 515, 6),
+])
+def test_rows_off_16_bytes(ctx, dtype_ab, dtype_c, accumulate, M, N, pitch, offset):
+    """The one-CTA kernel's whole-row accesses: all of C, nothing beside it (pitch columns and guard zones keep their bytes)."""
+    import torch
+    if dtype_c == "fp32":
+        offset *= 2  # in elements
+    K = 192
+    a, b = inputs.gemm_inputs(M, N, K, dtype_ab, False, True, 7 * M + N)
+    ga, gb = Guarded(a.shape, dtype_ab, fill=a), Guarded(b.shape, dtype_ab, fill=b)
+    rng = np.random.default_rng(M + N + pitch)
+    old = to_storage(rng.standard_normal((M, pitch), dtype=np.float32), dtype_c)
+    gc = Guarded((M, pitch), dtype_c, fill=old, offset=offset)
+    desc = capi.gemm_desc(M, N, K, dtype_ab, dtype_c, False, True, clear_accum=not accumulate, ldc=pitch, algo=capi.ALGO_TCGEN05)
+    s = torch.cuda.current_stream().cuda_stream
+    ctx.gemm(desc, ga.view.data_ptr(), gb.view.data_ptr(), gc.view.data_ptr(), stream=s)
+    ctx.check(s)
+    assert gc.guards_intact()
+    got = gc.host()
+    assert np.array_equal(got[:, N:], old[:, N:])
+    ref = gemm_oracle.gemm_fp64(a, b, dtype_ab, False, True, np.ascontiguousarray(old[:, :N]) if accumulate else None, dtype_c)
+    # every element by itself: one rounding to C's type of a sum of K products in fp32
+    unit = {"fp16": 2.0 ** -11, "bf16": 2.0 ** -8, "fp32": 2.0 ** -18}[dtype_c]
+    gotf = from_storage(np.ascontiguousarray(got[:, :N]), dtype_c)
+    bound = unit * np.abs(ref) + 2.0 ** -16 * np.sqrt(K)
+    assert (np.abs(gotf - ref) <= bound).all(), np.abs(gotf - ref).max()
+
+
 # ------------------------------------------------------------------ tiles of 64 columns
 @pytest.mark.parametrize("M,N,K,ta,tb,dtype_c", [
     (128, 2048, 2048, False, True, "bf16"),   # clusters of four, one box column: the parts are added up by all
