@@ -117,6 +117,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   // Normalised mode runs the key loop twice: pass 0 only gathers row maxima and row sums, pass 1
   // is the pass every mode has.  Barrier phases keep counting across passes and items.
   constexpr int first_pass = NORM ? 0 : 1;
+  // Where the row maximum is taken: before the group's turn, on the ALU while the other group keeps the special-function
+  // unit busy, or within it, run through the first exponentials.  Before is faster where the turns set the pace: D = 64, whose
+  // MMAs are half as long (8 x 32 heads x 2048 causal 274 -> 251 us, 3 x 16 x 1500 57.8 -> 51.7).  At
+  // D = 128 P.V and the next S set it, and long runs the power limit (930 W): 8 x 32 x 4096 causal 1173 -> 1183, 8 heads x 8192
+  // 279 -> 289.
+  constexpr bool kMaxFirst = D == 64;
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -435,8 +441,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       // on the same four schedulers and then both sit idle while their MMAs run; taking turns, one group works
       // alone (a third faster) while the other group's P.V and next S are in flight.  A group with fewer key
       // tiles than the other keeps passing the turn on until the other is done.
-      for (int j = 0; j < n_max; ++j) {
-        const bool mine = j < n_tiles;
+      for (int i = 0; i < n_max; ++i) {
+        const bool mine = i < n_tiles;
         uint32_t sr[4][32];
         if (mine) {
           if (!mbar_wait(&s_full[q], steps & 1, abort_flag, p.status, ST_ATTN_S)) {
@@ -448,6 +454,62 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(t_s + c * 32, sr[c]);
           tmem_ld_wait();
+
+          const int n0 = i * BN;
+          const bool needs_mask = (n0 + BN > p.S_kv) || (p.causal && (n0 + BN - 1 > m_tile + off));
+          if (needs_mask) {
+            int limit = p.S_kv - 1;
+            if (p.causal) limit = min(limit, g_row + off);
+            limit -= n0;  // columns > limit are hidden
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (c * 32 + i > limit) sr[c][i] = 0xff800000u;  // -inf
+          }
+        }
+        const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
+        float mxc[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four chains of the row maximum
+        auto max_step = [&](int i) {  // two keys of every 32
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            mxc[c] = max3f(mxc[c], __uint_as_float(sr[c][2 * i]), __uint_as_float(sr[c][2 * i + 1]));
+        };
+        // Takes the row maximum into the reference; true where that has moved (exponentials relative to the one before are
+        // void).  O is rescaled only when the maximum grew by more than the threshold: rare after the first tiles.
+        auto settle = [&]() -> bool {
+          const float mx = max3f(mxc[0], mxc[1], fmaxf(mxc[2], mxc[3]));
+          float m_new = fmaxf(m_ref, mx * p.scale_log2);
+          if (m_new == -INFINITY) m_new = 0.f;  // a row that sees no key yet: keep everything finite
+          if (i == 0) {
+            m_ref = m_new;
+            return true;
+          }
+          // (warp-uniform decision because the TMEM accesses are warp-collective)
+          if (!__any_sync(0xffffffffu, m_new - m_ref > kRescaleThreshold)) return false;
+          const float factor = ex2f(m_ref - m_new);
+          m_ref = m_new;
+          l_sum *= factor;
+          // O_q must be complete up to the key tile before this one before it is scaled
+          ok = mbar_wait(&o_done[q], (pv_base + i - 1) & 1, abort_flag, p.status, ST_ATTN_O);
+          if (!ok) return true;
+          tc_fence_after_sync();
+#pragma unroll
+          for (int c = 0; c < D / 32; ++c) {
+            uint32_t o[32];
+            tmem_ld_32x32b_x32(t_o + c * 32, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * factor);
+            tmem_st_32x32b_x32(t_o + c * 32, o);
+          }
+          return true;
+        };
+        if (kMaxFirst && mine) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) max_step(e);
+          settle();
+          if (!ok) break;
         }
         if (!mbar_wait(&turn[q], q == 0 ? ((turns & 1) ^ 1) : (turns & 1), abort_flag, p.status, ST_ATTN_S)) {
           ok = false;
@@ -459,86 +521,41 @@ __global__ void __launch_bounds__(kThreads, 1)
           continue;
         }
 
-        const int n0 = j * BN;
-        const bool needs_mask = (n0 + BN > p.S_kv) || (p.causal && (n0 + BN - 1 > m_tile + off));
-        if (needs_mask) {
-          int limit = p.S_kv - 1;
-          if (p.causal) limit = min(limit, g_row + off);
-          limit -= n0;  // columns > limit are hidden
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (c * 32 + i > limit) sr[c][i] = 0xff800000u;  // -inf
-        }
         // P = 2^(s*scale_log2 - m_ref) with packed fp32 FMAs, row sum in fp32, P rounded to 16 bits.
         // Two 32-key chunks at a time, interleaved pair by pair so that the special-function unit always has
-        // independent work.  WITH_MAX also runs the row maximum of all 128 keys (four chains of three-input
-        // max, two keys of every chunk per step) through the same loop: the maximum is a chain on the ALU, the
-        // exponentials are bound by the special-function unit, and neither waits for the other.
-        const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
-        float mxc[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-        auto exp_chunks = [&](int c0, float mref, uint32_t (&pa)[16], uint32_t (&pb)[16], float2& sum, auto with_max) {
-          const float2 negm2 = make_float2(-mref, -mref);
+        // independent work.  WITH_MAX also runs the row maximum of all 128 keys through the same loop: the maximum is a
+        // chain on the ALU, the exponentials are bound by the special-function unit, and neither waits for the other.
+        auto exp_chunks = [&](int c0, uint32_t (&pa)[16], uint32_t (&pb)[16], float2& sum, auto with_max) {
+          const float2 negm2 = make_float2(-m_ref, -m_ref);
           float2 sa = make_float2(0.f, 0.f), sb = make_float2(0.f, 0.f);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float2 xa = fma2(make_float2(__uint_as_float(sr[c0][2 * i]), __uint_as_float(sr[c0][2 * i + 1])), scale2, negm2);
-            const float2 xb = fma2(make_float2(__uint_as_float(sr[c0 + 1][2 * i]), __uint_as_float(sr[c0 + 1][2 * i + 1])), scale2, negm2);
-            if (decltype(with_max)::value) {
-#pragma unroll
-              for (int c = 0; c < 4; ++c)
-                mxc[c] = max3f(mxc[c], __uint_as_float(sr[c][2 * i]), __uint_as_float(sr[c][2 * i + 1]));
-            }
+          for (int e = 0; e < 16; ++e) {
+            const float2 xa = fma2(make_float2(__uint_as_float(sr[c0][2 * e]), __uint_as_float(sr[c0][2 * e + 1])), scale2, negm2);
+            const float2 xb = fma2(make_float2(__uint_as_float(sr[c0 + 1][2 * e]), __uint_as_float(sr[c0 + 1][2 * e + 1])), scale2, negm2);
+            if (decltype(with_max)::value) max_step(e);
             const float2 ea = make_float2(ex2f(xa.x), ex2f(xa.y));
             const float2 eb = make_float2(ex2f(xb.x), ex2f(xb.y));
             sa = add2(sa, ea);
             sb = add2(sb, eb);
-            pa[i] = pack16<BF16>(ea.x, ea.y);
-            pb[i] = pack16<BF16>(eb.x, eb.y);
+            pa[e] = pack16<BF16>(ea.x, ea.y);
+            pb[e] = pack16<BF16>(eb.x, eb.y);
           }
           sum = add2(sa, sb);
         };
-
-        // Optimistic first half: the exponentials of keys 0-63 are taken relative to the reference maximum
-        // the row already has, so they do not wait for the row maximum.  Only when the maximum turns out to
-        // have grown by more than the threshold (rare after the first tiles; always on the first tile, whose
-        // reference is -infinity) is O rescaled and the half recomputed.  The stale reference cannot overflow
-        // what is kept: a value that would exceed 2^threshold is by construction one that triggers the
-        // recomputation.
         uint32_t pk0[16], pk1[16];
         float2 sum01;
-        exp_chunks(0, m_ref, pk0, pk1, sum01, std::true_type());
-        const float mx = max3f(mxc[0], mxc[1], fmaxf(mxc[2], mxc[3]));
-        float m_new = fmaxf(m_ref, mx * p.scale_log2);
-        if (m_new == -INFINITY) m_new = 0.f;  // a row that sees no key yet: keep everything finite
-        // lazy rescale: warp-uniform decision because the TMEM accesses are warp-collective
-        const bool grow = (j > 0) && (m_new - m_ref > kRescaleThreshold);
-        bool redo = j == 0;
-        if (j == 0) {
-          m_ref = m_new;
-        } else if (__any_sync(0xffffffffu, grow)) {
-          const float factor = ex2f(m_ref - m_new);
-          m_ref = m_new;
-          l_sum *= factor;
-          redo = true;
-          // O_q must be complete up to tile j-1 before it is scaled
-          if (!mbar_wait(&o_done[q], (pv_base + j - 1) & 1, abort_flag, p.status, ST_ATTN_O)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after_sync();
-#pragma unroll
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t o[32];
-            tmem_ld_32x32b_x32(t_o + c * 32, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
-            tmem_st_32x32b_x32(t_o + c * 32, o);
-          }
+        if (kMaxFirst) {
+          exp_chunks(0, pk0, pk1, sum01, std::false_type());
+        } else {
+          // Optimistic first half: the exponentials of keys 0-63 are taken relative to the reference maximum the row
+          // already has, so they do not wait for the row maximum, and are computed again where that moves it (always on
+          // the first tile, whose reference is -infinity).  The stale reference cannot overflow what is kept: a value
+          // that would exceed 2^threshold is by construction one that moves it.
+          exp_chunks(0, pk0, pk1, sum01, std::true_type());
+          const bool redo = settle();
+          if (!ok) break;
+          if (redo) exp_chunks(0, pk0, pk1, sum01, std::false_type());
         }
-        if (redo) exp_chunks(0, m_ref, pk0, pk1, sum01, std::false_type());
         // P is written back over S chunk by chunk; a half of P (64 keys) that is complete lets the MMA warp start on it
         tmem_st_32x32b_x16(t_s, pk0);
         tmem_st_32x32b_x16(t_s + 16, pk1);
@@ -546,7 +563,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         tc_fence_before_sync();
         mbar_arrive(&p_ready[q]);
         float2 sum23;
-        exp_chunks(2, m_ref, pk0, pk1, sum23, std::false_type());
+        exp_chunks(2, pk0, pk1, sum23, std::false_type());
         tmem_st_32x32b_x16(t_s + 32, pk0);
         tmem_st_32x32b_x16(t_s + 48, pk1);
         tmem_st_wait();
