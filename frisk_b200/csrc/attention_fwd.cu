@@ -55,7 +55,9 @@ struct AttnSmem {
 };
 
 
-template <bool BF16, int D, bool OUT_F32, bool NORM>
+// SPLIT: an item is ONE query tile, whose key tiles the two softmax groups (and MMA threads) take in turn, even and odd
+// ones, each with its own S, P, O and statistics; at the end the halves are put together.
+template <bool BF16, int D, bool OUT_F32, bool NORM, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
     attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                          const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
@@ -80,7 +82,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* item_full = bars + 20;      // [2] the producer has published the id of a work item
   uint64_t* item_empty = bars + 22;     // [2] every consumer has read it
   uint64_t* q_empty = bars + 24;        // [1] both MMA threads are done with the Q tiles
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
+  uint64_t* xchg = bars + 26;           // [1] the two softmax groups meet (SPLIT only)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile int* item_slot = reinterpret_cast<volatile int*>(tmem_slot + 2);  // [2]
 
@@ -89,7 +92,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   // together); inside a chunk the heavy (late) query tiles of every head first, so that the machine
   // drains on light items.
   struct Item {
-    int bh, m0, nq[2], n_max;
+    int bh, m0;
+    int nq[2];  // key tiles of softmax group 0 and 1
+    int n_max;  // key tiles that are loaded
   };
   const int bh_total = (int)(p.total_items / p.n_groups);
   auto decode = [&](int t) {
@@ -101,9 +106,16 @@ __global__ void __launch_bounds__(kThreads, 1)
     Item it;
     it.bh = chunk * kHeadChunk + within % heads_here;
     it.m0 = group * p.group_rows;
-    it.nq[0] = kv_tiles_for(it.m0, p.S_q, p.S_kv, p.causal);
-    it.nq[1] = p.group_rows > BM ? kv_tiles_for(it.m0 + BM, p.S_q, p.S_kv, p.causal) : 0;
-    it.n_max = max(it.nq[0], it.nq[1]);
+    const int n0 = kv_tiles_for(it.m0, p.S_q, p.S_kv, p.causal);
+    if (SPLIT) {
+      it.nq[0] = (n0 + 1) / 2;
+      it.nq[1] = n0 / 2;
+      it.n_max = n0;
+    } else {
+      it.nq[0] = n0;
+      it.nq[1] = p.group_rows > BM ? kv_tiles_for(it.m0 + BM, p.S_q, p.S_kv, p.causal) : 0;
+      it.n_max = max(it.nq[0], it.nq[1]);
+    }
     return it;
   };
   // Consumers (the two MMA threads, the softmax warps) learn the n-th item of this CTA from the producer:
@@ -119,18 +131,18 @@ __global__ void __launch_bounds__(kThreads, 1)
   constexpr int first_pass = NORM ? 0 : 1;
   // Where the row maximum is taken: before the group's turn, on the ALU while the other group keeps the special-function
   // unit busy, or within it, run through the first exponentials.  Before is faster where the turns set the pace: D = 64, whose
-  // MMAs are half as long (8 x 32 heads x 2048 causal 274 -> 251 us, 3 x 16 x 1500 57.8 -> 51.7).  At
-  // D = 128 P.V and the next S set it, and long runs the power limit (930 W): 8 x 32 x 4096 causal 1173 -> 1183, 8 heads x 8192
-  // 279 -> 289.
-  constexpr bool kMaxFirst = D == 64;
+  // MMAs are half as long (8 x 32 heads x 2048 causal 274 -> 251 us, 3 x 16 x 1500 57.8 -> 51.7), and a lone query tile.  At
+  // D = 128 P.V and the next S set it, and long runs the power limit (930 W): before is slower there (8 x 32 x 4096 causal 1120
+  // -> 1145 us, 8 heads x 8192 272 -> 284).
+  constexpr bool kMaxFirst = D == 64 || SPLIT;
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], 2);  // one arrival per MMA-issuing thread
+      mbar_init(&k_empty[i], SPLIT ? 1 : 2);  // one arrival per MMA-issuing thread that reads the stage
       mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], 2);
+      mbar_init(&v_empty[i], SPLIT ? 1 : 2);
       mbar_init(&s_full[i], 1);
       mbar_init(&p_ready[i], 128);
       mbar_init(&p_ready_hi[i], 128);
@@ -140,6 +152,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(&item_empty[i], 10);  // two MMA threads, one lane of each of the eight softmax warps
     }
     mbar_init(q_empty, 2);
+    mbar_init(xchg, 256);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_q);
@@ -178,7 +191,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const Item it = decode(t);
         // the Q tiles of the item before are free when both MMA threads have issued their last S of it
         if (n > 0 && !mbar_wait(q_empty, (n - 1) & 1, abort_flag, p.status, ST_ATTN_Q)) break;
-        const int q_tiles = it.nq[1] > 0 ? 2 : 1;  // (nothing reads the second tile's place where there is none)
+        const int q_tiles = it.nq[1] > 0 && !SPLIT ? 2 : 1;  // (no query reads the second tile's place where there is none)
         mbar_expect_tx(q_full, q_tiles * L::kTileBytes);
         for (int q = 0; q < q_tiles; ++q)
 #pragma unroll
@@ -226,20 +239,22 @@ __global__ void __launch_bounds__(kThreads, 1)
       constexpr uint32_t idesc_o = umma_idesc_f16(BM, D, BF16, false, true);
       const uint32_t sq = smem_u32(smem + L::kQ), sk = smem_u32(smem + L::kK), sv = smem_u32(smem + L::kV);
       // descriptors are built once; the k16 slices only add a constant to the start-address field
-      const uint64_t dq = umma_desc_kmajor_sw128(sq + mq * L::kTileBytes);
+      const uint64_t dq = umma_desc_kmajor_sw128(sq + (SPLIT ? 0 : mq * L::kTileBytes));
       const uint64_t dk[2] = {umma_desc_kmajor_sw128(sk), umma_desc_kmajor_sw128(sk + L::kTileBytes)};
       const uint64_t dv[2] = {umma_desc_mnmajor_sw128(sv, kBoxBytes, 1024),
                               umma_desc_mnmajor_sw128(sv + L::kTileBytes, kBoxBytes, 1024)};
       const uint32_t t_sq = tmem_base + mq * 128;        // S_q; P_q aliases its first 64 columns (8 per k16 slice)
       const uint32_t t_oq = tmem_base + 256 + mq * 128;  // O_q
-      int kt = 0, vt = 0;  // K / V tiles seen so far, over all items (ring positions; K is streamed once per pass)
-      int steps = 0;       // (pass, key tile) steps of THIS query tile so far: the phase of s_full / p_ready
+      int kt0 = 0, vt0 = 0;  // K / V tiles of earlier passes and items (ring positions; K is streamed once per pass)
+      int steps = 0;         // (pass, key tile) steps of THIS softmax group so far: the phase of s_full / p_ready
+      const int j_first = SPLIT ? mq : 0, j_step = SPLIT ? 2 : 1;
       bool ok = true;
       for (int n = 0; ok; ++n) {
         const int t = next_item(n, true);
         if (t < 0) break;
         const Item it = decode(t);
         const int n_mine = it.nq[mq], n_max = it.n_max;
+        const int j_end = j_first + n_mine * j_step;  // one step beyond the last key tile of this group
         ok = mbar_wait(q_full, n & 1, abort_flag, p.status, ST_ATTN_Q);
         for (int pass = first_pass; pass < 2 && ok; ++pass) {
           const bool stats_pass = pass == 0;  // the pass that only gathers statistics issues no P.V
@@ -249,12 +264,13 @@ __global__ void __launch_bounds__(kThreads, 1)
           // MMAs of S(j+1) have been issued (a commit covers everything issued before it, so they only fire a
           // little later than strictly possible).
           bool have_k = false;  // K(j) of the current pass is known to have landed
-          for (int j = 0; j < n_max && ok; ++j, ++kt) {
+          for (int j = j_first; j < n_max && ok; j += j_step) {
+            const int kt = kt0 + j, vt = vt0 + j;
             const int ks = kt % kStagesKV;
             if (!have_k) ok = mbar_wait(&k_full[ks], (kt / kStagesKV) & 1, abort_flag, p.status, ST_ATTN_KV);
             have_k = false;
             if (!ok) break;
-            if (j < n_mine) {
+            if (j < j_end) {
               tc_fence_after_sync();
 #pragma unroll
               for (int kk = 0; kk < D / 16; ++kk) {
@@ -263,19 +279,20 @@ __global__ void __launch_bounds__(kThreads, 1)
               }
               umma_commit(&s_full[mq]);
               umma_commit(&k_empty[ks]);  // this tile's use of the K stage ends when these MMAs have read it
-              if (j > 0 && !stats_pass) {  // (deferred from the previous tile)
+              if (j > 0 && !stats_pass && !SPLIT) {  // (deferred from the previous tile)
                 umma_commit(&o_done[mq]);
                 umma_commit(&v_empty[(vt - 1) % kStagesKV]);
               }
-              if (pass == 1 && j == n_mine - 1) umma_commit(q_empty);  // this thread's last use of the Q tiles
+              if (pass == 1 && j + j_step == j_end) umma_commit(q_empty);  // this thread's last use of the Q tiles
             } else {
               mbar_arrive(&k_empty[ks]);  // a key tile only the other query tile needs
             }
             const int vs = vt % kStagesKV;
-            if (j < n_mine) {
+            if (j < j_end) {
               // the next K tile, while the softmax group works on this one
-              if (j + 1 < n_max) {
-                ok = mbar_wait(&k_full[(kt + 1) % kStagesKV], ((kt + 1) / kStagesKV) & 1, abort_flag, p.status, ST_ATTN_KV);
+              if (j + j_step < n_max) {
+                const int kn = kt + j_step;
+                ok = mbar_wait(&k_full[kn % kStagesKV], (kn / kStagesKV) & 1, abort_flag, p.status, ST_ATTN_KV);
                 have_k = ok;
               }
               if (!stats_pass && ok) ok = mbar_wait(&v_full[vs], (vt / kStagesKV) & 1, abort_flag, p.status, ST_ATTN_KV);
@@ -293,10 +310,11 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                 for (int kk = half * 4; kk < half * 4 + 4; ++kk)
                   umma_f16_ts(t_oq, t_sq + kk * 8, dv[vs] + static_cast<uint64_t>((kk * 2048) >> 4), idesc_o,
-                              (j | kk) != 0);
+                              j != j_first || kk != 0);
               }
               if (!ok) break;
-              if (!stats_pass && (j + 1 >= n_mine)) {  // no further S of this item follows: publish now
+              // no further S of this item follows, or the next V tile of this group waits for the stage: publish now
+              if (!stats_pass && (SPLIT || j + 1 >= n_mine)) {
                 umma_commit(&o_done[mq]);
                 umma_commit(&v_empty[vs]);
               }
@@ -304,8 +322,9 @@ __global__ void __launch_bounds__(kThreads, 1)
               ok = mbar_wait(&v_full[vs], (vt / kStagesKV) & 1, abort_flag, p.status, ST_ATTN_KV);
               if (ok) mbar_arrive(&v_empty[vs]);
             }
-            if (!stats_pass) ++vt;
           }
+          kt0 += n_max;
+          if (!stats_pass) vt0 += n_max;
         }
         if (ok && n_mine == 0) mbar_arrive(q_empty);  // (a query tile beyond the end of the sequence)
       }
@@ -314,7 +333,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
     // ------------------------------------------------------------------ softmax groups
-    const int q = warp >> 2;         // query tile of this group
+    const int q = warp >> 2;         // this group: its query tile, or its share of the key tiles
     const int quad = warp & 3;       // TMEM lane quadrant this warp may touch
     const int row = quad * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
@@ -324,15 +343,31 @@ __global__ void __launch_bounds__(kThreads, 1)
     int steps = 0;    // (pass, key tile) steps of this query tile so far, over all items: the phase of s_full
     int turns = 0;    // key-tile iterations so far: the phase of the turn barriers
     int pv_base = 0;  // key tiles whose P.V was issued for earlier items: the phase of o_done
+    int meets = 0;    // meetings of the two groups so far: the phase of xchg
     bool ok = true;
+    // Split keys: the two groups meet, and each thread learns what the other group's thread of its row brings.  The
+    // statistics lie in the second query tile's place, which nothing else uses then, in two sets that alternate: a set is
+    // written again only when everybody has arrived at the meeting in between, after reading it.
+    auto meet = [&](float2 mine_v) -> float2 {
+      float2* set = reinterpret_cast<float2*>(smem + L::kQ + L::kTileBytes) + (meets & 1) * 2 * BM;
+      set[q * BM + row] = mine_v;
+      tc_fence_before_sync();
+      mbar_arrive(xchg);
+      if (!mbar_wait(xchg, meets & 1, abort_flag, p.status, ST_ATTN_O)) ok = false;
+      ++meets;
+      tc_fence_after_sync();
+      return set[(q ^ 1) * BM + row];
+    };
 
     for (int n = 0; ok; ++n) {
       const int item_id = next_item(n, lane == 0);
       if (item_id < 0) break;
       const Item it = decode(item_id);
-      const int bh = it.bh, n_max = it.n_max;
+      const int bh = it.bh, n_max = max(it.nq[0], it.nq[1]);
       const int n_tiles = it.nq[q];
-      const int m_tile = it.m0 + q * BM;
+      const int m_tile = it.m0 + (SPLIT ? 0 : q * BM);
+      // (both groups have read both O of the item before)
+      if (SPLIT && n > 0) meet(make_float2(0.f, 0.f));
       const int g_row = m_tile + row;  // query index within the head
       float m_ref = -INFINITY;  // reference maximum (scaled, log2 units) the stored P and O are relative to
       float l_sum = 0.f;
@@ -349,9 +384,22 @@ __global__ void __launch_bounds__(kThreads, 1)
         auto exp2_of = [](float x) { return BF16 ? ex2f_ieee_range(x) : ex2f(x); };
         float m_run = -INFINITY, l_run = 0.f;
         for (int pass = 0; pass < 2 && ok; ++pass) {
+          if (SPLIT && pass == 1) {
+            // the other group's half of the keys
+            const float2 o = meet(make_float2(m_run, l_run));
+            const float m_all = fmaxf(m_run, o.x);
+            auto share = [&](float m, float l) {
+              return m == -INFINITY ? 0.f : l * ex2f_ieee_range(__fmul_rn(__fsub_rn(m, m_all), kLog2e));
+            };
+            const float a = share(m_run, l_run), b = share(o.x, o.y);
+            l_run = a + b;
+            m_run = m_all;
+            if (!ok) break;
+          }
           const float inv_l = __frcp_rn(l_run);  // (of use in pass 1 only)
           const float2 inv2 = make_float2(inv_l, inv_l), negl2 = make_float2(-l_run, -l_run);
-          for (int j = 0; j < n_tiles; ++j) {
+          for (int i = 0; i < n_tiles; ++i) {
+            const int j = SPLIT ? 2 * i + q : i;
             if (!mbar_wait(&s_full[q], steps & 1, abort_flag, p.status, ST_ATTN_S)) {
               ok = false;
               break;
@@ -433,6 +481,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
         l_sum = 1.0f;  // P is already normalised
+        m_ref = 0.f;
       } else
       // The two softmax groups take turns: group 1 starts the arithmetic of its key tile j when group 0 has
       // finished that of its tile j (all 128 keys: handing over after the first 64 measured 3 % slower), and group 0
@@ -455,7 +504,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(t_s + c * 32, sr[c]);
           tmem_ld_wait();
 
-          const int n0 = i * BN;
+          const int n0 = (SPLIT ? 2 * i + q : i) * BN;
           const bool needs_mask = (n0 + BN > p.S_kv) || (p.causal && (n0 + BN - 1 > m_tile + off));
           if (needs_mask) {
             int limit = p.S_kv - 1;
@@ -576,17 +625,55 @@ __global__ void __launch_bounds__(kThreads, 1)
 
       // ---- epilogue: O / l
       if (ok && n_tiles > 0) ok = mbar_wait(&o_done[q], (pv_base + n_tiles - 1) & 1, abort_flag, p.status, ST_ATTN_O);
-      if (ok && n_tiles > 0) {
+      float f_first = 0.f, f_second = 0.f;
+      int c_begin = 0, c_end = D / 32;  // 32-column chunks of O this group stores
+      if (SPLIT) {
+        const float2 other = meet(make_float2(m_ref, l_sum));
+        if (NORM) {
+          f_first = f_second = 1.0f;
+        } else {
+          // O = (O0 2^(m0 - m) + O1 2^(m1 - m)) / (l0 2^(m0 - m) + l1 2^(m1 - m)); a half that saw no key counts for nothing
+          const float l0 = q == 0 ? l_sum : other.y, l1 = q == 0 ? other.y : l_sum;
+          const float m0 = l0 == 0.f ? -INFINITY : (q == 0 ? m_ref : other.x);
+          const float m1 = l1 == 0.f ? -INFINITY : (q == 0 ? other.x : m_ref);
+          const float m = fmaxf(m0, m1);
+          const float w0 = m0 == -INFINITY ? 0.f : ex2f(m0 - m), w1 = m1 == -INFINITY ? 0.f : ex2f(m1 - m);
+          const float l = l0 * w0 + l1 * w1;
+          f_first = w0 / l;
+          f_second = w1 / l;
+        }
+        // each group stores half of the columns, but a 16-bit row of D = 64 is one box, which group 0 stores
+        if (D == 64 && !OUT_F32) {
+          c_end = q == 0 ? D / 32 : 0;
+        } else {
+          c_begin = q * (D / 64);
+          c_end = c_begin + D / 64;
+        }
+      }
+      if (ok && (SPLIT || n_tiles > 0)) {
         tc_fence_after_sync();
-        const float inv = 1.0f / l_sum;
+        const float inv = SPLIT ? 1.0f : 1.0f / l_sum;  // (the halves are scaled as they are put together)
         const bool valid = g_row < p.S_q;
         const size_t row_off = ((size_t)bh * p.S_q + (size_t)min(g_row, p.S_q - 1)) * D;
         uint32_t packed[32];
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
+          if (SPLIT && (c < c_begin || c >= c_end)) continue;
           uint32_t o[32];
-          tmem_ld_32x32b_x32(t_o + c * 32, o);
+          tmem_ld_32x32b_x32((SPLIT ? t_o - q * 128 : t_o) + c * 32, o);
           tmem_ld_wait();
+          if (SPLIT) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f_first);
+            if (it.nq[1] > 0) {  // (group 0 always has a key tile)
+              uint32_t o1[32];
+              tmem_ld_32x32b_x32(t_o - q * 128 + 128 + c * 32, o1);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                o[i] = __float_as_uint(__fmaf_rn(__uint_as_float(o1[i]), f_second, __uint_as_float(o[i])));
+            }
+          }
           if (valid) {
             if (OUT_F32) {
               float4* dst = reinterpret_cast<float4*>(static_cast<float*>(p.O) + row_off + c * 32);
@@ -649,7 +736,15 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-template <bool BF16, int D, bool OUT_F32, bool NORM>
+// Items of ONE query tile where that still leaves at most one item per SM: half the items' SMs would stand idle
+// otherwise, and a tile alone on its SM takes about 0.6 of the time two tiles take side by side (so from one item
+// per SM upwards pairs are the better use of it).
+bool one_tile_items(const frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d) {
+  const int64_t tiles = (d.S_q + BM - 1) / BM;
+  return tiles * d.B * d.H <= ctx->num_sms;
+}
+
+template <bool BF16, int D, bool OUT_F32, bool NORM, bool SPLIT>
 int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K, const void* V,
                void* O, cudaStream_t s) {
   CUtensorMap tq, tk, tv;
@@ -668,11 +763,7 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q
   AttnParams p;
   p.S_q = d.S_q;
   p.S_kv = d.S_kv;
-  // Items of ONE query tile where that still leaves at most one item per SM: half the items' SMs would stand idle
-  // otherwise, and a tile alone on its SM takes about 0.6 of the time two tiles take side by side (so from one item
-  // per SM upwards pairs are the better use of it).
-  const int64_t tiles = (d.S_q + BM - 1) / BM;
-  p.group_rows = tiles * bh <= ctx->num_sms ? BM : 2 * BM;
+  p.group_rows = one_tile_items(ctx, d) ? BM : 2 * BM;
   p.n_groups = (d.S_q + p.group_rows - 1) / p.group_rows;
   p.causal = d.causal ? 1 : 0;
   p.total_items = (int64_t)p.n_groups * bh;
@@ -683,7 +774,7 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q
   p.status = ctx->d_status;
   p.work = ctx->d_status + 16;  // work counter and exit counter of the persistent grid (zero between launches)
   if (p.total_items > INT32_MAX) return FRISK_B200_E_ATTN_SHAPE;
-  auto kern = attention_fwd_kernel<BF16, D, OUT_F32, NORM>;
+  auto kern = attention_fwd_kernel<BF16, D, OUT_F32, NORM, SPLIT>;
   using L = AttnSmem<D>;
   // setmaxnreg.inc waits (without a bound) until the CTA's own register pool holds what it
   // asks for: the registers the TMA/MMA warpgroup (128 threads) gives up must cover what the
@@ -716,15 +807,26 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q
   return 0;
 }
 
+template <bool BF16, int D, bool OUT_F32, bool NORM>
+int launch_split(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K, const void* V,
+                 void* O, cudaStream_t s) {
+  // A lone query tile's key tiles go to the two softmax groups in turn, where there are two at all: one group alone is
+  // bound by the chain S -> softmax -> P.V -> next S (1.4 us a key tile at D = 64 normalised), and two such chains overlap.
+  // 16 heads x 1025 normalised 29.3 -> 24.9 us; single pass, D = 128: 4 heads x 4096 causal 62.2 -> 45.9, 2 x 8192 121.6 -> 86.7,
+  // 8 x 1000 19.7 -> 16.4; one key tile has nothing to share.
+  if (one_tile_items(ctx, d) && d.S_kv > BN) return launch_cfg<BF16, D, OUT_F32, NORM, true>(ctx, d, Q, K, V, O, s);
+  return launch_cfg<BF16, D, OUT_F32, NORM, false>(ctx, d, Q, K, V, O, s);
+}
+
 template <bool BF16, int D>
 int launch_out(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K, const void* V,
                void* O, cudaStream_t s) {
   if (d.normalize_p) {
-    if (d.dtype_out == FRISK_B200_F32) return launch_cfg<BF16, D, true, true>(ctx, d, Q, K, V, O, s);
-    return launch_cfg<BF16, D, false, true>(ctx, d, Q, K, V, O, s);
+    if (d.dtype_out == FRISK_B200_F32) return launch_split<BF16, D, true, true>(ctx, d, Q, K, V, O, s);
+    return launch_split<BF16, D, false, true>(ctx, d, Q, K, V, O, s);
   }
-  if (d.dtype_out == FRISK_B200_F32) return launch_cfg<BF16, D, true, false>(ctx, d, Q, K, V, O, s);
-  return launch_cfg<BF16, D, false, false>(ctx, d, Q, K, V, O, s);
+  if (d.dtype_out == FRISK_B200_F32) return launch_split<BF16, D, true, false>(ctx, d, Q, K, V, O, s);
+  return launch_split<BF16, D, false, false>(ctx, d, Q, K, V, O, s);
 }
 
 }  // namespace

@@ -392,3 +392,58 @@ def test_execution_packet_runs_on_the_attention_kernel(ctx):
     torch.cuda.synchronize()
     assert torch.equal(a, b)
     assert np.array_equal(b.cpu().numpy().view(np.uint32), g[key + "/strict"][0, 1].view(np.uint32))
+
+
+# ------------------------------------------------------------------ a lone query tile's keys, split between the softmax groups
+@pytest.mark.parametrize("s_q,s_kv,causal", [
+    (128, 129, False),   # two key tiles, the second with one key
+    (17, 256, False),
+    (128, 257, True),    # three key tiles: the groups have two and one
+    (100, 150, True),    # rows that see no key of the second tile
+    (300, 300, True),    # the first query tile has one key tile: the second group has none
+    (129, 1025, True),
+    (40, 2100, False),
+])
+@pytest.mark.parametrize("D,dtype,out_dtype", [(64, "fp16", "fp16"), (64, "bf16", "fp32"), (128, "bf16", "bf16"), (128, "fp16", "fp32")])
+def test_lone_tiles_split_their_keys(ctx, s_q, s_kv, causal, D, dtype, out_dtype):
+    check(ctx, 1, 3, s_q, s_kv, D, dtype, causal, 60 + s_q + s_kv, out_dtype=out_dtype)
+
+
+@pytest.mark.parametrize("normalize_p", [0, 1])
+@pytest.mark.parametrize("high", [0, 1])
+def test_split_halves_with_far_maxima(ctx, high, normalize_p):
+    """Scores of one group's keys about 2^380 times the other's: the lower half must vanish without a NaN."""
+    import torch
+    rng = np.random.default_rng(77 + high)
+    from oracle.numerics import to_storage
+    S, D = 512, 64
+    q = to_storage(np.full((1, 2, 128, D), 1.0, np.float32), "fp16")
+    sign = np.where(np.arange(S) // 128 % 2 == high, 1.0, -1.0).astype(np.float32)
+    k = to_storage((sign[None, None, :, None] * 2.0625 + 0.05 * rng.standard_normal((1, 2, S, D))).astype(np.float32), "fp16")
+    v = to_storage(rng.standard_normal((1, 2, S, D), dtype=np.float32), "fp16")
+    gq, gk, gv = (Guarded(x.shape, "fp16", fill=x) for x in (q, k, v))
+    go = Guarded((1, 2, 128, D), "fp32")
+    go.view.fill_(float("nan"))
+    desc = capi.attn_desc(1, 2, 128, S, D, 1.0, False, "fp16", "fp32", normalize_p=normalize_p)
+    s = torch.cuda.current_stream().cuda_stream
+    ctx.attention_fwd(desc, gq.view.data_ptr(), gk.view.data_ptr(), gv.view.data_ptr(), go.view.data_ptr(), stream=s)
+    ctx.check(s)
+    assert go.guards_intact()
+    got, ref = go.host(), ao.attention_fwd(q, k, v, "fp16", 1.0, causal=False, mode="fp64")
+    assert np.isfinite(got).all() and rel_frobenius(got, ref) <= TOL
+
+
+def test_split_rows_with_nan_stay_their_own(ctx):
+    """A NaN in one query row reaches that row's results (through either group's keys) and no other row's."""
+    import torch
+    rng = np.random.default_rng(78)
+    q, k, v = (torch.tensor(rng.standard_normal((1, 1, 384, 128), dtype=np.float32)).to("cuda", torch.bfloat16) for _ in range(3))
+    q = q[:, :, :128].contiguous()
+    q[0, 0, 5, 3] = float("nan")
+    o = torch.empty_like(q)
+    desc = capi.attn_desc(1, 1, 128, 384, 128, 128 ** -0.5, False, "bf16", "bf16")
+    s = torch.cuda.current_stream().cuda_stream
+    ctx.attention_fwd(desc, q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), stream=s)
+    ctx.check(s)
+    bad = torch.isnan(o[0, 0]).all(1).cpu().numpy()
+    assert bad[5] and np.isfinite(o[0, 0].float().cpu().numpy()[np.arange(128) != 5]).all()
