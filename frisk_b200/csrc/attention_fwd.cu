@@ -126,6 +126,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (arrive) mbar_arrive(&item_empty[n & 1]);
     return t;
   };
+  // The ring of K and V: tile n goes to stage n % 2, and both MMA threads follow every tile.  SPLIT: each stage belongs to one MMA
+  // thread and n counts that stage's tiles, because a thread that does not follow all uses of a stage can mistake an earlier
+  // phase of its barrier for its own (with an odd number of key tiles the threads would change stages from pass to pass).
+  auto ring_phase = [](int n) -> uint32_t { return (SPLIT ? n : n / kStagesKV) & 1; };
   // Normalised mode runs the key loop twice: pass 0 only gathers row maxima and row sums, pass 1
   // is the pass every mode has.  Barrier phases keep counting across passes and items.
   constexpr int first_pass = NORM ? 0 : 1;
@@ -178,7 +182,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == kWarpTma) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      int kt = 0, vt = 0;  // K / V tiles loaded so far, over all items (K is streamed once per pass)
+      // K / V tiles loaded so far, over all items (K is streamed once per pass); SPLIT: into either stage
+      int kt = 0, vt = 0, kt_odd = 0, vt_odd = 0;
       bool ok = true;
       for (int n = 0; ok; ++n) {
         // take the next item and tell the other roles (slot n & 1 was last used by item n - 2)
@@ -199,8 +204,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             tma_load_3d(smem + L::kQ + q * L::kTileBytes + b * kBoxBytes, &tmap_q, q_full, b * 64, it.m0 + q * BM, it.bh);
         for (int pass = first_pass; pass < 2 && ok; ++pass) {
           for (int j = 0; j < it.n_max; ++j) {
-            const int ks = kt % kStagesKV;
-            if (!mbar_wait(&k_empty[ks], ((kt / kStagesKV) & 1) ^ 1, abort_flag, p.status, ST_ATTN_KV)) {
+            const bool odd = SPLIT && (j & 1);  // the second group's key tile
+            const int kp = odd ? kt_odd++ : kt++, vp = odd ? vt_odd : vt;
+            const int ks = SPLIT ? (int)odd : kp % kStagesKV;
+            if (!mbar_wait(&k_empty[ks], ring_phase(kp) ^ 1, abort_flag, p.status, ST_ATTN_KV)) {
               ok = false;
               break;
             }
@@ -208,10 +215,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int b = 0; b < kBoxes; ++b)
               tma_load_3d(smem + L::kK + ks * L::kTileBytes + b * kBoxBytes, &tmap_k, &k_full[ks], b * 64, j * BN, it.bh);
-            ++kt;
             if (pass == 0) continue;  // the statistics pass needs no values
-            const int vs = vt % kStagesKV;
-            if (!mbar_wait(&v_empty[vs], ((vt / kStagesKV) & 1) ^ 1, abort_flag, p.status, ST_ATTN_KV)) {
+            (odd ? vt_odd : vt)++;
+            const int vs = SPLIT ? (int)odd : vp % kStagesKV;
+            if (!mbar_wait(&v_empty[vs], ring_phase(vp) ^ 1, abort_flag, p.status, ST_ATTN_KV)) {
               ok = false;
               break;
             }
@@ -219,7 +226,6 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int b = 0; b < kBoxes; ++b)
               tma_load_3d(smem + L::kV + vs * L::kTileBytes + b * kBoxBytes, &tmap_v, &v_full[vs], b * 64, j * BN, it.bh);
-            ++vt;
           }
         }
       }
@@ -245,16 +251,15 @@ __global__ void __launch_bounds__(kThreads, 1)
                               umma_desc_mnmajor_sw128(sv + L::kTileBytes, kBoxBytes, 1024)};
       const uint32_t t_sq = tmem_base + mq * 128;        // S_q; P_q aliases its first 64 columns (8 per k16 slice)
       const uint32_t t_oq = tmem_base + 256 + mq * 128;  // O_q
-      int kt0 = 0, vt0 = 0;  // K / V tiles of earlier passes and items (ring positions; K is streamed once per pass)
+      int kt = 0, vt = 0;    // K / V tiles seen so far, over all items (ring positions; K is streamed once per pass)
       int steps = 0;         // (pass, key tile) steps of THIS softmax group so far: the phase of s_full / p_ready
-      const int j_first = SPLIT ? mq : 0, j_step = SPLIT ? 2 : 1;
+      auto ring_stage = [&](int n) -> int { return SPLIT ? mq : n % kStagesKV; };
       bool ok = true;
       for (int n = 0; ok; ++n) {
         const int t = next_item(n, true);
         if (t < 0) break;
         const Item it = decode(t);
-        const int n_mine = it.nq[mq], n_max = it.n_max;
-        const int j_end = j_first + n_mine * j_step;  // one step beyond the last key tile of this group
+        const int n_mine = it.nq[mq], n_max = SPLIT ? n_mine : it.n_max;  // key tiles: used, followed
         ok = mbar_wait(q_full, n & 1, abort_flag, p.status, ST_ATTN_Q);
         for (int pass = first_pass; pass < 2 && ok; ++pass) {
           const bool stats_pass = pass == 0;  // the pass that only gathers statistics issues no P.V
@@ -264,13 +269,12 @@ __global__ void __launch_bounds__(kThreads, 1)
           // MMAs of S(j+1) have been issued (a commit covers everything issued before it, so they only fire a
           // little later than strictly possible).
           bool have_k = false;  // K(j) of the current pass is known to have landed
-          for (int j = j_first; j < n_max && ok; j += j_step) {
-            const int kt = kt0 + j, vt = vt0 + j;
-            const int ks = kt % kStagesKV;
-            if (!have_k) ok = mbar_wait(&k_full[ks], (kt / kStagesKV) & 1, abort_flag, p.status, ST_ATTN_KV);
+          for (int j = 0; j < n_max && ok; ++j, ++kt) {
+            const int ks = ring_stage(kt);
+            if (!have_k) ok = mbar_wait(&k_full[ks], ring_phase(kt), abort_flag, p.status, ST_ATTN_KV);
             have_k = false;
             if (!ok) break;
-            if (j < j_end) {
+            if (j < n_mine) {
               tc_fence_after_sync();
 #pragma unroll
               for (int kk = 0; kk < D / 16; ++kk) {
@@ -283,19 +287,19 @@ __global__ void __launch_bounds__(kThreads, 1)
                 umma_commit(&o_done[mq]);
                 umma_commit(&v_empty[(vt - 1) % kStagesKV]);
               }
-              if (pass == 1 && j + j_step == j_end) umma_commit(q_empty);  // this thread's last use of the Q tiles
+              if (pass == 1 && j == n_mine - 1) umma_commit(q_empty);  // this thread's last use of the Q tiles
             } else {
               mbar_arrive(&k_empty[ks]);  // a key tile only the other query tile needs
             }
-            const int vs = vt % kStagesKV;
-            if (j < j_end) {
-              // the next K tile, while the softmax group works on this one
-              if (j + j_step < n_max) {
-                const int kn = kt + j_step;
-                ok = mbar_wait(&k_full[kn % kStagesKV], (kn / kStagesKV) & 1, abort_flag, p.status, ST_ATTN_KV);
+            const int vs = ring_stage(vt);
+            if (j < n_mine) {
+              // the next K tile, while the softmax group works on this one (SPLIT: it comes behind a V tile whose stage the
+              // other thread has yet to release, and must not hold up this thread's P.V)
+              if (!SPLIT && j + 1 < n_max) {
+                ok = mbar_wait(&k_full[ring_stage(kt + 1)], ring_phase(kt + 1), abort_flag, p.status, ST_ATTN_KV);
                 have_k = ok;
               }
-              if (!stats_pass && ok) ok = mbar_wait(&v_full[vs], (vt / kStagesKV) & 1, abort_flag, p.status, ST_ATTN_KV);
+              if (!stats_pass && ok) ok = mbar_wait(&v_full[vs], ring_phase(vt), abort_flag, p.status, ST_ATTN_KV);
               // O_q += P_q(j) . V(j).  The softmax group publishes P in two halves (64 keys each), so the first
               // four k16 slices start while the second half is still being exponentiated.  In the statistics
               // pass the two waits only tell that the softmax group is done with S_q.
@@ -310,7 +314,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                 for (int kk = half * 4; kk < half * 4 + 4; ++kk)
                   umma_f16_ts(t_oq, t_sq + kk * 8, dv[vs] + static_cast<uint64_t>((kk * 2048) >> 4), idesc_o,
-                              j != j_first || kk != 0);
+                              (j | kk) != 0);
               }
               if (!ok) break;
               // no further S of this item follows, or the next V tile of this group waits for the stage: publish now
@@ -319,12 +323,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 umma_commit(&v_empty[vs]);
               }
             } else if (!stats_pass) {
-              ok = mbar_wait(&v_full[vs], (vt / kStagesKV) & 1, abort_flag, p.status, ST_ATTN_KV);
+              ok = mbar_wait(&v_full[vs], ring_phase(vt), abort_flag, p.status, ST_ATTN_KV);
               if (ok) mbar_arrive(&v_empty[vs]);
             }
+            if (!stats_pass) ++vt;
           }
-          kt0 += n_max;
-          if (!stats_pass) vt0 += n_max;
         }
         if (ok && n_mine == 0) mbar_arrive(q_empty);  // (a query tile beyond the end of the sequence)
       }
@@ -812,8 +815,8 @@ int launch_split(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void*
                  void* O, cudaStream_t s) {
   // A lone query tile's key tiles go to the two softmax groups in turn, where there are two at all: one group alone is
   // bound by the chain S -> softmax -> P.V -> next S (1.4 us a key tile at D = 64 normalised), and two such chains overlap.
-  // 16 heads x 1025 normalised 29.3 -> 24.9 us; single pass, D = 128: 4 heads x 4096 causal 62.2 -> 45.9, 2 x 8192 121.6 -> 86.7,
-  // 8 x 1000 19.7 -> 16.4; one key tile has nothing to share.
+  // 16 heads x 1025 normalised 29.2 -> 23.4 us; single pass, D = 128: 4 heads x 4096 causal 62.1 -> 40.4, 2 x 8192 121.4 -> 75.3,
+  // 8 x 1000 19.8 -> 15.2; D = 64: 4 x 3000 42.5 -> 27.5; one key tile has nothing to share.
   if (one_tile_items(ctx, d) && d.S_kv > BN) return launch_cfg<BF16, D, OUT_F32, NORM, true>(ctx, d, Q, K, V, O, s);
   return launch_cfg<BF16, D, OUT_F32, NORM, false>(ctx, d, Q, K, V, O, s);
 }

@@ -447,3 +447,18 @@ def test_split_rows_with_nan_stay_their_own(ctx):
     ctx.check(s)
     bad = torch.isnan(o[0, 0]).all(1).cpu().numpy()
     assert bad[5] and np.isfinite(o[0, 0].float().cpu().numpy()[np.arange(128) != 5]).all()
+
+
+def test_split_keys_odd_tile_counts_repeat(ctx):
+    """Nine and three key tiles, two passes: every launch gives the same bytes (each group follows its own stages of K and V)."""
+    import torch
+    rng = np.random.default_rng(79)
+    for heads, n in ((16, 1025), (37, 300)):
+        q, k, v = (torch.tensor(rng.standard_normal((1, heads, n, 64), dtype=np.float32)).to("cuda", torch.float16) for _ in range(3))
+        desc = capi.attn_desc(1, heads, n, n, 64, 0.125, False, "fp16", "fp32", normalize_p=1)
+        s = torch.cuda.current_stream().cuda_stream
+        out = [torch.empty(1, heads, n, 64, dtype=torch.float32, device="cuda") for _ in range(40)]
+        for o in out:
+            ctx.attention_fwd(desc, q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), stream=s)
+        ctx.check(s)
+        assert all(torch.equal(o, out[0]) for o in out[1:])
