@@ -739,12 +739,37 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-// Items of ONE query tile where that still leaves at most one item per SM: half the items' SMs would stand idle
-// otherwise, and a tile alone on its SM takes about 0.6 of the time two tiles take side by side (so from one item
-// per SM upwards pairs are the better use of it).
+// Items of ONE query tile or of two.  A lone tile has half of its SM's softmax and MMA threads idle where it cannot be split
+// (one key tile), but more items balance better.  So lone tiles are taken where that leaves at most one item per SM, and
+// beyond that where this estimate is clearly better: in steps (one key tile of two query tiles side by side, 2.1 us at D = 128), a pair of
+// tiles takes its key tiles, a split lone tile 0.56 a key tile (304 us for 8 x 8192 where pairs take 273), either 1.9 more to
+// begin and end; equal items go round by round, causal ones heavy first.  Estimated / measured ratios: 12 heads x 2048 causal 0.66 / 0.66
+// (44.2 -> 29.0 us; D = 64 34.9 -> 21.5), 15 x 2013 causal 0.79 / 0.72, 10 x 4096 causal 0.87 / 0.78, 64 x 700 normalised 0.93 / 0.84,
+// 64 x 1025 0.80 / 0.85; 24 x 1000 1.29 / 1.18, 8 x 8192 1.14 / 1.12, 64 x 2048 causal 1.14 / 1.23.  Of 68 shapes the estimate
+// is too low only for causal ones of few key tiles (50 x 612 0.93 / 1.18), and too high in the normalised mode (36 x 978 1.21 / 1.06):
+// hence 0.9 and 0.95.
+double items_estimate(const frisk_b200_attn_desc& d, int sms, int tiles_per_item) {
+  constexpr double kSplitStep = 0.56, kItem = 1.9;
+  const int64_t heads = (int64_t)d.B * d.H, tiles = (d.S_q + BM - 1) / BM;
+  const int64_t groups = (tiles + tiles_per_item - 1) / tiles_per_item, items = groups * heads;
+  const double step = (tiles_per_item == 1 ? kSplitStep : 1.0) * (d.normalize_p ? 2 : 1);
+  const int64_t all = (d.S_kv + BN - 1) / BN, off = (int64_t)d.S_kv - d.S_q;
+  const double heaviest = step * (double)all + kItem;
+  if (!d.causal) return (double)((items + sms - 1) / sms) * heaviest;
+  if (items <= sms) return heaviest;
+  double total = 0;
+  for (int64_t g = 0; g < groups; ++g) {
+    const int64_t last_row = std::min<int64_t>((g + 1) * tiles_per_item * BM, d.S_q) - 1;
+    total += step * (double)std::min<int64_t>(all, std::max<int64_t>(0, last_row + off) / BN + 1) + kItem;
+  }
+  return std::max(heaviest, (double)heads * total / sms + 0.5 * total / (double)groups);
+}
 bool one_tile_items(const frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d) {
-  const int64_t tiles = (d.S_q + BM - 1) / BM;
-  return tiles * d.B * d.H <= ctx->num_sms;
+  const int64_t tiles = (d.S_q + BM - 1) / BM * d.B * d.H;
+  if (tiles <= ctx->num_sms) return true;
+  // (four rounds of pairs balance by themselves)
+  if (d.S_kv <= BN || tiles > 8 * (int64_t)ctx->num_sms) return false;
+  return items_estimate(d, ctx->num_sms, 1) < (d.normalize_p ? 0.95 : 0.9) * items_estimate(d, ctx->num_sms, 2);
 }
 
 template <bool BF16, int D, bool OUT_F32, bool NORM, bool SPLIT>

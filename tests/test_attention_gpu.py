@@ -462,3 +462,33 @@ def test_split_keys_odd_tile_counts_repeat(ctx):
             ctx.attention_fwd(desc, q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), stream=s)
         ctx.check(s)
         assert all(torch.equal(o, out[0]) for o in out[1:])
+
+
+@pytest.mark.parametrize("shape,normalize_p", [
+    ((1, 12, 2048, 64, True), 0),   # 192 causal tiles: pairs would leave the SMs to their heaviest items
+    ((1, 10, 2304, 128, True), 0),  # 180 tiles, 18 key tiles
+    ((4, 16, 650, 64, False), 1),   # 384 equal tiles: three rounds of lone ones against two of pairs
+])
+def test_lone_tiles_beyond_one_a_cta(ctx, shape, normalize_p):
+    """More lone tiles than SMs, so a CTA takes several: the ring, the meetings and O's phases go on from item to item."""
+    import torch
+    B, H, S, D, causal = shape
+    rng = np.random.default_rng(80)
+    from oracle.numerics import to_storage
+    q, k, v = (to_storage(rng.standard_normal((B, H, S, D), dtype=np.float32), "fp16") for _ in range(3))
+    gq, gk, gv = (Guarded(x.shape, "fp16", fill=x) for x in (q, k, v))
+    go = Guarded((B, H, S, D), "fp16")
+    go.view.fill_(float("nan"))
+    desc = capi.attn_desc(B, H, S, S, D, D ** -0.5, causal, "fp16", "fp16", normalize_p=normalize_p)
+    s = torch.cuda.current_stream().cuda_stream
+    first = None
+    for _ in range(5):
+        ctx.attention_fwd(desc, gq.view.data_ptr(), gk.view.data_ptr(), gv.view.data_ptr(), go.view.data_ptr(), stream=s)
+        ctx.check(s)
+        first = go.host().copy() if first is None else first
+        assert np.array_equal(go.host(), first)
+    assert go.guards_intact()
+    heads = [0, 5, B * H - 1]
+    ref = ao.attention_fwd(q, k, v, "fp16", D ** -0.5, causal=causal, mode="fp64", heads=heads)
+    got = from_storage(first, "fp16").reshape(B * H, S, D)[heads]
+    assert np.isfinite(got).all() and rel_frobenius(got, ref) <= TOL
