@@ -692,10 +692,13 @@ Plan plan_of(const GemmDims& g, int64_t tiles, int sms, int bn, int splits, int 
 template <typename F>
 Plan make_plan(const GemmDims& g, int sms, F&& clusters) {
   Plan best{256, 1, 0, 0, 1e300};
+  const int64_t kb = (g.K + BK - 1) / BK;
   for (int bn : {256, 128, 64}) {
     const int64_t tiles = ((g.M + BM - 1) / BM) * ((g.N + bn - 1) / bn);
     if (tiles > INT32_MAX / 2) continue;
+    if (bn == 64 && tiles > 2 * sms) continue;  // (wider ones fill the SMs; the call that asks has a launch to make)
     for (int splits : {1, 2, 4, 8}) {
+      if (splits > 1 && kb < 2 * splits) break;
       const Plan p = plan_of(g, tiles, sms, bn, splits, splits > 1 ? clusters(bn, splits) : 0);
       if (p.clocks < best.clocks) best = p;
     }
