@@ -764,11 +764,15 @@ double items_estimate(const frisk_b200_attn_desc& d, int sms, int tiles_per_item
   }
   return std::max(heaviest, (double)heads * total / sms + 0.5 * total / (double)groups);
 }
+// A lone tile's key tiles are worth sharing from two on in the normalised mode (33 heads x 251 11.8 -> 10.4 us) and from three
+// on in the single pass, where with two the meeting of the groups costs what it saves (48 heads x 159 9.4 us, 9.7 split).
+bool split_keys_pay(const frisk_b200_attn_desc& d) { return d.S_kv > (d.normalize_p ? BN : 2 * BN); }
+
 bool one_tile_items(const frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d) {
   const int64_t tiles = (d.S_q + BM - 1) / BM * d.B * d.H;
   if (tiles <= ctx->num_sms) return true;
   // (four rounds of pairs balance by themselves)
-  if (d.S_kv <= BN || tiles > 8 * (int64_t)ctx->num_sms) return false;
+  if (!split_keys_pay(d) || tiles > 8 * (int64_t)ctx->num_sms) return false;
   return items_estimate(d, ctx->num_sms, 1) < (d.normalize_p ? 0.95 : 0.9) * items_estimate(d, ctx->num_sms, 2);
 }
 
@@ -838,11 +842,11 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q
 template <bool BF16, int D, bool OUT_F32, bool NORM>
 int launch_split(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K, const void* V,
                  void* O, cudaStream_t s) {
-  // A lone query tile's key tiles go to the two softmax groups in turn, where there are two at all: one group alone is
+  // A lone query tile's key tiles go to the two softmax groups in turn: one group alone is
   // bound by the chain S -> softmax -> P.V -> next S (1.4 us a key tile at D = 64 normalised), and two such chains overlap.
   // 16 heads x 1025 normalised 29.2 -> 23.4 us; single pass, D = 128: 4 heads x 4096 causal 62.1 -> 40.4, 2 x 8192 121.4 -> 75.3,
-  // 8 x 1000 19.8 -> 15.2; D = 64: 4 x 3000 42.5 -> 27.5; one key tile has nothing to share.
-  if (one_tile_items(ctx, d) && d.S_kv > BN) return launch_cfg<BF16, D, OUT_F32, NORM, true>(ctx, d, Q, K, V, O, s);
+  // 8 x 1000 19.8 -> 15.2; D = 64: 4 x 3000 42.5 -> 27.5.
+  if (split_keys_pay(d) && one_tile_items(ctx, d)) return launch_cfg<BF16, D, OUT_F32, NORM, true>(ctx, d, Q, K, V, O, s);
   return launch_cfg<BF16, D, OUT_F32, NORM, false>(ctx, d, Q, K, V, O, s);
 }
 
