@@ -28,6 +28,7 @@
 // 64 columns of S_q (two 16-bit values per column).
 // Every mbarrier wait is bounded (ptx.cuh); no TMA load uses cluster multicast.
 #include <algorithm>
+#include <cfloat>
 #include <type_traits>
 
 #include "common.cuh"
@@ -532,7 +533,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         auto settle = [&]() -> bool {
           const float mx = max3f(mxc[0], mxc[1], fmaxf(mxc[2], mxc[3]));
           float m_new = fmaxf(m_ref, mx * p.scale_log2);
-          if (m_new == -INFINITY) m_new = 0.f;  // a row that sees no key yet: keep everything finite
+          // A row that has seen no key, or only scores of -inf: the lowest finite reference, so that its exponentials are 0 and the
+          // first finite score moves it (0 would let lower scores vanish; a group's first key tile may be any row's -inf).
+          if (m_new == -INFINITY) m_new = -FLT_MAX;
           if (i == 0) {
             m_ref = m_new;
             return true;

@@ -492,3 +492,36 @@ def test_lone_tiles_beyond_one_a_cta(ctx, shape, normalize_p):
     ref = ao.attention_fwd(q, k, v, "fp16", D ** -0.5, causal=causal, mode="fp64", heads=heads)
     got = from_storage(first, "fp16").reshape(B * H, S, D)[heads]
     assert np.isfinite(got).all() and rel_frobenius(got, ref) <= TOL
+
+
+@pytest.mark.parametrize("hidden", [(0,), (1,), (0, 1), (2,)])
+@pytest.mark.parametrize("heads,s_q,D,dtype", [
+    (2, 128, 64, "fp16"), (2, 128, 128, "bf16"),    # lone query tiles: tile 0 and tile 1 are the first of a softmax group
+    (80, 256, 64, "bf16"), (80, 256, 128, "fp16"),  # pairs of query tiles
+    (2, 8, 128, "fp16"),                            # few queries: split over the keys
+])
+@pytest.mark.parametrize("normalize_p", [0, 1])
+def test_key_tiles_at_minus_infinity(ctx, hidden, heads, s_q, D, dtype, normalize_p):
+    """Keys padded with -inf in one column, whole key tiles of them, and scores far below 0 elsewhere (2^-40, beyond fp16's
+    range, or 2^-173, beyond bf16's): the padding counts for nothing, wherever it lies, and the low scores count as any others."""
+    import torch
+    rng = np.random.default_rng(81)
+    from oracle.numerics import to_storage
+    S = 512
+    q = 0.1 * rng.standard_normal((1, heads, s_q, D), dtype=np.float32)
+    k = 0.5 * rng.standard_normal((1, heads, S, D), dtype=np.float32)
+    q[..., :2], k[..., 0], k[..., 1] = 1.0, 0.0, -28.0 if dtype == "fp16" else -120.0
+    for tile in hidden:
+        k[..., tile * 128:(tile + 1) * 128, 0] = -np.inf
+    q, k, v = (to_storage(x, dtype) for x in (q, k, rng.standard_normal((1, heads, S, D), dtype=np.float32)))
+    gq, gk, gv = (Guarded(x.shape, dtype, fill=x) for x in (q, k, v))
+    go = Guarded((1, heads, s_q, D), "fp32")
+    go.view.fill_(float("nan"))
+    desc = capi.attn_desc(1, heads, s_q, S, D, 1.0, False, dtype, "fp32", normalize_p=normalize_p)
+    s = torch.cuda.current_stream().cuda_stream
+    ctx.attention_fwd(desc, gq.view.data_ptr(), gk.view.data_ptr(), gv.view.data_ptr(), go.view.data_ptr(), stream=s)
+    ctx.check(s)
+    some = [0, heads - 1]
+    got = go.host().reshape(heads, s_q, D)[some]
+    ref = ao.attention_fwd(q, k, v, dtype, 1.0, causal=False, mode="fp64", heads=some)
+    assert go.guards_intact() and np.isfinite(ref).all() and np.isfinite(got).all() and rel_frobenius(got, ref) <= TOL
