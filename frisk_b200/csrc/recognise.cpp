@@ -353,7 +353,10 @@ struct Graph {
     }
     return v;
   }
-  // the global kernel argument whose data a memref operand holds, staged or not
+  // a global kernel argument
+  bool global_arg(const Value& v) const { return v.is_arg && v.owner.get() == k.entry.get() && v.t.space == 1; }  // 1: GLOBAL
+  // the global kernel argument whose data a memref operand holds, staged or not, and of the operand's extents: the kernel reads
+  // those from the argument's address, and a copy's verifier does not compare the two sides
   bool root(const Value& operand, Value* out) const {
     Value v = strip(operand);
     if (producer(v, kUpstream, "memref.alloc")) {
@@ -366,7 +369,7 @@ struct Graph {
       if (!from) return false;
       v = strip(from->in[0]);
     }
-    if (!v.is_arg || v.owner.get() != k.entry.get() || v.t.space != 1) return false;  // 1: GLOBAL
+    if (!global_arg(v) || v.t.rank != operand.t.rank || v.t.e[0] != operand.t.e[0] || v.t.e[1] != operand.t.e[1]) return false;
     *out = v;
     return true;
   }
@@ -400,7 +403,9 @@ PyObject* attention(const Kernel& k) {
     }
   }
   Value o, v, q, key_arg;
-  if (!store || !g.root(store->in[1], &o)) return nullptr;
+  if (!store) return nullptr;
+  o = g.strip(store->in[1]);  // (a copy INTO a buffer does not say where the buffer's contents go)
+  if (!g.global_arg(o)) return nullptr;
   const Value* result = &store->in[0];
   if (const Op* t = g.producer(*result, kUpstream, "arith.truncf")) result = &t->in[0];
   const Op* pv = g.producer(*result, kMma);

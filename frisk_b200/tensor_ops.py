@@ -330,16 +330,29 @@ def attention_plan(kernel, ops=None):
             v = v.owner.operands[0]
         return v
 
+    def global_arg(v):
+        if not (v.is_arg and v.owner is entry) or v.type.space != MemorySpace.GLOBAL:
+            _fail("matrix operands must come from global kernel arguments")
+        return v
+
     def root_arg(v):
         """The global kernel argument a (possibly staged) memref operand holds the data of."""
-        v = strip_view(v)
+        tile = list(v.type.shape)
+        v, copy = strip_view(v), None
         if not v.is_arg and isinstance(v.owner, UpstreamOp) and v.owner.op_name == "memref.alloc":
             src = [c for c in copies if strip_view(c.operands[1]) is v]
             if len(src) != 1:
                 _fail("a staging buffer must be filled by exactly one frisk.copy")
-            v = strip_view(src[0].operands[0])
-        if not (v.is_arg and v.owner is entry) or v.type.space != MemorySpace.GLOBAL:
-            _fail("matrix operands must come from global kernel arguments")
+            copy = src[0]
+            v = strip_view(copy.operands[0])
+        global_arg(v)
+        # A frisk.copy states no extents of its own: the argument must hold the tile, at its beginning and without gaps (the kernel
+        # reads the tile's extents from the argument's address)
+        shape = list(v.type.shape)
+        if shape[:-len(tile)] + tile != shape or any(e != 1 for e in shape[:-len(tile)]):
+            if (copy is None or len(copy.operands) != 2 or copy.attrs["srcMap"].get_num_results() or len(shape) < len(tile)
+                    or shape[-1] != tile[-1] or shape[-2] < tile[-2]):
+                _fail(f"an argument of extents {shape} does not hold a tile of {tile}")
         return v
 
     def producer(v, cls=None, name=None):
@@ -370,7 +383,7 @@ def attention_plan(kernel, ops=None):
     if len(stores) != 1:
         _fail(f"expected one frisk.tile_store, found {len(stores)}")
     out_val, out_ref = stores[0].operands
-    o_arg = root_arg(out_ref)
+    o_arg = global_arg(strip_view(out_ref))  # (a copy INTO a buffer does not say where the buffer's contents go)
     if isinstance(out_val.owner, UpstreamOp) and out_val.owner.op_name == "arith.truncf":
         out_val = out_val.owner.operands[0]
     pv = producer(out_val, MmaOp)

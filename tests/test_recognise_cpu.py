@@ -151,3 +151,68 @@ def test_unusual_kernels_are_left_to_python():
     assert recognise.plan(kernel) is None and by_execute(kernel) == by_python(kernel)
     assert recognise.plan(gemm_kernel(fill=None, reduce=None, clear=True, trips=3)) is None
     assert recognise.plan(F.create_session().module) is None
+
+
+def change_argument(kernel, index, shape):
+    """Argument `index` and its views take another shape; the staging buffer and the ops on it stay as they are."""
+    old = kernel.regions[0].front().arguments[index].type
+    new = ir.type("memref", shape=list(shape), element=old.element, map=old.map, space=old.space)
+    for v in parts_of(kernel)[1]:
+        if v.type is old:
+            v.type = new
+    kernel.attrs["function_type"].inputs[index] = new
+    return kernel
+
+
+def store_through_buffer(shape, to_argument=False):
+    """The result is stored to a staging buffer, which the output argument, of `shape`, was copied into (or is copied to)."""
+    kernel = attention_kernel(64, 64, 64)
+    store = next(op for op in tensor_ops._ops_of(kernel) if isinstance(op, tensor_ops.TileStoreOp))
+    view = store.operands[1]
+    buffer = tensor_ops.UpstreamOp("memref.alloc", (), [ir.type("memref", shape=[64, 64], element=view.type.element, map=None,
+                                                                space=ir.MemorySpace.SHARED)])
+    ends = [view, buffer.results[0]]
+    copy = ir.CopyOp(operands=ends[::-1] if to_argument else ends, attrs={
+        "srcMap": ir.AffineMap(empty=True), "dstMap": ir.AffineMap(empty=True), "srcExtents": [64, 64], "dstExtents": [64, 64], "_nsrc": 0})
+    ops = store.parent_block.operations
+    at = ops.index(store)
+    ops[at:at + 1] = [buffer, store, copy] if to_argument else [buffer, copy, store]
+    for op in (buffer, copy):
+        op.parent_block = store.parent_block
+    store.operands[1] = buffer.results[0]
+    return change_argument(kernel, 3, shape)
+
+
+@needs_build
+@pytest.mark.parametrize("index,shape", [(0, [32, 64]), (1, [64, 64]), (2, [64, 64]), (1, [128, 32]), (2, [256, 32]), (0, [64, 128]), (1, [8192]),
+                                         (1, [2, 64, 64])])
+def test_an_argument_must_hold_the_tile_that_is_staged_from_it(index, shape):
+    """The kernel would read the buffer's extents from the argument's address: beyond its end, or with another pitch."""
+    kernel = change_argument(attention_kernel(64, 128, 64), index, shape)
+    assert recognise.plan(kernel) is None
+    with pytest.raises(ValueError, match="does not hold a tile"):
+        execute._plan_of(kernel, capi.ALGO_AUTO)
+
+
+@needs_build
+@pytest.mark.parametrize("index,shape", [(0, [256, 64]), (1, [1, 128, 64]), (2, [129, 64]), (2, [3, 128, 64])])
+def test_an_argument_may_hold_more_than_the_tile(index, shape):
+    kernel = change_argument(attention_kernel(64, 128, 64), index, shape)
+    plan = by_execute(kernel)
+    assert plan == by_python(kernel) and plan[1:] == by_execute(attention_kernel(64, 128, 64))[1:]
+    # but not where the copy names a place in it
+    copy = [op for op in tensor_ops._ops_of(kernel) if isinstance(op, ir.CopyOp)][index]
+    if shape[0] > 1:
+        copy.attrs["srcMap"] = ir.AffineMap(num_dims=0, results=[ir.get_affine_constant_expr(64), ir.get_affine_constant_expr(0)])
+        assert by_python(kernel) is None and recognise.plan(kernel) is None
+
+
+@needs_build
+@pytest.mark.parametrize("shape", [[32, 64], [64, 64]])
+@pytest.mark.parametrize("to_argument", [False, True])
+def test_a_result_is_stored_to_an_argument(shape, to_argument):
+    """A buffer that an argument was copied into is not that argument."""
+    kernel = store_through_buffer(shape, to_argument)
+    assert recognise.plan(kernel) is None
+    with pytest.raises(ValueError, match="global kernel arguments"):
+        execute._plan_of(kernel, capi.ALGO_AUTO)
