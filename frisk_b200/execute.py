@@ -214,6 +214,10 @@ def execute(module_or_kernel, *tensors, stream=None, name=None, algo=capi.ALGO_A
     arg_types = kernel.attrs["function_type"].inputs
     if len(tensors) != len(arg_types):
         raise ValueError(f"frisk-b200-execute: kernel takes {len(arg_types)} tensors, got {len(tensors)}")
+    # the plan is read off the entry block's arguments, the tensors are checked against the function type
+    arguments = kernel.regions[0].front().arguments
+    if len(arguments) != len(arg_types) or any(a.type is not t and a.type != t for a, t in zip(arguments, arg_types)):
+        raise ValueError("frisk-b200-execute: the entry block's arguments are not those of the kernel's function type")
     dtypes = {"f16": torch.float16, "bf16": torch.bfloat16, "f32": torch.float32}
     for t, ty in zip(tensors, arg_types):
         if t is None:

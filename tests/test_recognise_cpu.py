@@ -216,3 +216,24 @@ def test_a_result_is_stored_to_an_argument(shape, to_argument):
     assert recognise.plan(kernel) is None
     with pytest.raises(ValueError, match="global kernel arguments"):
         execute._plan_of(kernel, capi.ALGO_AUTO)
+
+
+@pytest.mark.parametrize("name", ["attention", "fused"])
+def test_entry_arguments_are_those_of_the_function_type(name):
+    """The tensors are checked against the function type, and the plan comes from the entry block's arguments: both must agree."""
+    import torch
+    kernel = KERNELS[name]()
+    inputs = kernel.attrs["function_type"].inputs
+    dtypes = {"f16": torch.float16, "f32": torch.float32}
+
+    def run():
+        execute.execute(kernel, *[torch.zeros(t.shape, dtype=dtypes[t.element.name]) for t in inputs])
+    inputs[0] = ir.type("memref", shape=list(inputs[0].shape), element=inputs[0].element, map=inputs[0].map, space=inputs[0].space)
+    with pytest.raises(ValueError, match="no CPU path"):  # (equal types; the tensors are not on a GPU)
+        run()
+    inputs[0].shape = [16, 64]
+    with pytest.raises(ValueError, match="entry block"):
+        run()
+    inputs.append(inputs[1])
+    with pytest.raises(ValueError, match="entry block"):
+        run()
