@@ -5,9 +5,10 @@
 Each ``csrc/*.cu`` is compiled to an object (in parallel, only when it or a header
 is newer than the object) and linked into ``frisk_b200/lib/libfrisk_b200.so``.
 nvcc cross-compiles without a GPU.  ``csrc/recognise.cpp``, a host-only CPython module, is compiled by g++ into
-``frisk_b200/lib/_recognise.so``.
+``frisk_b200/lib/_recognise`` + the interpreter's extension suffix; where g++ or Python's headers are missing the package does without.
 """
 import concurrent.futures
+import importlib.machinery
 import os
 import pathlib
 import shutil
@@ -19,7 +20,7 @@ PKG = pathlib.Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "build"
 LIB = PKG / "lib" / "libfrisk_b200.so"
-RECOGNISE = PKG / "lib" / "_recognise.so"
+RECOGNISE = PKG / "lib" / ("_recognise" + importlib.machinery.EXTENSION_SUFFIXES[0])  # (names the interpreter's ABI)
 INCLUDE = PKG.parent / "include"
 
 NVCC_FLAGS = [
@@ -40,6 +41,25 @@ def _stale(target, deps):
         return True
     t = target.stat().st_mtime
     return any(d.stat().st_mtime > t for d in deps)
+
+
+def build_recognise(force=False):
+    """The native recogniser, or None where it cannot be built here: ``execute`` then recognises in Python, more slowly."""
+    source, target = CSRC / "recognise.cpp", RECOGNISE
+    if not force and not _stale(target, [source]):
+        return target
+    gxx, headers = shutil.which("g++"), sysconfig.get_paths()["include"]
+    if gxx is None or not os.path.exists(os.path.join(headers, "Python.h")) or sys.version_info < (3, 10):
+        sys.stderr.write("frisk_b200: no g++ or no headers of Python 3.10 or newer: built without the native recogniser\n")
+        target.unlink(missing_ok=True)  # (one of an older source)
+        return None
+    target.parent.mkdir(exist_ok=True)
+    res = subprocess.run([gxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-I", headers, str(source), "-o", str(target)],
+                         capture_output=True, text=True)
+    if res.returncode:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("g++ failed on recognise.cpp")
+    return target
 
 
 def build(force=False, verbose=False):
@@ -74,14 +94,7 @@ def build(force=False, verbose=False):
         if res.returncode:
             sys.stderr.write(res.stdout + res.stderr)
             raise RuntimeError("link of libfrisk_b200.so failed")
-    host = CSRC / "recognise.cpp"
-    if force or _stale(RECOGNISE, [host]):
-        cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"],
-               str(host), "-o", str(RECOGNISE)]
-        res = subprocess.run(cmd, capture_output=True, text=True)
-        if res.returncode:
-            sys.stderr.write(res.stdout + res.stderr)
-            raise RuntimeError("g++ failed on recognise.cpp")
+    build_recognise(force)
     return LIB
 
 

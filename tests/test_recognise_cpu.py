@@ -1,15 +1,17 @@
 """The native recogniser (csrc/recognise.cpp) against the Python ones: what it accepts they resolve to the same plan, also after
 any single part of a built kernel has been changed, removed or put in another's place."""
 import importlib
+import os
 import random
+import sysconfig
 
 import pytest
 
 import frisk_b200 as F
-from frisk_b200 import capi, ir, recognise, tensor_ops
+from frisk_b200 import build, capi, ir, recognise, tensor_ops
 
 execute = importlib.import_module("frisk_b200.execute")
-needs_build = pytest.mark.skipif(not recognise.PATH.exists(), reason="_recognise.so is not built")
+needs_build = pytest.mark.skipif(not recognise.PATH.exists(), reason="the native recogniser is not built")
 
 
 def attention_kernel(n_q=64, n_kv=128, d=64, element="f16", out="f32", scale=0.125):
@@ -237,3 +239,24 @@ def test_entry_arguments_are_those_of_the_function_type(name):
     inputs.append(inputs[1])
     with pytest.raises(ValueError, match="entry block"):
         run()
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_plans_are_the_same_without_the_extension(name, monkeypatch, tmp_path):
+    monkeypatch.setattr(recognise, "PATH", tmp_path / "_recognise.so")
+    monkeypatch.setattr(recognise, "_plan", None)
+    kernel = KERNELS[name]()
+    assert recognise.plan(kernel) is None and by_execute(kernel) == by_python(kernel)
+
+
+def test_the_extension_is_built_for_this_interpreter_or_not_at_all(monkeypatch, tmp_path, capsys):
+    assert recognise.PATH.name == "_recognise" + sysconfig.get_config_var("EXT_SUFFIX") and build.RECOGNISE == recognise.PATH
+    target = tmp_path / recognise.PATH.name
+    monkeypatch.setattr(build, "RECOGNISE", target)
+    with monkeypatch.context() as m:
+        m.setattr(build.sysconfig, "get_paths", lambda: {"include": str(tmp_path)})  # no Python.h there
+        assert build.build_recognise() is None and "without the native recogniser" in capsys.readouterr().err
+    target.write_bytes(b"of an older source")
+    os.utime(target, (0, 0))
+    monkeypatch.setattr(build.shutil, "which", lambda name: None)  # no g++
+    assert build.build_recognise() is None and not target.exists()
