@@ -583,7 +583,12 @@ int frisk_b200_gemm_host(frisk_b200_ctx* ctx, const frisk_b200_gemm_desc* d, con
     if (rc) return rc;
     FB_CUDA(ctx, cudaEventRecord(ctx->ev[2 * p + 1], s));
     FB_CUDA(ctx, cudaStreamWaitEvent(s3, ctx->ev[2 * p + 1], 0));
-    FB_CUDA(ctx, cudaMemcpyAsync(static_cast<unsigned char*>(C) + c_off, dC, c_bytes, cudaMemcpyDeviceToHost, s3));
+    // (what lies between the rows of a wider buffer is the caller's: the device has no bytes for it)
+    if (g.ldc == g.N || rows == 1)
+      FB_CUDA(ctx, cudaMemcpyAsync(static_cast<unsigned char*>(C) + c_off, dC, c_bytes, cudaMemcpyDeviceToHost, s3));
+    else
+      FB_CUDA(ctx, cudaMemcpy2DAsync(static_cast<unsigned char*>(C) + c_off, g.ldc * cs, dC, g.ldc * cs, g.N * cs, (size_t)rows,
+                                     cudaMemcpyDeviceToHost, s3));
   }
   FB_CUDA(ctx, cudaEventRecord(ctx->ev[23], s3));
   FB_CUDA(ctx, cudaStreamWaitEvent(s, ctx->ev[23], 0));

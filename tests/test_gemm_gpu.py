@@ -549,6 +549,25 @@ def test_gemm_host_entry_short_last_panel_and_explicit_algo(ctx):
         assert np.isfinite(c).all() and rel_frobenius(c, ref) <= TOL["fp16"], algo
 
 
+@pytest.mark.parametrize("M,N,K,pitch,dtype", [
+    (1, 24, 64, 40, "fp16"), (16, 512, 512, 520, "bf16"), (300, 130, 192, 136, "bf16"), (130, 126, 100, 128, "fp32"),
+    (2100, 1000, 64, 1024, "fp32"),  # moved in row panels
+    (2100, 1024, 64, 1027, "fp16"),
+])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_gemm_host_into_part_of_a_wider_buffer(ctx, M, N, K, pitch, dtype, accumulate):
+    """What lies between C's rows in the host buffer keeps its bytes, also where C is not read."""
+    a, b = inputs.gemm_inputs(M, N, K, dtype, False, True, 47, "uniform" if dtype == "fp32" else "normal_rsqrt_k")
+    old = to_storage(np.random.default_rng(M + pitch).standard_normal((M, pitch), dtype=np.float32), dtype)
+    c = old.copy()
+    ctx.gemm_host(capi.gemm_desc(M, N, K, dtype, dtype, False, True, clear_accum=not accumulate, ldc=pitch), a.ctypes.data,
+                  b.ctypes.data, c.ctypes.data)
+    assert np.array_equal(c[:, N:].view(np.uint8), old[:, N:].view(np.uint8))
+    mine = [np.ascontiguousarray(x[:, :N]) for x in (c, old)]
+    ref = gemm_oracle.gemm_fp64(a, b, dtype, False, True, mine[1] if accumulate else None, dtype)
+    assert rel_frobenius(from_storage(mine[0], dtype), ref) <= TOL[dtype]
+
+
 @pytest.mark.parametrize("M,N,K,dtype,ta,tb", [
     (515, 771, 1003, "fp32", True, True),     # tensor cores, though no extent is a multiple of 8
     (64, 1024, 4096, "bf16", False, True),    # K shared by clusters of the one-CTA kernel
