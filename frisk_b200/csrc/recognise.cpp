@@ -44,7 +44,7 @@ class Ref {
   X(regions) X(blocks) X(operations) X(operands) X(results) X(attrs) X(type) X(owner) X(index) X(is_arg) X(kind) X(name)  \
   X(shape) X(element) X(space) X(map) X(op_name) X(arguments) X(m) X(n) X(k) X(trans_a) X(trans_b) X(dim) X(dimensions)   \
   X(threads) X(ranges) X(srcMap) X(dstMap) X(_nsrc) X(num_dims) X(num_symbols) X(_value) X(transA) X(transB) X(M) X(N)    \
-  X(K) X(policy) X(clear_accum) X(value) X(clear) X(lower) X(upper) X(step)
+  X(K) X(policy) X(clear_accum) X(value) X(clear) X(lower) X(upper) X(step) X(function_type) X(inputs)
 struct Names {
 #define X(n) PyObject* n = nullptr;
   NAMES(X)
@@ -336,6 +336,17 @@ bool walk(Kernel& k, const Ref& op, int depth) {
   return true;
 }
 
+// The plan is read off the entry block's arguments, execute checks the tensors against the function type: the same type objects
+// (others that are equal are for the Python side to compare).
+bool arguments_match(const Ref& kernel, const Ref& entry) {
+  const Ref inputs = attr(key(attr(kernel, names.attrs), names.function_type), names.inputs), arguments = attr(entry, names.arguments);
+  const Py_ssize_t n = length(inputs);
+  if (n < 0 || length(arguments) != n) return false;
+  for (Py_ssize_t i = 0; i < n; ++i)
+    if (attr(item(arguments, i), names.type).get() != item(inputs, i).get()) return false;
+  return true;
+}
+
 // ------------------------------------------------------------------------ the attention graph
 struct Graph {
   const Kernel& k;
@@ -492,7 +503,7 @@ PyObject* plan(PyObject*, PyObject* arg) {
   try {
     Kernel k;
     const Ref kernel(Py_NewRef(arg));
-    if (walk(k, kernel, 0)) {
+    if (walk(k, kernel, 0) && arguments_match(kernel, k.entry)) {
       bool mma = false;
       for (const Op& op : k.ops) mma = mma || op.cls == kMma;
       PyObject* out = mma ? attention(k) : fused(k);

@@ -184,11 +184,17 @@ def _plan_of(kernel, algo):
     known = recognise.plan(kernel)
     if known is None:
         ops = tensor_ops._ops_of(kernel)
-        if any(isinstance(op, tensor_ops.MmaOp) for op in ops):
+        attention = any(isinstance(op, tensor_ops.MmaOp) for op in ops)
+        if attention:
             spec, idx = tensor_ops.attention_plan(kernel, ops)
-            return True, (capi.attn_desc(1, 1, spec["S_q"], spec["S_kv"], spec["D"], spec["scale"], False, spec["dtype_in"],
-                                         spec["dtype_out"], normalize_p=True), idx)
-        return False, fused_plan(kernel, algo=algo)
+            plan = capi.attn_desc(1, 1, spec["S_q"], spec["S_kv"], spec["D"], spec["scale"], False, spec["dtype_in"],
+                                  spec["dtype_out"], normalize_p=True), idx
+        else:
+            plan = fused_plan(kernel, algo=algo)
+        # the plan is read off the entry block's arguments, the tensors are checked against the function type
+        if [a.type for a in kernel.regions[0].front().arguments] != list(kernel.attrs["function_type"].inputs):
+            raise ValueError("frisk-b200-execute: the entry block's arguments are not those of the kernel's function type")
+        return attention, plan
     if not known[0]:
         _, s_q, s_kv, d, scale, e_in, e_out, *idx = known
         return True, (capi.attn_desc(1, 1, s_q, s_kv, d, scale, False, _ELEMENTS[e_in], _ELEMENTS[e_out], normalize_p=True), idx)
@@ -214,10 +220,6 @@ def execute(module_or_kernel, *tensors, stream=None, name=None, algo=capi.ALGO_A
     arg_types = kernel.attrs["function_type"].inputs
     if len(tensors) != len(arg_types):
         raise ValueError(f"frisk-b200-execute: kernel takes {len(arg_types)} tensors, got {len(tensors)}")
-    # the plan is read off the entry block's arguments, the tensors are checked against the function type
-    arguments = kernel.regions[0].front().arguments
-    if len(arguments) != len(arg_types) or any(a.type is not t and a.type != t for a, t in zip(arguments, arg_types)):
-        raise ValueError("frisk-b200-execute: the entry block's arguments are not those of the kernel's function type")
     dtypes = {"f16": torch.float16, "bf16": torch.bfloat16, "f32": torch.float32}
     for t, ty in zip(tensors, arg_types):
         if t is None:
