@@ -8,17 +8,20 @@
 // Unlike the reference's three-pass schedule (tiled_attention.py:697-698) this is a single
 // pass with an online softmax, so K and V are read once per query tile:
 //
-//   * the kernel is persistent: one CTA per SM takes work items (TWO 128-row query tiles of one
-//     (batch, head)) from an atomic counter, heavy items first, until none is left.  Barriers, tensor
+//   * the kernel is persistent: one CTA per SM takes work items from an atomic counter, heavy items first, until none is
+//     left.  An item is TWO 128-row query tiles of one (batch, head), each with a softmax group and an MMA thread of its own, or
+//     ONE (items_estimate, below), whose key tiles the two groups share out (SPLIT) or group 0 takes alone.  Barriers, tensor
 //     memory and the K/V ring live across items, so the next item's Q, K and V are already on their
 //     way, and its first scores are computed, while the softmax warps still store the last item's O;
-//   * 128-key K/V tiles stream through a 2-stage TMA ring (K and V have separate full/empty mbarriers);
-//   * warp 8 is the TMA producer; warps 9 and 10 issue the tcgen05.mma of query tile 0 and 1: S_q =
+//   * 128-key K/V tiles stream through a 2-stage TMA ring (K and V have separate full/empty mbarriers).  Both MMA threads read
+//     every tile; SPLIT: the even key tiles are in stage 0, for the first thread alone, the odd ones in stage 1, for the second;
+//   * warp 8 is the TMA producer; warps 9 and 10 issue the tcgen05.mma of softmax group 0 and 1: S_q =
 //     Q_q.K^T (SS form, both operands K-major, 128-byte swizzle) into tensor memory and O_q += P_q.V
 //     (P read from tensor memory, V as an MN-major shared-memory operand);
 //   * warps 0-3 and 4-7 are the two softmax groups: thread r owns row r of its query tile
-//     (TMEM lane r), so row max / row sum need no shuffles.  The two groups alternate, so
-//     the tensor core works on one tile's MMAs while the other group exponentiates;
+//     (TMEM lane r), so row max / row sum need no shuffles.  In the single pass the two groups take turns, so
+//     the tensor core works on one group's MMAs while the other exponentiates.  The row maximum is taken within the turn, through
+//     the first exponentials, or before it (kMaxFirst);
 //   * the running maximum is applied lazily: O is rescaled in tensor memory only when the
 //     maximum grew by more than 2^8, which keeps P within bf16/fp16 range and makes most
 //     iterations rescale-free;
@@ -742,8 +745,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-// Items of ONE query tile or of two.  A lone tile has half of its SM's softmax and MMA threads idle where it cannot be split
-// (one key tile), but more items balance better.  So lone tiles are taken where that leaves at most one item per SM, and
+// Items of ONE query tile or of two.  A lone tile has half of its SM's softmax and MMA threads idle where its keys are not split
+// (split_keys_pay: one key tile, two in the single pass), but more items balance better.  So lone tiles are taken where that leaves at most one item per SM, and
 // beyond that where this estimate is clearly better: in steps (one key tile of two query tiles side by side, 2.1 us at D = 128), a pair of
 // tiles takes its key tiles, a split lone tile 0.56 a key tile (304 us for 8 x 8192 where pairs take 273), either 1.9 more to
 // begin and end; equal items go round by round, causal ones heavy first.  Estimated / measured ratios: 12 heads x 2048 causal 0.66 / 0.66

@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          tma_store_2d(&tmap_c, box, c0, r0);  // clipped at the edges of C
+          tma_store_2d(&tmap_c, box, c0, r0);  // clipped at the edges of C (its rows end on 16 bytes, tma_writes_c)
           tma_store_commit();
         }
       } else {

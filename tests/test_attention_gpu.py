@@ -24,7 +24,7 @@ def ctx():
     c.close()
 
 
-def run_attention(ctx, q, k, v, dtype, scale, causal, out_dtype=None):
+def run_attention(ctx, q, k, v, dtype, scale, causal, out_dtype=None, normalize_p=0):
     import torch
     out_dtype = out_dtype or dtype
     B, H, S_q, D = q.shape
@@ -33,7 +33,7 @@ def run_attention(ctx, q, k, v, dtype, scale, causal, out_dtype=None):
     go = Guarded((B, H, S_q, D), out_dtype)
     go.view.fill_(float("nan"))
     before = [g.raw.clone() for g in (gq, gk, gv)]
-    desc = capi.attn_desc(B, H, S_q, S_kv, D, scale, causal, dtype, out_dtype)
+    desc = capi.attn_desc(B, H, S_q, S_kv, D, scale, causal, dtype, out_dtype, normalize_p)
     s = torch.cuda.current_stream().cuda_stream
     ctx.attention_fwd(desc, gq.view.data_ptr(), gk.view.data_ptr(), gv.view.data_ptr(), go.view.data_ptr(), stream=s)
     ctx.check(s)
@@ -41,14 +41,14 @@ def run_attention(ctx, q, k, v, dtype, scale, causal, out_dtype=None):
     return go.host(), ok
 
 
-def check(ctx, B, H, S_q, S_kv, D, dtype, causal, seed, out_dtype=None, scale=None):
+def check(ctx, B, H, S_q, S_kv, D, dtype, causal, seed, out_dtype=None, scale=None, normalize_p=0):
     scale = scale if scale is not None else D ** -0.5
     rng = np.random.default_rng(seed)
     from oracle.numerics import to_storage
     q = to_storage(rng.standard_normal((B, H, S_q, D), dtype=np.float32), dtype)
     k = to_storage(rng.standard_normal((B, H, S_kv, D), dtype=np.float32), dtype)
     v = to_storage(rng.standard_normal((B, H, S_kv, D), dtype=np.float32), dtype)
-    got, ok = run_attention(ctx, q, k, v, dtype, scale, causal, out_dtype)
+    got, ok = run_attention(ctx, q, k, v, dtype, scale, causal, out_dtype, normalize_p)
     assert ok, "guard zone or input changed"
     ref = ao.attention_fwd(q, k, v, dtype, scale, causal=causal, mode="fp64")
     gotf = from_storage(got, out_dtype or dtype)
@@ -395,18 +395,21 @@ def test_execution_packet_runs_on_the_attention_kernel(ctx):
 
 
 # ------------------------------------------------------------------ a lone query tile's keys, split between the softmax groups
+# (from two key tiles on in the normalised mode, from three on in the single pass: two are left to one group there)
 @pytest.mark.parametrize("s_q,s_kv,causal", [
     (128, 129, False),   # two key tiles, the second with one key
     (17, 256, False),
+    (100, 150, True),    # two key tiles; rows that see no key of the second
     (128, 257, True),    # three key tiles: the groups have two and one
-    (100, 150, True),    # rows that see no key of the second tile
     (300, 300, True),    # the first query tile has one key tile: the second group has none
+    (300, 350, True),    # the first query tile has two, and rows that see no key of the second group's only one
     (129, 1025, True),
     (40, 2100, False),
 ])
 @pytest.mark.parametrize("D,dtype,out_dtype", [(64, "fp16", "fp16"), (64, "bf16", "fp32"), (128, "bf16", "bf16"), (128, "fp16", "fp32")])
-def test_lone_tiles_split_their_keys(ctx, s_q, s_kv, causal, D, dtype, out_dtype):
-    check(ctx, 1, 3, s_q, s_kv, D, dtype, causal, 60 + s_q + s_kv, out_dtype=out_dtype)
+@pytest.mark.parametrize("normalize_p", [0, 1])
+def test_lone_tiles_split_their_keys(ctx, s_q, s_kv, causal, D, dtype, out_dtype, normalize_p):
+    check(ctx, 1, 3, s_q, s_kv, D, dtype, causal, 60 + s_q + s_kv, out_dtype=out_dtype, normalize_p=normalize_p)
 
 
 @pytest.mark.parametrize("normalize_p", [0, 1])
