@@ -5,8 +5,8 @@
 //                 | (True, M, N, K, type of A, type of C, trans_a, trans_b, clear_accum, policy, ia, ib, ic,
 //                    fill or None, reduce kind or None, reduce argument, reduce_clear)        one gemm, its fill and reduce
 //
-// Walking and verifying a built kernel op by op in Python took most of a small call (a 64 x 64 attention tile 53.1 us, 21.3 with
-// this module, whose part is 12; a 512 x 384 x 256 gemm with fill and reduce 28.8 and 13.8, of which 3.6), and nothing may be
+// Walking and verifying a built kernel op by op in Python took most of a small call (a 64 x 64 attention tile 53.1 us, 22.0 with
+// this module, whose part is 12; a 512 x 384 x 256 gemm with fill and reduce 28.8 and 14.3, of which 3.6), and nothing may be
 // remembered between calls, since every list and attribute of the IR can be changed at any time.  So the same walk and
 // the checks of ir._verify and of tensor_ops.attention_plan / execute.fused_plan are made here, read off the same objects.
 //
