@@ -8,7 +8,6 @@ namespace fb {
 namespace attn {
 
 constexpr int BM = 128;        // query rows per tile (two tiles or one per work item)
-constexpr int BN = 128;        // keys per K/V tile
 constexpr int kThreads = 384;  // warps 0-3, 4-7: softmax groups; warp 8: TMA; warps 9, 10: MMA of softmax group 0, 1; 11 idle
 constexpr int kRegsSoftmax = 208, kRegsOther = 72;  // per-thread register budgets after setmaxnreg
 constexpr int kWarpTma = 8, kWarpMma = 9;
@@ -18,6 +17,7 @@ enum : unsigned { ST_ATTN_S = 0x201, ST_ATTN_P = 0x202, ST_ATTN_O = 0x203, ST_AT
 
 struct AttnParams {
   int S_q, S_kv, causal;
+  int heads;                 // batch x heads
   int n_groups, group_rows;  // work items per (batch, head), and the query rows of one: two 128-row tiles or one
   int normalized;  // 1: two passes over the keys, P divided by the complete row sum before it is rounded
   int64_t total_items;
@@ -109,15 +109,6 @@ __device__ __forceinline__ uint32_t pack16(float a, float b) {
     __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
   }
-}
-
-// number of key tiles query tile `m0` needs
-__device__ __forceinline__ int kv_tiles_for(int m0, int S_q, int S_kv, int causal) {
-  if (m0 >= S_q) return 0;
-  int all = (S_kv + BN - 1) / BN;
-  if (!causal) return all;
-  int last_key = min(S_kv - 1, m0 + BM - 1 + (S_kv - S_q));  // visible to the tile's last row
-  return min(all, last_key / BN + 1);
 }
 
 }  // namespace attn

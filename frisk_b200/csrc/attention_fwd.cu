@@ -9,30 +9,34 @@
 // pass with an online softmax, so K and V are read once per query tile:
 //
 //   * the kernel is persistent: one CTA per SM takes work items from an atomic counter, heavy items first, until none is
-//     left.  An item is TWO 128-row query tiles of one (batch, head), each with a softmax group and an MMA thread of its own, or
-//     ONE (items_estimate, below), whose key tiles the two groups share out (SPLIT) or group 0 takes alone.  Barriers, tensor
-//     memory and the K/V ring live across items, so the next item's Q, K and V are already on their
+//     left.  An item is TWO 128-row query tiles, of one (batch, head) or of two, each with a softmax group and an MMA thread of
+//     its own, or ONE (items_estimate, below), whose key tiles the two groups share out (kSplit) or group 0 takes alone.
+//     Barriers, tensor memory and the K/V ring live across items, so the next item's Q, K and V are already on their
 //     way, and its first scores are computed, while the softmax warps still store the last item's O;
-//   * 128-key K/V tiles stream through a 2-stage TMA ring (K and V have separate full/empty mbarriers).  Both MMA threads read
-//     every tile; SPLIT: the even key tiles are in stage 0, for the first thread alone, the odd ones in stage 1, for the second;
+//   * key tiles are 64 keys, and every query tile has two buffers of scores: S of tile b + 2 follows P(b).V on the tensor core
+//     while the softmax group works on tile b + 1, whose scores are there.  With one buffer of 128 keys every tile waited for the
+//     chain P -> P.V -> next S -> softmax.  An MMA of S takes 49 clk for 64 keys and 65 for 128 (it
+//     reads Q's rows from shared memory either way): 1270 clk for both query tiles' step of 64 keys against 1050, the price;
+//   * K and V stream through a TMA ring of 4 stages, each what one step of the MMA threads takes;
 //   * warp 8 is the TMA producer; warps 9 and 10 issue the tcgen05.mma of softmax group 0 and 1: S_q =
 //     Q_q.K^T (SS form, both operands K-major, 128-byte swizzle) into tensor memory and O_q += P_q.V
 //     (P read from tensor memory, V as an MN-major shared-memory operand);
 //   * warps 0-3 and 4-7 are the two softmax groups: thread r owns row r of its query tile
-//     (TMEM lane r), so row max / row sum need no shuffles.  In the single pass the two groups take turns, so
-//     the tensor core works on one group's MMAs while the other exponentiates.  The row maximum is taken within the turn, through
-//     the first exponentials, or before it (kMaxFirst);
+//     (TMEM lane r), so row max / row sum need no shuffles.  They work freely, one filling the gaps of the other;
 //   * the running maximum is applied lazily: O is rescaled in tensor memory only when the
 //     maximum grew by more than 2^8, which keeps P within bf16/fp16 range and makes most
 //     iterations rescale-free;
 //   * causal: key tiles wholly above the diagonal are never loaded; only tiles that touch the
 //     diagonal (or the ragged end of the keys) are masked.
-// TMEM columns: S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [384,384+D); P_q aliases the first
-// 64 columns of S_q (two 16-bit values per column).
+// TMEM columns: S0 [0,64) and [64,128), S1 [128,192) and [192,256), O0 [256,256+D) O1 [384,384+D); P_q of a key tile
+// aliases the first 32 columns of its scores (two 16-bit values per column).
+//
+// What bounds it: 8 x 32 heads x 4096 causal at D = 128 (1000 us; 1120 with 128-key tiles, one buffer and softmax groups in turn)
+// the power limit, at which it runs at 1.5 instead of 1.7 GHz; short runs the softmax groups, 1700 clk for a step of both
+// where the exponentials take 1024 and the MMAs 1270.
 // Every mbarrier wait is bounded (ptx.cuh); no TMA load uses cluster multicast.
 #include <algorithm>
 #include <cfloat>
-#include <type_traits>
 
 #include "common.cuh"
 #include "ptx.cuh"
@@ -43,15 +47,27 @@ namespace fb {
 namespace {
 using namespace attn;
 
-constexpr int kStagesKV = 2;
+constexpr int BN = 64;  // keys per K/V tile
+
+// number of key tiles query tile `m0` needs
+__device__ __forceinline__ int kv_tiles_for(int m0, int S_q, int S_kv, int causal) {
+  if (m0 >= S_q) return 0;
+  int all = (S_kv + BN - 1) / BN;
+  if (!causal) return all;
+  int last_key = min(S_kv - 1, m0 + BM - 1 + (S_kv - S_q));  // visible to the tile's last row
+  return min(all, last_key / BN + 1);
+}
+
 constexpr int kHeadChunk = 16;  // heads whose K and V are worked on together (they stay in L2: 16 x 2 MB at S = 4096)
 template <int D>
 struct AttnSmem {
-  static constexpr int kTileBytes = BM * D * 2;       // one Q, K or V tile
+  static constexpr int kTileBytes = BM * D * 2;        // one Q tile
+  static constexpr int kKvBytes = BN * D * 2;          // one K or V tile
+  static constexpr int kStagesKV = 4;                  // of the K/V ring; two may belong to either MMA thread
   static constexpr int kQ = 0;                         // Q0, Q1
-  static constexpr int kK = 2 * kTileBytes;            // K stages
-  static constexpr int kV = kK + kStagesKV * kTileBytes;
-  static constexpr int kBar = kV + kStagesKV * kTileBytes;
+  static constexpr int kStageBytes = 2 * kKvBytes;     // a K tile, then a V tile
+  static constexpr int kKV = 2 * kTileBytes;           // the ring
+  static constexpr int kBar = kKV + kStagesKV * kStageBytes;
   // 16-bit outputs: one [32 rows][128 bytes] box per softmax warp for the TMA stores of O, 1024-byte aligned
   static constexpr int kOut = kBar + 1024;
   static constexpr int kTotal = kOut + 8 * (32 * 128) + 1024;
@@ -59,35 +75,41 @@ struct AttnSmem {
 };
 
 
-// SPLIT: an item is ONE query tile, whose key tiles the two softmax groups (and MMA threads) take in turn, even and odd
-// ones, each with its own S, P, O and statistics; at the end the halves are put together.
-template <bool BF16, int D, bool OUT_F32, bool NORM, bool SPLIT>
+// What the two softmax groups (and MMA threads) make of a work item
+enum Mode {
+  kPair,   // two query tiles of one head, which share the K and V tiles
+  kSplit,  // ONE query tile, whose key tiles they take in turn, even and odd ones, each with its own S, P, O and statistics; at the
+           // end the halves are put together
+  kTwin    // two heads of one query tile each, with K and V of their own
+};
+
+template <bool BF16, int D, bool OUT_F32, bool NORM, Mode MODE>
 __global__ void __launch_bounds__(kThreads, 1)
     attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                          const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
                          const AttnParams p) {
+  constexpr bool SPLIT = MODE == kSplit, TWIN = MODE == kTwin;
+  constexpr bool OWN_KV = MODE != kPair;  // each MMA thread has key tiles, and stages of the ring, of its own
   using L = AttnSmem<D>;
   constexpr int kBoxes = D / 64;            // 64-element (128-byte) column blocks per tile
-  constexpr int kBoxBytes = BM * 128;       // one [128 rows][128 B] block
+  constexpr int kBoxBytes = BM * 128;       // one [128 rows][128 B] block of Q
+  constexpr int kKvBoxBytes = BN * 128;     // one [64 keys][128 B] block of K or V
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~static_cast<uintptr_t>(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBar);
   uint64_t* q_full = bars;              // [1]
-  uint64_t* k_full = bars + 1;          // [2]
-  uint64_t* k_empty = bars + 3;         // [2]
-  uint64_t* v_full = bars + 5;          // [2]
-  uint64_t* v_empty = bars + 7;         // [2]
-  uint64_t* s_full = bars + 9;          // [2] per query tile
-  uint64_t* p_ready = bars + 11;        // [2] first half of P_q (keys 0-63) written
-  uint64_t* p_ready_hi = bars + 16;     // [2] second half written
-  uint64_t* o_done = bars + 13;         // [2]
-  uint64_t* turn = bars + 18;           // [2] hand-over of the exponential section between the two softmax groups
-  uint64_t* item_full = bars + 20;      // [2] the producer has published the id of a work item
-  uint64_t* item_empty = bars + 22;     // [2] every consumer has read it
-  uint64_t* q_empty = bars + 24;        // [1] both MMA threads are done with the Q tiles
-  uint64_t* xchg = bars + 26;           // [1] the two softmax groups meet (SPLIT only)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 27);
+  uint64_t* q_empty = bars + 1;         // [1] both MMA threads are done with the Q tiles
+  uint64_t* kv_full = bars + 2;         // [4]
+  uint64_t* kv_empty = bars + 6;        // [4]
+  uint64_t* s_full = bars + 10;         // [2 groups][2 buffers] the scores of a key tile are complete
+  uint64_t* p_ready = bars + 14;        // [2 groups][2 buffers] its probabilities are written (statistics pass: the scores read)
+  uint64_t* o_done = bars + 18;         // [2 groups][2] of an item all P.V but the last, all P.V are complete
+  uint64_t* item_full = bars + 22;      // [2] the producer has published the id of a work item
+  uint64_t* item_empty = bars + 24;     // [2] every consumer has read it
+  uint64_t* turn = bars + 26;           // [2] the MMA threads issue in turn
+  uint64_t* xchg = bars + 28;           // [1] the two softmax groups meet (SPLIT only)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 29);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile int* item_slot = reinterpret_cast<volatile int*>(tmem_slot + 2);  // [2]
 
@@ -108,6 +130,13 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int heads_here = min(kHeadChunk, bh_total - chunk * kHeadChunk);
     const int group = p.n_groups - 1 - within / heads_here;
     Item it;
+    if (TWIN) {
+      it.bh = 2 * t;
+      it.m0 = 0;
+      it.nq[0] = it.n_max = kv_tiles_for(0, p.S_q, p.S_kv, p.causal);
+      it.nq[1] = it.bh + 1 < p.heads ? it.nq[0] : 0;
+      return it;
+    }
     it.bh = chunk * kHeadChunk + within % heads_here;
     it.m0 = group * p.group_rows;
     const int n0 = kv_tiles_for(it.m0, p.S_q, p.S_kv, p.causal);
@@ -130,32 +159,29 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (arrive) mbar_arrive(&item_empty[n & 1]);
     return t;
   };
-  // The ring of K and V: tile n goes to stage n % 2, and both MMA threads follow every tile.  SPLIT: each stage belongs to one MMA
-  // thread and n counts that stage's tiles, because a thread that does not follow all uses of a stage can mistake an earlier
-  // phase of its barrier for its own (with an odd number of key tiles the threads would change stages from pass to pass).
-  auto ring_phase = [](int n) -> uint32_t { return (SPLIT ? n : n / kStagesKV) & 1; };
+  // The ring of K and V.  What an MMA thread takes in one step, the V of key tile b and the K of tile b + 2, makes a stage: one
+  // barrier to wait for and one to release (each costs the thread about a hundred clocks).  The n-th goes to stage n % kStages, and
+  // both MMA threads follow all of them.  OWN_KV: two stages belong to either MMA thread and n counts that thread's,
+  // because a thread that does not follow all uses of a stage can mistake an earlier phase of its barrier for its own.
+  constexpr int kStages = L::kStagesKV, kOwnStages = OWN_KV ? kStages / 2 : kStages;
+  auto ring_stage = [](int n, int group) -> int { return (OWN_KV ? group * kOwnStages : 0) + n % kOwnStages; };
+  auto ring_phase = [](int n) -> uint32_t { return (n / kOwnStages) & 1; };
   // Normalised mode runs the key loop twice: pass 0 only gathers row maxima and row sums, pass 1
   // is the pass every mode has.  Barrier phases keep counting across passes and items.
   constexpr int first_pass = NORM ? 0 : 1;
-  // Where the row maximum is taken: before the group's turn, on the ALU while the other group keeps the special-function
-  // unit busy, or within it, run through the first exponentials.  Before is faster where the turns set the pace: D = 64, whose
-  // MMAs are half as long (8 x 32 heads x 2048 causal 274 -> 251 us, 3 x 16 x 1500 57.8 -> 51.7), and a lone query tile.  At
-  // D = 128 P.V and the next S set it, and long runs the power limit (930 W): before is slower there (8 x 32 x 4096 causal 1120
-  // -> 1145 us, 8 heads x 8192 272 -> 284).
-  constexpr bool kMaxFirst = D == 64 || SPLIT;
-
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], SPLIT ? 1 : 2);  // one arrival per MMA-issuing thread that reads the stage
-      mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], SPLIT ? 1 : 2);
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(&kv_full[i], 1);
+      mbar_init(&kv_empty[i], OWN_KV ? 1 : 2);  // one arrival per MMA-issuing thread that reads the stage
+    }
+    for (int i = 0; i < 4; ++i) {
       mbar_init(&s_full[i], 1);
       mbar_init(&p_ready[i], 128);
-      mbar_init(&p_ready_hi[i], 128);
       mbar_init(&o_done[i], 1);
-      mbar_init(&turn[i], 128);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&turn[i], 1);
       mbar_init(&item_full[i], 1);
       mbar_init(&item_empty[i], 10);  // two MMA threads, one lane of each of the eight softmax warps
     }
@@ -186,8 +212,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == kWarpTma) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      // K / V tiles loaded so far, over all items (K is streamed once per pass); SPLIT: into either stage
-      int kt = 0, vt = 0, kt_odd = 0, vt_odd = 0;
+      int loaded[2] = {0, 0};  // stages filled so far, over all items; OWN_KV: for either MMA thread
       bool ok = true;
       for (int n = 0; ok; ++n) {
         // take the next item and tell the other roles (slot n & 1 was last used by item n - 2)
@@ -205,136 +230,123 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int q = 0; q < q_tiles; ++q)
 #pragma unroll
           for (int b = 0; b < kBoxes; ++b)
-            tma_load_3d(smem + L::kQ + q * L::kTileBytes + b * kBoxBytes, &tmap_q, q_full, b * 64, it.m0 + q * BM, it.bh);
+            tma_load_3d(smem + L::kQ + q * L::kTileBytes + b * kBoxBytes, &tmap_q, q_full, b * 64, TWIN ? 0 : it.m0 + q * BM,
+                        it.bh + (TWIN ? q : 0));
         for (int pass = first_pass; pass < 2 && ok; ++pass) {
-          for (int j = 0; j < it.n_max; ++j) {
-            const bool odd = SPLIT && (j & 1);  // the second group's key tile
-            const int kp = odd ? kt_odd++ : kt++, vp = odd ? vt_odd : vt;
-            const int ks = SPLIT ? (int)odd : kp % kStagesKV;
-            if (!mbar_wait(&k_empty[ks], ring_phase(kp) ^ 1, abort_flag, p.status, ST_ATTN_KV)) {
-              ok = false;
-              break;
-            }
-            mbar_expect_tx(&k_full[ks], L::kTileBytes);
+          const int n_keys = OWN_KV ? it.nq[0] : it.n_max;  // (group 0 has no fewer key tiles than group 1)
+          for (int b = -2; b < n_keys && ok; ++b) {
 #pragma unroll
-            for (int b = 0; b < kBoxes; ++b)
-              tma_load_3d(smem + L::kK + ks * L::kTileBytes + b * kBoxBytes, &tmap_k, &k_full[ks], b * 64, j * BN, it.bh);
-            if (pass == 0) continue;  // the statistics pass needs no values
-            (odd ? vt_odd : vt)++;
-            const int vs = SPLIT ? (int)odd : vp % kStagesKV;
-            if (!mbar_wait(&v_empty[vs], ring_phase(vp) ^ 1, abort_flag, p.status, ST_ATTN_KV)) {
-              ok = false;
-              break;
-            }
-            mbar_expect_tx(&v_full[vs], L::kTileBytes);
+            for (int g = 0; g < (OWN_KV ? 2 : 1); ++g) {
+              const int n_mine = OWN_KV ? it.nq[g] : it.n_max, bh = it.bh + (TWIN ? g : 0);
+              const bool has_k = b + 2 < n_mine, has_v = pass == 1 && b >= 0 && b < n_mine;  // (statistics need no values)
+              if (!ok || !(has_k || has_v)) continue;
+              const int st = ring_stage(loaded[g], g);
+              ok = mbar_wait(&kv_empty[st], ring_phase(loaded[g]) ^ 1, abort_flag, p.status, ST_ATTN_KV);
+              if (!ok) continue;
+              ++loaded[g];
+              mbar_expect_tx(&kv_full[st], (has_k && has_v ? 2 : 1) * L::kKvBytes);
+              unsigned char* at = smem + L::kKV + st * L::kStageBytes;
 #pragma unroll
-            for (int b = 0; b < kBoxes; ++b)
-              tma_load_3d(smem + L::kV + vs * L::kTileBytes + b * kBoxBytes, &tmap_v, &v_full[vs], b * 64, j * BN, it.bh);
+              for (int x = 0; x < kBoxes; ++x) {
+                if (has_k)
+                  tma_load_3d(at + x * kKvBoxBytes, &tmap_k, &kv_full[st], x * 64, (SPLIT ? 2 * (b + 2) + g : b + 2) * BN, bh);
+                if (has_v)
+                  tma_load_3d(at + L::kKvBytes + x * kKvBoxBytes, &tmap_v, &kv_full[st], x * 64, (SPLIT ? 2 * b + g : b) * BN, bh);
+              }
+            }
           }
         }
       }
     }
   } else if (warp == kWarpMma || warp == kWarpMma + 1) {
-    // ------------------------------------------------------------------ MMA issuers, one thread per query tile
-    // Each query tile has its own issuing thread (warps 9 and 10).  One thread for both tiles was the
-    // kernel's bottleneck: besides the 32 MMAs of a key tile it has a dozen barrier waits, fences and commits
-    // to execute, each a round trip of ~100 clocks for a single thread, and the two tiles' chains
-    // (S -> softmax -> P.V -> next S) queued behind each other in it.  tcgen05 operations of ONE thread execute
-    // in issue order, which is all the ordering a query tile needs (S_q(j+1) overwrites P_q(j) only after
-    // P_q(j).V(j) has read it); the two tiles share only the read-only K and V stages, which each thread
-    // releases with its own arrival (the empty barriers count two).
-    const int mq = warp - kWarpMma;
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = umma_idesc_f16(BM, BN, BF16, false, false);
-      constexpr uint32_t idesc_o = umma_idesc_f16(BM, D, BF16, false, true);
-      const uint32_t sq = smem_u32(smem + L::kQ), sk = smem_u32(smem + L::kK), sv = smem_u32(smem + L::kV);
-      // descriptors are built once; the k16 slices only add a constant to the start-address field
-      const uint64_t dq = umma_desc_kmajor_sw128(sq + (SPLIT ? 0 : mq * L::kTileBytes));
-      const uint64_t dk[2] = {umma_desc_kmajor_sw128(sk), umma_desc_kmajor_sw128(sk + L::kTileBytes)};
-      const uint64_t dv[2] = {umma_desc_mnmajor_sw128(sv, kBoxBytes, 1024),
-                              umma_desc_mnmajor_sw128(sv + L::kTileBytes, kBoxBytes, 1024)};
-      const uint32_t t_sq = tmem_base + mq * 128;        // S_q; P_q aliases its first 64 columns (8 per k16 slice)
-      const uint32_t t_oq = tmem_base + 256 + mq * 128;  // O_q
-      int kt = 0, vt = 0;    // K / V tiles seen so far, over all items (ring positions; K is streamed once per pass)
-      int steps = 0;         // (pass, key tile) steps of THIS softmax group so far: the phase of s_full / p_ready
-      auto ring_stage = [&](int n) -> int { return SPLIT ? mq : n % kStagesKV; };
-      bool ok = true;
-      for (int n = 0; ok; ++n) {
-        const int t = next_item(n, true);
-        if (t < 0) break;
-        const Item it = decode(t);
-        const int n_mine = it.nq[mq], n_max = SPLIT ? n_mine : it.n_max;  // key tiles: used, followed
-        ok = mbar_wait(q_full, n & 1, abort_flag, p.status, ST_ATTN_Q);
-        for (int pass = first_pass; pass < 2 && ok; ++pass) {
-          const bool stats_pass = pass == 0;  // the pass that only gathers statistics issues no P.V
-          // Per key tile and query tile the dependent chain is: softmax publishes P(j) -> P(j).V(j) -> S(j+1) ->
-          // softmax.  Everything this thread can do off that chain is done off it: the wait for K(j+1) happens
-          // before the wait for P(j), and the commits that release V(j), K(j+1) and publish O come after the
-          // MMAs of S(j+1) have been issued (a commit covers everything issued before it, so they only fire a
-          // little later than strictly possible).
-          bool have_k = false;  // K(j) of the current pass is known to have landed
-          for (int j = 0; j < n_max && ok; ++j, ++kt) {
-            const int ks = ring_stage(kt);
-            if (!have_k) ok = mbar_wait(&k_full[ks], ring_phase(kt), abort_flag, p.status, ST_ATTN_KV);
-            have_k = false;
-            if (!ok) break;
-            if (j < n_mine) {
-              tc_fence_after_sync();
+    // ------------------------------------------------------------------ MMA issuers, one warp per query tile
+    // tcgen05 operations of ONE thread execute in issue order, which is all the ordering a query tile needs: S_q(b + 2) overwrites
+    // P_q(b) after P_q(b).V(b) has read it.  The tensor core queues only a few MMAs, so an issuing thread is busy for as long as
+    // its MMAs run and everything else it does (a wait or a commit costs 100 clk or more, ~500 a step) leaves the pipe idle,
+    // unless the other thread issues meanwhile.  Two threads that issue freely fall into step, MMA by MMA, and do everything
+    // else at the same time too: 1840 clk a step.  So they issue in turn (1240 clk where the softmax is left out), and there
+    // is little else to do: one wait for P and the stage of the ring, two commits.  The loop is run by whole warps, so that
+    // descriptors and counters are uniform; one elected lane issues.
+    const int mq = __shfl_sync(0xffffffffu, warp - kWarpMma, 0);
+    constexpr uint32_t idesc_s = umma_idesc_f16(BM, BN, BF16, false, false);
+    constexpr uint32_t idesc_o = umma_idesc_f16(BM, D, BF16, false, true);
+    // descriptors differ only in the start address
+    const uint64_t dq = umma_desc_kmajor_sw128(smem_u32(smem + L::kQ) + (SPLIT ? 0 : mq * L::kTileBytes));
+    const uint64_t dk = umma_desc_kmajor_sw128(smem_u32(smem + L::kKV));
+    const uint64_t dv = umma_desc_mnmajor_sw128(smem_u32(smem + L::kKV + L::kKvBytes), kKvBoxBytes, 1024);
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+    const uint32_t t_sq = tmem + mq * 128;        // the two buffers of S_q, 64 columns each
+    const uint32_t t_oq = tmem + 256 + mq * 128;  // O_q
+    int turns = 0;     // steps in turn so far, over all items
+    int taken = 0;     // stages of the ring followed so far, over all items
+    int begun = 0;     // S_q begun so far, over all items: its buffer
+    int finished = 0;  // P_q taken so far, over all items: its buffer and the phase of p_ready
+    bool ok = true;
+    for (int n = 0; ok; ++n) {
+      const int t = __shfl_sync(0xffffffffu, next_item(n, lane == 0), 0);
+      if (t < 0) break;
+      const Item it = decode(t);
+      const int n_mine = it.nq[mq], n_max = OWN_KV ? n_mine : it.n_max;  // key tiles: used, followed
+      const int n_steps = OWN_KV ? it.nq[0] : it.n_max;  // the same for both MMA threads
+      const bool in_turn = it.nq[1] > 0;                // a lone thread issues as it comes
+      ok = mbar_wait(q_full, n & 1, abort_flag, p.status, ST_ATTN_Q);
+      for (int pass = first_pass; pass < 2 && ok; ++pass) {
+        const bool stats_pass = pass == 0;  // the pass that only gathers statistics issues no P.V
+        // S runs two key tiles ahead of P.V: the scores of tile b + 1 are complete (or on their way) while the softmax
+        // group works on tile b, and those of tile b + 2 take their place as soon as P(b).V has read P(b) there.
+        for (int b = -2; b < n_steps && ok; ++b) {
+          const bool staged = b + 2 < n_max || (!stats_pass && b >= 0 && b < n_max);  // a stage of the ring comes with this step
+          const bool use_p = b >= 0 && b < n_mine, use_s = b + 2 < n_mine;
+          const int st = ring_stage(taken, mq), buf = finished & 1;
+          uint64_t* const p_bar = &p_ready[2 * mq + buf];
+          if (use_p && staged)
+            ok = mbar_wait_both(p_bar, (finished >> 1) & 1, &kv_full[st], ring_phase(taken), abort_flag, p.status, ST_ATTN_P,
+                                ST_ATTN_KV);
+          else if (use_p)
+            ok = mbar_wait(p_bar, (finished >> 1) & 1, abort_flag, p.status, ST_ATTN_P);
+          else if (staged)
+            ok = mbar_wait(&kv_full[st], ring_phase(taken), abort_flag, p.status, ST_ATTN_KV);
+          if (ok && in_turn) ok = mbar_wait(&turn[mq], (turns & 1) ^ (mq ^ 1), abort_flag, p.status, ST_ATTN_S);
+          turns += in_turn;
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after_sync();
+          const uint64_t at = static_cast<uint64_t>((st * L::kStageBytes) >> 4);
+          if (use_p) {
+            ++finished;
+            if (!stats_pass && elect_one()) {
 #pragma unroll
-              for (int kk = 0; kk < D / 16; ++kk) {
-                const uint64_t off = static_cast<uint64_t>(((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4);
-                umma_f16_ss(t_sq, dq + off, dk[ks] + off, idesc_s, kk != 0);
-              }
-              umma_commit(&s_full[mq]);
-              umma_commit(&k_empty[ks]);  // this tile's use of the K stage ends when these MMAs have read it
-              if (j > 0 && !stats_pass && !SPLIT) {  // (deferred from the previous tile)
-                umma_commit(&o_done[mq]);
-                umma_commit(&v_empty[(vt - 1) % kStagesKV]);
-              }
-              if (pass == 1 && j == n_mine - 1) umma_commit(q_empty);  // this thread's last use of the Q tiles
-            } else {
-              mbar_arrive(&k_empty[ks]);  // a key tile only the other query tile needs
+              for (int kk = 0; kk < BN / 16; ++kk)
+                umma_f16_ts(t_oq, t_sq + buf * BN + kk * 8, dv + at + static_cast<uint64_t>((kk * 2048) >> 4), idesc_o,
+                            (b > 0 || kk > 0) ? 1u : 0u);
             }
-            const int vs = ring_stage(vt);
-            if (j < n_mine) {
-              // the next K tile, while the softmax group works on this one (SPLIT: it comes behind a V tile whose stage the
-              // other thread has yet to release, and must not hold up this thread's P.V)
-              if (!SPLIT && j + 1 < n_max) {
-                ok = mbar_wait(&k_full[ring_stage(kt + 1)], ring_phase(kt + 1), abort_flag, p.status, ST_ATTN_KV);
-                have_k = ok;
-              }
-              if (!stats_pass && ok) ok = mbar_wait(&v_full[vs], ring_phase(vt), abort_flag, p.status, ST_ATTN_KV);
-              // O_q += P_q(j) . V(j).  The softmax group publishes P in two halves (64 keys each), so the first
-              // four k16 slices start while the second half is still being exponentiated.  In the statistics
-              // pass the two waits only tell that the softmax group is done with S_q.
-              const uint32_t parity = steps & 1;
-              ++steps;
+          }
+          if (use_s) {
+            const int s_buf = begun & 1;
+            ++begun;
+            if (elect_one()) {
 #pragma unroll
-              for (int half = 0; half < 2; ++half) {
-                if (ok) ok = mbar_wait(half ? &p_ready_hi[mq] : &p_ready[mq], parity, abort_flag, p.status, ST_ATTN_P);
-                if (stats_pass) continue;
-                if (!ok) break;
-                tc_fence_after_sync();
-#pragma unroll
-                for (int kk = half * 4; kk < half * 4 + 4; ++kk)
-                  umma_f16_ts(t_oq, t_sq + kk * 8, dv[vs] + static_cast<uint64_t>((kk * 2048) >> 4), idesc_o,
-                              (j | kk) != 0);
-              }
-              if (!ok) break;
-              // no further S of this item follows, or the next V tile of this group waits for the stage: publish now
-              if (!stats_pass && (SPLIT || j + 1 >= n_mine)) {
-                umma_commit(&o_done[mq]);
-                umma_commit(&v_empty[vs]);
-              }
-            } else if (!stats_pass) {
-              ok = mbar_wait(&v_full[vs], ring_phase(vt), abort_flag, p.status, ST_ATTN_KV);
-              if (ok) mbar_arrive(&v_empty[vs]);
+              for (int kk = 0; kk < D / 16; ++kk)
+                umma_f16_ss(t_sq + s_buf * BN, dq + static_cast<uint64_t>(((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4),
+                            dk + at + static_cast<uint64_t>(((kk / 4) * kKvBoxBytes + (kk % 4) * 32) >> 4), idesc_s, kk != 0);
+              if (in_turn) mbar_arrive(&turn[mq ^ 1]);
+              umma_commit(&s_full[2 * mq + s_buf]);
+              if (pass == 1 && b + 2 == n_mine - 1) umma_commit(q_empty);  // this thread's last use of the Q tiles
             }
-            if (!stats_pass) ++vt;
+          } else if (in_turn && elect_one()) {
+            mbar_arrive(&turn[mq ^ 1]);
+          }
+          if (use_p && !stats_pass && b >= n_mine - 2 && elect_one()) umma_commit(&o_done[2 * mq + (b == n_mine - 1)]);
+          if (staged) {
+            // this thread's use of the stage ends when these MMAs have read it
+            if (elect_one()) {
+              if (use_p || use_s) umma_commit(&kv_empty[st]); else mbar_arrive(&kv_empty[st]);
+            }
+            ++taken;
           }
         }
-        if (ok && n_mine == 0) mbar_arrive(q_empty);  // (a query tile beyond the end of the sequence)
       }
+      if (ok && n_mine == 0 && lane == 0) mbar_arrive(q_empty);  // (a query tile beyond the end of the sequence)
     }
   }
   } else {
@@ -347,9 +359,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t t_s = tmem_base + q * 128 + lane_addr;
     const uint32_t t_o = tmem_base + 256 + q * 128 + lane_addr;
     const int off = p.S_kv - p.S_q;
-    int steps = 0;    // (pass, key tile) steps of this query tile so far, over all items: the phase of s_full
-    int turns = 0;    // key-tile iterations so far: the phase of the turn barriers
-    int pv_base = 0;  // key tiles whose P.V was issued for earlier items: the phase of o_done
+    int steps = 0;    // (pass, key tile) steps of this group so far, over all items: buffer and phase of s_full
+    int ends[2] = {0, 0};  // items with two key tiles or more, with one or more so far: the phases of o_done
     int meets = 0;    // meetings of the two groups so far: the phase of xchg
     bool ok = true;
     // Split keys: the two groups meet, and each thread learns what the other group's thread of its row brings.  The
@@ -370,14 +381,47 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int item_id = next_item(n, lane == 0);
       if (item_id < 0) break;
       const Item it = decode(item_id);
-      const int bh = it.bh, n_max = max(it.nq[0], it.nq[1]);
+      const int bh = it.bh + (TWIN ? q : 0);
       const int n_tiles = it.nq[q];
-      const int m_tile = it.m0 + (SPLIT ? 0 : q * BM);
+      const int m_tile = it.m0 + (MODE == kPair ? q * BM : 0);
       // (both groups have read both O of the item before)
       if (SPLIT && n > 0) meet(make_float2(0.f, 0.f));
       const int g_row = m_tile + row;  // query index within the head
       float m_ref = -INFINITY;  // reference maximum (scaled, log2 units) the stored P and O are relative to
       float l_sum = 0.f;
+
+      uint32_t sr[2][32];  // the scores of a key tile
+      auto load_scores = [&]() {  // of step `steps`
+        tc_fence_after_sync();
+#pragma unroll
+        for (int c = 0; c < 2; ++c) tmem_ld_32x32b_x32(t_s + (steps & 1) * BN + c * 32, sr[c]);
+      };
+      auto scores_there = [&](bool more) -> bool {  // (the vote is taken in any case: behind a branch on `more` the loop is 13 % slower)
+        return __all_sync(0xffffffffu, more && mbar_test(&s_full[2 * q + (steps & 1)], (steps >> 1) & 1));
+      };
+      auto wait_scores = [&]() {
+        if (ok) ok = mbar_wait(&s_full[2 * q + (steps & 1)], (steps >> 1) & 1, abort_flag, p.status, ST_ATTN_S);
+        if (ok) load_scores();
+      };
+      auto mask_scores = [&](int n0) {  // of keys n0..
+        if ((n0 + BN > p.S_kv) || (p.causal && (n0 + BN - 1 > m_tile + off))) {
+          int limit = p.S_kv - 1;
+          if (p.causal) limit = min(limit, g_row + off);
+          limit -= n0;  // columns > limit are hidden
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (c * 32 + i > limit) sr[c][i] = 0xff800000u;  // -inf
+        }
+      };
+      auto row_max = [&](float (&m)[4]) {  // in four chains
+#pragma unroll
+        for (int e = 0; e < 16; ++e)
+#pragma unroll
+          for (int c = 0; c < 2; ++c)
+            m[2 * c + (e & 1)] = max3f(m[2 * c + (e & 1)], __uint_as_float(sr[c][2 * e]), __uint_as_float(sr[c][2 * e + 1]));
+      };
 
       if (NORM) {
         // The reference's semantics (benchmark/layout/execution/tiled_attention.py:697-698,
@@ -406,34 +450,17 @@ __global__ void __launch_bounds__(kThreads, 1)
           const float inv_l = __frcp_rn(l_run);  // (of use in pass 1 only)
           const float2 inv2 = make_float2(inv_l, inv_l), negl2 = make_float2(-l_run, -l_run);
           for (int i = 0; i < n_tiles; ++i) {
-            const int j = SPLIT ? 2 * i + q : i;
-            if (!mbar_wait(&s_full[q], steps & 1, abort_flag, p.status, ST_ATTN_S)) {
-              ok = false;
-              break;
-            }
+            const int buf = steps & 1;
+            wait_scores();
+            if (!ok) break;
             ++steps;
-            tc_fence_after_sync();
-            uint32_t sr[4][32];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(t_s + c * 32, sr[c]);
             tmem_ld_wait();
             if (pass == 0) {
-              // S_q is in registers: the MMA warp may overwrite it
+              // the scores are in registers: the MMA warp may overwrite them
               tc_fence_before_sync();
-              mbar_arrive(&p_ready[q]);
-              mbar_arrive(&p_ready_hi[q]);
+              mbar_arrive(&p_ready[2 * q + buf]);
             }
-            const int n0 = j * BN;
-            if ((n0 + BN > p.S_kv) || (p.causal && (n0 + BN - 1 > m_tile + off))) {
-              int limit = p.S_kv - 1;
-              if (p.causal) limit = min(limit, g_row + off);
-              limit -= n0;  // columns > limit are hidden
-#pragma unroll
-              for (int c = 0; c < 4; ++c)
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                  if (c * 32 + i > limit) sr[c][i] = 0xff800000u;  // -inf
-            }
+            mask_scores((SPLIT ? 2 * i + q : i) * BN);
             // (score - m) * log2e of a pair, rounded step by step; the scale is positive, so it keeps the order and
             // the maximum of the scaled scores is the scaled maximum
             auto arg2 = [&](int c, int i, float2 negm2) {
@@ -442,11 +469,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             };
             if (pass == 0) {
               float mxc[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-              for (int i = 0; i < 16; ++i)
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                  mxc[c] = max3f(mxc[c], __uint_as_float(sr[c][2 * i]), __uint_as_float(sr[c][2 * i + 1]));
+              row_max(mxc);
               const float mx = __fmul_rn(max3f(mxc[0], mxc[1], fmaxf(mxc[2], mxc[3])), p.scale);
               const float m_new = fmaxf(m_run, mx);
               if (m_new != -INFINITY) {
@@ -457,9 +480,9 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
                 for (int i = 0; i < 16; ++i)
 #pragma unroll
-                  for (int c = 0; c < 4; ++c) {
+                  for (int c = 0; c < 2; ++c) {
                     const float2 x = arg2(c, i, negm2);
-                    sum[c] = add2_rn(sum[c], make_float2(exp2_of(x.x), exp2_of(x.y)));
+                    sum[2 * c + (i & 1)] = add2_rn(sum[2 * c + (i & 1)], make_float2(exp2_of(x.x), exp2_of(x.y)));
                   }
                 const float2 all = add2_rn(add2_rn(sum[0], sum[1]), add2_rn(sum[2], sum[3]));
                 const float carry = (m_run == -INFINITY) ? 0.f : l_run * ex2f_ieee_range(__fmul_rn(__fsub_rn(m_run, m_new), kLog2e));
@@ -469,7 +492,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             } else {
               const float2 negm2 = make_float2(-m_run, -m_run);
 #pragma unroll
-              for (int c = 0; c < 4; ++c) {
+              for (int c = 0; c < 2; ++c) {
                 uint32_t pk[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
@@ -477,80 +500,71 @@ __global__ void __launch_bounds__(kThreads, 1)
                   const float2 pv = div2_by(make_float2(exp2_of(x.x), exp2_of(x.y)), negl2, inv2);
                   pk[i] = pack16<BF16>(pv.x, pv.y);
                 }
-                tmem_st_32x32b_x16(t_s + c * 16, pk);
-                if (c & 1) {
-                  tmem_st_wait();
-                  tc_fence_before_sync();
-                  mbar_arrive(c == 1 ? &p_ready[q] : &p_ready_hi[q]);
-                }
+                tmem_st_32x32b_x16(t_s + buf * BN + c * 16, pk);
               }
+              tmem_st_wait();
+              tc_fence_before_sync();
+              mbar_arrive(&p_ready[2 * q + buf]);
             }
           }
         }
         l_sum = 1.0f;  // P is already normalised
         m_ref = 0.f;
-      } else
-      // The two softmax groups take turns: group 1 starts the arithmetic of its key tile j when group 0 has
-      // finished that of its tile j (all 128 keys: handing over after the first 64 measured 3 % slower), and group 0
-      // starts tile j+1 when group 1 has finished tile j.  Left alone the
-      // two groups fall into step (they share the K/V ring and the tensor pipe), exponentiate at the same time
-      // on the same four schedulers and then both sit idle while their MMAs run; taking turns, one group works
-      // alone (a third faster) while the other group's P.V and next S are in flight.  A group with fewer key
-      // tiles than the other keeps passing the turn on until the other is done.
-      for (int i = 0; i < n_max; ++i) {
-        const bool mine = i < n_tiles;
-        uint32_t sr[4][32];
-        if (mine) {
-          if (!mbar_wait(&s_full[q], steps & 1, abort_flag, p.status, ST_ATTN_S)) {
-            ok = false;
-            break;
-          }
-          ++steps;
+      } else {
+      // The scores of a key tile are read as soon as those of the tile before are used up, if they are there by then (usually
+      // they are), and else after that tile's P has been handed over.
+      if (n_tiles > 0) {
+        // The first reference is the maximum of two key tiles: more rows then have their largest probability at 1, which loses
+        // nothing when it is rounded (2.10e-3 from 64 bits at 8 x 32 x 4096; with one key tile's 2.11e-3).
+        float mx = -INFINITY;
+        for (int t = 0; t < min(n_tiles, 2); ++t) {
+          const int n0 = (SPLIT ? 2 * t + q : t) * BN, step = steps + t;
+          ok = mbar_wait(&s_full[2 * q + (step & 1)], (step >> 1) & 1, abort_flag, p.status, ST_ATTN_S);
+          if (!ok) break;
           tc_fence_after_sync();
 #pragma unroll
-          for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(t_s + c * 32, sr[c]);
+          for (int c = 0; c < 2; ++c) tmem_ld_32x32b_x32(t_s + (step & 1) * BN + c * 32, sr[c]);
           tmem_ld_wait();
-
-          const int n0 = (SPLIT ? 2 * i + q : i) * BN;
-          const bool needs_mask = (n0 + BN > p.S_kv) || (p.causal && (n0 + BN - 1 > m_tile + off));
-          if (needs_mask) {
-            int limit = p.S_kv - 1;
-            if (p.causal) limit = min(limit, g_row + off);
-            limit -= n0;  // columns > limit are hidden
+          mask_scores(n0);
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (c * 32 + i > limit) sr[c][i] = 0xff800000u;  // -inf
+          for (int e = 0; e < 32; ++e) mx = max3f(mx, __uint_as_float(sr[0][e]), __uint_as_float(sr[1][e]));
+        }
+        // A row that has seen no key, or only scores of -inf: the lowest finite reference, so that its exponentials are 0 and the
+        // first finite score moves it (0 would let lower scores vanish; a group's first key tiles may be any row's -inf).
+        m_ref = fmaxf(mx * p.scale_log2, -FLT_MAX);
+        // The groups begin a CTA's first item at the same time, and two that work in step leave the special-function unit idle
+        // together between their key tiles.  So group 1 begins later, by about a third of its work on a tile.  (Later items begin
+        // as far apart as the ones before ended; where tiles are short and equally many it pays for every item.)
+        // 8 x 8192, D = 128 265 -> 255 us, causal 138 -> 128; D = 64, 12 x 2048 36.2 -> 32.2, 15 x 11 x 479 30.2 -> 29.2.
+        if (q == 1 && n_tiles > 3 && (n == 0 || (D == 64 && !p.causal))) {
+          const long long from = clock64();
+          while (clock64() - from < 300) {
           }
         }
+        if (ok) load_scores();
+      }
+      for (int i = 0; i < n_tiles && ok; ++i) {
+        const int buf = steps & 1;
+        ++steps;
+        tmem_ld_wait();
+        mask_scores((SPLIT ? 2 * i + q : i) * BN);
+        const bool more = i + 1 < n_tiles;
         const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
         float mxc[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four chains of the row maximum
-        auto max_step = [&](int i) {  // two keys of every 32
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            mxc[c] = max3f(mxc[c], __uint_as_float(sr[c][2 * i]), __uint_as_float(sr[c][2 * i + 1]));
-        };
-        // Takes the row maximum into the reference; true where that has moved (exponentials relative to the one before are
-        // void).  O is rescaled only when the maximum grew by more than the threshold: rare after the first tiles.
-        auto settle = [&]() -> bool {
+        // Takes the row maximum into the reference.  O is rescaled only when the maximum grew by more than the threshold: rare.
+        auto settle = [&]() {
           const float mx = max3f(mxc[0], mxc[1], fmaxf(mxc[2], mxc[3]));
-          float m_new = fmaxf(m_ref, mx * p.scale_log2);
-          // A row that has seen no key, or only scores of -inf: the lowest finite reference, so that its exponentials are 0 and the
-          // first finite score moves it (0 would let lower scores vanish; a group's first key tile may be any row's -inf).
-          if (m_new == -INFINITY) m_new = -FLT_MAX;
-          if (i == 0) {
-            m_ref = m_new;
-            return true;
-          }
+          const float m_new = fmaxf(m_ref, mx * p.scale_log2);
           // (warp-uniform decision because the TMEM accesses are warp-collective)
-          if (!__any_sync(0xffffffffu, m_new - m_ref > kRescaleThreshold)) return false;
+          if (!__any_sync(0xffffffffu, m_new - m_ref > kRescaleThreshold)) return;
           const float factor = ex2f(m_ref - m_new);
           m_ref = m_new;
           l_sum *= factor;
           // O_q must be complete up to the key tile before this one before it is scaled
-          ok = mbar_wait(&o_done[q], (pv_base + i - 1) & 1, abort_flag, p.status, ST_ATTN_O);
-          if (!ok) return true;
+          // (the scores of the next key tile come after that product)
+          ok = i + 1 < n_tiles ? mbar_wait(&s_full[2 * q + (buf ^ 1)], (steps >> 1) & 1, abort_flag, p.status, ST_ATTN_S)
+                               : mbar_wait(&o_done[2 * q], ends[0] & 1, abort_flag, p.status, ST_ATTN_O);
+          if (!ok) return;
           tc_fence_after_sync();
 #pragma unroll
           for (int c = 0; c < D / 32; ++c) {
@@ -561,79 +575,42 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * factor);
             tmem_st_32x32b_x32(t_o + c * 32, o);
           }
-          return true;
         };
-        if (kMaxFirst && mine) {
-#pragma unroll
-          for (int e = 0; e < 16; ++e) max_step(e);
-          settle();
-          if (!ok) break;
-        }
-        if (!mbar_wait(&turn[q], q == 0 ? ((turns & 1) ^ 1) : (turns & 1), abort_flag, p.status, ST_ATTN_S)) {
-          ok = false;
-          break;
-        }
-        ++turns;
-        if (!mine) {
-          mbar_arrive(&turn[q ^ 1]);
-          continue;
-        }
-
-        // P = 2^(s*scale_log2 - m_ref) with packed fp32 FMAs, row sum in fp32, P rounded to 16 bits.
-        // Two 32-key chunks at a time, interleaved pair by pair so that the special-function unit always has
-        // independent work.  WITH_MAX also runs the row maximum of all 128 keys through the same loop: the maximum is a
-        // chain on the ALU, the exponentials are bound by the special-function unit, and neither waits for the other.
-        auto exp_chunks = [&](int c0, uint32_t (&pa)[16], uint32_t (&pb)[16], float2& sum, auto with_max) {
-          const float2 negm2 = make_float2(-m_ref, -m_ref);
-          float2 sa = make_float2(0.f, 0.f), sb = make_float2(0.f, 0.f);
-#pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            const float2 xa = fma2(make_float2(__uint_as_float(sr[c0][2 * e]), __uint_as_float(sr[c0][2 * e + 1])), scale2, negm2);
-            const float2 xb = fma2(make_float2(__uint_as_float(sr[c0 + 1][2 * e]), __uint_as_float(sr[c0 + 1][2 * e + 1])), scale2, negm2);
-            if (decltype(with_max)::value) max_step(e);
-            const float2 ea = make_float2(ex2f(xa.x), ex2f(xa.y));
-            const float2 eb = make_float2(ex2f(xb.x), ex2f(xb.y));
-            sa = add2(sa, ea);
-            sb = add2(sb, eb);
-            pa[e] = pack16<BF16>(ea.x, ea.y);
-            pb[e] = pack16<BF16>(eb.x, eb.y);
-          }
-          sum = add2(sa, sb);
-        };
+        row_max(mxc);
+        settle();
+        if (!ok) break;
+        // P = 2^(s*scale_log2 - m_ref) with packed fp32 FMAs, row sum in fp32, P rounded to 16 bits.  The two 32-key halves are
+        // interleaved pair by pair so that the special-function unit always has independent work.
         uint32_t pk0[16], pk1[16];
-        float2 sum01;
-        if (kMaxFirst) {
-          exp_chunks(0, pk0, pk1, sum01, std::false_type());
-        } else {
-          // Optimistic first half: the exponentials of keys 0-63 are taken relative to the reference maximum the row
-          // already has, so they do not wait for the row maximum, and are computed again where that moves it (always on
-          // the first tile, whose reference is -infinity).  The stale reference cannot overflow what is kept: a value
-          // that would exceed 2^threshold is by construction one that moves it.
-          exp_chunks(0, pk0, pk1, sum01, std::true_type());
-          const bool redo = settle();
-          if (!ok) break;
-          if (redo) exp_chunks(0, pk0, pk1, sum01, std::false_type());
+        const float2 negm2 = make_float2(-m_ref, -m_ref);
+        float2 sa = make_float2(0.f, 0.f), sb = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          const float2 xa = fma2(make_float2(__uint_as_float(sr[0][2 * e]), __uint_as_float(sr[0][2 * e + 1])), scale2, negm2);
+          const float2 xb = fma2(make_float2(__uint_as_float(sr[1][2 * e]), __uint_as_float(sr[1][2 * e + 1])), scale2, negm2);
+          const float2 ea = make_float2(ex2f(xa.x), ex2f(xa.y));
+          const float2 eb = make_float2(ex2f(xb.x), ex2f(xb.y));
+          sa = add2(sa, ea);
+          sb = add2(sb, eb);
+          pk0[e] = pack16<BF16>(ea.x, ea.y);
+          pk1[e] = pack16<BF16>(eb.x, eb.y);
         }
-        // P is written back over S chunk by chunk; a half of P (64 keys) that is complete lets the MMA warp start on it
-        tmem_st_32x32b_x16(t_s, pk0);
-        tmem_st_32x32b_x16(t_s + 16, pk1);
+        const float2 tot = add2(sa, sb);
+        const bool ahead = scores_there(more);
+        if (ahead) load_scores();
+        // P is written over the first half of the scores it comes from
+        tmem_st_32x32b_x16(t_s + buf * BN, pk0);
+        tmem_st_32x32b_x16(t_s + buf * BN + 16, pk1);
         tmem_st_wait();
         tc_fence_before_sync();
-        mbar_arrive(&p_ready[q]);
-        float2 sum23;
-        exp_chunks(2, pk0, pk1, sum23, std::false_type());
-        tmem_st_32x32b_x16(t_s + 32, pk0);
-        tmem_st_32x32b_x16(t_s + 48, pk1);
-        tmem_st_wait();
-        tc_fence_before_sync();
-        mbar_arrive(&p_ready_hi[q]);
-        mbar_arrive(&turn[q ^ 1]);  // the other group's turn: its scores arrived while this one worked alone
-        const float2 tot = add2(sum01, sum23);
+        mbar_arrive(&p_ready[2 * q + buf]);
         l_sum += tot.x + tot.y;
+        if (more && !ahead) wait_scores();
+      }
       }
 
       // ---- epilogue: O / l
-      if (ok && n_tiles > 0) ok = mbar_wait(&o_done[q], (pv_base + n_tiles - 1) & 1, abort_flag, p.status, ST_ATTN_O);
+      if (ok && n_tiles > 0) ok = mbar_wait(&o_done[2 * q + 1], ends[1] & 1, abort_flag, p.status, ST_ATTN_O);
       float f_first = 0.f, f_second = 0.f;
       int c_begin = 0, c_end = D / 32;  // 32-column chunks of O this group stores
       if (SPLIT) {
@@ -718,7 +695,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
-      pv_base += n_tiles;
+      ends[0] += n_tiles > 1;
+      ends[1] += n_tiles > 0;
     }
   }
 
@@ -747,32 +725,31 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // Items of ONE query tile or of two.  A lone tile has half of its SM's softmax and MMA threads idle where its keys are not split
 // (split_keys_pay: one key tile, two in the single pass), but more items balance better.  So lone tiles are taken where that leaves at most one item per SM, and
-// beyond that where this estimate is clearly better: in steps (one key tile of two query tiles side by side, 2.1 us at D = 128), a pair of
-// tiles takes its key tiles, a split lone tile 0.56 a key tile (304 us for 8 x 8192 where pairs take 273), either 1.9 more to
-// begin and end; equal items go round by round, causal ones heavy first.  Estimated / measured ratios: 12 heads x 2048 causal 0.66 / 0.66
-// (44.2 -> 29.0 us; D = 64 34.9 -> 21.5), 15 x 2013 causal 0.79 / 0.72, 10 x 4096 causal 0.87 / 0.78, 64 x 700 normalised 0.93 / 0.84,
-// 64 x 1025 0.80 / 0.85; 24 x 1000 1.29 / 1.18, 8 x 8192 1.14 / 1.12, 64 x 2048 causal 1.14 / 1.23.  Of 68 shapes the estimate
-// is too low only for causal ones of few key tiles (50 x 612 0.93 / 1.18), and too high in the normalised mode (36 x 978 1.21 / 1.06):
-// hence 0.9 and 0.95.
+// beyond that where this estimate is clearly better: in steps (128 keys of two query tiles side by side, 1.8 us at D = 128), a pair of
+// tiles takes its key tiles, a split lone tile 0.56 a step, either 1.9 more to begin and end; equal items go round by round,
+// causal ones heavy first.  Estimated / measured ratios: 12 heads x 2048 causal 0.67 / 0.61 (34.5 against 21.2 us; D = 64 32.5
+// against 20.9), 15 x 2013 causal 0.79 / 0.65, 10 x 4096 causal 0.87 / 0.72, 64 x 700 normalised 0.93 / 0.88, 64 x 1025 0.80 / 0.85;
+// 64 x 2048 causal 1.14 / 1.16.  Of 63 shapes the choice costs more than 2 % in 6, at most 8 %.  The estimate is too low for
+// causal ones of few key tiles (50 x 612 0.93 / 1.16) and too high in the normalised mode (36 x 978 1.21 / 1.05): hence 0.9 and 0.95.
 double items_estimate(const frisk_b200_attn_desc& d, int sms, int tiles_per_item) {
   constexpr double kSplitStep = 0.56, kItem = 1.9;
   const int64_t heads = (int64_t)d.B * d.H, tiles = (d.S_q + BM - 1) / BM;
   const int64_t groups = (tiles + tiles_per_item - 1) / tiles_per_item, items = groups * heads;
   const double step = (tiles_per_item == 1 ? kSplitStep : 1.0) * (d.normalize_p ? 2 : 1);
-  const int64_t all = (d.S_kv + BN - 1) / BN, off = (int64_t)d.S_kv - d.S_q;
+  const int64_t all = (d.S_kv + 127) / 128, off = (int64_t)d.S_kv - d.S_q;
   const double heaviest = step * (double)all + kItem;
   if (!d.causal) return (double)((items + sms - 1) / sms) * heaviest;
   if (items <= sms) return heaviest;
   double total = 0;
   for (int64_t g = 0; g < groups; ++g) {
     const int64_t last_row = std::min<int64_t>((g + 1) * tiles_per_item * BM, d.S_q) - 1;
-    total += step * (double)std::min<int64_t>(all, std::max<int64_t>(0, last_row + off) / BN + 1) + kItem;
+    total += step * (double)std::min<int64_t>(all, std::max<int64_t>(0, last_row + off) / 128 + 1) + kItem;
   }
   return std::max(heaviest, (double)heads * total / sms + 0.5 * total / (double)groups);
 }
-// A lone tile's key tiles are worth sharing from two on in the normalised mode (33 heads x 251 11.8 -> 10.4 us) and from three
-// on in the single pass, where with two the meeting of the groups costs what it saves (48 heads x 159 9.4 us, 9.7 split).
-bool split_keys_pay(const frisk_b200_attn_desc& d) { return d.S_kv > (d.normalize_p ? BN : 2 * BN); }
+// A lone tile's keys are worth sharing beyond 128 in the normalised mode (33 heads x 251 11.8 -> 10.4 us) and beyond 256 in the
+// single pass, where with fewer the meeting of the groups costs what it saves (16 heads x 256 and 48 x 159 as fast either way).
+bool split_keys_pay(const frisk_b200_attn_desc& d) { return d.S_kv > (d.normalize_p ? 128 : 256); }
 
 bool one_tile_items(const frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d) {
   const int64_t tiles = (d.S_q + BM - 1) / BM * d.B * d.H;
@@ -782,7 +759,7 @@ bool one_tile_items(const frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d) {
   return items_estimate(d, ctx->num_sms, 1) < (d.normalize_p ? 0.95 : 0.9) * items_estimate(d, ctx->num_sms, 2);
 }
 
-template <bool BF16, int D, bool OUT_F32, bool NORM, bool SPLIT>
+template <bool BF16, int D, bool OUT_F32, bool NORM, Mode MODE>
 int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K, const void* V,
                void* O, cudaStream_t s) {
   CUtensorMap tq, tk, tv;
@@ -801,10 +778,11 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q
   AttnParams p;
   p.S_q = d.S_q;
   p.S_kv = d.S_kv;
-  p.group_rows = one_tile_items(ctx, d) ? BM : 2 * BM;
+  p.group_rows = MODE == kTwin || one_tile_items(ctx, d) ? BM : 2 * BM;
   p.n_groups = (d.S_q + p.group_rows - 1) / p.group_rows;
   p.causal = d.causal ? 1 : 0;
-  p.total_items = (int64_t)p.n_groups * bh;
+  p.heads = bh;
+  p.total_items = MODE == kTwin ? ((int64_t)bh + 1) / 2 : (int64_t)p.n_groups * bh;
   p.scale_log2 = d.scale * 1.4426950408889634f;
   p.scale = d.scale;
   p.normalized = d.normalize_p ? 1 : 0;
@@ -812,7 +790,7 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q
   p.status = ctx->d_status;
   p.work = ctx->d_status + 16;  // work counter and exit counter of the persistent grid (zero between launches)
   if (p.total_items > INT32_MAX) return FRISK_B200_E_ATTN_SHAPE;
-  auto kern = attention_fwd_kernel<BF16, D, OUT_F32, NORM, SPLIT>;
+  auto kern = attention_fwd_kernel<BF16, D, OUT_F32, NORM, MODE>;
   using L = AttnSmem<D>;
   // setmaxnreg.inc waits (without a bound) until the CTA's own register pool holds what it
   // asks for: the registers the TMA/MMA warpgroup (128 threads) gives up must cover what the
@@ -846,25 +824,28 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q
 }
 
 template <bool BF16, int D, bool OUT_F32, bool NORM>
-int launch_split(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K, const void* V,
+int launch_mode(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K, const void* V,
                  void* O, cudaStream_t s) {
-  // A lone query tile's key tiles go to the two softmax groups in turn: one group alone is
-  // bound by the chain S -> softmax -> P.V -> next S (1.4 us a key tile at D = 64 normalised), and two such chains overlap.
-  // 16 heads x 1025 normalised 29.2 -> 23.4 us; single pass, D = 128: 4 heads x 4096 causal 62.1 -> 40.4, 2 x 8192 121.4 -> 75.3,
-  // 8 x 1000 19.8 -> 15.2; D = 64: 4 x 3000 42.5 -> 27.5.
-  if (split_keys_pay(d) && one_tile_items(ctx, d)) return launch_cfg<BF16, D, OUT_F32, NORM, true>(ctx, d, Q, K, V, O, s);
-  return launch_cfg<BF16, D, OUT_F32, NORM, false>(ctx, d, Q, K, V, O, s);
+  // A lone query tile's key tiles go to the two softmax groups in turn: one group alone leaves the schedulers idle while it
+  // waits for tensor memory and barriers (with one buffer of scores: 16 heads x 1025 normalised 29.2 -> 23.4 us, 4 heads x 4096
+  // causal at D = 128 62.1 -> 40.4; with two 22.1 and 32.9).
+  if (split_keys_pay(d) && one_tile_items(ctx, d)) return launch_cfg<BF16, D, OUT_F32, NORM, kSplit>(ctx, d, Q, K, V, O, s);
+  // Heads of one query tile, more of them than SMs: two at a time, since a pair's second group would be idle (512 heads x 128,
+  // D = 64 13.9 -> 11.9 us, D = 128 19.2 -> 16.5).  In the normalised mode a lone tile is as fast.
+  if (!NORM && d.S_q <= BM && (int64_t)d.B * d.H > ctx->num_sms)
+    return launch_cfg<BF16, D, OUT_F32, NORM, NORM ? kPair : kTwin>(ctx, d, Q, K, V, O, s);
+  return launch_cfg<BF16, D, OUT_F32, NORM, kPair>(ctx, d, Q, K, V, O, s);
 }
 
 template <bool BF16, int D>
 int launch_out(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K, const void* V,
                void* O, cudaStream_t s) {
   if (d.normalize_p) {
-    if (d.dtype_out == FRISK_B200_F32) return launch_split<BF16, D, true, true>(ctx, d, Q, K, V, O, s);
-    return launch_split<BF16, D, false, true>(ctx, d, Q, K, V, O, s);
+    if (d.dtype_out == FRISK_B200_F32) return launch_mode<BF16, D, true, true>(ctx, d, Q, K, V, O, s);
+    return launch_mode<BF16, D, false, true>(ctx, d, Q, K, V, O, s);
   }
-  if (d.dtype_out == FRISK_B200_F32) return launch_split<BF16, D, true, false>(ctx, d, Q, K, V, O, s);
-  return launch_split<BF16, D, false, false>(ctx, d, Q, K, V, O, s);
+  if (d.dtype_out == FRISK_B200_F32) return launch_mode<BF16, D, true, false>(ctx, d, Q, K, V, O, s);
+  return launch_mode<BF16, D, false, false>(ctx, d, Q, K, V, O, s);
 }
 
 }  // namespace

@@ -66,6 +66,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Bounded wait.  `abort_flag` is a shared-memory word any role sets when it gives up, so
 // that the other roles stop waiting too.  Returns false when the wait was abandoned.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag,
@@ -84,6 +95,25 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
       }
     }
   }
+}
+
+// Waits for two barriers: where both phases are complete, the usual case for a thread that is behind its suppliers, the two
+// tests' latencies overlap.
+__device__ __forceinline__ bool mbar_wait_both(uint64_t* bar_a, uint32_t parity_a, uint64_t* bar_b, uint32_t parity_b,
+                                               volatile uint32_t* abort_flag, unsigned* status, unsigned code_a,
+                                               unsigned code_b) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+      "and.pred p, p, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar_a)), "r"(parity_a), "r"(smem_u32(bar_b)), "r"(parity_b)
+      : "memory");
+  return ok != 0 || (mbar_wait(bar_a, parity_a, abort_flag, status, code_a) &&
+                     mbar_wait(bar_b, parity_b, abort_flag, status, code_b));
 }
 
 // ---------------------------------------------------------------- fences
