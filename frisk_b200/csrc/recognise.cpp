@@ -5,8 +5,8 @@
 //                 | (True, M, N, K, type of A, type of C, trans_a, trans_b, clear_accum, policy, ia, ib, ic,
 //                    fill or None, reduce kind or None, reduce argument, reduce_clear)        one gemm, its fill and reduce
 //
-// Walking and verifying a built kernel op by op in Python took most of a small call (a 64 x 64 attention tile 53.1 us, 22.0 with
-// this module, whose part is 12; a 512 x 384 x 256 gemm with fill and reduce 28.8 and 14.3, of which 3.6), and nothing may be
+// Walking and verifying a built kernel op by op in Python took most of a small call (a 64 x 64 attention tile 53.1 us, 17.1 with
+// this module, whose part is 8; a 512 x 384 x 256 gemm with fill and reduce 28.8 and 13.5, of which 3), and nothing may be
 // remembered between calls, since every list and attribute of the IR can be changed at any time.  So the same walk and
 // the checks of ir._verify and of tensor_ops.attention_plan / execute.fused_plan are made here, read off the same objects.
 //
@@ -16,6 +16,8 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <cstring>
+#include <deque>
 #include <utility>
 #include <vector>
 
@@ -61,6 +63,33 @@ Ref attr(const Ref& o, PyObject* name) {
   if (!v) PyErr_Clear();
   return Ref(v);
 }
+// The attributes of one object.  The IR's objects hold theirs in the instance's dictionary, where one costs a third of
+// PyObject_GetAttr, which looks through the classes first; what is not there is asked for the usual way.
+class Fields {
+ public:
+  explicit Fields(const Ref& o) : o_(o.get()), dict_(o ? PyObject_GenericGetDict(o.get(), nullptr) : nullptr) {
+    if (o_ && !dict_) PyErr_Clear();
+  }
+  Ref operator()(PyObject* name) const {
+    if (!o_) return Ref();
+    PyObject* v = dict_ ? PyDict_GetItemWithError(dict_.get(), name) : nullptr;
+    if (v) return Ref(Py_NewRef(v));
+    PyErr_Clear();
+    v = PyObject_GetAttr(o_, name);
+    if (!v) PyErr_Clear();
+    return Ref(v);
+  }
+  bool holds(PyObject* name) const {  // in the instance itself
+    if (!dict_) return true;
+    const int has = PyDict_Contains(dict_.get(), name);
+    if (has < 0) PyErr_Clear();
+    return has != 0;
+  }
+
+ private:
+  PyObject* o_;  // (the caller keeps it)
+  Ref dict_;
+};
 Ref key(const Ref& dict, PyObject* name) {
   if (!dict || !PyDict_CheckExact(dict.get())) return Ref();
   PyObject* v = PyDict_GetItemWithError(dict.get(), name);
@@ -73,7 +102,9 @@ Ref item(const Ref& list, Py_ssize_t i) {
 }
 Py_ssize_t length(const Ref& list) { return list && PyList_CheckExact(list.get()) ? PyList_GET_SIZE(list.get()) : -1; }
 bool text_is(const Ref& s, const char* t) {
-  return s && PyUnicode_CheckExact(s.get()) && PyUnicode_CompareWithASCIIString(s.get(), t) == 0;
+  if (!s || !PyUnicode_CheckExact(s.get()) || !PyUnicode_IS_COMPACT_ASCII(s.get())) return false;  // (the names are ASCII)
+  const size_t n = strlen(t);
+  return (size_t)PyUnicode_GET_LENGTH(s.get()) == n && memcmp(PyUnicode_DATA(s.get()), t, n) == 0;
 }
 bool to_int(const Ref& o, long long* out) {
   if (!o || !PyLong_CheckExact(o.get())) return false;
@@ -120,74 +151,111 @@ struct Value {
   bool is_arg = false;
 };
 
+struct Values {  // up to three, which the kernel's list of known values holds
+  const Value* at[3] = {nullptr, nullptr, nullptr};
+  size_t n = 0;
+  const Value& operator[](size_t i) const { return *at[i]; }
+  size_t size() const { return n; }
+  bool empty() const { return n == 0; }
+};
+
 struct Op {
   Ref op, attrs, name;  // name: op_name of an upstream op
   Class cls = kOther;
-  std::vector<Value> in, out;
+  Values in, out;
+};
+
+// What has been read in this call already (an object appears many times), and the objects it was read from.
+template <typename T>
+struct Known {
+  std::vector<PyObject*> ids;  // looked through from the end: most operands have just been results
+  std::deque<T> what;          // (does not move)
+  std::vector<Ref> keep;
+  Known() {
+    ids.reserve(64);
+    keep.reserve(64);
+  }
+  const T* find(PyObject* id) const {
+    for (size_t j = ids.size(); j > 0; --j)
+      if (ids[j - 1] == id) return &what[j - 1];
+    return nullptr;
+  }
+  const T* add(const Ref& o, T&& t) {
+    what.push_back(std::move(t));
+    keep.push_back(o);
+    ids.push_back(o.get());
+    return &what.back();
+  }
 };
 
 struct Kernel {
   std::vector<Op> ops;  // nested ones, in program order
   Ref entry;
-  std::vector<std::pair<PyObject*, Shaped>> types;  // read in this call already (an object appears many times)
-  std::vector<Value> values;                        // likewise
-  std::vector<Ref> keep;
+  Known<Shaped> types;
+  Known<Value> values;
+  Known<Element> elements;
+  bool class_has_place = false;  // the class of the types itself has a `space` or a `map`
 };
+
+bool read_element(Kernel& k, const Ref& e, Element* out) {
+  if (!is_a(e, type_class)) return false;
+  if (const Element* known = k.elements.find(e.get())) {
+    *out = *known;
+    return true;
+  }
+  const Fields of(e);
+  if (!text_is(of(names.kind), "float")) return false;
+  const Ref name = of(names.name);
+  *out = text_is(name, "f16") ? kF16 : text_is(name, "bf16") ? kBF16 : text_is(name, "f32") ? kF32 : text_is(name, "f64") ? kF64 : kNone;
+  if (*out == kNone) return false;
+  k.elements.add(e, Element(*out));
+  return true;
+}
 
 bool read_type(Kernel& k, const Ref& t, Shaped* out) {
   if (!is_a(t, type_class)) return false;
-  for (const auto& known : k.types)
-    if (known.first == t.get()) {
-      *out = known.second;
-      return true;
-    }
+  if (const Shaped* known = k.types.find(t.get())) {
+    *out = *known;
+    return true;
+  }
   Shaped s;
-  const Ref kind = attr(t, names.kind);
+  const Fields of(t);
+  const Ref kind = of(names.kind);
   s.memref = text_is(kind, "memref");
   if (!s.memref && !text_is(kind, "tensor")) return false;
-  const Ref shape = attr(t, names.shape), element = attr(t, names.element);
+  const Ref shape = of(names.shape), element = of(names.element);
   s.rank = (int)length(shape);
   if (s.rank < 1 || s.rank > 2) return false;
   for (int i = 0; i < s.rank; ++i)
     if (!to_int(item(shape, i), &s.e[i]) || s.e[i] <= 0 || s.e[i] > (1LL << 40)) return false;
-  if (!is_a(element, type_class) || !text_is(attr(element, names.kind), "float")) return false;
-  const Ref name = attr(element, names.name);
-  s.element = text_is(name, "f16") ? kF16 : text_is(name, "bf16") ? kBF16 : text_is(name, "f32") ? kF32 : text_is(name, "f64") ? kF64 : kNone;
-  if (s.element == kNone) return false;
+  if (!read_element(k, element, &s.element)) return false;
   if (s.memref) {
-    if (!to_enum(attr(t, names.space), space_class, &s.space)) return false;
-    s.map = attr(t, names.map);
+    if (!to_enum(of(names.space), space_class, &s.space)) return false;
+    s.map = of(names.map);
     if (!s.map) return false;
-  } else if (PyObject_HasAttr(t.get(), names.space) || PyObject_HasAttr(t.get(), names.map)) {
+  } else if (k.class_has_place || of.holds(names.space) || of.holds(names.map)) {
     return false;  // (a tensor has neither; types are compared with them)
   }
-  k.types.emplace_back(t.get(), s);
-  k.keep.push_back(t);
-  *out = s;
+  *out = *k.types.add(t, std::move(s));
   return true;
 }
 
-bool read_values(Kernel& k, const Ref& list, std::vector<Value>* out) {
+bool read_values(Kernel& k, const Ref& list, Values* out) {
   const Py_ssize_t n = length(list);
   if (n < 0 || n > 3) return false;
-  out->resize(n);
+  out->n = (size_t)n;
   for (Py_ssize_t i = 0; i < n; ++i) {
     const Ref v = item(list, i);
-    Value& x = (*out)[i];
-    bool known = false;
-    for (size_t j = k.values.size(); j > 0 && !known; --j)  // (most operands have just been results)
-      if (k.values[j - 1].id == v.get()) {
-        x = k.values[j - 1];
-        known = true;
-      }
-    if (known) continue;
-    if (!is_a(v, value_class) || !read_type(k, attr(v, names.type), &x.t) || !to_bool(attr(v, names.is_arg), &x.is_arg) ||
-        !to_int(attr(v, names.index), &x.index))
+    if (!v) return false;
+    if ((out->at[i] = k.values.find(v.get()))) continue;
+    if (!is_a(v, value_class)) return false;
+    const Fields of(v);
+    Value x;
+    if (!read_type(k, of(names.type), &x.t) || !to_bool(of(names.is_arg), &x.is_arg) || !to_int(of(names.index), &x.index))
       return false;
-    x.owner = attr(v, names.owner);
+    x.owner = of(names.owner);
     x.id = v.get();
-    k.values.push_back(x);
-    k.keep.push_back(v);
+    out->at[i] = k.values.add(v, std::move(x));
   }
   return true;
 }
@@ -320,14 +388,15 @@ bool walk(Kernel& k, const Ref& op, int depth) {
     for (int c = 1; c < kClasses; ++c)
       if (is_a(x.op, classes[c])) x.cls = static_cast<Class>(c);
     if (x.cls == kOther) return false;
-    x.attrs = attr(x.op, names.attrs);
-    if (x.cls == kUpstream) x.name = attr(x.op, names.op_name);
+    const Fields of(x.op);
+    x.attrs = of(names.attrs);
+    if (x.cls == kUpstream) x.name = of(names.op_name);
     const bool holds = x.cls == kParallel || x.cls == kFor;
     long long n_args = 0;
-    const Ref r = attr(x.op, names.regions);
+    const Ref r = of(names.regions);
     if (length(r) != (holds ? 1 : 0)) return false;
     if (holds) n_args = length(attr(item(attr(item(r, 0), names.blocks), 0), names.arguments));
-    if (!read_values(k, attr(x.op, names.operands), &x.in) || !read_values(k, attr(x.op, names.results), &x.out)) return false;
+    if (!read_values(k, of(names.operands), &x.in) || !read_values(k, of(names.results), &x.out)) return false;
     if (!verify_op(x, n_args)) return false;
     const Ref self = x.op;
     k.ops.push_back(std::move(x));
@@ -482,8 +551,8 @@ PyObject* fused(const Kernel& k) {
   const Value& c = gemm->in[2];
   if ((fill && fill->in[0].id != c.id) || (reduce && reduce->in[0].id != c.id)) return nullptr;
   auto global_arg = [&](const Value& v) { return v.is_arg && v.owner.get() == k.entry.get() && v.t.space == 1; };
-  for (const Value& v : gemm->in)
-    if (!global_arg(v)) return nullptr;
+  for (size_t i = 0; i < gemm->in.size(); ++i)
+    if (!global_arg(gemm->in[i])) return nullptr;
   if (reduce && !global_arg(reduce->in[1])) return nullptr;
   bool ta = false, tb = false, clear = false, reduce_clear = true;
   if (!flag(*gemm, names.transA, &ta) || !flag(*gemm, names.transB, &tb) || !flag(*gemm, names.clear_accum, &clear)) return nullptr;
@@ -502,6 +571,7 @@ PyObject* plan(PyObject*, PyObject* arg) {
   if (!type_class) Py_RETURN_NONE;
   try {
     Kernel k;
+    k.class_has_place = PyObject_HasAttr(type_class, names.space) || PyObject_HasAttr(type_class, names.map);
     const Ref kernel(Py_NewRef(arg));
     if (walk(k, kernel, 0) && arguments_match(kernel, k.entry)) {
       bool mma = false;

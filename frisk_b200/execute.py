@@ -26,12 +26,14 @@ import math
 from . import capi, ir, recognise, tensor_ops
 
 _TORCH_DTYPE = None
+_ELEMENT_DTYPE = None
 
 
 def _torch():
     import torch
-    global _TORCH_DTYPE
+    global _TORCH_DTYPE, _ELEMENT_DTYPE
     if _TORCH_DTYPE is None:
+        _ELEMENT_DTYPE = {"f16": torch.float16, "bf16": torch.bfloat16, "f32": torch.float32}
         _TORCH_DTYPE = {torch.float32: capi.F32, torch.float16: capi.F16, torch.bfloat16: capi.BF16}
     return torch
 
@@ -210,7 +212,7 @@ def _plan_of(kernel, algo):
 
 def execute(module_or_kernel, *tensors, stream=None, name=None, algo=capi.ALGO_AUTO):
     """Run the kernel on CUDA tensors bound positionally to its memref arguments."""
-    torch = _torch()
+    _torch()
     kernel = _kernel_of(module_or_kernel, name)
     attention, plan = _plan_of(kernel, algo)
     if attention:
@@ -220,13 +222,13 @@ def execute(module_or_kernel, *tensors, stream=None, name=None, algo=capi.ALGO_A
     arg_types = kernel.attrs["function_type"].inputs
     if len(tensors) != len(arg_types):
         raise ValueError(f"frisk-b200-execute: kernel takes {len(arg_types)} tensors, got {len(tensors)}")
-    dtypes = {"f16": torch.float16, "bf16": torch.bfloat16, "f32": torch.float32}
+    dtypes = _ELEMENT_DTYPE
     for t, ty in zip(tensors, arg_types):
         if t is None:
             continue
         if not t.is_cuda:
             raise ValueError("frisk-b200-execute: tensors must live on a CUDA device (there is no CPU path)")
-        if list(t.shape) != list(ty.shape) or not t.is_contiguous():
+        if t.shape != tuple(ty.shape) or not t.is_contiguous():
             raise ValueError(f"frisk-b200-execute: tensor of shape {list(t.shape)} does not match {ty}")
         if t.dtype != dtypes.get(ty.element.name):
             raise ValueError(f"frisk-b200-execute: tensor dtype {t.dtype} does not match {ty}")
