@@ -300,26 +300,29 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_f16(BM, BN, BF16, A_MN, B_MN);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      TileItem it;
-      for (int i = 0; ok && get_item(i, it); ++i) {
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.status, ST_TIMEOUT_ACC_EMPTY)) break;
+    // Run by the whole warp, so that descriptors and counters are uniform; one elected lane issues.  A k-block of 128 columns takes
+    // 427 clk so, 501 as one lane's code (wait, four MMAs of 65, commit; with 256 columns the MMAs hide the rest): 512 x 512 x 4096
+    // 11.6 -> 11.1 us, 128 x 2048 x 2048 9.1 -> 8.8.  One wait and one commit for two k-blocks were slower (256 x 4096 x 4096 18.3 -> 19.2).
+    constexpr uint32_t idesc = umma_idesc_f16(BM, BN, BF16, A_MN, B_MN);
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true;
+    TileItem it;
+    for (int i = 0; ok && get_item(i, it); ++i) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.status, ST_TIMEOUT_ACC_EMPTY));
+      if (!ok) break;
+      tc_fence_after_sync();
+      const uint32_t d_tmem = tmem + acc * BN;
+      for (int kb = it.kb0; kb < it.kb1; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_flag, p.status, ST_TIMEOUT_FULL));
+        if (!ok) break;
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = it.kb0; kb < it.kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, ST_TIMEOUT_FULL)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after_sync();
-          const uint32_t sa = smem_u32(smem + stage * L::kStageBytes);
-          const uint32_t sb = sa + L::kABytes;
+        const uint32_t sa = smem_u32(smem + stage * L::kStageBytes);
+        const uint32_t sb = sa + L::kABytes;
+        if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             uint64_t da = A_MN ? umma_desc_mnmajor_sw128(sa + k * (UMMA_K * 128), BK * 128, 1024)
@@ -328,18 +331,18 @@ __global__ void __launch_bounds__(kThreads, 1)
                                : umma_desc_kmajor_sw128(sb + k * (UMMA_K * 2));
             umma_f16_ss(d_tmem, da, db, idesc, (kb > it.kb0 || k != 0) ? 1u : 0u);
           }
-          umma_commit(&empty_bar[stage]);  // stage reusable once these MMAs have read it
-          if (++stage == kStages) {
-            stage = 0;
-            phase ^= 1;
-          }
+          umma_commit(&empty_bar[stage]);                     // stage reusable once these MMAs have read it
+          if (kb + 1 == it.kb1) umma_commit(&acc_full[acc]);  // accumulator complete (an item has a k-block or more)
         }
-        if (!ok) break;
-        umma_commit(&acc_full[acc]);  // accumulator complete
-        if (++acc == 2) {
-          acc = 0;
-          acc_phase ^= 1;
+        __syncwarp();
+        if (++stage == kStages) {
+          stage = 0;
+          phase ^= 1;
         }
+      }
+      if (++acc == 2) {
+        acc = 0;
+        acc_phase ^= 1;
       }
     }
   } else {
