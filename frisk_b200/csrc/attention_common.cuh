@@ -66,30 +66,6 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
   return d;
 }
 
-// the same pairs with subnormals kept and every operation rounded by itself (the normalised mode's arithmetic)
-__device__ __forceinline__ float2 mul2_rn(float2 a, float2 b) {
-  float2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;"
-      : "=l"(*reinterpret_cast<unsigned long long*>(&d))
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
-  return d;
-}
-__device__ __forceinline__ float2 add2_rn(float2 a, float2 b) {
-  float2 d;
-  asm("add.rn.f32x2 %0, %1, %2;"
-      : "=l"(*reinterpret_cast<unsigned long long*>(&d))
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
-  return d;
-}
-__device__ __forceinline__ float2 fma2_rn(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(*reinterpret_cast<unsigned long long*>(&d))
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
-        "l"(*reinterpret_cast<unsigned long long*>(&c)));
-  return d;
-}
-
 // a / l for a pair of numerators, without the branch a division per element brings (128 of them in a row of a key
 // tile ran one after the other).  Markstein's correction (IBM J. Res. Dev. 34(1), 1990): with inv the correctly
 // rounded reciprocal of l, q = a*inv is corrected by its exact remainder, and the result is the correctly rounded

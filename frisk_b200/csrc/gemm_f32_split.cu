@@ -20,14 +20,15 @@
 // gives them.
 //
 // One CTA per SM, 16 warps with fixed roles (128 registers each, all of the SM's):
-//   warps 0-7   promotion: tensor memory -> fp32 registers (64 columns of one row per thread), stores.  One thread of
-//               warp 0 also issues the MMAs, of block i before the warp adds up block i - 1
+//   warps 0-7   promotion: tensor memory -> fp32 registers (64 columns of one row per thread), stores.  Warp 0 also issues
+//               the MMAs of block i, a quarter at a time between the quarters of block i - 1 that it adds up
 //   warps 8-15  loaders: global -> registers (one block ahead) -> split -> shared memory, in the 128-byte-swizzle image
-//               tcgen05 reads (K-major or MN-major, whichever way the operand lies in global memory)
-// Shared memory would allow a block in 2300 clk (96 KB of planes written, 192 KB read by 24 MMAs, at 128 B/clk; 1540 clk of
-// tensor pipe).  4096^3 takes 3700 (886 us, 155 TFLOP/s of fp32).  No single part is the limit: 2048^3 takes 126 us, 118
-// without the conversions, 120 without the loads, 112 with a sixth of the MMAs; four stages of 32 k instead of two of 64
-// take 154.
+//               tcgen05 reads (K-major or MN-major, whichever way the operand lies in global memory), or tensor memory
+// What bounds a block is the loaders: two warps a scheduler take 3100 clk for their ~550 instructions a block, wherever the terms
+// go and in whatever order they are made; the MMAs take 1560 (2000 as issued), shared memory 2300, or 1150 with A in tensor
+// memory.  1024^3 22.0 us with the MMAs of a block issued in one piece, 21.1 in quarters; 2000 x 2000 x 400 38.1 and 34.6;
+// 4096^3 runs at 155 TFLOP/s of fp32.  Tried: four stages of 32 k instead of two of 64 (2048^3 126 -> 154 us), 16 warps that load,
+// split and add up (1024^3 27.0), a warp of its own for the MMAs (96 registers a thread then: spills).
 //
 // Where the tiles are fewer than half the SMs a cluster of 2 to 8 CTAs shares a tile's K; every CTA leaves its fp32 part
 // in its own shared memory and each finishes a share of the tile's 32-row pieces, adding the parts over distributed
@@ -37,6 +38,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 #include "gemm_common.cuh"
@@ -84,18 +86,60 @@ struct SplitArgs {
   unsigned* status;
 };
 
-// (x, y) 2^24 as three pairs of bf16 terms
+// (x, y) 2^24 as three pairs of bf16 terms (packed arithmetic: 10 instructions instead of 14)
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&w)[3]) {
-  x *= kScale;
-  y *= kScale;
+  float2 v = mul2_rn(make_float2(x, y), make_float2(kScale, kScale));
 #pragma unroll
   for (int t = 0; t < 3; ++t) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
     w[t] = *reinterpret_cast<const uint32_t*>(&h);
-    x -= __uint_as_float(w[t] << 16);          // exact
-    y -= __uint_as_float(w[t] & 0xffff0000u);  // exact
+    // exact
+    if (t < 2) v = fma2_rn(make_float2(__uint_as_float(w[t] << 16), __uint_as_float(w[t] & 0xffff0000u)), make_float2(-1.f, -1.f), v);
   }
 }
+
+// An A whose terms go to tensor memory: 128 rows of a tile are its lanes, two k of a plane a column.  It is contiguous along
+// its rows, so a loader warp reads 32 rows of one k at a time and nothing is turned round on the way: warp w has rows
+// 32 (w % 4).., the first or the second 32 k of the block.  Any alignment.
+struct LaneLoader {
+  float r[32];
+  const float* base;  // this thread's first element of the block the next fetch() takes
+  int k, row;         // its place
+
+  __device__ __forceinline__ void place(const Operand& o, int row0, int k0, int tid) {
+    row = row0 + (tid & 127);
+    k = k0 + (tid >> 7) * 32;
+    base = o.p + (int64_t)k * o.ld + row;
+  }
+  __device__ __forceinline__ void fetch(const Operand& o, bool inside) {
+    if (inside) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) r[j] = __ldg(base + j * o.ld);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) r[j] = row < o.cols && k + j < o.rows ? __ldg(base + j * o.ld) : 0.f;
+    }
+    base += BK * o.ld;
+    k += BK;
+  }
+  // the three planes of the block, 32 columns each from `tmem` on (this warp's lanes)
+  __device__ __forceinline__ void store(uint32_t tmem, int tid) const {
+    const uint32_t at = tmem + (tid >> 7) * 16;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t w[3][8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        uint32_t x[3];
+        split_pair(r[h * 16 + 2 * j], r[h * 16 + 2 * j + 1], x);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) w[t][j] = x[t];
+      }
+#pragma unroll
+      for (int t = 0; t < 3; ++t) tmem_st_32x32b_x8(at + t * 32 + h * 8, w[t]);
+    }
+  }
+};
 
 // A block of an operand is 128 box rows of 64 elements: rows = MN and columns = k for an operand contiguous along K;
 // for one contiguous along MN, 64 rows = k of columns mn0..+63, then 64 rows of columns mn0+64..+127.  A loader thread
@@ -297,14 +341,20 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_unaligned) + 1023) & ~static_cast<uintptr_t>(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kBarOffset);
-  uint64_t* empty_bar = full_bar + kStages;
-  uint64_t* acc_full = empty_bar + kStages;  // [2]
-  uint64_t* acc_empty = acc_full + 2;        // [2]
+  uint64_t* done_bar = full_bar + kStages;   // [2] a block's MMAs are complete: its stage is free, its accumulator full
+  uint64_t* acc_empty = done_bar + kStages;  // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   volatile uint32_t* any_noted = tmem_slot + 2;
   uint32_t* noted = reinterpret_cast<uint32_t*>(smem + kRedoOffset);  // pieces of each of this CTA's tiles to compute again
   constexpr int kHalves = TWO ? 2 : 1, kAccCols = kHalves * BT;  // of an accumulator
+  // The terms of an A that is stored transposed go to tensor memory, behind the two accumulators, where there is room (two
+  // stages of three planes): their MMAs then read only B from shared memory.  1024^3 21.0 -> 20.4 us, 515 x 771 x 1003 21.6 -> 20.1,
+  // 128 x 1500 x 700 15.4 -> 14.9.  (Any operand contiguous along its rows would do, with the product turned round for B; for an
+  // A contiguous along K that was no faster: 21.1 and 21.4 us at 1024^3.)
+  constexpr bool LANES = A_MN && !TWO;
+  constexpr uint32_t kPlanesAt = 2 * BT, kPlanesCols = 3 * BK / 2, kTmemCols = LANES ? 512 : 2 * kAccCols;
+  static_assert(kPlanesAt + 2 * kPlanesCols <= 512, "accumulators and planes must fit");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int splits = p.splits, rank = splits > 1 ? (int)cluster_ctarank() : 0;
   // this CTA's tiles (one, if K is shared) and its blocks of each
@@ -316,10 +366,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; ++i) {
       mbar_init(&full_bar[i], kLoadWarps);
-      mbar_init(&empty_bar[i], 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&acc_full[i], 1);
+      mbar_init(&done_bar[i], 1);
       mbar_init(&acc_empty[i], kPromoWarps);
     }
     *abort_flag = 0;
@@ -328,7 +375,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
   }
   for (int i = threadIdx.x; i < n_mine; i += kThreads) noted[i] = 0;
   if (warp == 0) {
-    tmem_alloc(tmem_slot, 2 * kAccCols);
+    tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
@@ -353,60 +400,81 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
         *any_noted = 1;
       }
     };
-    // the MMAs of the next block: stage and accumulator alternate with the block's number
-    auto issue = [&]() {
-      constexpr uint32_t idesc = umma_idesc_f16(BT, BT, true, A_MN, B_MN);
+    // The MMAs of the next block, by warp 0: stage and accumulator alternate with the block's number.  The tensor core queues
+    // only a few of them, so the warp is busy for as long as they run, and what else it did in one piece left the tensor core
+    // idle.  So it issues a quarter of a block, adds up a quarter of the one before, which the queue covers, and so on.
+    constexpr uint32_t idesc = umma_idesc_f16(BT, BT, true, A_MN && !LANES, B_MN);
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+    constexpr int kParts = 4, kPartMmas = 6 * (BK / 16) / kParts;
+    auto may_issue = [&]() -> bool {
+      const int i = issued & 1;
+      const uint32_t phase = (issued >> 1) & 1;
+      const bool there = __all_sync(0xffffffffu, mbar_wait_both(&full_bar[i], phase, &acc_empty[i], phase ^ 1, abort_flag, p.status,
+                                                                ST_TIMEOUT_FULL, ST_TIMEOUT_ACC_EMPTY));
+      tc_fence_after_sync();
+      return there;
+    };
+    auto issue_part = [&](int part) {
       // term products, smallest first; (term of A, term of B)
       constexpr int ta[6] = {2, 0, 1, 1, 0, 0}, tb[6] = {0, 2, 1, 0, 1, 0};
       const int i = issued & 1;
-      const uint32_t phase = (issued >> 1) & 1;
-      if (lane == 0 && mbar_wait(&full_bar[i], phase, abort_flag, p.status, ST_TIMEOUT_FULL) &&
-          mbar_wait(&acc_empty[i], phase ^ 1, abort_flag, p.status, ST_TIMEOUT_ACC_EMPTY)) {
-        tc_fence_after_sync();
-        const uint32_t sa = smem_u32(smem + i * kStageBytes), sb = sa + 3 * kPlane;
-        // descriptors differ only in the start address
-        const uint64_t da = A_MN ? umma_desc_mnmajor_sw128(sa, BK * 128, 1024) : umma_desc_kmajor_sw128(sa);
-        const uint64_t db = B_MN ? umma_desc_mnmajor_sw128(sb, BK * 128, 1024) : umma_desc_kmajor_sw128(sb);
+      const uint32_t sa = smem_u32(smem + i * kStageBytes), sb = sa + 3 * kPlane;
+      // descriptors differ only in the start address
+      const uint64_t da = A_MN ? umma_desc_mnmajor_sw128(sa, BK * 128, 1024) : umma_desc_kmajor_sw128(sa);
+      const uint64_t db = B_MN ? umma_desc_mnmajor_sw128(sb, BK * 128, 1024) : umma_desc_kmajor_sw128(sb);
+      if (elect_one()) {
 #pragma unroll
-        for (int t = 0; t < 6; ++t)
-#pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            umma_f16_ss(tmem_base + i * kAccCols + (TWO && k >= 2 ? BT : 0), da + ((ta[t] * kPlane + k * (A_MN ? 16 * 128 : 32)) >> 4),
-                        db + ((tb[t] * kPlane + k * (B_MN ? 16 * 128 : 32)) >> 4), idesc, (t | (TWO ? k & 1 : k)) != 0 ? 1u : 0u);
-        umma_commit(&empty_bar[i]);
-        umma_commit(&acc_full[i]);
+        for (int m = part * kPartMmas; m < (part + 1) * kPartMmas; ++m) {
+          const int t = m / (BK / 16), k = m % (BK / 16);
+          const uint32_t acc = tmem + i * kAccCols + (TWO && k >= 2 ? BT : 0), add = (t | (TWO ? k & 1 : k)) != 0 ? 1u : 0u;
+          const uint64_t b = db + ((tb[t] * kPlane + k * (B_MN ? 16 * 128 : 32)) >> 4);
+          if (LANES)
+            umma_f16_ts(acc, tmem + kPlanesAt + i * kPlanesCols + ta[t] * (BK / 2) + k * 8, b, idesc, add);
+          else
+            umma_f16_ss(acc, da + ((ta[t] * kPlane + k * (A_MN ? 16 * 128 : 32)) >> 4), b, idesc, add);
+        }
+        if (part == kParts - 1) umma_commit(&done_bar[i]);
       }
       __syncwarp();
-      ++issued;
     };
-    if (warp == 0 && total > 0) issue();
+    if (warp == 0 && total > 0 && may_issue()) {
+#pragma unroll
+      for (int part = 0; part < kParts; ++part) issue_part(part);
+      ++issued;
+    }
     for (int tile = tile_first; tile < tiles && ok; tile += tile_step) {
       float v[64];
 #pragma unroll
       for (int i = 0; i < 64; ++i) v[i] = 0.f;
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (warp == 0 && issued < total) issue();
+        const bool issues = warp == 0 && issued < total && may_issue();
         const int acc = blocks & 1;
-        if (!mbar_wait(&acc_full[acc], (blocks >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACC_FULL)) {
-          ok = false;
-          break;
-        }
-        ++blocks;
-        tc_fence_after_sync();
-        __syncwarp();
 #pragma unroll
-        for (int h = 0; h < 2 * kHalves; ++h) {
-          uint32_t t[32];
-          tmem_ld_32x32b_x32(tmem_base + acc * kAccCols + (h >> 1) * BT + half * 64 + (h & 1) * 32 + lane_addr, t);
+        for (int part = 0; part < kParts; ++part) {
+          if (issues) issue_part(part);
+          if (part == 0) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&done_bar[acc], (blocks >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACC_FULL));
+            if (!ok) break;
+            tc_fence_after_sync();
+          }
+          uint32_t t[kHalves][16];
+#pragma unroll
+          for (int h = 0; h < kHalves; ++h)
+            tmem_ld_32x32b_x16(tmem_base + acc * kAccCols + h * BT + half * 64 + part * 16 + lane_addr, t[h]);
           tmem_ld_wait();
-          if (h == 2 * kHalves - 1) {
+          if (part == kParts - 1) {
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[acc]);
           }
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[(h & 1) * 32 + i] += __uint_as_float(t[i]);
+          for (int h = 0; h < kHalves; ++h)
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[part * 16 + i] += __uint_as_float(t[h][i]);
         }
+        if (issues) ++issued;
+        if (!ok) break;
+        ++blocks;
       }
       if (!ok) break;
       if (splits > 1) {
@@ -455,7 +523,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
   } else {
     // ------------------------------------------------------------------ loaders
     const int tid = threadIdx.x - kPromoWarps * 32;
-    Loader<A_MN, VEC> la;
+    std::conditional_t<LANES, LaneLoader, Loader<A_MN, VEC>> la;
+    const uint32_t planes = tmem_base + kPlanesAt + (static_cast<uint32_t>((warp & 3) * 32) << 16);  // (LANES)
     Loader<B_MN, VEC> lb;
     int tile = tile_first, kb = kb0, stage = 0;
     uint32_t phase = 0;
@@ -481,15 +550,24 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
         more = tile < tiles;
         if (more) place();
       }
-      if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+      if (!mbar_wait(&done_bar[stage], phase ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
       __syncwarp();
       unsigned char* sa = smem + stage * kStageBytes;
       const bool k_in = (unsigned)(kb + 1) * BK <= (unsigned)p.K;
-      la.store(sa, tid);
+      if constexpr (LANES) {
+        tc_fence_after_sync();
+        la.store(planes + stage * kPlanesCols, tid);
+      } else {
+        la.store(sa, tid);
+      }
       if (more) la.fetch(p.a, a_in && k_in);
       lb.store(sa + 3 * kPlane, tid);
       if (more) lb.fetch(p.b, b_in && k_in);
       fence_proxy_async_smem();  // the planes are read by the tensor core
+      if (LANES) {
+        tmem_st_wait();
+        tc_fence_before_sync();
+      }
       __syncwarp();
       if (lane == 0) mbar_arrive(&full_bar[stage]);
       if (++stage == kStages) {
@@ -518,7 +596,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
   if (warp == 0) {
     __syncwarp();
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 2 * kAccCols);
+    tmem_dealloc(tmem_base, kTmemCols);
   }
 }
 

@@ -94,6 +94,18 @@ def test_f32_auto_on_the_tensor_cores(ctx, M, N, K, acc):
         assert check(ctx, M, N, K, "fp32", "fp32", ta, tb, 23, accumulate=acc) < 2.0 ** -24 * max(8, K ** 0.5)
 
 
+@pytest.mark.parametrize("M,N,K,acc,offset", [
+    (8, 8, 640, False, 0),       # the shortest K whose A goes to tensor memory, eight of 128 rows
+    (136, 264, 648, True, 4),    # eight k in the last block, unaligned operands
+    (2056, 1160, 704, False, 0),  # more tiles than SMs
+])
+def test_f32_transposed_a_in_tensor_memory(ctx, M, N, K, acc, offset):
+    """A stored transposed, K >= 640, either layout of B; the bound is that of plain fp32 accumulation."""
+    for tb in (False, True):
+        err = check(ctx, M, N, K, "fp32", "fp32", True, tb, 27, accumulate=acc, algo=capi.ALGO_F32_SPLIT, offset=offset)
+        assert err < 2.0 ** -24 * K ** 0.5
+
+
 def test_f32_auto_short_k_is_the_cuda_cores_sum(ctx):
     """Below K = 320 (other than multiples of 8 from 256 up) an AUTO call adds in fp32 with round-to-nearest, whatever the
     other kernel would take: K = 1 is the correctly rounded product."""
