@@ -152,12 +152,23 @@ __global__ void __launch_bounds__(kThreads, 1)
     return it;
   };
   // Consumers (the two MMA threads, the softmax warps) learn the n-th item of this CTA from the producer:
-  // returns its id, or -1 when the work has run out or a wait was abandoned.
-  auto next_item = [&](int n, bool arrive) -> int {
-    if (!mbar_wait(&item_full[n & 1], (n >> 1) & 1, abort_flag, p.status, ST_ATTN_Q)) return -1;
-    const int t = item_slot[n & 1];
-    if (arrive) mbar_arrive(&item_empty[n & 1]);
-    return t;
+  // returns its id, or -1 when the work has run out or a wait was abandoned.  The slot is written again once the warp's one arrival
+  // is in, so no lane may read it after that: lane 0 reads it for the warp, or all lanes before the arrival (the normalised mode's
+  // two passes are compiled better so: 16 heads x 1025 22.1 against 22.4 us).
+  auto next_item = [&](int n) -> int {
+    int t = -1;
+    if (NORM) {
+      if (!__all_sync(0xffffffffu, mbar_wait(&item_full[n & 1], (n >> 1) & 1, abort_flag, p.status, ST_ATTN_Q))) return -1;
+      t = item_slot[n & 1];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&item_empty[n & 1]);
+      return t;
+    }
+    if (lane == 0 && mbar_wait(&item_full[n & 1], (n >> 1) & 1, abort_flag, p.status, ST_ATTN_Q)) {
+      t = item_slot[n & 1];
+      mbar_arrive(&item_empty[n & 1]);
+    }
+    return __shfl_sync(0xffffffffu, t, 0);
   };
   // The ring of K and V.  What an MMA thread takes in one step, the V of key tile b and the K of tile b + 2, makes a stage: one
   // barrier to wait for and one to release (each costs the thread about a hundred clocks).  The n-th goes to stage n % kStages, and
@@ -283,7 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     int finished = 0;  // P_q taken so far, over all items: its buffer and the phase of p_ready
     bool ok = true;
     for (int n = 0; ok; ++n) {
-      const int t = __shfl_sync(0xffffffffu, next_item(n, lane == 0), 0);
+      const int t = next_item(n);
       if (t < 0) break;
       const Item it = decode(t);
       const int n_mine = it.nq[mq], n_max = OWN_KV ? n_mine : it.n_max;  // key tiles: used, followed
@@ -378,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     };
 
     for (int n = 0; ok; ++n) {
-      const int item_id = next_item(n, lane == 0);
+      const int item_id = next_item(n);
       if (item_id < 0) break;
       const Item it = decode(item_id);
       const int bh = it.bh + (TWIN ? q : 0);
