@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kDecThreads, 1)
     bool ok = true;
     auto meet = [&]() {  // bounded meeting point of the consumer threads
       mbar_arrive(meet_bar);
-      if (ok) ok = mbar_wait(meet_bar, meet_phase, abort_flag, p.status, ST_TIMEOUT_MISC);
+      if (ok) ok = mbar_wait_warp(meet_bar, meet_phase, abort_flag, p.status, ST_TIMEOUT_MISC);
       meet_phase ^= 1;
     };
     // ldmatrix rows of this lane: K as [16 keys][16 d] (key blocks outer), V as [16 keys][16 d] (d blocks outer)
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(kDecThreads, 1)
       float m_ref[2] = {-INFINITY, -INFINITY}, l_sum[2] = {0.f, 0.f};  // rows g and g + 8 (l: this lane's columns)
 
       for (unsigned tile = tile0; tile < tile1; ++tile) {
-        if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, ST_ATTN_KV)) {
+        if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.status, ST_ATTN_KV)) {
           ok = false;
           break;
         }

@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
         for (int part = 0; part < kParts; ++part) {
           if (issues) issue_part(part);
           if (part == 0) {
-            ok = __all_sync(0xffffffffu, mbar_wait(&done_bar[acc], (blocks >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACC_FULL));
+            ok = mbar_wait_warp(&done_bar[acc], (blocks >> 1) & 1, abort_flag, p.status, ST_TIMEOUT_ACC_FULL);
             if (!ok) break;
             tc_fence_after_sync();
           }
@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
         more = tile < tiles;
         if (more) place();
       }
-      if (!mbar_wait(&done_bar[stage], phase ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
+      if (!mbar_wait_warp(&done_bar[stage], phase ^ 1, abort_flag, p.status, ST_TIMEOUT_EMPTY)) break;
       __syncwarp();
       unsigned char* sa = smem + stage * kStageBytes;
       const bool k_in = (unsigned)(kb + 1) * BK <= (unsigned)p.K;

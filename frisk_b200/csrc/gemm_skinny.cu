@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool epi_ok = true;
     auto epi_sync = [&]() {
       mbar_arrive(epi_bar);
-      if (epi_ok) epi_ok = mbar_wait(epi_bar, epi_phase, abort_flag, status, ST_TIMEOUT_MISC);
+      if (epi_ok) epi_ok = mbar_wait_warp(epi_bar, epi_phase, abort_flag, status, ST_TIMEOUT_MISC);
       epi_phase ^= 1;
     };
     auto store_column = [&](int tile, const float (&v)[TM]) {
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const Seg sg = segs.get(si);
       const int tile = sg.tile;
       const int t0 = tile * num_kg, t1 = t0 + num_kg;
-      if (!mbar_wait(&acc_full[acc], acc_phase, abort_flag, status, ST_TIMEOUT_ACC_FULL)) break;
+      if (!mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag, status, ST_TIMEOUT_ACC_FULL)) break;
       tc_fence_after_sync();
       uint32_t raw[TM];
       tmem_ld_32x32b_x16(tmem_base + acc * TM + (static_cast<uint32_t>(quad * 32) << 16), raw);

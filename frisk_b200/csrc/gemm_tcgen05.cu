@@ -312,12 +312,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool ok = true;
     TileItem it;
     for (int i = 0; ok && get_item(i, it); ++i) {
-      ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.status, ST_TIMEOUT_ACC_EMPTY));
+      ok = mbar_wait_warp(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.status, ST_TIMEOUT_ACC_EMPTY);
       if (!ok) break;
       tc_fence_after_sync();
       const uint32_t d_tmem = tmem + acc * BN;
       for (int kb = it.kb0; kb < it.kb1; ++kb) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_flag, p.status, ST_TIMEOUT_FULL));
+        ok = mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.status, ST_TIMEOUT_FULL);
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t sa = smem_u32(smem + stage * L::kStageBytes);
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // bounded meeting point of this CTA's 128 epilogue threads
     auto epi_sync = [&]() {
       mbar_arrive(epi_bar);
-      if (ok) ok = mbar_wait(epi_bar, epi_phase, abort_flag, p.status, ST_TIMEOUT_MISC);
+      if (ok) ok = mbar_wait_warp(epi_bar, epi_phase, abort_flag, p.status, ST_TIMEOUT_MISC);
       epi_phase ^= 1;
     };
     // byte offset of column j of a box's row r: 128-byte rows in the 128-byte-swizzle image
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         values(h, v);
         if (accumulate) {
           if (h == 0 && tma_c) {
-            if (ok) ok = mbar_wait(&bars[box_sel], (box_phases >> box_sel) & 1, abort_flag, p.status, ST_TIMEOUT_MISC);
+            if (ok) ok = mbar_wait_warp(&bars[box_sel], (box_phases >> box_sel) & 1, abort_flag, p.status, ST_TIMEOUT_MISC);
             box_phases ^= 1u << box_sel;
             __syncwarp();
           }
@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int i = 0; ok && get_item(i, it); ++i) {
       const TileCoord tc = tile_coord(it.tile, tiles_m, tiles_n);
       const int m0 = tc.m * BM, n0 = tc.n * BN;
-      if (!mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.status, ST_TIMEOUT_ACC_FULL)) break;
+      if (!mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag, p.status, ST_TIMEOUT_ACC_FULL)) break;
       tc_fence_after_sync();
       __syncwarp();
       const uint32_t taddr = tmem_base + acc * BN + (static_cast<uint32_t>(quad * 32) << 16);

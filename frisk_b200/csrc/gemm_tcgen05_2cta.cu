@@ -310,14 +310,14 @@ __global__ void __launch_bounds__(kThreads2, 1)
     // bounded meeting point of this CTA's 128 epilogue threads
     auto epi_sync = [&]() {
       mbar_arrive(epi_bar);
-      if (epi_ok) epi_ok = mbar_wait(epi_bar, epi_phase, abort_flag, status, ST_TIMEOUT_MISC);
+      if (epi_ok) epi_ok = mbar_wait_warp(epi_bar, epi_phase, abort_flag, status, ST_TIMEOUT_MISC);
       epi_phase ^= 1;
     };
     for (int t = pair; t < n_items; t += num_pairs) {
       const Item2 it = get_item2(t, n_full, num_kb);
       TileCoord tc = tile_coord(it.tile, tiles_m, tiles_n);
       const int m0 = tc.m * BM2 + (int)rank * BMC, n0 = tc.n * TILE_N;
-      if (!mbar_wait(&acc_full[acc], acc_phase, abort_flag, status, ST_TIMEOUT_ACC_FULL)) break;
+      if (!mbar_wait_warp(&acc_full[acc], acc_phase, abort_flag, status, ST_TIMEOUT_ACC_FULL)) break;
       tc_fence_after_sync();
       const int row_local = quad * 32 + lane;
       const int row = m0 + row_local;
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kThreads2, 1)
           if (c0 >= N || r0 >= M) break;  // wholly outside C (warp-uniform)
           if (ADD_OLD) {
             if (lane == 0 && u + 1 < TILE_N / kUnitCols && c0 + kUnitCols < N) fetch_old(box_sel ^ 1, c0 + kUnitCols, r0);
-            if (epi_ok) epi_ok = mbar_wait(&bars[box_sel], (box_phases >> box_sel) & 1, abort_flag, status, ST_TIMEOUT_MISC);
+            if (epi_ok) epi_ok = mbar_wait_warp(&bars[box_sel], (box_phases >> box_sel) & 1, abort_flag, status, ST_TIMEOUT_MISC);
             box_phases ^= 1u << box_sel;
             __syncwarp();
           }

@@ -1,8 +1,11 @@
-"""What the kernels' barriers order, as their sources state it (no GPU needed)."""
+"""What the kernels' barriers order and what follows their bounded waits, as their sources state it (no GPU needed)."""
 import pathlib
 import re
 
+import pytest
+
 CSRC = pathlib.Path(__file__).resolve().parents[1] / "frisk_b200" / "csrc"
+KERNELS = sorted(p.name for p in CSRC.glob("*.cu") if "mbar_wait" in p.read_text())
 
 
 class Block:
@@ -43,3 +46,22 @@ def test_no_lane_reads_an_item_after_the_warp_has_released_it():
     for block, at in reads:
         release = block.own.find("mbar_arrive(&item_empty", at)
         assert release >= 0 and (block.one_lane() or "__syncwarp()" in block.own[at:release])
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_waits_of_whole_warps_are_voted_on(name):
+    """A wait may run out for some lanes only, and votes, tensor-memory loads and __syncwarp need all of them.  So a per-lane wait belongs
+    to code of one lane, or to a vote, or its outcome is voted on in the same block before anything else needs the warp, or it goes to a
+    variable that nothing but votes reads."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+    for block, at in places(name, r"\bmbar_wait(_both)?\("):
+        before, after = block.own[:at], block.own[at:]
+        if block.one_lane() or before.endswith("__all_sync(0xffffffffu, ") or re.search(r"lane == 0 && $", before):
+            continue
+        kept = re.search(r"(\w+) (&=|=) $", before)
+        if kept and kept[1] != "ok":
+            uses = re.findall(rf"(?:bool |__a(?:ny|ll)_sync\(0xffffffffu, !?)?\b{kept[1]}\b(?: &?= )?", text)
+            assert all(re.match(r"bool |__a", use) or use.endswith("= ") for use in uses), (name, uses)
+            continue
+        vote = after.find("ok = __all_sync(0xffffffffu, ok)")
+        assert vote >= 0 and not re.search(r"\{\}|break|return|_sync\(|__syncwarp|tmem_|elect_one", after[:vote]), (name, after[:80])
