@@ -559,6 +559,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           while (clock64() - from < 300) {
           }
         }
+        __syncwarp();
         load_scores();
       }
       for (int i = 0; i < n_tiles && ok; ++i) {
@@ -664,6 +665,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t packed[32];
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
+          __syncwarp();
           if (SPLIT && (c < c_begin || c >= c_end)) continue;
           uint32_t o[32];
           tmem_ld_32x32b_x32((SPLIT ? t_o - q * 128 : t_o) + c * 32, o);

@@ -375,6 +375,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
   }
   for (int i = threadIdx.x; i < n_mine; i += kThreads) noted[i] = 0;
   if (warp == 0) {
+    __syncwarp();
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
@@ -518,6 +519,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
         }
         if (!store_piece(p, v, out, tc.m * BT + g * 32, tc.n * BT + u * 16, lane)) note(tile_first, x);
       }
+      __syncwarp();
       cluster_sync_all();  // the peers have read this CTA's part
     }
   } else {
@@ -565,6 +567,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
       if (more) lb.fetch(p.b, b_in && k_in);
       fence_proxy_async_smem();  // the planes are read by the tensor core
       if (LANES) {
+        __syncwarp();  // (at an edge of B every lane loads as far as it goes)
         tmem_st_wait();
         tc_fence_before_sync();
       }

@@ -383,14 +383,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       float row_acc = reduce_identity(reduce_kind);
       if (tma_c) {
         if (!accumulate && lane == 0) tma_store_wait_read<1>();  // the store before the last one used this box
-        __syncwarp();
       } else if (accumulate) {
         // old values of C, a row at a time, into the same image; all loads are on their way before the first is stored
         load_box_rows(C + (int64_t)r0 * p.ldc + c0, p.ldc, min(32, p.M - r0), min(U, p.N - c0), lane, [&](int r, uint32_t w) {
           *reinterpret_cast<uint32_t*>(box + box_at(r, lane * kPer)) = w;
         });
-        __syncwarp();
       }
+      __syncwarp();
       uint32_t w[32];
 #pragma unroll
       for (int h = 0; h < U / 32; ++h) {

@@ -387,8 +387,8 @@ __global__ void __launch_bounds__(kThreads2, 1)
             if (lane == 0 && u + 1 < TILE_N / kUnitCols && c0 + kUnitCols < N) fetch_old(box_sel ^ 1, c0 + kUnitCols, r0);
             if (epi_ok) epi_ok = mbar_wait_warp(&bars[box_sel], (box_phases >> box_sel) & 1, abort_flag, status, ST_TIMEOUT_MISC);
             box_phases ^= 1u << box_sel;
-            __syncwarp();
           }
+          __syncwarp();
           const uint4* old_row = reinterpret_cast<const uint4*>(boxes + box_sel * (32 * 128) + lane * 128);
           uint32_t w[32];
           if (sizeof(TO) == 4) {
@@ -469,6 +469,7 @@ __global__ void __launch_bounds__(kThreads2, 1)
       } else if (write_c) {
 #pragma unroll 1
         for (int c = 0; c < TILE_N / 32; ++c) {
+          __syncwarp();
           uint32_t v[32];
           tmem_ld_32x32b_x32(taddr + c * 32, v);
           tmem_ld_wait();

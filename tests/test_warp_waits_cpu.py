@@ -65,3 +65,48 @@ def test_waits_of_whole_warps_are_voted_on(name):
             continue
         vote = after.find("ok = __all_sync(0xffffffffu, ok)")
         assert vote >= 0 and not re.search(r"\{\}|break|return|_sync\(|__syncwarp|tmem_|elect_one", after[:vote]), (name, after[:80])
+
+
+ALIGNED = r"\b(?:tmem_(?:ld|st)_32x32b_x\d+|tmem_st_wait|tmem_alloc(?:_pair)?|cluster_sync_all|load_scores|values|la\.store)\("
+MEET = r"__sync(?:warp|threads)\(|_sync\(|\b(?:mbar_wait_warp|epi_sync|meet|combine_rows|cluster_sync_all|may_issue|issue_part|scores_there)\("
+APART = r"if \([^;{}]*\b(?:lane|row|grow|threadIdx\.x) [<>=!]=?|if \(valid\)|clock64|\b[abl]+\.fetch\(|\bnote\("
+
+
+def meets(text):
+    """Where in a piece of source the warp meets, whichever way it goes (a block that begins and ends in the piece may be left out)."""
+    opened, closed = [], []
+    for i, c in enumerate(text):
+        if c == "{":
+            opened.append(i)
+        elif c == "}" and opened:
+            closed.append((opened.pop(), i))
+    return [m.end() for m in re.finditer(MEET, text) if not any(a < m.start() < b for a, b in closed)]
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_warps_meet_before_what_needs_all_lanes(name):
+    """Instructions that a warp executes as one (tcgen05 loads, stores, waits and allocations, cluster barriers) come after a meeting of its
+    lanes wherever code of single lanes comes before, in program order or in the loop's last round."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+    opened, blocks = [], []
+    for i, c in enumerate(text):
+        if c == "{":
+            opened.append(i)
+        elif c == "}":
+            blocks.append((opened.pop(), i))
+    for m in re.finditer(ALIGNED, text):
+        for begin, end in sorted((b for b in blocks if b[0] < m.start() < b[1]), reverse=True):  # from the innermost block outwards
+            head = text[text.rfind("\n", 0, begin):begin]
+            if re.search(r"warp == (?!0)", head) and m.group().startswith("tmem_alloc"):
+                break  # (thread 0's set-up is another warp's)
+            before = text[begin:m.start()]
+            met = meets(before)
+            piece = before[met[-1]:] if met else before
+            if not met and re.search(r"\b(for|while) \(", head):
+                rest = text[m.start():end]
+                met_later = meets(rest)
+                piece = (rest[met_later[-1]:] if met_later else rest) + piece
+            apart = re.search(APART, piece)
+            assert not apart, (name, text.count("\n", 0, m.start()) + 1, m.group(), apart.group())
+            if met or re.search(r"__device__|\[&\]\(|\[\]\(|__launch_bounds__", head):
+                break  # (a function is judged where it is called)
