@@ -12,6 +12,7 @@ import pathlib
 
 F32, F16, BF16 = 0, 1, 2
 ALGO_AUTO, ALGO_SIMT_F32, ALGO_TCGEN05, ALGO_SKINNY, ALGO_TCGEN05_PAIR, ALGO_F32_SPLIT = 0, 1, 2, 3, 4, 5
+ATTN_PAIRS, ATTN_SPLIT_KEYS, ATTN_TWO_HEADS, ATTN_FEW_QUERIES = 0, 1, 2, 3
 DTYPE_CODE = {"fp32": F32, "fp16": F16, "bf16": BF16}
 DTYPE_NAME = {v: k for k, v in DTYPE_CODE.items()}
 ITEMSIZE = {F32: 4, F16: 2, BF16: 2}
@@ -28,7 +29,7 @@ EXPORTS = (
     "frisk_b200_gemm_skinny_static", "frisk_b200_gemm_push", "frisk_b200_sum_slots",
     "frisk_b200_peer_buffer_create", "frisk_b200_peer_buffer_open", "frisk_b200_peer_buffer_close",
     "frisk_b200_gemm_fused_select", "frisk_b200_gemm_fused_workspace_bytes", "frisk_b200_gemm_fused",
-    "frisk_b200_gemm_plan",
+    "frisk_b200_gemm_plan", "frisk_b200_attention_form",
 )
 
 
@@ -107,6 +108,7 @@ def load():
         "frisk_b200_gemm_host": (ctypes.c_int, [vp, gd, vp, vp, vp]),
         "frisk_b200_attention_validate": (ctypes.c_int, [ad]),
         "frisk_b200_attention_workspace_bytes": (sz, [ad]),
+        "frisk_b200_attention_form": (ctypes.c_int, [vp, ad, ctypes.POINTER(i32)]),
         "frisk_b200_attention_fwd": (ctypes.c_int, [vp, ad, vp, vp, vp, vp, vp, sz, vp]),
         "frisk_b200_attention_fwd_host": (ctypes.c_int, [vp, ad, vp, vp, vp, vp]),
         "frisk_b200_convert_f32": (ctypes.c_int, [vp, vp, vp, i64, i32, vp]),
@@ -205,6 +207,12 @@ class Context:
 
     def gemm_host(self, desc, a_ptr, b_ptr, c_ptr):
         raise_for(load().frisk_b200_gemm_host(self.handle, ctypes.byref(desc), a_ptr, b_ptr, c_ptr), self._h)
+
+    def attention_form(self, desc):
+        """How ``attention_fwd`` shares this descriptor's work out (``ATTN_*``); launches nothing."""
+        form = ctypes.c_int32()
+        raise_for(load().frisk_b200_attention_form(self.handle, ctypes.byref(desc), ctypes.byref(form)), self._h)
+        return form.value
 
     def attention_fwd(self, desc, q, k, v, o, stream=None):
         rc = load().frisk_b200_attention_fwd(self.handle, ctypes.byref(desc), q, k, v, o, None, 0, stream)

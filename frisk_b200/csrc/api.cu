@@ -621,6 +621,14 @@ size_t frisk_b200_attention_workspace_bytes(const frisk_b200_attn_desc* d) {
   return 0;  // the 5th "scratch" argument of the reference ABI is unused there as well
 }
 
+int frisk_b200_attention_form(frisk_b200_ctx* ctx, const frisk_b200_attn_desc* d, int32_t* form) {
+  if (!ctx || !d || !form) return FRISK_B200_E_ARG;
+  const int rc = frisk_b200_attention_validate(d);
+  if (rc) return rc;
+  *form = attention_form(ctx, *d);
+  return 0;
+}
+
 int frisk_b200_attention_fwd(frisk_b200_ctx* ctx, const frisk_b200_attn_desc* d, const void* Q, const void* K,
                              const void* V, void* O, void* workspace, size_t workspace_bytes, void* stream) {
   (void)workspace;

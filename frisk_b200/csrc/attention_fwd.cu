@@ -845,18 +845,27 @@ int launch_cfg(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q
   return 0;
 }
 
-template <bool BF16, int D, bool OUT_F32, bool NORM>
-int launch_mode(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K, const void* V,
-                 void* O, cudaStream_t s) {
+Mode mode_of(const frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d) {
   // A lone query tile's key tiles go to the two softmax groups in turn: one group alone leaves the schedulers idle while it
   // waits for tensor memory and barriers (with one buffer of scores: 16 heads x 1025 normalised 29.2 -> 23.4 us, 4 heads x 4096
   // causal at D = 128 62.1 -> 40.4; with two 22.1 and 32.9).
-  if (split_keys_pay(d) && one_tile_items(ctx, d)) return launch_cfg<BF16, D, OUT_F32, NORM, kSplit>(ctx, d, Q, K, V, O, s);
-  // Heads of one query tile, more of them than SMs: two at a time, since a pair's second group would be idle (512 heads x 128,
-  // D = 64 13.9 -> 11.9 us, D = 128 19.2 -> 16.5).  In the normalised mode a lone tile is as fast.
-  if (!NORM && d.S_q <= BM && (int64_t)d.B * d.H > ctx->num_sms)
-    return launch_cfg<BF16, D, OUT_F32, NORM, NORM ? kPair : kTwin>(ctx, d, Q, K, V, O, s);
-  return launch_cfg<BF16, D, OUT_F32, NORM, kPair>(ctx, d, Q, K, V, O, s);
+  if (split_keys_pay(d) && one_tile_items(ctx, d)) return kSplit;
+  // Heads of one query tile, more of them than SMs, whose keys are not split: two at a time, since a pair's second group would be
+  // idle (512 heads x 128, D = 64 13.9 -> 11.9 us, D = 128 19.2 -> 16.5).  That is up to 256 keys, or more than 8 heads an SM:
+  // between, the estimate above knows no item of two heads and always prefers split keys.  In the normalised mode a lone tile is
+  // as fast.
+  if (!d.normalize_p && d.S_q <= BM && (int64_t)d.B * d.H > ctx->num_sms) return kTwin;
+  return kPair;
+}
+
+template <bool BF16, int D, bool OUT_F32, bool NORM>
+int launch_mode(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K, const void* V,
+                 void* O, cudaStream_t s) {
+  switch (mode_of(ctx, d)) {
+    case kSplit: return launch_cfg<BF16, D, OUT_F32, NORM, kSplit>(ctx, d, Q, K, V, O, s);
+    case kTwin: return launch_cfg<BF16, D, OUT_F32, NORM, NORM ? kPair : kTwin>(ctx, d, Q, K, V, O, s);
+    default: return launch_cfg<BF16, D, OUT_F32, NORM, kPair>(ctx, d, Q, K, V, O, s);
+  }
 }
 
 template <bool BF16, int D>
@@ -871,6 +880,12 @@ int launch_out(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q
 }
 
 }  // namespace
+
+int attention_form(const frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d) {
+  if (attention_decode_preferred(d)) return FRISK_B200_ATTN_FEW_QUERIES;
+  const Mode mode = mode_of(ctx, d);
+  return mode == kSplit ? FRISK_B200_ATTN_SPLIT_KEYS : mode == kTwin ? FRISK_B200_ATTN_TWO_HEADS : FRISK_B200_ATTN_PAIRS;
+}
 
 int launch_attention_fwd(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K,
                          const void* V, void* O, cudaStream_t s) {

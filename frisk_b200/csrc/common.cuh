@@ -296,6 +296,8 @@ int launch_fill(void* C, int64_t M, int64_t N, int64_t ldc, float value, int dty
 int launch_attention_fwd(frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d, const void* Q, const void* K,
                          const void* V, void* O, cudaStream_t s);
 
+int attention_form(const frisk_b200_ctx* ctx, const frisk_b200_attn_desc& d);  // FRISK_B200_ATTN_*: what the launch takes
+
 // a few queries per head against a long key/value cache (attention_decode.cu)
 bool attention_decode_preferred(const frisk_b200_attn_desc& d);
 size_t attention_decode_scratch_bytes();

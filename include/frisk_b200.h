@@ -196,6 +196,15 @@ int frisk_b200_gemm_skinny_static(int device, const frisk_b200_gemm_desc* desc, 
  * (benchmark/layout/execution/tiled_attention.py:56-61: args q,k,v,out,scratch). */
 int frisk_b200_attention_validate(const frisk_b200_attn_desc* desc);
 size_t frisk_b200_attention_workspace_bytes(const frisk_b200_attn_desc* desc);
+/* How frisk_b200_attention_fwd shares this descriptor's work out on this context's device (FRISK_B200_ATTN_*).  Launches
+ * nothing. */
+enum {
+  FRISK_B200_ATTN_PAIRS = 0,       /* two 128-row query tiles of a head side by side, or one alone */
+  FRISK_B200_ATTN_SPLIT_KEYS = 1,  /* one query tile, its keys halved */
+  FRISK_B200_ATTN_TWO_HEADS = 2,   /* two heads of one query tile each side by side */
+  FRISK_B200_ATTN_FEW_QUERIES = 3  /* up to 16 queries a head, keys shared out over all SMs */
+};
+int frisk_b200_attention_form(frisk_b200_ctx* ctx, const frisk_b200_attn_desc* desc, int32_t* form);
 int frisk_b200_attention_fwd(frisk_b200_ctx* ctx, const frisk_b200_attn_desc* desc, const void* Q,
                              const void* K, const void* V, void* O, void* workspace,
                              size_t workspace_bytes, void* stream);
