@@ -15,6 +15,7 @@
 // gives None, and the Python recognisers decide and word the error.  No exception leaves this file.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
+#include <structmember.h>
 
 #include <cstring>
 #include <deque>
@@ -56,6 +57,12 @@ struct Names {
 enum Class { kOther, kEnd, kParallel, kFor, kCopy, kFill, kReduce, kGemm, kMma, kReduceTensor, kView, kStore, kUpstream, kClasses };
 PyObject* classes[kClasses];  // the Python classes, in the order of Class
 PyObject *type_class, *value_class, *map_class, *space_class, *policy_class;
+struct {
+  Py_ssize_t type, owner, index, is_arg;
+} value_at;  // places of a value's slots
+struct {
+  Py_ssize_t operands, results, attrs, regions;
+} op_at[kClasses];
 
 Ref attr(const Ref& o, PyObject* name) {
   if (!o) return Ref();
@@ -63,8 +70,27 @@ Ref attr(const Ref& o, PyObject* name) {
   if (!v) PyErr_Clear();
   return Ref(v);
 }
-// The attributes of one object.  The IR's objects hold theirs in the instance's dictionary, where one costs a third of
-// PyObject_GetAttr, which looks through the classes first; what is not there is asked for the usual way.
+// An attribute that every object of a class holds in a slot: the descriptor's place in the object, 0 if there is none.
+Py_ssize_t slot_of(PyObject* cls, PyObject* name) {
+  const Ref d(PyObject_GetAttr(cls, name));
+  if (!d) PyErr_Clear();
+  if (!d || !Py_IS_TYPE(d.get(), &PyMemberDescr_Type)) return 0;
+  const PyMemberDef* member = reinterpret_cast<PyMemberDescrObject*>(d.get())->d_member;
+  return member->type == T_OBJECT_EX ? member->offset : 0;
+}
+// Read there, without PyObject_GetAttr, which looks through the classes first: a 64 x 64 attention graph takes 8.1 us, and 10.5 in its
+// first call.  (Out of the objects' instance dictionaries it took 9.3, but they have none until somebody asks: a first call of 15.7,
+// 4 KB a kernel that stayed, and ir._verify 7 % slower from then on.)
+Ref slot(const Ref& o, Py_ssize_t at, PyObject* name) {
+  if (o && at) {
+    PyObject* v = *reinterpret_cast<PyObject**>(reinterpret_cast<char*>(o.get()) + at);
+    if (v) return Ref(Py_NewRef(v));
+  }
+  return attr(o, name);
+}
+
+// The attributes of a type.  Its constructor fills the instance's dictionary, so there is one; an attribute costs a third of
+// PyObject_GetAttr there.  What is not there is asked for the usual way.
 class Fields {
  public:
   explicit Fields(const Ref& o) : o_(o.get()), dict_(o ? PyObject_GenericGetDict(o.get(), nullptr) : nullptr) {
@@ -249,11 +275,11 @@ bool read_values(Kernel& k, const Ref& list, Values* out) {
     if (!v) return false;
     if ((out->at[i] = k.values.find(v.get()))) continue;
     if (!is_a(v, value_class)) return false;
-    const Fields of(v);
     Value x;
-    if (!read_type(k, of(names.type), &x.t) || !to_bool(of(names.is_arg), &x.is_arg) || !to_int(of(names.index), &x.index))
+    if (!read_type(k, slot(v, value_at.type, names.type), &x.t) || !to_bool(slot(v, value_at.is_arg, names.is_arg), &x.is_arg) ||
+        !to_int(slot(v, value_at.index, names.index), &x.index))
       return false;
-    x.owner = of(names.owner);
+    x.owner = slot(v, value_at.owner, names.owner);
     x.id = v.get();
     out->at[i] = k.values.add(v, std::move(x));
   }
@@ -388,15 +414,17 @@ bool walk(Kernel& k, const Ref& op, int depth) {
     for (int c = 1; c < kClasses; ++c)
       if (is_a(x.op, classes[c])) x.cls = static_cast<Class>(c);
     if (x.cls == kOther) return false;
-    const Fields of(x.op);
-    x.attrs = of(names.attrs);
-    if (x.cls == kUpstream) x.name = of(names.op_name);
+    const auto& at = op_at[x.cls];
+    x.attrs = slot(x.op, at.attrs, names.attrs);
+    if (x.cls == kUpstream) x.name = attr(x.op, names.op_name);
     const bool holds = x.cls == kParallel || x.cls == kFor;
     long long n_args = 0;
-    const Ref r = of(names.regions);
+    const Ref r = slot(x.op, at.regions, names.regions);
     if (length(r) != (holds ? 1 : 0)) return false;
     if (holds) n_args = length(attr(item(attr(item(r, 0), names.blocks), 0), names.arguments));
-    if (!read_values(k, of(names.operands), &x.in) || !read_values(k, of(names.results), &x.out)) return false;
+    if (!read_values(k, slot(x.op, at.operands, names.operands), &x.in) ||
+        !read_values(k, slot(x.op, at.results, names.results), &x.out))
+      return false;
     if (!verify_op(x, n_args)) return false;
     const Ref self = x.op;
     k.ops.push_back(std::move(x));
@@ -593,7 +621,12 @@ PyObject* set_classes(PyObject*, PyObject* args) {
     PyErr_SetString(PyExc_ValueError, "recognise: wrong number of classes");
     return nullptr;
   }
-  for (int i = 1; i < kClasses; ++i) Py_XSETREF(classes[i], Py_NewRef(PyList_GET_ITEM(ops, i - 1)));
+  for (int i = 1; i < kClasses; ++i) {
+    PyObject* c = PyList_GET_ITEM(ops, i - 1);
+    op_at[i] = {slot_of(c, names.operands), slot_of(c, names.results), slot_of(c, names.attrs), slot_of(c, names.regions)};
+    Py_XSETREF(classes[i], Py_NewRef(c));
+  }
+  value_at = {slot_of(v, names.type), slot_of(v, names.owner), slot_of(v, names.index), slot_of(v, names.is_arg)};
   Py_XSETREF(value_class, Py_NewRef(v));
   Py_XSETREF(map_class, Py_NewRef(m));
   Py_XSETREF(space_class, Py_NewRef(s));

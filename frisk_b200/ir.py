@@ -144,7 +144,23 @@ from .affine import (AffineExpr, AffineExprKind, AffineMap, get_affine_binary_op
 # ------------------------------------------------------------------------ IR skeleton
 
 
-class value:  # noqa: N801
+class _Slotted:
+    """Objects whose usual attributes lie in slots, saved and read back as those that have a dictionary only."""
+    __slots__ = ()
+
+    def __reduce_ex__(self, protocol):
+        return super().__reduce_ex__(max(protocol, 2))  # (the older protocols know no slots)
+
+    def __setstate__(self, state):
+        for part in state if isinstance(state, tuple) else (state,):  # (a dictionary: saved when there were no slots)
+            for name, v in (part or {}).items():
+                setattr(self, name, v)
+
+
+class value(_Slotted):  # noqa: N801
+    # slots for what every call of a built kernel reads (and a dictionary for anything else, made when something is put there)
+    __slots__ = ("type", "owner", "index", "is_arg", "__dict__", "__weakref__")
+
     def __init__(self, ty, owner, index, is_arg):
         self.type, self.owner, self.index, self.is_arg = ty, owner, index, is_arg
 
@@ -191,9 +207,10 @@ class region:  # noqa: N801
         return self.blocks[0]
 
 
-class OpState:
+class OpState(_Slotted):
     """An operation: name, operands, results, attributes, regions."""
     op_name = "builtin.unknown"
+    __slots__ = ("operands", "results", "attrs", "regions", "parent_block", "__dict__", "__weakref__")
 
     def __init__(self, operands=(), result_types=(), attrs=None, num_regions=0):
         self.operands = list(operands)

@@ -1,9 +1,13 @@
 """The native recogniser (csrc/recognise.cpp) against the Python ones: what it accepts they resolve to the same plan, also after
 any single part of a built kernel has been changed, removed or put in another's place."""
+import copy
+import gc
 import importlib
 import os
+import pickle
 import random
 import sysconfig
+import tracemalloc
 
 import pytest
 
@@ -261,3 +265,30 @@ def test_the_extension_is_built_for_this_interpreter_or_not_at_all(monkeypatch, 
     os.utime(target, (0, 0))
     monkeypatch.setattr(build.shutil, "which", lambda name: None)  # no g++
     assert build.build_recognise() is None and not target.exists()
+
+
+@needs_build
+@pytest.mark.parametrize("make", [attention_kernel, gemm_kernel])
+def test_recognising_leaves_nothing_in_the_kernel(make):
+    """A kernel's objects hold no more memory after a call than before (an instance dictionary is made when somebody asks for it)."""
+    assert recognise.plan(make()) is not None  # (sets up what a process keeps)
+    kernel = make()
+    gc.collect()
+    tracemalloc.start()
+    try:
+        recognise.plan(kernel)
+        assert tracemalloc.get_traced_memory()[0] < 200  # (the interpreter's own; a dictionary takes 100 and more, and there are dozens)
+    finally:
+        tracemalloc.stop()
+
+
+@pytest.mark.parametrize("protocol", range(pickle.HIGHEST_PROTOCOL + 1))
+def test_kernels_are_saved_and_copied_whole(protocol):
+    kernel = gemm_kernel()
+    kernel.note = "kept"
+    for other in (pickle.loads(pickle.dumps(kernel, protocol)), copy.deepcopy(kernel)):
+        assert str(other) == str(kernel) and other.note == "kept" and by_python(other) == by_python(kernel) is not None
+    v = kernel.regions[0].blocks[0].arguments[1]
+    old = ir.value.__new__(ir.value)
+    old.__setstate__({"type": v.type, "owner": v.owner, "index": 1, "is_arg": True})  # as it was saved without slots
+    assert (old.type, old.owner, old.index, old.is_arg) == (v.type, v.owner, 1, True)
