@@ -551,10 +551,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         // first finite score moves it (0 would let lower scores vanish; a group's first key tiles may be any row's -inf).
         m_ref = fmaxf(mx * p.scale_log2, -FLT_MAX);
         // The groups begin a CTA's first item at the same time, and two that work in step leave the special-function unit idle
-        // together between their key tiles.  So group 1 begins later, by about a third of its work on a tile.  (Later items begin
-        // as far apart as the ones before ended; where tiles are short and equally many it pays for every item.)
-        // 8 x 8192, D = 128 265 -> 255 us, causal 138 -> 128; D = 64, 12 x 2048 36.2 -> 32.2, 15 x 11 x 479 30.2 -> 29.2.
-        if (q == 1 && n_tiles > 3 && (n == 0 || (D == 64 && !p.causal))) {
+        // together between their key tiles.  So at D = 64 group 1 begins later, by about a third of its work on a tile.  (Later items
+        // begin as far apart as the ones before ended; where tiles are short and equally many it pays for every item.)  Without and
+        // with: 12 x 2048 34.1 and 33.1 us, 16 x 1025 14.6 and 13.8, 48 x 300 against 1024 keys 13.9 and 13.1, 150 x 2586 404 and
+        // 398, 132 x 1075 causal 59.2 and 59.3.  At D = 128 it costs more than it gives (8 x 8192 261 and 268, causal 137.5 and 140,
+        // 62 x 6308 causal 599 and 605, but 24 x 1000 22.5 and 22.2), as with two heads an item (512 x 128 against 256 15.75 and 16.05).
+        if (D == 64 && !TWIN && q == 1 && n_tiles > 3 && (n == 0 || !p.causal)) {
           const long long from = clock64();
           while (clock64() - from < 300) {
           }
