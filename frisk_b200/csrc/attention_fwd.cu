@@ -153,11 +153,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   };
   // Consumers (the two MMA threads, the softmax warps) learn the n-th item of this CTA from the producer:
   // returns its id, or -1 when the work has run out or a wait was abandoned.  The slot is written again once the warp's one arrival
-  // is in, so no lane may read it after that: lane 0 reads it for the warp, or all lanes before the arrival (the normalised mode's
-  // two passes are compiled better so: 16 heads x 1025 22.1 against 22.4 us).
+  // is in, so no lane may read it after that: lane 0 reads it for the warp, or all lanes before the arrival.  The latter is compiled into
+  // faster loops for the normalised mode (16 heads x 1025 22.1 against 22.4 us) and for split keys at D = 64 (13.4 and 13.6; 2 heads x
+  // 512 8.9 and 9.2), the former at D = 128 (4 heads x 4096 causal 32.6 against 33.4).
   auto next_item = [&](int n) -> int {
     int t = -1;
-    if (NORM) {
+    if (NORM || (SPLIT && D == 64)) {
       if (!mbar_wait_warp(&item_full[n & 1], (n >> 1) & 1, abort_flag, p.status, ST_ATTN_Q)) return -1;
       t = item_slot[n & 1];
       __syncwarp();
@@ -374,6 +375,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     int ends[2] = {0, 0};  // items with two key tiles or more, with one or more so far: the phases of o_done
     int meets = 0;    // meetings of the two groups so far: the phase of xchg
     bool ok = true;
+    // Waits of this lane that have not run out.  A vote of its own on every wait costs up to 3 % (16 heads x 1025, D = 64 13.4 -> 13.8 us;
+    // on the single pass's waits for scores 0.7 % at 8 x 32 x 4096 causal, 3 % at 150 x 2586).  So a lane whose wait has run out goes on
+    // with what it finds until the warp next votes: on whether to rescale, for every key tile, and before O is read.
+    bool there = true;
     // Split keys: the two groups meet, and each thread learns what the other group's thread of its row brings.  The
     // statistics lie in the second query tile's place, which nothing else uses then, in two sets that alternate: a set is
     // written again only when everybody has arrived at the meeting in between, after reading it.
@@ -382,7 +387,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       set[q * BM + row] = mine_v;
       tc_fence_before_sync();
       mbar_arrive(xchg);
-      if (!mbar_wait_warp(xchg, meets & 1, abort_flag, p.status, ST_ATTN_O)) ok = false;
+      there &= mbar_wait(xchg, meets & 1, abort_flag, p.status, ST_ATTN_O);
       ++meets;
       tc_fence_after_sync();
       return set[(q ^ 1) * BM + row];
@@ -410,9 +415,6 @@ __global__ void __launch_bounds__(kThreads, 1)
       auto scores_there = [&](bool more) -> bool {  // (the vote is taken in any case: behind a branch on `more` the loop is 13 % slower)
         return __all_sync(0xffffffffu, more && mbar_test(&s_full[2 * q + (steps & 1)], (steps >> 1) & 1));
       };
-      // Single pass: a vote on every wait for scores costs 0.7 % (8 x 32 x 4096 causal) to 3 % (150 x 2586).  So a lane whose wait has
-      // run out goes on with what it finds, and the warp learns of it where it votes on whether to rescale, for every key tile.
-      bool there = true;
       auto wait_scores = [&]() {
         if (NORM) {
           if (ok) ok = mbar_wait_warp(&s_full[2 * q + (steps & 1)], (steps >> 1) & 1, abort_flag, p.status, ST_ATTN_S);
@@ -464,6 +466,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const float a = share(m_run, l_run), b = share(o.x, o.y);
             l_run = a + b;
             m_run = m_all;
+            if (!__all_sync(0xffffffffu, there)) ok = false;
             if (!ok) break;
           }
           const float inv_l = __frcp_rn(l_run);  // (of use in pass 1 only)
@@ -633,7 +636,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
 
       // ---- epilogue: O / l
-      if (ok && n_tiles > 0) ok = mbar_wait_warp(&o_done[2 * q + 1], ends[1] & 1, abort_flag, p.status, ST_ATTN_O);
+      if (ok && n_tiles > 0) {
+        if (SPLIT) there &= mbar_wait(&o_done[2 * q + 1], ends[1] & 1, abort_flag, p.status, ST_ATTN_O);
+        else ok = mbar_wait_warp(&o_done[2 * q + 1], ends[1] & 1, abort_flag, p.status, ST_ATTN_O);
+      }
       float f_first = 0.f, f_second = 0.f;
       int c_begin = 0, c_end = D / 32;  // 32-column chunks of O this group stores
       if (SPLIT) {
@@ -659,6 +665,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           c_end = c_begin + D / 64;
         }
       }
+      if (SPLIT && !__all_sync(0xffffffffu, there)) ok = false;
       if (ok && (SPLIT || n_tiles > 0)) {
         tc_fence_after_sync();
         const float inv = SPLIT ? 1.0f : 1.0f / l_sum;  // (the halves are scaled as they are put together)
