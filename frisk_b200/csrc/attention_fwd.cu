@@ -154,11 +154,11 @@ __global__ void __launch_bounds__(kThreads, 1)
   // Consumers (the two MMA threads, the softmax warps) learn the n-th item of this CTA from the producer:
   // returns its id, or -1 when the work has run out or a wait was abandoned.  The slot is written again once the warp's one arrival
   // is in, so no lane may read it after that: lane 0 reads it for the warp, or all lanes before the arrival.  The latter is compiled into
-  // faster loops for the normalised mode (16 heads x 1025 22.1 against 22.4 us) and for split keys at D = 64 (13.4 and 13.6; 2 heads x
-  // 512 8.9 and 9.2), the former at D = 128 (4 heads x 4096 causal 32.6 against 33.4).
+  // faster loops for the normalised mode (16 heads x 1025 22.1 against 22.4 us), the former for the others (split keys, 4 heads x 4096 at
+  // D = 64 33.1 against 35.1, causal at D = 128 32.6 against 33.4).
   auto next_item = [&](int n) -> int {
     int t = -1;
-    if (NORM || (SPLIT && D == 64)) {
+    if (NORM) {
       if (!mbar_wait_warp(&item_full[n & 1], (n >> 1) & 1, abort_flag, p.status, ST_ATTN_Q)) return -1;
       t = item_slot[n & 1];
       __syncwarp();
@@ -375,10 +375,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     int ends[2] = {0, 0};  // items with two key tiles or more, with one or more so far: the phases of o_done
     int meets = 0;    // meetings of the two groups so far: the phase of xchg
     bool ok = true;
-    // Waits of this lane that have not run out.  A vote of its own on every wait costs up to 3 % (16 heads x 1025, D = 64 13.4 -> 13.8 us;
-    // on the single pass's waits for scores 0.7 % at 8 x 32 x 4096 causal, 3 % at 150 x 2586).  So a lane whose wait has run out goes on
-    // with what it finds until the warp next votes: on whether to rescale, for every key tile, and before O is read.
+    // Waits of this lane that have not run out.  A vote of its own on every wait for scores costs the single pass 0.7 % (8 x 32 x 4096
+    // causal) to 3 % (150 x 2586).  So a lane whose wait has run out goes on with what it finds until the warp votes on whether to
+    // rescale, for every key tile.  Split keys at D = 64 have such a vote for the waits at the end of an item too, before O is read
+    // (16 heads x 1025 14.2 -> 14.0 us, 12 x 2048 causal 18.9 -> 18.7); at D = 128 each of those waits is voted on, which is as fast.
     bool there = true;
+    constexpr bool END_VOTE = SPLIT && D == 64;
     // Split keys: the two groups meet, and each thread learns what the other group's thread of its row brings.  The
     // statistics lie in the second query tile's place, which nothing else uses then, in two sets that alternate: a set is
     // written again only when everybody has arrived at the meeting in between, after reading it.
@@ -387,7 +389,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       set[q * BM + row] = mine_v;
       tc_fence_before_sync();
       mbar_arrive(xchg);
-      there &= mbar_wait(xchg, meets & 1, abort_flag, p.status, ST_ATTN_O);
+      if (END_VOTE)
+        there &= mbar_wait(xchg, meets & 1, abort_flag, p.status, ST_ATTN_O);
+      else if (!mbar_wait_warp(xchg, meets & 1, abort_flag, p.status, ST_ATTN_O))
+        ok = false;
       ++meets;
       tc_fence_after_sync();
       return set[(q ^ 1) * BM + row];
@@ -400,6 +405,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int bh = it.bh + (TWIN ? q : 0);
       const int n_tiles = it.nq[q];
       const int m_tile = it.m0 + (MODE == kPair ? q * BM : 0);
+      // (only END_VOTE carries it on to the next item; said so, the loops are faster here, 12 x 2048 at D = 64 33.9 -> 33.5 us, and slower
+      // elsewhere: 24 x 1000 at D = 128 21.9 -> 22.1)
+      if (SPLIT ? D == 128 : D == 64) there = true;
       // (both groups have read both O of the item before)
       if (SPLIT && n > 0) meet(make_float2(0.f, 0.f));
       const int g_row = m_tile + row;  // query index within the head
@@ -466,7 +474,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             const float a = share(m_run, l_run), b = share(o.x, o.y);
             l_run = a + b;
             m_run = m_all;
-            if (!__all_sync(0xffffffffu, there)) ok = false;
+            if (END_VOTE && !__all_sync(0xffffffffu, there)) ok = false;
             if (!ok) break;
           }
           const float inv_l = __frcp_rn(l_run);  // (of use in pass 1 only)
@@ -554,12 +562,13 @@ __global__ void __launch_bounds__(kThreads, 1)
         // first finite score moves it (0 would let lower scores vanish; a group's first key tiles may be any row's -inf).
         m_ref = fmaxf(mx * p.scale_log2, -FLT_MAX);
         // The groups begin a CTA's first item at the same time, and two that work in step leave the special-function unit idle
-        // together between their key tiles.  So at D = 64 group 1 begins later, by about a third of its work on a tile.  (Later items
-        // begin as far apart as the ones before ended; where tiles are short and equally many it pays for every item.)  Without and
-        // with: 12 x 2048 34.1 and 33.1 us, 16 x 1025 14.6 and 13.8, 48 x 300 against 1024 keys 13.9 and 13.1, 150 x 2586 404 and
-        // 398, 132 x 1075 causal 59.2 and 59.3.  At D = 128 it costs more than it gives (8 x 8192 261 and 268, causal 137.5 and 140,
-        // 62 x 6308 causal 599 and 605, but 24 x 1000 22.5 and 22.2), as with two heads an item (512 x 128 against 256 15.75 and 16.05).
-        if (D == 64 && !TWIN && q == 1 && n_tiles > 3 && (n == 0 || !p.causal)) {
+        // together between their key tiles.  So at D = 64 and with split keys group 1 begins later, by about a third of its work on a
+        // tile.  (Later items begin as far apart as the ones before ended; where tiles are short and equally many it pays for every item.)
+        // Without and with: 12 x 2048 34.1 and 33.1 us, 16 x 1025 14.6 and 13.8, 48 x 300 against 1024 keys 13.9 and 13.1, 150 x 2586 404
+        // and 398, 132 x 1075 causal 59.2 and 59.3; split at D = 128, 4 x 4096 37.6 and 36.6, causal 32.9 and 32.6, 2 x 8192 causal 58.1
+        // and 57.8.  Pairs at D = 128 it costs more than it gives (8 x 8192 261 and 268, causal 137.5 and 140, 62 x 6308 causal 599 and
+        // 605), and two heads an item (512 x 128 against 256 15.75 and 16.05).
+        if ((SPLIT || (D == 64 && !TWIN)) && q == 1 && n_tiles > 3 && (n == 0 || (D == 64 && !p.causal))) {
           const long long from = clock64();
           while (clock64() - from < 300) {
           }
@@ -637,7 +646,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
       // ---- epilogue: O / l
       if (ok && n_tiles > 0) {
-        if (SPLIT) there &= mbar_wait(&o_done[2 * q + 1], ends[1] & 1, abort_flag, p.status, ST_ATTN_O);
+        if (END_VOTE) there &= mbar_wait(&o_done[2 * q + 1], ends[1] & 1, abort_flag, p.status, ST_ATTN_O);
         else ok = mbar_wait_warp(&o_done[2 * q + 1], ends[1] & 1, abort_flag, p.status, ST_ATTN_O);
       }
       float f_first = 0.f, f_second = 0.f;
@@ -665,7 +674,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           c_end = c_begin + D / 64;
         }
       }
-      if (SPLIT && !__all_sync(0xffffffffu, there)) ok = false;
+      if (END_VOTE && !__all_sync(0xffffffffu, there)) ok = false;
       if (ok && (SPLIT || n_tiles > 0)) {
         tc_fence_after_sync();
         const float inv = SPLIT ? 1.0f : 1.0f / l_sum;  // (the halves are scaled as they are put together)
