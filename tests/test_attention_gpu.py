@@ -536,14 +536,12 @@ def test_key_tiles_at_minus_infinity(ctx, hidden, heads, s_q, D, dtype, normaliz
     (299, 100, 200, 64, "fp16", "fp16", True),   # several items a CTA, a ragged last key tile
     (151, 127, 65, 128, "bf16", "fp32", False),  # one key in the second tile
     (300, 128, 256, 128, "bf16", "bf16", True),
-    (1185, 33, 700, 64, "fp16", "fp32", False),  # eleven key tiles (above 256 keys only from 8 heads an SM on)
 ])
 def test_heads_two_at_a_time(ctx, heads, s_q, s_kv, D, dtype, out, causal):
     """More heads of one query tile than SMs: an item is two heads, with K and V of their own."""
     rng = np.random.default_rng(91)
     from oracle.numerics import to_storage
     q, k, v = (to_storage(rng.standard_normal((1, heads, s, D), dtype=np.float32), dtype) for s in (s_q, s_kv, s_kv))
-    assert ctx.attention_form(capi.attn_desc(1, heads, s_q, s_kv, D, D ** -0.5, causal, dtype, out)) == capi.ATTN_TWO_HEADS
     got, ok = run_attention(ctx, q, k, v, dtype, D ** -0.5, causal, out)
     ref = ao.attention_fwd(q, k, v, dtype, D ** -0.5, causal=causal, mode="fp64")
     got = from_storage(got, out).reshape(heads, s_q, D)
@@ -553,15 +551,49 @@ def test_heads_two_at_a_time(ctx, heads, s_q, s_kv, D, dtype, out, causal):
 
 
 @pytest.mark.parametrize("high", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("heads,s_q,D", [
+    (2, 100, 64),    # a lone query tile, its keys split
+    (75, 256, 128),  # two query tiles an item
+    (149, 128, 64),  # more such tiles than SMs
+])
+def test_maximum_in_a_late_key_tile(ctx, high, heads, s_q, D):
+    """Scores that rise by 2^20 in one of five 64-key tiles (the last has 44): O is rescaled before it, also before the last."""
+    rng = np.random.default_rng(92)
+    from oracle.numerics import to_storage
+    q, k, v = (rng.standard_normal((1, heads, s, D), dtype=np.float32) for s in (s_q, 300, 300))
+    q[..., 0], k[..., 0] = 2.0, 0.0
+    k[:, :, high * 64:high * 64 + 64, 0] = 7.0
+    k[:, :, :high * 64, 1:] *= 0.25
+    q, k, v = (to_storage(x, "bf16") for x in (q, k, v))
+    got, ok = run_attention(ctx, q, k, v, "bf16", 1.0, False, "fp32")
+    some = [0, 1, heads - 1]
+    ref = ao.attention_fwd(q, k, v, "bf16", 1.0, causal=False, mode="fp64", heads=some)
+    got = got.reshape(heads, s_q, D)[some]
+    assert ok and np.isfinite(got).all() and rel_frobenius(got, ref.reshape(got.shape)) <= TOL
+
+
 @pytest.mark.parametrize("heads,s_q,s_kv,D,form", [
     (2, 100, 300, 64, "SPLIT_KEYS"),
     (149, 128, 300, 64, "SPLIT_KEYS"),
     (75, 256, 300, 128, "PAIRS"),
-    (150, 128, 236, 128, "TWO_HEADS"),  # (four key tiles: no tile is high where `high` is 4)
-    (1185, 40, 300, 64, "TWO_HEADS"),
+    (149, 128, 128, 64, "TWO_HEADS"),
+    (150, 17, 64, 128, "TWO_HEADS"),
+    (299, 100, 200, 64, "TWO_HEADS"),
+    (151, 127, 65, 128, "TWO_HEADS"),
+    (300, 128, 256, 128, "TWO_HEADS"),
 ])
-def test_maximum_in_a_late_key_tile(ctx, high, heads, s_q, s_kv, D, form):
-    """Scores that rise by 2^20 in one of four or five 64-key tiles (the last has 44): O is rescaled before it, also before the last."""
+def test_forms_of_the_cases_above(ctx, heads, s_q, s_kv, D, form):
+    assert ctx.attention_form(capi.attn_desc(1, heads, s_q, s_kv, D, 1.0, False, "bf16", "fp32")) == getattr(capi, "ATTN_" + form)
+
+
+@pytest.mark.parametrize("high", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("heads,s_q,s_kv,D", [
+    (150, 128, 236, 128),  # four key tiles (no tile is high where `high` is 4)
+    (1185, 40, 300, 64),   # five (above 256 keys only from 8 heads an SM on)
+    (1185, 33, 700, 64),   # eleven
+])
+def test_maximum_in_a_late_key_tile_of_two_heads(ctx, high, heads, s_q, s_kv, D):
+    """The same with two heads an item, which have keys and rescalings of their own."""
     rng = np.random.default_rng(92)
     from oracle.numerics import to_storage
     q, k, v = (rng.standard_normal((1, heads, s, D), dtype=np.float32) for s in (s_q, s_kv, s_kv))
@@ -569,7 +601,7 @@ def test_maximum_in_a_late_key_tile(ctx, high, heads, s_q, s_kv, D, form):
     k[:, :, high * 64:high * 64 + 64, 0] = 7.0
     k[:, :, :high * 64, 1:] *= 0.25
     q, k, v = (to_storage(x, "bf16") for x in (q, k, v))
-    assert ctx.attention_form(capi.attn_desc(1, heads, s_q, s_kv, D, 1.0, False, "bf16", "fp32")) == getattr(capi, "ATTN_" + form)
+    assert ctx.attention_form(capi.attn_desc(1, heads, s_q, s_kv, D, 1.0, False, "bf16", "fp32")) == capi.ATTN_TWO_HEADS
     got, ok = run_attention(ctx, q, k, v, "bf16", 1.0, False, "fp32")
     some = [0, 1, heads - 2, heads - 1]
     ref = ao.attention_fwd(q, k, v, "bf16", 1.0, causal=False, mode="fp64", heads=some)
