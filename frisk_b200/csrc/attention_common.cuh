@@ -1,5 +1,5 @@
 // Pieces shared by the attention kernels: tile sizes, launch parameters, the packed-fp32 and
-// exponential helpers of the softmax, and the number of key tiles a query tile needs.
+// exponential helpers of the softmax.
 #pragma once
 #include "common.cuh"
 #include "ptx.cuh"
@@ -66,8 +66,8 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
   return d;
 }
 
-// a / l for a pair of numerators, without the branch a division per element brings (128 of them in a row of a key
-// tile ran one after the other).  Markstein's correction (IBM J. Res. Dev. 34(1), 1990): with inv the correctly
+// a / l for a pair of numerators, without the branch a division per element brings (those of a key tile's row
+// ran one after the other).  Markstein's correction (IBM J. Res. Dev. 34(1), 1990): with inv the correctly
 // rounded reciprocal of l, q = a*inv is corrected by its exact remainder, and the result is the correctly rounded
 // quotient as long as the remainder is representable, a >= 2^-100 (here a <= 1 <= l, so nothing overflows); below
 // that the quotient, smaller than 2^-100, may be off by one unit of its last fp32 place before it is rounded to 16 bits.

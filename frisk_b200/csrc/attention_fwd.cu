@@ -16,7 +16,8 @@
 //   * key tiles are 64 keys, and every query tile has two buffers of scores: S of tile b + 2 follows P(b).V on the tensor core
 //     while the softmax group works on tile b + 1, whose scores are there.  With one buffer of 128 keys every tile waited for the
 //     chain P -> P.V -> next S -> softmax.  An MMA of S takes 49 clk for 64 keys and 65 for 128 (it
-//     reads Q's rows from shared memory either way): 1270 clk for both query tiles' step of 64 keys against 1050, the price;
+//     reads Q's rows from shared memory either way): 1240 clk for both query tiles' step of 64 keys, as measured with the softmax
+//     left out, against 1050, the price;
 //   * K and V stream through a TMA ring of 4 stages, each what one step of the MMA threads takes;
 //   * warp 8 is the TMA producer; warps 9 and 10 issue the tcgen05.mma of softmax group 0 and 1: S_q =
 //     Q_q.K^T (SS form, both operands K-major, 128-byte swizzle) into tensor memory and O_q += P_q.V
@@ -31,9 +32,9 @@
 // TMEM columns: S0 [0,64) and [64,128), S1 [128,192) and [192,256), O0 [256,256+D) O1 [384,384+D); P_q of a key tile
 // aliases the first 32 columns of its scores (two 16-bit values per column).
 //
-// What bounds it: 8 x 32 heads x 4096 causal at D = 128 (1000 us; 1120 with 128-key tiles, one buffer and softmax groups in turn)
-// the power limit, at which it runs at 1.5 instead of 1.7 GHz; short runs the softmax groups, 1700 clk for a step of both
-// where the exponentials take 1024 and the MMAs 1270.
+// What bounds it: 8 x 32 heads x 4096 causal at D = 128 (1050 us, 1120 with 128-key tiles, one buffer and softmax groups in
+// turn) the power limit, at which it runs at 1.5 instead of 1.7 GHz; short runs the softmax groups, 1700 clk for a step of both
+// where the exponentials take 1024 and the MMAs 1240.
 // Every mbarrier wait is bounded (ptx.cuh); no TMA load uses cluster multicast.
 #include <algorithm>
 #include <cfloat>

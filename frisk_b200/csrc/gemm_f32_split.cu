@@ -12,7 +12,7 @@
 // summed in tensor memory, small terms first, so that only the four A0B0 steps see a large accumulator, and then
 // added to fp32 registers with round-to-nearest: 1.0e-7 at K = 1024, 2.6e-7 on the CUDA cores.  Sums whose terms share a
 // sign feel the truncations more: below K = 640 a block is summed in two halves, each in an accumulator of its own
-// (TWO; 22.4 us instead of 21.8 at 1024^3), and below K = 320 the CUDA cores are the more accurate (split_accurate).
+// (TWO; 2.7 % of the time at 1024^3), and below K = 320 the CUDA cores are the more accurate (split_accurate).
 //
 // An element that is not finite, or so large that x 2^24 or a sum overflows, makes the result non-finite.  The 32 x 16
 // piece of C it lies in is noted, and when a CTA's tiles are done (no wait of the pipeline is open any more, however long
@@ -24,11 +24,13 @@
 //               the MMAs of block i, a quarter at a time between the quarters of block i - 1 that it adds up
 //   warps 8-15  loaders: global -> registers (one block ahead) -> split -> shared memory, in the 128-byte-swizzle image
 //               tcgen05 reads (K-major or MN-major, whichever way the operand lies in global memory), or tensor memory
-// What bounds a block is the loaders: two warps a scheduler take 3100 clk for their ~550 instructions a block, wherever the terms
-// go and in whatever order they are made; the MMAs take 1560 (2000 as issued), shared memory 2300, or 1150 with A in tensor
-// memory.  1024^3 22.0 us with the MMAs of a block issued in one piece, 21.1 in quarters; 2000 x 2000 x 400 38.1 and 34.6;
-// 4096^3 runs at 155 TFLOP/s of fp32.  Tried: four stages of 32 k instead of two of 64 (2048^3 126 -> 154 us), 16 warps that load,
-// split and add up (1024^3 27.0), a warp of its own for the MMAs (96 registers a thread then: spills).
+// What bounds a block is the loaders' chain: a warp makes the terms of A, asks for the next A, does the same for B, waits and fences,
+// one after the other, 3100 clk a block wherever the terms go and in whatever order they are made.  It is latency: a scheduler's
+// two warps fill 1100 of its 3100 issue slots with ~550 instructions each; the MMAs take 1560 (2000 as issued), shared memory
+// 2300, or 1150 with A in tensor memory.  1024^3 takes 21.1 us (22.0 with the MMAs of a block issued in one piece instead of
+// quarters; 23.1 with operands from HBM), 2000 x 2000 x 400 35.4 (38.1), 2048^3 126, 4096^3 840 to 930 (448 blocks a CTA, at the
+// power limit).  Tried: four stages of 32 k instead of two of 64 (2048^3 154), 16 warps that load, split and add up (1024^3 27.0), a
+// warp of its own for the MMAs (96 registers a thread then: spills).
 //
 // Where the tiles are fewer than half the SMs a cluster of 2 to 8 CTAs shares a tile's K; every CTA leaves its fp32 part
 // in its own shared memory and each finishes a share of the tile's 32-row pieces, adding the parts over distributed
@@ -252,7 +254,7 @@ __device__ __forceinline__ bool store_piece(const SplitArgs& p, float (&v)[16], 
 // columns 64h + 16 (w / 4), rows 32 (w % 4).  Plain fp32 sums by all 16 warps, half a tile at a time, a lane with 4 x 4
 // results of a piece; where few pieces are noted, two or four warps share a block's k and their sums are added in order.
 // 4096^3 takes 0.83 ms, with one infinite element 1.5 and with every result above 2^80 8.4 (53 and 451 when the thread that
-// met such a result summed it up on the spot); 1024^3 24 us, 167 and 232.
+// met such a result summed it up on the spot); 1024^3 21 us, 167 and 232.
 template <bool A_MN, bool B_MN>
 __device__ __noinline__ void redo_pieces(const SplitArgs& p, unsigned char* smem, const uint32_t* noted, int first, int step,
                                          int count) {
@@ -349,9 +351,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_split_kernel(const __gri
   uint32_t* noted = reinterpret_cast<uint32_t*>(smem + kRedoOffset);  // pieces of each of this CTA's tiles to compute again
   constexpr int kHalves = TWO ? 2 : 1, kAccCols = kHalves * BT;  // of an accumulator
   // The terms of an A that is stored transposed go to tensor memory, behind the two accumulators, where there is room (two
-  // stages of three planes): their MMAs then read only B from shared memory.  1024^3 21.0 -> 20.4 us, 515 x 771 x 1003 21.6 -> 20.1,
-  // 128 x 1500 x 700 15.4 -> 14.9.  (Any operand contiguous along its rows would do, with the product turned round for B; for an
-  // A contiguous along K that was no faster: 21.1 and 21.4 us at 1024^3.)
+  // stages of three planes): their MMAs then read only B from shared memory: 3 % at 1024^3 with both operands transposed,
+  // 515 x 771 x 1003 21.6 -> 20.0 us, 128 x 1500 x 700 15.4 -> 14.9.  (Any operand contiguous along its rows would do, with the
+  // product turned round for B; for an A contiguous along K that was 1 % slower at 1024^3.)
   constexpr bool LANES = A_MN && !TWO;
   constexpr uint32_t kPlanesAt = 2 * BT, kPlanesCols = 3 * BK / 2, kTmemCols = LANES ? 512 : 2 * kAccCols;
   static_assert(kPlanesAt + 2 * kPlanesCols <= 512, "accumulators and planes must fit");
@@ -678,8 +680,10 @@ bool split_accurate(const frisk_b200_gemm_desc& d) { return d.K >= 320 || f32_sp
 
 // Both kernels estimated in microseconds from measurements.  CUDA cores: 4.3 for 64 x 64 x 64 and about 2.0 more for
 // every further 64 x 64 x 64 unit an SM takes, 2 to add up the parts of a shared tile (512^3 13.5, 1024^3 57, 2048^3 401).
-// Tensor cores: 5.5 and 2.1 for every 128 x 128 x 64 block a CTA takes, 2 more to add up the parts of a shared tile (64^3
-// 7.6, 128^3 9.9, 512^3 11.6, 1024^3 22.9, 2048^3 128); 2.4 per block where rows are not 16-byte aligned (1151 x 2047 x 1023 43).
+// Tensor cores: 5.5 and 2.1 for every 128 x 128 x 64 block a CTA takes, 2 more to add up the parts of a shared tile; 2.4 per block
+// where rows are not 16-byte aligned.  That was fitted when a block's MMAs were issued in one piece and is 5 to 15 % too much today (512^3
+// 11.1, 1024^3 21.1, 2048^3 126, 1151 x 2047 x 1023 43), more for a transposed A off 16 bytes from K = 640 on, whose lane-wise loads do
+// not care: where the two are close the CUDA cores are taken a little too often.
 bool f32_split_beats_simt(const frisk_b200_gemm_desc& d) {
   if (d.dtype_ab != FRISK_B200_F32 || d.dtype_c != FRISK_B200_F32 || !split_accurate(d)) return false;
   if (d.M > INT32_MAX / 4 || d.N > INT32_MAX / 4 || d.K > INT32_MAX / 4) return false;

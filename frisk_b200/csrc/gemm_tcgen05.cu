@@ -658,12 +658,13 @@ struct Plan {
   double clocks;
 };
 // The plan for tiles of bn columns and clusters of `splits` CTAs, of which the device runs `clusters`.  A 64-k block takes
-// its MMAs (512 clk at 256 columns, 256 at 128) and, the more SMs are at it, what L2 adds: 770 at 2048^3 and 4096^3 with
-// the chip full, 1100 where rows begin off 128-byte lines (3000^3: two requests of the TMA unit a row).  Sharing costs
+// its MMAs (512 clk at 256 columns) or the issuing warp's work (below) and, the more SMs are at it, what L2 adds: 770 at 2048^3
+// and 4096^3 with the chip full, 1100 where rows begin off 128-byte lines (3000^3: two requests of the TMA unit a row).  Sharing costs
 // barriers, parts and sums: 3.5 us at 128 rows (128 x 512 x 512 over clusters of four took 8.7 us, whole 6.7), less
 // with fewer rows (17 x 1024 x 1024 6.8, 128 x 1024 x 1024 9.1 over clusters of eight).  Tiles of 64 columns take as long for a
-// block (MMAs paced by the 6 KB of operands each) but put twice the SMs to work and have half the parts to add up: they are for products
-// with few columns and rows (128 x 2048 x 2048 in clusters of four 9.9 us, 11.2 with 128 columns; 64 x 2048 x 4096 11.4, 12.3;
+// block (410 clk, 427 with 128 columns: the issuing warp's wait, four MMAs and commit set the pace, not the MMAs) but put twice the SMs
+// to work and have half the parts to add up: they are for products with few columns and rows (128 x 2048 x 2048
+// in clusters of four 9.9 us, 11.2 with 128 columns; 64 x 2048 x 4096 11.4, 12.3;
 // 256 x 1024 x 4096 12.1, 13.4; whole 300 x 1000 x 1000 9.2, 9.9).
 Plan plan_of(const GemmDims& g, int64_t tiles, int sms, int bn, int splits, int clusters) {
   const int64_t kb = (g.K + BK - 1) / BK;
@@ -686,6 +687,8 @@ Plan plan_of(const GemmDims& g, int64_t tiles, int sms, int bn, int splits, int 
     extra = (bn == 256 ? 4500 : bn == 128 ? 3500 : 2500) + (bn == 64 ? 1500.0 : 3000.0) * (double)std::min<int64_t>(g.M, BM) / BM;
   }
   const double busy = (double)p.grid / sms;
+  // (Fitted to whole calls together with `l2` and `extra`, when one lane issued the MMAs: 270 and 250 are shares of an estimate, and lie
+  // below the 427 and 410 clk that a block takes an issuing warp.)
   const double mma = bn == 256 ? 520 : bn == 128 ? 270 : 250;
   const double l2 = bn == 256 ? (aligned ? 250 : 580) : bn == 128 ? (aligned ? 200 : 450) : aligned ? 150 : 340;
   p.clocks = blocks * (mma + l2 * busy) + extra;

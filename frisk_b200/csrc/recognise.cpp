@@ -5,8 +5,8 @@
 //                 | (True, M, N, K, type of A, type of C, trans_a, trans_b, clear_accum, policy, ia, ib, ic,
 //                    fill or None, reduce kind or None, reduce argument, reduce_clear)        one gemm, its fill and reduce
 //
-// Walking and verifying a built kernel op by op in Python took most of a small call (a 64 x 64 attention tile 53.1 us, 17.1 with
-// this module, whose part is 8; a 512 x 384 x 256 gemm with fill and reduce 28.8 and 13.5, of which 3), and nothing may be
+// Walking and verifying a built kernel op by op in Python took most of a small call (a 64 x 64 attention tile 53.1 us, 16.2 with
+// this module, whose part is 8; a 512 x 384 x 256 gemm with fill and reduce 28.8 and 13.4, of which 3), and nothing may be
 // remembered between calls, since every list and attribute of the IR can be changed at any time.  So the same walk and
 // the checks of ir._verify and of tensor_ops.attention_plan / execute.fused_plan are made here, read off the same objects.
 //
